@@ -189,9 +189,10 @@ __global__ void jacobi_setup_kernel(int n, const int* __restrict__ offsets,
     const double bm = block_max(ratio, scratch, -(double)INFINITY);
     if (threadIdx.x == 0) maxima[blockIdx.x] = bm;
     if (!last_block_arrived(counter, &last)) return;
-    if (threadIdx.x != 0) return;
     double maximum = -INFINITY;
-    for (int b = 0; b < (int)gridDim.x; ++b) maximum = fmax(maximum, __ldcg(&maxima[b]));
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) maximum = fmax(maximum, __ldcg(&maxima[b]));
+    maximum = block_max(maximum, scratch, -(double)INFINITY);
+    if (threadIdx.x != 0) return;
     const double relative = fmin(kChebyshevInterval / (double)max(n, 1), kIntervalCap);
     const double dominance = fmax(maximum, 1e-3);
     const double lower = fmax(relative, 1.0 - dominance);
@@ -462,13 +463,15 @@ __global__ void __launch_bounds__(kThreads, 8) settle_kernel(long long total, co
     const double bs = block_sum(reached, scratch);
     if (threadIdx.x == 0) partials[blockIdx.x] = make_double2(bm, bs);
     if (!last_block_arrived(counter, &last)) return;
-    if (threadIdx.x != 0) return;
     double m = 0.0, cnt = 0.0;
-    for (int b = 0; b < (int)gridDim.x; ++b) {
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
         const double2 p = __ldcg(&partials[b]);
         m = fmax(m, p.x);
         cnt += p.y;
     }
+    m = block_max(m, scratch, 0.0);
+    cnt = block_sum(cnt, scratch);  // whole numbers: exact in any order
+    if (threadIdx.x != 0) return;
     const double checks = settle->checks + 1.0;
     settle->checks = checks;
     const double count = cnt + 1.0;
@@ -527,11 +530,22 @@ __global__ void backward_error_kernel(int n, int k, const int* __restrict__ offs
     }
 }
 
+}  // namespace
+}  // namespace ob
+
+#include "ob_pcg_resident.cuh"
+
+namespace ob {
+namespace {
+
 int next_pow2(int v) {
     int p = 1;
     while (p < v) p <<= 1;
     return p;
 }
+
+constexpr size_t kStateBytes = 64;  // of the state in its allocation, the scalars after it
+static_assert(sizeof(LoopState) <= kStateBytes, "the state is followed by the columns' scalars");
 
 struct Solver {
     int n = 0, k_live = 0, k = 0, precond = 0, narrow = 0;
@@ -542,6 +556,7 @@ struct Solver {
     // The sliced-ELL copy the iteration's mat-vecs read (its float32 values when narrow), grown
     // when a rebound operator's slices need more entries than it holds.
     int n_slices = 0;
+    bool sell_bound = false;  // the copy holds the bound operator
     long long* sell_start = nullptr;
     int* sell_columns = nullptr;
     double* sell_values = nullptr;
@@ -557,9 +572,18 @@ struct Solver {
     LoopState* state = nullptr;
     SettleState* settle = nullptr;
     unsigned int* counters = nullptr;  // [0] matvec, [1] settle, [2] reset, [3] setup
-    LoopState* host_state = nullptr;   // pinned
+    // The device's state and scalars are one allocation, its host image pinned: one copy back.
+    LoopState* host_state = nullptr;
     ColumnScalars* host_scalars = nullptr;
     int blocks = 0;
+    bool loop_ready = false;  // the loop graph's vectors are allocated
+    // The resident form (ob_pcg_resident.cuh), when the system fits it.
+    const void* resident = nullptr;
+    int resident_form = 0, resident_threads = 0, resident_ctas = 0, resident_width = 0, resident_pushes = 0;
+    size_t resident_smem = 0;
+    double* published = nullptr;  // kGrid: two buffers of n
+    double* resident_partials = nullptr;
+    unsigned int* arrivals = nullptr;  // the counter and the abort flag
     cudaStream_t capture = nullptr;
     // Cached loop graphs: key = (settle?, rounds per body, maxiter, params).
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
@@ -626,6 +650,7 @@ int build_sell(Solver* S, cudaStream_t stream) {
         S->sell_capacity = total;
     }
     S->sell_entries = total;
+    S->sell_bound = true;
     slice_fill_kernel<<<ceil_div(S->n, kThreads), kThreads, 0, stream>>>(
         S->n, S->offsets, S->columns, S->values, S->sell_start, S->sell_columns, S->sell_values,
         S->narrow ? S->sell_values32 : nullptr);
@@ -643,7 +668,8 @@ Sell<float> sell32(const Solver* S) {
 }
 
 // Copies an operator of the solver's shape into its own arrays and derives what the iteration
-// reads from it: the inverse diagonal, the Chebyshev steps and the sliced-ELL copy.
+// reads from it: the inverse diagonal and the Chebyshev steps (the sliced-ELL copy is made when
+// the loop graph first needs it).
 int bind_operator(Solver* S, const int* offsets, const int* columns, const double* values,
                   cudaStream_t stream) {
     const int n = S->n;
@@ -661,7 +687,8 @@ int bind_operator(Solver* S, const int* offsets, const int* columns, const doubl
         n, S->offsets, S->columns, S->values, S->inv_diag, S->maxima, S->counters + 3,
         kChebyshevDegree - 1, S->steps);
     OB_CHECK_LAUNCH("pcg setup");
-    return build_sell(S, stream);
+    S->sell_bound = false;
+    return OB_OK;
 }
 
 int solver_alloc(Solver* S, void** out, size_t bytes, cudaStream_t stream) {
@@ -675,9 +702,166 @@ void solver_release(Solver* S) {
     release_sell(S);
     for (void* p : S->owned) cudaFree(p);
     if (S->host_state) cudaFreeHost(S->host_state);
-    if (S->host_scalars) cudaFreeHost(S->host_scalars);
     if (S->capture) cudaStreamDestroy(S->capture);
     delete S;
+}
+
+// What the loop graph needs and the resident form does not: its vectors, its partial sums, the
+// capture stream (once), and the sliced-ELL copy of the bound operator (after each rebind; its
+// size is read back, which synchronises the stream).
+int ensure_loop(Solver* S, cudaStream_t stream) {
+    if (!S->loop_ready) {
+        const size_t vec = sizeof(double) * (size_t)S->n * S->k;
+        int st = OB_OK;
+        auto A = [&](void** p, size_t bytes) {
+            if (st == OB_OK && *p == nullptr) st = solver_alloc(S, p, bytes, stream);
+        };
+        for (double** v : {&S->b, &S->x, &S->r, &S->u, &S->w, &S->p, &S->s, &S->previous}) A((void**)v, vec);
+        if (S->precond == 1)
+            for (double** v : {&S->scaled, &S->t0, &S->t1}) A((void**)v, vec);
+        A((void**)&S->partials, sizeof(double) * 3 * (size_t)S->blocks * S->k);
+        A((void**)&S->settle_partials, sizeof(double2) * (size_t)S->blocks);
+        A((void**)&S->sell_start, sizeof(long long) * ((size_t)S->n_slices + 1));
+        if (st) return st;
+        if (S->capture == nullptr) OB_CUDA(cudaStreamCreateWithFlags(&S->capture, cudaStreamNonBlocking));
+        S->loop_ready = true;
+    }
+    return S->sell_bound ? OB_OK : build_sell(S, stream);
+}
+
+template <int R, int FORM>
+const void* resident_kernel_of(bool cheb) {
+    return cheb ? (const void*)resident_pcg_kernel<R, FORM, true> : (const void*)resident_pcg_kernel<R, FORM, false>;
+}
+
+cudaLaunchConfig_t resident_config(const Solver* S, cudaLaunchAttribute* attribute, cudaStream_t stream) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3((unsigned)S->resident_ctas);
+    config.blockDim = dim3((unsigned)S->resident_threads);
+    config.dynamicSmemBytes = S->resident_smem;
+    config.stream = stream;
+    config.attrs = attribute;
+    if (S->resident_form == kCluster) {
+        attribute->id = cudaLaunchAttributeClusterDimension;
+        attribute->val.clusterDim.x = (unsigned)S->resident_ctas;
+        attribute->val.clusterDim.y = attribute->val.clusterDim.z = 1;
+        config.numAttrs = 1;
+    } else if (S->resident_form == kGrid) {
+        attribute->id = cudaLaunchAttributeCooperative;
+        attribute->val.cooperative = 1;
+        config.numAttrs = 1;
+    }
+    return config;
+}
+
+// Takes one form for the solver if the system fits it and the device can hold all its CTAs at once.
+bool take_resident(Solver* S, int form, int rows_a_cta, int rows_a_thread) {
+    const int per_warp = 32 * rows_a_thread;
+    int threads = (rows_a_cta + per_warp - 1) / per_warp * 32;
+    if (form == kGrid) threads = std::max(threads, 96);  // a warp for each of the three sums
+    if (threads > resident_threads(rows_a_thread)) return false;
+    int device = 0, limit = 0;
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
+        return false;
+    const size_t owned = (size_t)threads * rows_a_thread;
+    const int registers = register_entries(rows_a_thread);
+    const int pushes = form == kCluster ? (int)(2 * owned) : 0;
+    const size_t fixed = (form == kGrid ? 0 : 16 * (owned + (form == kCluster ? kHalo : 0))) +
+                         8 * (6 * kClusterMax + 3 * 32 + 4) +
+                         (form == kCluster ? sizeof(int2) * pushes + sizeof(int) * (2 * kHaloTable + 4) : 0);
+    const size_t entry = owned * (sizeof(unsigned) + sizeof(double));
+    if (fixed + (registers ? 0 : 7) * entry > (size_t)limit) return false;
+    S->resident_form = form;
+    S->resident_threads = threads;
+    S->resident_ctas = (int)((S->n + owned - 1) / owned);
+    S->resident_pushes = pushes;
+    S->resident_width = (int)std::min<size_t>(kResidentWidth, registers + ((size_t)limit - fixed) / entry);
+    S->resident_smem = fixed + (S->resident_width - registers) * entry;
+    const bool cheb = S->precond == 1;
+    const void* kernel = form == kBlock ? resident_kernel_of<2, kBlock>(cheb)
+                         : form == kCluster
+                             ? (rows_a_thread == 2 ? resident_kernel_of<2, kCluster>(cheb)
+                                                   : resident_kernel_of<4, kCluster>(cheb))
+                             : (rows_a_thread == 2 ? resident_kernel_of<2, kGrid>(cheb)
+                                                   : resident_kernel_of<4, kGrid>(cheb));
+    // The device's limit, whatever this solver needs: the attribute is the kernel's, not the launch's.
+    bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) == cudaSuccess;
+    if (ok && form == kCluster) {
+        ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        cudaLaunchAttribute attribute;
+        const cudaLaunchConfig_t config = resident_config(S, &attribute, nullptr);
+        int clusters = 0;
+        ok = ok && cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) == cudaSuccess && clusters >= 1;
+    }
+    if (ok && form == kGrid) {
+        int per_sm = 0;
+        ok = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, S->resident_smem) ==
+                 cudaSuccess &&
+             (long long)per_sm * sm_count() >= S->resident_ctas;
+    }
+    if (!ok) {
+        cudaGetLastError();
+        return false;
+    }
+    S->resident = kernel;
+    return true;
+}
+
+// The form by size: one CTA to 1 024 rows, a cluster of up to 16 CTAs while their shared memory holds
+// the rows (about 26 000), then a grid of one CTA an SM; two rows a thread (their entries in
+// registers) to 1 024 rows a CTA, four (in shared memory) to 2 048. Larger systems, and several
+// columns, take the loop graph, whose kernels then run for longer than their launch.
+void choose_resident(Solver* S) {
+    if (S->k != 1) return;
+    if (S->n <= 1024 && take_resident(S, kBlock, S->n, 2)) return;
+    const int cluster_rows = std::max((S->n + kClusterMax - 1) / kClusterMax, 64);
+    if (cluster_rows <= 2048 && take_resident(S, kCluster, cluster_rows, cluster_rows <= 1280 ? 2 : 4)) return;
+    const int grid_rows = std::max((S->n + sm_count() - 1) / sm_count(), 256);
+    if (grid_rows <= 2048) take_resident(S, kGrid, grid_rows, grid_rows <= 1280 ? 2 : 4);
+}
+
+// One solve by the resident form; check_rounds 0 stops by the residual.
+int launch_resident(Solver* S, const double* rhs, double* x, double tol, int maxiter, int check_rounds,
+                    double change_tolerance, int settle_rounds, cudaStream_t stream) {
+    if (S->resident_form == kGrid) {
+        if (S->published == nullptr) {
+            if (int st = solver_alloc(S, (void**)&S->published, sizeof(double) * 2 * (size_t)S->n, stream)) return st;
+            if (int st = solver_alloc(S, (void**)&S->resident_partials, sizeof(double) * 6 * S->resident_ctas, stream))
+                return st;
+            if (int st = solver_alloc(S, (void**)&S->arrivals, 2 * sizeof(int), stream)) return st;
+        }
+        OB_CUDA(cudaMemsetAsync(S->arrivals, 0, 2 * sizeof(int), stream));
+    }
+    ResidentArgs a = {};
+    a.n = S->n;
+    a.offsets = S->offsets;
+    a.columns = S->columns;
+    a.values = S->values;
+    a.inv_diag = S->inv_diag;
+    a.steps = S->steps;
+    a.rhs = rhs;
+    a.x = x;
+    a.tol = tol;
+    a.maxiter = maxiter;
+    a.check_rounds = check_rounds;
+    a.change_tolerance = change_tolerance;
+    a.settle_rounds = settle_rounds;
+    a.state = S->state;
+    a.scalars = S->scalars;
+    a.narrow = S->narrow;
+    a.width = S->resident_width;
+    a.pushes = S->resident_pushes;
+    a.published = S->published;
+    a.partials = S->resident_partials;
+    a.counter = S->arrivals;
+    a.abort = reinterpret_cast<int*>(S->arrivals + 1);
+    cudaLaunchAttribute attribute;
+    const cudaLaunchConfig_t config = resident_config(S, &attribute, stream);
+    void* args[] = {&a};
+    OB_CUDA(cudaLaunchKernelExC(&config, S->resident, args));
+    OB_CHECK_LAUNCH("pcg resident solve");
+    return OB_OK;
 }
 
 // Enqueues one round (mat-vec with dots, update, and the polynomial when preconditioned by it).
@@ -869,11 +1053,29 @@ int finish_solve(Solver* S, double* x, cudaStream_t stream) {
         OB_CUDA(cudaMemcpy2DAsync(x, sizeof(double) * S->k_live, S->x, sizeof(double) * S->k,
                                   sizeof(double) * S->k_live, S->n, cudaMemcpyDeviceToDevice,
                                   stream));
-    OB_CUDA(cudaMemcpyAsync(S->host_state, S->state, sizeof(LoopState), cudaMemcpyDeviceToHost,
-                            stream));
-    OB_CUDA(cudaMemcpyAsync(S->host_scalars, S->scalars, sizeof(ColumnScalars) * S->k,
-                            cudaMemcpyDeviceToHost, stream));
     return OB_OK;
+}
+
+// The state and the columns' scalars to their host image (the caller waits for the stream).
+int read_back(Solver* S, cudaStream_t stream) {
+    OB_CUDA(cudaMemcpyAsync(S->host_state, S->state, kStateBytes + sizeof(ColumnScalars) * S->k,
+                            cudaMemcpyDeviceToHost, stream));
+    OB_CUDA(cudaStreamSynchronize(stream));
+    if (S->host_state->status == kStatusAborted)
+        return fail(OB_ERR_TIMEOUT, "pcg: a wait between the solver's blocks gave up");
+    return OB_OK;
+}
+
+// One solve by the loop graph.
+int run_loop(Solver* S, const double* rhs, double* x, double tol, int mode, int rounds_per_body, int maxiter,
+             int check_rounds, double change_tolerance, int settle_rounds, cudaStream_t stream) {
+    int st = ensure_loop(S, stream);
+    if (st == OB_OK) st = start_solve(S, rhs, x, tol, stream);
+    if (st == OB_OK)
+        st = loop_graph(S, mode, rounds_per_body, maxiter, check_rounds, change_tolerance, settle_rounds);
+    if (st) return st;
+    OB_CUDA(cudaGraphLaunch(S->exec[mode], stream));
+    return finish_solve(S, x, stream);
 }
 
 }  // namespace
@@ -910,7 +1112,6 @@ int ob_pcg_create(int n, const int32_t* offsets, const int32_t* columns, const d
     const long long total = (long long)n * S->k;
     S->blocks = (int)std::max(1LL, std::min((total + kThreads - 1) / kThreads,
                                             (long long)8 * sm_count()));
-    const size_t vec = sizeof(double) * (size_t)total;
     int st = OB_OK;
     auto A = [&](void** p, size_t bytes) {
         if (st == OB_OK) st = solver_alloc(S, p, bytes, stream);
@@ -923,31 +1124,23 @@ int ob_pcg_create(int n, const int32_t* offsets, const int32_t* columns, const d
     A((void**)&own_columns, sizeof(int) * (size_t)std::max(nnz, 1));
     A((void**)&own_values, sizeof(double) * (size_t)std::max(nnz, 1));
     A((void**)&S->inv_diag, sizeof(double) * n);
-    for (double** v : {&S->b, &S->x, &S->r, &S->u, &S->w, &S->p, &S->s, &S->previous})
-        A((void**)v, vec);
-    if (precond == 1)
-        for (double** v : {&S->scaled, &S->t0, &S->t1}) A((void**)v, vec);
-    A((void**)&S->partials, sizeof(double) * 3 * (size_t)S->blocks * S->k);
     A((void**)&S->maxima, sizeof(double) * (size_t)S->blocks);
-    A((void**)&S->settle_partials, sizeof(double2) * (size_t)S->blocks);
     A((void**)&S->steps, sizeof(double4) * kChebyshevDegree);
-    A((void**)&S->scalars, sizeof(ColumnScalars) * S->k);
-    A((void**)&S->state, sizeof(LoopState));
+    A((void**)&S->state, kStateBytes + sizeof(ColumnScalars) * S->k);
     A((void**)&S->settle, sizeof(SettleState));
     A((void**)&S->counters, sizeof(unsigned int) * 8);
     S->n_slices = ceil_div(n, kSlice);
-    A((void**)&S->sell_start, sizeof(long long) * ((size_t)S->n_slices + 1));
     if (st != OB_OK) {
         solver_release(S);
         return st;
     }
-    if (cudaMallocHost((void**)&S->host_state, sizeof(LoopState)) != cudaSuccess ||
-        cudaMallocHost((void**)&S->host_scalars, sizeof(ColumnScalars) * S->k) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&S->capture, cudaStreamNonBlocking) != cudaSuccess) {
+    S->scalars = reinterpret_cast<ColumnScalars*>(reinterpret_cast<char*>(S->state) + kStateBytes);
+    if (cudaMallocHost((void**)&S->host_state, kStateBytes + sizeof(ColumnScalars) * S->k) != cudaSuccess) {
         cudaGetLastError();
         solver_release(S);
         return fail(OB_ERR_NOMEM, "ob_pcg_create: host allocations failed");
     }
+    S->host_scalars = reinterpret_cast<ColumnScalars*>(reinterpret_cast<char*>(S->host_state) + kStateBytes);
     e = cudaMemsetAsync(S->counters, 0, sizeof(unsigned int) * 8, stream);
     if (e != cudaSuccess) {
         solver_release(S);
@@ -957,6 +1150,7 @@ int ob_pcg_create(int n, const int32_t* offsets, const int32_t* columns, const d
     S->columns = own_columns;
     S->values = own_values;
     st = bind_operator(S, offsets, columns, values, stream);
+    if (st == OB_OK) choose_resident(S);
     if (st == OB_OK) {
         e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) st = cuda_status(e, "ob_pcg_create: setup");
@@ -995,16 +1189,12 @@ int ob_pcg_solve(void* solver, const double* rhs, double* x, double tol, int max
     OB_REQUIRE(solver && rhs && x, "ob_pcg_solve: null pointer");
     OB_REQUIRE(tol >= 0.0 && maxiter >= 0, "ob_pcg_solve: bad tolerance or cap");
     Solver* S = static_cast<Solver*>(solver);
-    int st = start_solve(S, rhs, x, tol, stream);
-    if (st) return st;
-    st = loop_graph(S, 0, 4, maxiter, 0, 0.0, 0);
-    if (st) return st;
-    OB_CUDA(cudaGraphLaunch(S->exec[0], stream));
-    st = finish_solve(S, x, stream);
+    int st = S->resident ? launch_resident(S, rhs, x, tol, maxiter, 0, 0.0, 0, stream)
+                         : run_loop(S, rhs, x, tol, 0, 4, maxiter, 0, 0.0, 0, stream);
     if (st) return st;
     if (iterations || relative_residual) {
-        OB_CUDA(cudaStreamSynchronize(stream));
-        count_body_launches(S, 4, 0);
+        if ((st = read_back(S, stream))) return st;
+        if (!S->resident) count_body_launches(S, 4, 0);
         for (int c = 0; c < S->k_live; ++c) {
             if (iterations) iterations[c] = S->host_state->iterations;
             if (relative_residual) {
@@ -1024,16 +1214,14 @@ int ob_pcg_settle(void* solver, const double* rhs, double* x, int check_rounds,
     OB_REQUIRE(check_rounds >= 1 && check_rounds <= 256, "ob_pcg_settle: check_rounds in [1, 256]");
     OB_REQUIRE(maxiter >= 0, "ob_pcg_settle: negative cap");
     Solver* S = static_cast<Solver*>(solver);
-    int st = start_solve(S, rhs, x, 0.0, stream);
-    if (st) return st;
-    st = loop_graph(S, 1, check_rounds, maxiter, check_rounds, change_tolerance, settle_rounds);
-    if (st) return st;
-    OB_CUDA(cudaGraphLaunch(S->exec[1], stream));
-    st = finish_solve(S, x, stream);
+    int st = S->resident ? launch_resident(S, rhs, x, 0.0, maxiter, check_rounds, change_tolerance, settle_rounds,
+                                           stream)
+                         : run_loop(S, rhs, x, 0.0, 1, check_rounds, maxiter, check_rounds, change_tolerance,
+                                    settle_rounds, stream);
     if (st) return st;
     if (rounds || status) {
-        OB_CUDA(cudaStreamSynchronize(stream));
-        count_body_launches(S, check_rounds, 1);
+        if ((st = read_back(S, stream))) return st;
+        if (!S->resident) count_body_launches(S, check_rounds, 1);
         if (rounds) *rounds = S->host_state->iterations;
         if (status) *status = S->host_state->status;
     }
@@ -1044,6 +1232,7 @@ int ob_pcg_time_matvec(void* solver, int reps, float* ms, ob_stream_t stream_) {
     cudaStream_t stream = as_stream(stream_);
     OB_REQUIRE(solver && ms && reps >= 1, "ob_pcg_time_matvec: bad argument");
     Solver* S = static_cast<Solver*>(solver);
+    if (int ready = ensure_loop(S, stream)) return ready;
     // Each launch is timed alone, its loop state reset before it (a launch that finds the loop
     // over returns at once, and a zero residual ends the loop after one launch).
     cudaEvent_t start, end;
@@ -1086,6 +1275,7 @@ int ob_pcg_time_matvec(void* solver, int reps, float* ms, ob_stream_t stream_) {
 int ob_pcg_info(void* solver, long long* info) {
     OB_REQUIRE(solver && info, "ob_pcg_info: bad argument");
     Solver* S = static_cast<Solver*>(solver);
+    if (int st = ensure_loop(S, nullptr)) return st;
     info[0] = S->n;
     info[1] = S->k;
     info[2] = S->nnz;

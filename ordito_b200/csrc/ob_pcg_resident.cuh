@@ -1,0 +1,601 @@
+// The conjugate gradient loop of ob_pcg.cu as ONE kernel that stays on the chip, for one right-hand
+// side on an operator small enough to share out over the SMs' registers and shared memory.
+//
+// What bounds a round of a small system is not its bytes but its chain: a mat-vec and an update
+// kernel (13 kernels under the Chebyshev polynomial), each with its launch, its first loads and
+// its drain (4-5 us a kernel measured inside the loop graph, whatever the size below ~100 k rows).
+// Here a thread owns R rows for the whole solve: their r, p, s, x, u and first seven entries (a
+// mesh row's usual count) sit in registers, further entries in shared memory, and a round's kernels
+// become barriers between the phases. Only the vector the next mat-vec gathers is published. Three
+// forms, by how far it has to travel:
+//
+//   kBlock    one CTA: shared memory, __syncthreads;
+//   kCluster  up to 16 CTAs, each holding its rows' values and a copy of the other CTAs' values its
+//             rows read (its halo). A CTA publishes by storing its own values and pushing those
+//             other CTAs hold copies of into their shared memory (a list made at the start), so
+//             every gather is local; barrier.cluster between phases. (Gathering from the other
+//             CTAs instead took 3 us a mat-vec on a 10 k-vertex icosphere, whose edge rows read
+//             nothing local; what does not fit the halo is still read so.)
+//   kGrid     up to one CTA an SM (a cooperative launch): global memory at L2, an arrival counter
+//             between phases. Its wait is bounded: a CTA that gives up raises `abort`, every CTA
+//             then leaves, and the host reports OB_ERR_TIMEOUT.
+//
+// Rows longer than the entries a thread holds read the rest from the CSR arrays. A round's float64
+// chain is kept short (two partial sums a row, one division behind the dots), since latency is what
+// is left: the sums a row and the scalars agree with the loop graph's to rounding. The dots are
+// folded thread, warp, CTA in a fixed order, so every run gives the same bits.
+#pragma once
+
+#include "ob_internal.cuh"
+
+namespace ob {
+namespace {
+
+enum ResidentForm : int { kBlock = 0, kCluster = 1, kGrid = 2 };
+constexpr int kClusterMax = 16;
+constexpr int kHalo = 1024;      // other CTAs' values a cluster CTA holds copies of
+constexpr int kHaloTable = 2048; // the hash table that numbers them
+constexpr int kResidentWidth = 16;      // entries a row kept on the chip, at most
+__host__ __device__ constexpr int register_entries(int rows_a_thread) { return rows_a_thread <= 2 ? 7 : 0; }
+__host__ __device__ constexpr int resident_threads(int) { return 512; }
+constexpr int kStatusAborted = -1;      // LoopState::status of a solve whose grid wait gave up
+constexpr unsigned kGridSpins = 1u << 22;  // polls (>= 0.3 us each) before a grid wait gives up
+
+struct ResidentArgs {
+    int n;
+    const int* offsets;
+    const int* columns;
+    const double* values;
+    const double* inv_diag;
+    const double4* steps;  // the polynomial's, when preconditioned by it
+    const double* rhs;
+    double* x;
+    double tol;
+    int maxiter;
+    int check_rounds;  // 0: stop by the residual
+    double change_tolerance;
+    int settle_rounds;
+    LoopState* state;
+    ColumnScalars* scalars;
+    int narrow;  // the operator's values are rounded to float32
+    int width;   // entries a row on the chip, those in registers among them
+    int pushes;  // kCluster: the capacity of a CTA's push list
+    // kGrid: the published vector (two buffers of n), the CTAs' partial sums (6 a CTA), the
+    // arrival counter and the abort flag (both zero at the launch).
+    double* published;
+    double* partials;
+    unsigned int* counter;
+    int* abort;
+};
+
+__device__ __forceinline__ unsigned shared_address(const void* p) {
+    return (unsigned)__cvta_generic_to_shared(p);
+}
+
+__device__ __forceinline__ unsigned cluster_address(unsigned local, int rank) {
+    unsigned out;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(local), "r"(rank));
+    return out;
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile(
+        "barrier.cluster.arrive.release.aligned;\n\t"
+        "barrier.cluster.wait.acquire.aligned;" ::
+            : "memory");
+}
+
+__device__ __forceinline__ void store_cluster(unsigned at, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+}
+
+// A value another SM has written: from L2, and read anew each time.
+__device__ __forceinline__ double load_l2(const double* p) {
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
+// Arrives at a grid barrier and waits until `goal` arrivals (monotonic, wrap-safe). False when
+// this wait, or another CTA's, gave up. Called by every thread.
+__device__ __forceinline__ bool grid_barrier(unsigned int* counter, unsigned int goal, int* abort, int* alive) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(counter, 1u);
+        unsigned seen, spins = 0;
+        int ok = 1;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+            if ((int)(seen - goal) >= 0) break;
+            if (++spins >= kGridSpins || ((spins & 255u) == 0u && *(volatile int*)abort != 0)) {
+                atomicExch(abort, 1);
+                ok = 0;
+                break;
+            }
+        }
+        __threadfence();
+        *alive = ok;
+    }
+    __syncthreads();
+    return *alive != 0;
+}
+
+// The warp's sums of three values: lane 8 q ends with the sum of value q (q < 3), in a fixed
+// order. Two exchange steps hand each quarter of the warp one of the values, the last three add
+// within the quarters: 6 shuffles where three plain sums take 15.
+__device__ __forceinline__ double packed_sum(double v0, double v1, double v2, int lane) {
+    const bool high = lane & 16, odd = lane & 8;
+    const double s0 = __shfl_xor_sync(0xffffffffu, high ? v0 : v2, 16);
+    const double s1 = __shfl_xor_sync(0xffffffffu, high ? v1 : 0.0, 16);
+    double a = (high ? v2 : v0) + s0, b = high ? 0.0 : v1 + s1;
+    a = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+    a += __shfl_xor_sync(0xffffffffu, a, 4);
+    a += __shfl_xor_sync(0xffffffffu, a, 2);
+    return a + __shfl_xor_sync(0xffffffffu, a, 1);
+}
+
+// The sums of three rows of `count` <= 32 values at `from` (rows `stride` apart): a quarter of the
+// warp a row. Every lane gets the three.
+__device__ __forceinline__ void row_sums(const double* from, int stride, int count, int lane, double& v0,
+                                         double& v1, double& v2) {
+    const int q = lane >> 3;
+    double v = 0.0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int w = (lane & 7) + 8 * j;
+        if (q < 3 && w < count) v += from[q * stride + w];
+    }
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v0 = __shfl_sync(0xffffffffu, v, 0);
+    v1 = __shfl_sync(0xffffffffu, v, 8);
+    v2 = __shfl_sync(0xffffffffu, v, 16);
+}
+
+template <int R, int FORM, bool CHEB>
+__global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(const ResidentArgs a) {
+    constexpr int E = register_entries(R);
+    extern __shared__ double resident_smem[];
+    const int T = blockDim.x, S = T * R, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int warps = T >> 5, cta = blockIdx.x, ctas = gridDim.x;
+    // Shared memory: the published vector's two buffers (own rows, then the halo), the cluster's
+    // partial sums (two rows of three values a CTA), the warps' (one), three totals, the entries past
+    // the registers' (values, places), then the halo's table and the push list.
+    const int buffer = FORM == kGrid ? 0 : S + (FORM == kCluster ? kHalo : 0);
+    double* pub = resident_smem;
+    double* parts = pub + 2 * buffer;
+    double* scratch = parts + 6 * kClusterMax;
+    double* totals = scratch + 3 * 32;
+    int* alive = reinterpret_cast<int*>(totals + 3);
+    double* vals = totals + 4;
+    const int more = a.width - E;
+    int2* push = reinterpret_cast<int2*>(vals + (size_t)more * S);  // (own row, address); kCluster
+    int* table = reinterpret_cast<int*>(push + (FORM == kCluster ? a.pushes : 0));
+    int* table_slot = table + kHaloTable;
+    int* counters = table_slot + kHaloTable;  // halo values, pushes, pulled entries
+    unsigned* places = FORM == kCluster ? reinterpret_cast<unsigned*>(counters + 4) : reinterpret_cast<unsigned*>(push);
+    const unsigned pub_at = FORM == kGrid ? 0u : shared_address(pub);
+    unsigned goal = 0;  // grid arrivals due
+    bool ok = true, pulls = false;
+    int pushed = 0;
+
+    auto barrier = [&]() {
+        if (FORM == kBlock) __syncthreads();
+        if (FORM == kCluster) cluster_barrier();
+        if (FORM == kGrid) {
+            goal += (unsigned)ctas;
+            ok = grid_barrier(a.counter, goal, a.abort, alive) && ok;
+        }
+    };
+    // Sums over every row of the system, in two halves around a barrier: `fold` leaves the CTA's
+    // three sums where `read` finds them after the next barrier(). `slot` 0: the dots; 1: the
+    // settle check's, a maximum and a sum -- the two may wait for the same barrier. (Between two
+    // folds lies a barrier() after which the first's scratch is not read; one CTA reads it later.)
+    auto fold = [&](double v0, double v1, double v2, int slot) {
+        if (FORM == kBlock && slot == 1) __syncthreads();
+        if (slot == 0) {
+            v0 = packed_sum(v0, v1, v2, lane);
+            if ((lane & 7) == 0 && lane < 24) scratch[4 * lane + warp] = v0;
+        } else {
+            v0 = warp_max(v0);
+            v1 = warp_sum(v1);
+            if (lane == 0) {
+                scratch[warp] = v0;
+                scratch[32 + warp] = v1;
+            }
+        }
+        if (FORM == kBlock) return;
+        __syncthreads();
+        if (warp != 0) return;
+        if (slot == 0) {
+            row_sums(scratch, 32, warps, lane, v0, v1, v2);
+        } else {
+            v0 = warp_max(lane < warps ? scratch[lane] : 0.0);
+            v1 = warp_sum(lane < warps ? scratch[32 + lane] : 0.0);
+            v2 = 0.0;
+        }
+        if (FORM == kCluster) {
+            if (lane < ctas) {
+                const unsigned at = cluster_address(shared_address(parts + 3 * kClusterMax * slot + cta), lane);
+                store_cluster(at, v0);
+                store_cluster(at + 8u * kClusterMax, v1);
+                store_cluster(at + 16u * kClusterMax, v2);
+            }
+        } else if (lane == 0) {
+            double* at = a.partials + (size_t)3 * ctas * slot + cta;
+            __stcg(at, v0);
+            __stcg(at + ctas, v1);
+            __stcg(at + 2 * ctas, v2);
+        }
+    };
+    auto read = [&](double& v0, double& v1, double& v2, int slot) {
+        if (FORM == kGrid) {
+            // A warp a sum, so the CTAs' partials are read once a CTA.
+            if (warp < 3) {
+                const double* from = a.partials + (size_t)ctas * (3 * slot + warp);
+                const bool largest = slot == 1 && warp == 0;
+                double v = 0.0;
+#pragma unroll 5
+                for (int b = lane; b < ctas; b += 32) {
+                    const double p = load_l2(from + b);
+                    v = largest ? fmax(v, p) : v + p;
+                }
+                __syncwarp();
+                v = largest ? warp_max(v) : warp_sum(v);
+                if (lane == 0) totals[warp] = v;
+            }
+            __syncthreads();
+            v0 = totals[0], v1 = totals[1], v2 = totals[2];
+            return;
+        }
+        const double* from = FORM == kBlock ? scratch : parts + 3 * kClusterMax * slot;
+        const int stride = FORM == kBlock ? 32 : kClusterMax, count = FORM == kBlock ? warps : ctas;
+        if (slot == 0) {
+            row_sums(from, stride, count, lane, v0, v1, v2);
+        } else {
+            v0 = warp_max(lane < count ? from[lane] : 0.0);
+            v1 = warp_sum(lane < count ? from[stride + lane] : 0.0);
+        }
+    };
+
+    // -- the rows: their entries, r = b - A x ----------------------------------------------------
+    double x[R], r[R], p[R], s[R], u[R], inv[R], scaled[R], previous[R];
+    double value[E ? E : 1][R];
+    unsigned place[E ? E : 1][R];  // a column until the places are known
+    int over = 0, span = 0;
+    double bb = 0.0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int row = cta * S + i * T + tid;
+        const bool live = row < a.n;
+        const int o = live ? a.offsets[row] : 0, d = live ? a.offsets[row + 1] - o : 0;
+        const unsigned self = (unsigned)min(row, a.n - 1);
+        double ax = 0.0;
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const bool has = e < d;
+            const int col = has ? a.columns[o + e] : (int)self;
+            const double v = has ? a.values[o + e] : 0.0;
+            if (has) ax = fma(v, a.x[col], ax);
+            value[e][i] = a.narrow ? (double)(float)v : v;
+            place[e][i] = (unsigned)col;
+        }
+        for (int e = E; e < d; ++e) {
+            const int col = a.columns[o + e];
+            const double v = a.values[o + e];
+            ax = fma(v, a.x[col], ax);
+            if (e < a.width) {
+                vals[((e - E) * R + i) * T + tid] = a.narrow ? (double)(float)v : v;
+                places[((e - E) * R + i) * T + tid] = (unsigned)col;
+            }
+        }
+        over |= d > a.width;
+        span = max(span, min(d, a.width));
+        const double b = live ? a.rhs[row] : 0.0;
+        bb = fma(b, b, bb);
+        x[i] = live ? a.x[row] : 0.0;
+        previous[i] = x[i];
+        r[i] = live ? b - ax : 0.0;
+        inv[i] = live ? a.inv_diag[row] : 0.0;
+        p[i] = s[i] = 0.0;
+        scaled[i] = u[i] = inv[i] * r[i];
+    }
+    // The warp's rows are padded to one span with zero entries on a live row.
+    __syncwarp();
+    over = __any_sync(0xffffffffu, over);
+    span = __reduce_max_sync(0xffffffffu, span);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int row = cta * S + i * T + tid;
+        const int d = row < a.n ? a.offsets[row + 1] - a.offsets[row] : 0;
+        for (int e = max(d, E); e < span; ++e) {
+            vals[((e - E) * R + i) * T + tid] = 0.0;
+            places[((e - E) * R + i) * T + tid] = (unsigned)min(row, a.n - 1);
+        }
+    }
+
+    // -- the halo: each other CTA's column numbered once, its owner told to push it ------------
+    auto mine = [&](int col) { return FORM != kCluster || (unsigned)(col - cta * S) < (unsigned)S; };
+    // A column's place in the table (-1: the table was full when it came).
+    auto find = [&](int col, bool insert) -> int {
+        unsigned h = ((unsigned)col * 2654435761u) >> 21;  // kHaloTable = 2^11
+        for (int probe = 0; probe < 64; ++probe, h = (h + 1) & (kHaloTable - 1)) {
+            const int was = insert ? atomicCAS(&table[h], -1, col) : table[h];
+            if (was == col || (insert && was == -1)) return (int)h;
+            if (was == -1) return -1;
+        }
+        return -1;
+    };
+    // A column's shared address (its own row's, its halo copy's, or its owner's), or the column.
+    auto place_of = [&](int col) -> unsigned {
+        if (FORM == kGrid) return (unsigned)col;
+        if (mine(col)) return pub_at + 8u * (unsigned)(FORM == kCluster ? col - cta * S : col);
+        const int h = find(col, false);
+        if (h >= 0 && table_slot[h] >= 0) return pub_at + 8u * (unsigned)(S + table_slot[h]);
+        return cluster_address(pub_at + 8u * (unsigned)(col % S), col / S);
+    };
+    if (FORM == kCluster) {
+        for (int h = tid; h < kHaloTable; h += T) table[h] = -1;
+        if (tid < 4) counters[tid] = 0;
+        for (int i = tid; i < 2 * kHalo; i += T) pub[(i / kHalo) * buffer + S + i % kHalo] = 0.0;
+        cluster_barrier();  // every CTA of the cluster runs, its table and counters are ready
+        bool pulled = false;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+                if (!mine((int)place[e][i])) pulled |= find((int)place[e][i], true) < 0;
+            for (int e = E; e < span; ++e) {
+                const int col = (int)places[((e - E) * R + i) * T + tid];
+                if (!mine(col)) pulled |= find(col, true) < 0;
+            }
+        }
+        __syncthreads();
+        for (int h = tid; h < kHaloTable; h += T) {
+            if (table[h] < 0) continue;
+            const int slot = atomicAdd(&counters[0], 1), owner = table[h] / S;
+            int taken = -1;
+            if (slot < kHalo) {
+                unsigned at;
+                asm volatile("atom.shared::cluster.add.u32 %0, [%1], 1;"
+                             : "=r"(at)
+                             : "r"(cluster_address(shared_address(counters + 1), owner))
+                             : "memory");
+                if ((int)at < a.pushes) {
+                    const unsigned entry = cluster_address(shared_address(push + at), owner);
+                    asm volatile("st.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(entry),
+                                 "r"(table[h] - owner * S), "r"((cta << 16) | slot)
+                                 : "memory");
+                    taken = slot;
+                }
+            }
+            table_slot[h] = taken;
+            pulled |= taken < 0;
+        }
+        if (over) pulled = true;  // entries read from the CSR arrays may lie anywhere
+        if (__any_sync(0xffffffffu, pulled) && lane == 0) atomicOr(&counters[2], 1);
+        cluster_barrier();  // every owner's list is whole
+        pulls = counters[2] != 0;
+        pushed = min(counters[1], a.pushes);
+        for (int q = tid; q < pushed; q += T) {
+            const int2 to = push[q];
+            push[q].y = (int)cluster_address(pub_at + 8u * (unsigned)(S + (to.y & 0xffff)), to.y >> 16);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) place[e][i] = place_of((int)place[e][i]);
+        for (int e = E; e < span; ++e) {
+            unsigned* at = places + ((e - E) * R + i) * T + tid;
+            *at = place_of((int)*at);
+        }
+    }
+
+    int parity = 0;
+    auto publish = [&](const double* v) {
+        parity ^= 1;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int at = i * T + tid;
+            if (FORM != kGrid)
+                pub[parity * buffer + at] = v[i];
+            else if (cta * S + at < a.n)
+                __stcg(a.published + (size_t)parity * a.n + cta * S + at, v[i]);
+        }
+        if (FORM == kCluster) {
+            __syncthreads();
+            for (int q = tid; q < pushed; q += T) {
+                const int2 to = push[q];
+                store_cluster((unsigned)to.y + 8u * (unsigned)(parity * buffer), pub[parity * buffer + to.x]);
+            }
+        }
+    };
+    auto gather = [&](unsigned at) -> double {
+        double v;
+        if (FORM == kGrid) {
+            v = load_l2(a.published + (size_t)parity * a.n + at);
+        } else if (FORM == kCluster && pulls) {
+            asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(at + 8u * (unsigned)(parity * buffer)));
+        } else {
+            asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(at + 8u * (unsigned)(parity * buffer)));
+        }
+        return v;
+    };
+    // out = A (the published vector): two partial sums a row halve the chain.
+    auto matvec = [&](double* out) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            double even = 0.0, odd = 0.0;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                if (e & 1) odd = fma(value[e][i], gather(place[e][i]), odd);
+                else even = fma(value[e][i], gather(place[e][i]), even);
+            }
+            out[i] = even + odd;
+        }
+        for (int e0 = E; e0 < span; e0 += 4) {
+#pragma unroll
+            for (int e1 = 0; e1 < 4; ++e1) {
+                const int e = e0 + e1;
+                if (e >= span) break;
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const int at = ((e - E) * R + i) * T + tid;
+                    out[i] = fma(vals[at], gather(places[at]), out[i]);
+                }
+            }
+        }
+        if (over) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int row = cta * S + i * T + tid;
+                const int o = row < a.n ? a.offsets[row] : 0, d = row < a.n ? a.offsets[row + 1] - o : 0;
+                for (int e = a.width; e < d; ++e) {
+                    const double v = a.narrow ? (double)(float)a.values[o + e] : a.values[o + e];
+                    out[i] = fma(v, gather(place_of(a.columns[o + e])), out[i]);
+                }
+            }
+            __syncwarp();
+        }
+    };
+    // u = the polynomial of the published `scaled` (which is u itself under Jacobi), published.
+    auto precondition = [&]() {
+        if (!CHEB) return;
+        double before[R], ax[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) u[i] = before[i] = scaled[i];
+        for (int index = 0; index < kChebyshevDegree - 1 && ok; ++index) {
+            const double4 st = a.steps[index];
+            const double slope = st.w * st.x;
+            double base[R];  // what the step takes from the vectors it has
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const double current = st.x * u[i];
+                base[i] = fma(st.w, scaled[i], fma(st.z, current - st.y * before[i], current));
+                before[i] = u[i];
+            }
+            matvec(ax);
+#pragma unroll
+            for (int i = 0; i < R; ++i) u[i] = fma(-slope * inv[i], ax[i], base[i]);
+            publish(u);
+            barrier();
+        }
+    };
+
+    // -- the start: |b|^2, u published ---------------------------------------------------------
+    double rr0 = 0.0, unused0, unused1;
+    fold(bb, 0.0, 0.0, 0);
+    publish(CHEB ? scaled : u);
+    barrier();
+    read(rr0, unused0, unused1, 0);
+    barrier();  // the sums are read before the next fold writes them
+    precondition();
+    const double atol_sq = a.tol * a.tol * rr0;
+    // 1 / gamma of the last step, formed beside its other division (0: its value has no such inverse).
+    double gamma_old = INFINITY, inverse_old = 0.0, denominator_old = 0.0, rr = rr0;
+    double settle_previous = 0.0, settle_reach = 0.0, settle_checks = 0.0;
+    int round = 0, iterations = 0, status = OB_STATUS_CAPPED;
+    bool done = false;
+    while (!done && ok) {
+        double w[R], ag = 0.0, ad = 0.0, ar = 0.0;
+        matvec(w);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            ag = fma(r[i], u[i], ag);
+            ad = fma(w[i], u[i], ad);
+            ar = fma(r[i], r[i], ar);
+        }
+        double gamma, delta;
+        fold(ag, ad, ar, 0);
+        barrier();
+        if (!ok) break;
+        read(gamma, delta, rr, 0);
+        double alpha = 0.0, beta = 0.0;
+        bool step = false;
+        if (rr > atol_sq && round <= a.maxiter && gamma != 0.0) {
+            // beta gamma / alpha_old of the loop graph, with alpha_old = gamma_old / denominator_old.
+            beta = inverse_old != 0.0 ? gamma * inverse_old : gamma / gamma_old;
+            const double denominator = delta - beta * beta * denominator_old;
+            if (denominator != 0.0) {
+                alpha = gamma / denominator;
+                const double inverse = 1.0 / gamma;
+                step = true;
+                inverse_old = gamma > 1e-290 && gamma < 1e290 ? inverse : 0.0;
+                gamma_old = gamma;
+                denominator_old = denominator;
+            }
+        }
+        iterations += step ? 1 : 0;
+        if (!step || round >= a.maxiter) {
+            done = true;
+            status = !(rr == rr) ? OB_STATUS_NONFINITE
+                     : (!step && round <= a.maxiter) ? OB_STATUS_CONVERGED
+                                                     : OB_STATUS_CAPPED;
+        }
+        ++round;
+        if (step) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                p[i] = fma(beta, p[i], u[i]);
+                s[i] = fma(beta, s[i], w[i]);
+                x[i] = fma(alpha, p[i], x[i]);
+                r[i] = fma(-alpha, s[i], r[i]);
+                scaled[i] = inv[i] * r[i];
+                if (!CHEB) u[i] = scaled[i];
+            }
+        }
+        if (done) break;
+        const bool check = a.check_rounds > 0 && round % a.check_rounds == 0;
+        if (check) {
+            double change = 0.0, reached = 0.0;
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                if (x[i] != 0.0) {
+                    change = fmax(change, fabs(x[i] - previous[i]) / fabs(x[i]));
+                    reached += 1.0;
+                }
+                previous[i] = x[i];
+            }
+            fold(change, reached, 0.0, 1);
+        }
+        publish(CHEB ? scaled : u);
+        barrier();
+        if (!ok) break;
+        if (check) {
+            double change, reached;
+            read(change, reached, unused0, 1);
+            settle_checks += 1.0;
+            if (reached + 1.0 != settle_previous) {
+                settle_previous = reached + 1.0;
+                settle_reach = settle_checks;
+            } else if (change < a.change_tolerance ||
+                       (settle_checks - settle_reach) * (double)a.check_rounds >= (double)a.settle_rounds) {
+                done = true;
+                status = change < a.change_tolerance ? OB_STATUS_SETTLED : OB_STATUS_SETTLE_BOUND;
+            }
+            if (FORM == kBlock) __syncthreads();  // the scratch is read before the next fold
+        }
+        if (!done) precondition();
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int row = cta * S + i * T + tid;
+        if (row < a.n) a.x[row] = x[i];
+    }
+    if (cta == 0 && tid == 0) {
+        a.state->round = round;
+        a.state->iterations = iterations;
+        a.state->done = 1;
+        a.state->status = ok ? status : kStatusAborted;
+        a.scalars->rr = rr;
+        a.scalars->rr0 = rr0;
+    }
+    if (FORM == kCluster) cluster_barrier();  // no CTA leaves while another may still read its memory
+}
+
+}  // namespace
+}  // namespace ob

@@ -1,0 +1,115 @@
+"""The resident conjugate-gradient form at the edges of its sizes, against direct solves."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import scipy.sparse as sp
+import scipy.sparse.linalg as spla
+
+from ordito_b200 import linalg
+from ordito_b200.array import CsrMatrix
+from ordito_b200.device import DeviceArray
+
+pytestmark = pytest.mark.gpu
+
+
+def _operator(n: int, seed: int) -> sp.csr_matrix:
+    """A diagonally dominant symmetric operator of neighbours at distance 1 and ~sqrt(n) (a
+    dominance of 1.25: condition below 9) with one row and column of 40 entries, more than a
+    thread of the resident form keeps in shared memory."""
+    rng = np.random.default_rng(seed)
+    far = max(2, int(n**0.5))
+    rows, cols = [], []
+    for step in (1, far):
+        at = np.arange(max(0, n - step))
+        rows.append(at)
+        cols.append(at + step)
+    if n > 64:
+        to = rng.choice(np.arange(2, n), size=40, replace=False)
+        rows.append(np.full(40, 0))
+        cols.append(to)
+    i, j = np.concatenate(rows), np.concatenate(cols)
+    off = sp.coo_matrix((-rng.uniform(0.5, 1.0, i.size), (i, j)), shape=(n, n)).tocsr()
+    off = off + off.T
+    diagonal = 1.25 * np.maximum(-np.asarray(off.sum(axis=1)).ravel(), 1.0)
+    matrix = (off + sp.diags(diagonal)).tocsr()
+    matrix.sort_indices()
+    return matrix
+
+
+# One CTA (1 to 1024 rows), a cluster (to 16 x 1024 at two rows a thread, then four), the grid at two
+# rows a thread (148 x 1024), at four (148 x 2048), and the loop graph past it.
+_SIZES = (1, 2, 31, 33, 1024, 1025, 2049, 16384, 16385, 26001, 32769, 151552, 151553, 303104, 303105)
+
+
+@pytest.mark.parametrize("kind", ["diag", "chebyshev"])
+@pytest.mark.parametrize("n", _SIZES)
+def test_solve_at_every_form_edge(gpu, n: int, kind: str) -> None:
+    host = _operator(n, n)
+    matrix = CsrMatrix.from_host(host.indptr, host.indices, host.data, host.shape)
+    rng = np.random.default_rng(n + 1)
+    rhs, start = rng.normal(size=n), rng.normal(size=n)
+    preconditioner = (linalg.chebyshev_preconditioner if kind == "chebyshev"
+                      else linalg.jacobi_preconditioner)(matrix)
+    tol = 1e-10
+    results = []
+    for _ in range(2):
+        x = DeviceArray.from_host(start)
+        _, residual, _ = linalg.solve_spd(matrix, DeviceArray.from_host(rhs), x, tol=tol,
+                                          preconditioner=preconditioner)
+        assert residual <= tol
+        results.append(x.numpy())
+    np.testing.assert_array_equal(results[0], results[1])
+    # |b - A x| <= tol |b| (the recurrence's residual; its drift from the true one is of the order
+    # of the rounding, 1e-16 times the ~25 rounds' terms, far below tol).
+    assert np.linalg.norm(rhs - host @ results[0]) <= 1.01 * tol * np.linalg.norm(rhs)
+
+
+@pytest.mark.parametrize("n", [1500, 9000, 16384, 20000, 40000])
+def test_scattered_rows(gpu, n: int) -> None:
+    """Rows in random order: every CTA reads the others' rows, past what its halo and push list hold."""
+    rng = np.random.default_rng(n)
+    order = rng.permutation(n)
+    host = _operator(n, 3)[order][:, order].tocsr()
+    host.sort_indices()
+    matrix = CsrMatrix.from_host(host.indptr, host.indices, host.data, host.shape)
+    rhs = rng.normal(size=n)
+    for preconditioner in (linalg.jacobi_preconditioner(matrix), linalg.chebyshev_preconditioner(matrix)):
+        x = DeviceArray.zeros(n, np.float64)
+        linalg.solve_spd(matrix, DeviceArray.from_host(rhs), x, tol=1e-10, preconditioner=preconditioner)
+        assert np.linalg.norm(rhs - host @ x.numpy()) <= 1.01e-10 * np.linalg.norm(rhs)
+
+
+@pytest.mark.parametrize("n", [1, 33, 1024, 1025, 16385, 32769, 151553, 303105])
+def test_settle_at_every_form_edge(gpu, n: int) -> None:
+    """The settled solve reaches every entry in its own precision: verified by the componentwise
+    backward error the solver accepts iterates by, against a direct solve."""
+    host = _operator(n, n + 7)
+    matrix = CsrMatrix.from_host(host.indptr, host.indices, host.data, host.shape)
+    rhs = np.random.default_rng(n).uniform(0.5, 1.5, size=n)
+    x = DeviceArray.zeros(n, np.float64)
+    linalg.solve_spd_settled(matrix, DeviceArray.from_host(rhs), x, check_rounds=16, change_tolerance=1e-6,
+                             settle_rounds=192)
+    got = x.numpy()
+    # The iteration's operator holds float32 values (6e-8 each): a backward error of 1e-7, and a
+    # componentwise condition below 9 for this dominance.
+    scale = np.abs(host) @ np.abs(got) + np.abs(rhs)
+    assert np.max(np.abs(rhs - host @ got) / scale) <= 2e-7
+    if n <= 40000:
+        want = spla.splu(host.tocsc()).solve(rhs)
+        np.testing.assert_allclose(got, want, rtol=2e-6)
+
+
+def test_rebound_state_solves_the_new_operator(gpu) -> None:
+    """A kept state of the same shape takes another operator's values (and its wide row's)."""
+    n = 3000
+    first, second = _operator(n, 1), _operator(n, 1)
+    second.data = second.data * 1.5
+    rhs = np.random.default_rng(0).normal(size=n)
+    for host in (first, second, first):
+        matrix = CsrMatrix.from_host(host.indptr, host.indices, host.data, host.shape)
+        x = DeviceArray.zeros(n, np.float64)
+        linalg.solve_spd(matrix, DeviceArray.from_host(rhs), x, tol=1e-12)
+        assert np.linalg.norm(rhs - host @ x.numpy()) <= 1e-11 * np.linalg.norm(rhs)
+        matrix.release()
