@@ -39,7 +39,7 @@ namespace {
 constexpr int kPanel = 64;         // columns eliminated a panel step; tile edge of K2 / K3
 constexpr int kDiagThreads = 256;
 constexpr int kTileThreads = 128;  // four warps, each a 16-row strip of the 64 x 64 output
-constexpr int kSmemLd = kPanel + 1;
+constexpr int kSmemLd = kPanel + 4;
 constexpr int kTileSmem = 2 * kPanel * kSmemLd * (int)sizeof(double);
 constexpr int kExtendThreads = 256;
 constexpr int kExtendColumns = 32;  // child columns an extend-add task takes
@@ -51,24 +51,20 @@ struct ExtendTask {
     int child, parent, b0, b1;
 };
 
-// K1: the diagonal block (b x b) of a panel at front offset f (leading dimension fld), its
-// inverse written at z in the factor's values (leading dimension zld).
-struct DiagTask {
+// One panel of one front: its front (offset f, leading dimension fld, m rows), its stored block
+// (offset z, leading dimension zld), the panel's first column j0 and width b. K1 takes one task a
+// CTA; K2 and K3 take 64 x 64 output tiles of [j1, m), j1 = j0 + b, numbered within the task from
+// its first tile of the launch: K2 the row tiles of the panel below the diagonal, then the column
+// tiles of the stored block's panel rows; K3 the lower tiles of the trailing front (column by
+// column), then the tiles of the stored block below (row by row).
+struct StepTask {
     long long f, z;
-    int fld, zld, b, pad;
+    int fld, zld, m, j0, b;
+    int first_panel, first_trailing;
+    int pad;
 };
 
-// K2 / K3: C (rows x cols) = or -= A (rows x inner) B (inner x cols), inner <= 64.
-// A(i, kk) at a + i a_rs + kk a_ks, B(kk, c) at b + kk b_ks + c b_cs, C(i, c) at c + i c_rs +
-// c c_cs; each offset into the front arena (buffer 0) or the factor's values (buffer 1).
-struct ProductTile {
-    long long a, b, c;
-    int a_rs, a_ks, b_ks, b_cs, c_rs, c_cs;
-    int rows, cols, inner;
-    unsigned char a_buf, b_buf, c_buf, subtract;
-};
-
-enum LaunchKind : int { kExtend = 0, kDiag = 1, kProduct = 2 };
+enum LaunchKind : int { kExtend = 0, kDiag = 1, kPanelProduct = 2, kTrailing = 3 };
 
 }  // namespace
 
@@ -97,6 +93,7 @@ struct FactorPlan {
     struct Launch {
         int kind;
         const void* tasks;
+        const int* owner;  // K2 / K3: each tile's task
         int count;
     };
     std::vector<Launch> launches;  // the whole numeric schedule, in order
@@ -301,17 +298,18 @@ int build_plan(const CholAnalysis& A, FactorPlan* P, cudaStream_t stream) {
     std::vector<std::vector<int>> at_level(A.levels);
     for (int s = 0; s < ns; ++s) at_level[A.nodes[s].level].push_back(s);
     std::vector<ExtendTask> extend;
-    std::vector<DiagTask> diag;
-    std::vector<ProductTile> tiles;
-    // Task lists are gathered on the host per launch, then uploaded as one array each.
+    std::vector<StepTask> steps;
+    std::vector<int> owners;
+    // Task lists are gathered on the host, then uploaded as one array each.
     struct Pending {
         int kind;
-        size_t first, count;
+        size_t first, count, owner;
     };
     std::vector<Pending> pending;
-    auto add = [&](int kind, size_t first, size_t count) {
-        if (count > 0) pending.push_back(Pending{kind, first, count});
+    auto add = [&](int kind, size_t first, size_t count, size_t owner) {
+        if (count > 0) pending.push_back(Pending{kind, first, count, owner});
     };
+    const auto tiles_of = [](int extent) { return (extent + kPanel - 1) / kPanel; };
     for (int l = 0; l < A.levels; ++l) {
         const std::vector<int>& nodes = at_level[l];
         size_t ranks = 0;
@@ -324,119 +322,55 @@ int build_plan(const CholAnalysis& A, FactorPlan* P, cudaStream_t stream) {
                 for (int b0 = 0; b0 < noff[c]; b0 += kExtendColumns)
                     extend.push_back(ExtendTask{c, p, b0, std::min(noff[c], b0 + kExtendColumns)});
             }
-            add(kExtend, first, extend.size() - first);
+            add(kExtend, first, extend.size() - first, 0);
         }
-        int steps = 0;
-        for (int s : nodes) steps = std::max(steps, (nc[s] + kPanel - 1) / kPanel);
-        for (int step = 0; step < steps; ++step) {
-            const int j0 = step * kPanel;
-            const size_t d_first = diag.size(), k2_first = tiles.size();
+        int panels = 0;
+        for (int s : nodes) panels = std::max(panels, tiles_of(nc[s]));
+        for (int panel = 0; panel < panels; ++panel) {
+            const int j0 = panel * kPanel;
+            const size_t first = steps.size(), k2_first = owners.size();
+            size_t k2 = 0, k3 = 0;
             for (int s : nodes) {
                 if (nc[s] <= j0) continue;
-                const int b = std::min(kPanel, nc[s] - j0), j1 = j0 + b, m = nc[s] + noff[s];
-                const long long f = front_at[s];
-                const long long z = layout.inv_at[s];
-                const int ld = layout.ld_at[s], fl = fld[s];
-                diag.push_back(DiagTask{f + (long long)j0 * fl + j0, z + (long long)j0 * ld + j0, fl, ld, b, 0});
-                // K2: L = F D^-T for rows [j1, m) (in place), D^-1 from the stored block.
-                for (int rb = j1; rb < m; rb += kPanel) {
-                    ProductTile t{};
-                    t.a = f + (long long)j0 * fl + rb;
-                    t.a_rs = 1;
-                    t.a_ks = fl;
-                    t.b = z + (long long)j0 * ld + j0;  // B(kk, c) = D^-1(c, kk)
-                    t.b_ks = 1;
-                    t.b_cs = ld;
-                    t.c = t.a;
-                    t.c_rs = 1;
-                    t.c_cs = fl;
-                    t.rows = std::min(kPanel, m - rb);
-                    t.cols = b;
-                    t.inner = b;
-                    t.a_buf = 0, t.b_buf = 1, t.c_buf = 0, t.subtract = 0;
-                    tiles.push_back(t);
-                }
-                // K2: the panel's rows of the stored block, Z_p = D^-1 Z_p over columns [0, j0).
-                for (int cb = 0; cb < j0; cb += kPanel) {
-                    ProductTile t{};
-                    t.a = z + (long long)j0 * ld + j0;  // A(i, kk) = D^-1(i, kk)
-                    t.a_rs = ld;
-                    t.a_ks = 1;
-                    t.b = z + (long long)j0 * ld + cb;  // B(kk, c) = Z(j0 + kk, cb + c)
-                    t.b_ks = ld;
-                    t.b_cs = 1;
-                    t.c = t.b;
-                    t.c_rs = ld;
-                    t.c_cs = 1;
-                    t.rows = b;
-                    t.cols = std::min(kPanel, j0 - cb);
-                    t.inner = b;
-                    t.a_buf = 1, t.b_buf = 1, t.c_buf = 1, t.subtract = 0;
-                    tiles.push_back(t);
-                }
+                StepTask t{};
+                t.f = front_at[s];
+                t.z = layout.inv_at[s];
+                t.fld = fld[s];
+                t.zld = layout.ld_at[s];
+                t.m = nc[s] + noff[s];
+                t.j0 = j0;
+                t.b = std::min(kPanel, nc[s] - j0);
+                t.first_panel = (int)k2;
+                t.first_trailing = (int)k3;
+                const size_t below = tiles_of(t.m - j0 - t.b);
+                k2 += below + tiles_of(j0);
+                k3 += below * (below + 1) / 2 + below * tiles_of(j0 + t.b);
+                steps.push_back(t);
             }
-            add(kDiag, d_first, diag.size() - d_first);
-            add(kProduct, k2_first, tiles.size() - k2_first);
-            const size_t k3_first = tiles.size();
-            for (int s : nodes) {
-                if (nc[s] <= j0) continue;
-                const int b = std::min(kPanel, nc[s] - j0), j1 = j0 + b, m = nc[s] + noff[s];
-                const long long f = front_at[s];
-                const long long z = layout.inv_at[s];
-                const int ld = layout.ld_at[s], fl = fld[s];
-                // K3: F[rb, cb] -= L[rb] L[cb]^T over the lower tiles of [j1, m)^2.
-                for (int cb = j1; cb < m; cb += kPanel)
-                    for (int rb = cb; rb < m; rb += kPanel) {
-                        ProductTile t{};
-                        t.a = f + (long long)j0 * fl + rb;
-                        t.a_rs = 1;
-                        t.a_ks = fl;
-                        t.b = f + (long long)j0 * fl + cb;  // B(kk, c) = L(cb + c, kk)
-                        t.b_ks = fl;
-                        t.b_cs = 1;
-                        t.c = f + (long long)cb * fl + rb;
-                        t.c_rs = 1;
-                        t.c_cs = fl;
-                        t.rows = std::min(kPanel, m - rb);
-                        t.cols = std::min(kPanel, m - cb);
-                        t.inner = b;
-                        t.a_buf = 0, t.b_buf = 0, t.c_buf = 0, t.subtract = 1;
-                        tiles.push_back(t);
-                    }
-                // K3: Z[rb, cb] -= L[rb] Z_p[:, cb] for rows [j1, m), columns [0, j1).
-                for (int rb = j1; rb < m; rb += kPanel)
-                    for (int cb = 0; cb < j1; cb += kPanel) {
-                        ProductTile t{};
-                        t.a = f + (long long)j0 * fl + rb;
-                        t.a_rs = 1;
-                        t.a_ks = fl;
-                        t.b = z + (long long)j0 * ld + cb;
-                        t.b_ks = ld;
-                        t.b_cs = 1;
-                        t.c = z + (long long)rb * ld + cb;
-                        t.c_rs = ld;
-                        t.c_cs = 1;
-                        t.rows = std::min(kPanel, m - rb);
-                        t.cols = std::min(kPanel, j1 - cb);
-                        t.inner = b;
-                        t.a_buf = 0, t.b_buf = 1, t.c_buf = 1, t.subtract = 1;
-                        tiles.push_back(t);
-                    }
+            // Each tile's task, counted from the launch's first.
+            owners.resize(k2_first + k2 + k3);
+            for (size_t i = first; i < steps.size(); ++i) {
+                const size_t end2 = i + 1 < steps.size() ? steps[i + 1].first_panel : k2;
+                const size_t end3 = i + 1 < steps.size() ? steps[i + 1].first_trailing : k3;
+                std::fill(owners.begin() + k2_first + steps[i].first_panel, owners.begin() + k2_first + end2,
+                          (int)(i - first));
+                std::fill(owners.begin() + k2_first + k2 + steps[i].first_trailing,
+                          owners.begin() + k2_first + k2 + end3, (int)(i - first));
             }
-            add(kProduct, k3_first, tiles.size() - k3_first);
+            add(kDiag, first, steps.size() - first, 0);
+            add(kPanelProduct, first, k2, k2_first);
+            add(kTrailing, first, k3, k2_first + k2);
         }
     }
     ExtendTask* d_extend = nullptr;
-    DiagTask* d_diag = nullptr;
-    ProductTile* d_tiles = nullptr;
-    if ((st = upload(P, &d_extend, extend, stream)) || (st = upload(P, &d_diag, diag, stream)) ||
-        (st = upload(P, &d_tiles, tiles, stream)))
+    StepTask* d_steps = nullptr;
+    int* d_owners = nullptr;
+    if ((st = upload(P, &d_extend, extend, stream)) || (st = upload(P, &d_steps, steps, stream)) ||
+        (st = upload(P, &d_owners, owners, stream)))
         return st;
     for (const Pending& q : pending) {
-        const void* base = q.kind == kExtend ? (const void*)(d_extend + q.first)
-                           : q.kind == kDiag ? (const void*)(d_diag + q.first)
-                                             : (const void*)(d_tiles + q.first);
-        P->launches.push_back(FactorPlan::Launch{q.kind, base, (int)q.count});
+        const void* base = q.kind == kExtend ? (const void*)(d_extend + q.first) : (const void*)(d_steps + q.first);
+        P->launches.push_back(FactorPlan::Launch{q.kind, base, d_owners + q.owner, (int)q.count});
     }
     OB_CUDA(cudaStreamSynchronize(stream));  // the host tables go out of scope
     return OB_OK;
@@ -509,124 +443,282 @@ extend_add_kernel(const ExtendTask* __restrict__ tasks, const long long* __restr
     }
 }
 
-// K1: Cholesky of the panel's diagonal block and its inverse, in shared memory. Column j: the
-// pivot's square root, the column below scaled, then the trailing lower triangle and the
-// inverse's rows below updated (the inverse by forward elimination of the identity). A pivot
-// that is not positive sets *status and is replaced by 1, so the launch completes.
+// K1: the panel's diagonal block D = L L^T inverted to L^-1, in registers: a 16 x 16 grid of threads,
+// each with 16 entries of the block (rows tx + 16 a, columns ty + 16 c) and 16 of the identity
+// that forward elimination turns into the inverse (rows ty + 16 a, columns tx + 16 c). The
+// eliminations run unnormalised (column j and the inverse's row j leave as they are, the update
+// takes 1 / d_j once), so a step's chain is one reciprocal, one multiply-add and one barrier;
+// the rows are scaled by d_i^-1/2 at the end. The next column and row are updated and published
+// (two buffers) before the rest of a step's update, so the reciprocal of the next pivot runs
+// beside it. A step in shared memory with a square root, a division and three barriers took
+// 1.3 us (86 us a launch of any size on the 131k torus); this takes 0.2. A pivot that is not
+// positive sets *status and is replaced by 1, so the launch completes.
 __global__ void __launch_bounds__(kDiagThreads)
-diag_block_kernel(const DiagTask* __restrict__ tasks, const double* __restrict__ fronts, double* __restrict__ vals,
+diag_block_kernel(const StepTask* __restrict__ tasks, const double* __restrict__ fronts, double* __restrict__ vals,
                   int* __restrict__ status) {
-    extern __shared__ double diag_smem[];
-    double(*L)[kSmemLd] = reinterpret_cast<double(*)[kSmemLd]>(diag_smem);
-    double(*X)[kSmemLd] = reinterpret_cast<double(*)[kSmemLd]>(diag_smem + kPanel * kSmemLd);
-    const DiagTask t = tasks[blockIdx.x];
-    const int b = t.b;
-    const double* F = fronts + t.f;
-    for (int e = threadIdx.x; e < kPanel * kPanel; e += kDiagThreads) {
-        const int r = e % kPanel, c = e / kPanel;
-        L[r][c] = (r < b && c < b && r >= c) ? F[(size_t)c * t.fld + r] : 0.0;
-        X[r][c] = r == c ? 1.0 : 0.0;
+    __shared__ double col[2][kPanel], row[2][kPanel], reciprocal[2], pivot[kPanel];
+    const StepTask t = tasks[blockIdx.x];
+    const int b = t.b, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const double* F = fronts + t.f + (long long)t.j0 * t.fld + t.j0;
+    double A[4][4], X[4][4];  // A[a][c]: row tx + 16 a, column ty + 16 c; X[a][c]: row ty + 16 a, column tx + 16 c
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const int r = tx + 16 * a, k = ty + 16 * c;
+            A[a][c] = (r < b && k <= r) ? F[(size_t)k * t.fld + r] : 0.0;
+            X[a][c] = ty + 16 * a == tx + 16 * c ? 1.0 : 0.0;
+        }
+    auto take_pivot = [&](int j, double d) {
+        const bool bad = !(d > 0.0);
+        if (bad) *status = 1;
+        d = bad ? 1.0 : d;
+        pivot[j] = d;
+        reciprocal[j & 1] = 1.0 / d;
+    };
+    // Publishes column j of the block (zero above the diagonal) and row j of the inverse.
+    auto publish = [&](int j, const double (&column)[4], const double (&line)[4]) {
+        if (ty == (j & 15)) {
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                const int r = tx + 16 * a;
+                col[j & 1][r] = r > j ? column[a] : 0.0;
+                row[j & 1][r] = line[a];
+                if (r == j) take_pivot(j, column[a]);
+            }
+        }
+    };
+    {
+        const double column[4] = {A[0][0], A[1][0], A[2][0], A[3][0]};
+        publish(0, column, X[0]);
     }
     __syncthreads();
-    for (int j = 0; j < b; ++j) {
-        double d = L[j][j];
-        const bool bad = !(d > 0.0);
-        if (bad) d = 1.0;
-        const double root = sqrt(d), inv = 1.0 / root;
-        __syncthreads();  // every thread has read L[j][j]
-        if (threadIdx.x == 0) {
-            L[j][j] = root;
-            if (bad) *status = 1;
+#pragma unroll
+    for (int jb = 0; jb < 4; ++jb) {
+        for (int jj = 0; jj < 16; ++jj) {
+            const int j = 16 * jb + jj;
+            if (j >= b) break;
+            const double inv = reciprocal[j & 1];
+            double cr[4], ck[4], xr[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                cr[a] = col[j & 1][tx + 16 * a];
+                ck[a] = col[j & 1][ty + 16 * a] * inv;
+                xr[a] = row[j & 1][tx + 16 * a];
+            }
+            // Column j + 1 and the inverse's row j + 1 first.
+            if (j + 1 < b) {
+                double column[4], line[4];
+                if (jj < 15) {
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) {
+                        column[a] = fma(-cr[a], ck[jb], A[a][jb]);
+                        line[a] = fma(-ck[jb], xr[a], X[jb][a]);
+                    }
+                } else {
+                    const int next = jb < 3 ? jb + 1 : 3;
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) {
+                        column[a] = fma(-cr[a], ck[next], A[a][next]);
+                        line[a] = fma(-ck[next], xr[a], X[next][a]);
+                    }
+                }
+                publish(j + 1, column, line);
+            }
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    A[a][c] = fma(-cr[a], ck[c], A[a][c]);
+                    X[a][c] = fma(-ck[a], xr[c], X[a][c]);
+                }
+            __syncthreads();
         }
-        for (int i = j + 1 + threadIdx.x; i < b; i += kDiagThreads) L[i][j] *= inv;
-        for (int c = threadIdx.x; c <= j; c += kDiagThreads) X[j][c] *= inv;
-        __syncthreads();
-        const int rest = b - j - 1;
-        for (int e = threadIdx.x; e < rest * rest; e += kDiagThreads) {
-            const int i = j + 1 + e / rest, k = j + 1 + e % rest;
-            if (k <= i) L[i][k] -= L[i][j] * L[k][j];
-        }
-        for (int e = threadIdx.x; e < rest * (j + 1); e += kDiagThreads) {
-            const int i = j + 1 + e / (j + 1), c = e % (j + 1);
-            X[i][c] -= L[i][j] * X[j][c];
-        }
-        __syncthreads();
     }
-    double* Z = vals + t.z;
-    for (int e = threadIdx.x; e < b * b; e += kDiagThreads) {
-        const int i = e / b, c = e % b;
-        if (c <= i) Z[(size_t)i * t.zld + c] = X[i][c];
+    double* Z = vals + t.z + (long long)t.j0 * t.zld + t.j0;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const int r = ty + 16 * a;
+        if (r >= b) continue;
+        const double scale = rsqrt(pivot[r]);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int k = tx + 16 * c;
+            if (k <= r) Z[(size_t)r * t.zld + k] = X[a][c] * scale;
+        }
     }
 }
 
-// K2 / K3: one 64 x 64 output tile a CTA. A and B are staged whole in shared memory (zero past
-// their extents) before any output is written, so a tile may write the block it reads (the
-// in-place products of K2); no two tiles of a launch write the same entries, and none reads
-// what another writes.
-__global__ void __launch_bounds__(kTileThreads)
-front_product_kernel(const ProductTile* __restrict__ tiles, double* fronts, double* vals) {
+__device__ __forceinline__ void copy_async_8(double* to, const double* from, bool take) {
+    const unsigned at = (unsigned)__cvta_generic_to_shared(to);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(at), "l"(from), "r"(take ? 8 : 0) : "memory");
+}
+
+template <int N>
+__device__ __forceinline__ void copy_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// K2 (TRAILING false) / K3: one 64 x 64 output tile a CTA, C = or -= A (rows x inner) B (inner x
+// cols), inner <= 64. The tile's place in its front follows from its index (StepTask), so the
+// schedule holds one int a tile. A and B are staged by 8-byte asynchronous copies (a front's rows
+// begin at any column after a short panel) in four groups of 16 inner steps, the products of a
+// group running while the later ones arrive; C is fetched with them. Each operand lies in shared
+// memory with its contiguous direction contiguous and a leading dimension of 68, in either
+// orientation free of bank conflicts in the fragment loads (65 had four lanes to a bank). A tile
+// may write the block it reads (the in-place products of K2): every copy has landed before the
+// first store; no two tiles of a launch write the same entries, and none reads what another writes.
+template <bool TRAILING>
+__global__ void __launch_bounds__(kTileThreads, 3)
+front_product_kernel(const StepTask* __restrict__ tasks, const int* __restrict__ owner, double* fronts, double* vals) {
     extern __shared__ double smem[];
-    double* As = smem;                     // As[i * kSmemLd + kk]
-    double* Bs = smem + kPanel * kSmemLd;  // Bs[kk * kSmemLd + c]
-    const ProductTile t = tiles[blockIdx.x];
-    const double* A = (t.a_buf ? vals : fronts) + t.a;
-    const double* B = (t.b_buf ? vals : fronts) + t.b;
-    double* C = (t.c_buf ? vals : fronts) + t.c;
-    const int inner4 = (t.inner + 3) & ~3;
-    for (int e = threadIdx.x; e < kPanel * inner4; e += kTileThreads) {
-        int i, kk;
-        if (t.a_rs == 1) {
-            i = e % kPanel;
-            kk = e / kPanel;
+    double* As = smem;
+    double* Bs = smem + kPanel * kSmemLd;
+    const StepTask t = tasks[owner[blockIdx.x]];
+    const int j1 = t.j0 + t.b, below = (t.m - j1 + kPanel - 1) / kPanel;
+    double* F = fronts + t.f;
+    double* Z = vals + t.z;
+    const long long panel = (long long)t.j0 * t.fld;  // the panel's first column in the front
+    const double *A, *B;
+    double* C;
+    int a_ks, b_ld, c_rs, c_cs, rows, cols;
+    bool a_rows = true, b_cols = true;  // A contiguous down its rows, B along its columns (else along inner)
+    int q = blockIdx.x - (TRAILING ? t.first_trailing : t.first_panel);
+    if (!TRAILING) {
+        if (q < below) {
+            // L = F D^-T in place: B(kk, c) = D^-1(c, kk).
+            const int rb = j1 + q * kPanel;
+            A = F + panel + rb;
+            a_ks = t.fld;
+            B = Z + (long long)t.j0 * t.zld + t.j0;
+            b_ld = t.zld;
+            b_cols = false;
+            C = F + panel + rb;
+            c_rs = 1, c_cs = t.fld;
+            rows = min(kPanel, t.m - rb), cols = t.b;
         } else {
-            kk = e % inner4;
-            i = e / inner4;
+            // Z_p = D^-1 Z_p in place over columns [0, j0).
+            const int cb = (q - below) * kPanel;
+            A = Z + (long long)t.j0 * t.zld + t.j0;
+            a_ks = t.zld;
+            a_rows = false;
+            B = Z + (long long)t.j0 * t.zld + cb;
+            b_ld = t.zld;
+            C = Z + (long long)t.j0 * t.zld + cb;
+            c_rs = t.zld, c_cs = 1;
+            rows = t.b, cols = min(kPanel, t.j0 - cb);
         }
-        As[i * kSmemLd + kk] = (i < t.rows && kk < t.inner) ? A[(long long)i * t.a_rs + (long long)kk * t.a_ks] : 0.0;
-        int c;
-        if (t.b_cs == 1) {
-            c = e % kPanel;
-            kk = e / kPanel;
+    } else {
+        const int triangle = below * (below + 1) / 2;
+        a_ks = t.fld;
+        if (q < triangle) {
+            // F[rb, cb] -= L[rb] L[cb]^T over the lower tiles, column by column.
+            int ct = 0;
+            while (q >= below - ct) q -= below - ct, ++ct;
+            const int cb = j1 + ct * kPanel, rb = cb + q * kPanel;
+            A = F + panel + rb;
+            B = F + panel + cb;
+            b_ld = t.fld;
+            C = F + (long long)cb * t.fld + rb;
+            c_rs = 1, c_cs = t.fld;
+            rows = min(kPanel, t.m - rb), cols = min(kPanel, t.m - cb);
         } else {
-            kk = e % inner4;
-            c = e / inner4;
+            // Z[rb, cb] -= L[rb] Z_p[:, cb] for rows [j1, m), columns [0, j1).
+            q -= triangle;
+            const int across = (j1 + kPanel - 1) / kPanel;
+            const int rb = j1 + (q / across) * kPanel, cb = (q % across) * kPanel;
+            A = F + panel + rb;
+            B = Z + (long long)t.j0 * t.zld + cb;
+            b_ld = t.zld;
+            C = Z + (long long)rb * t.zld + cb;
+            c_rs = t.zld, c_cs = 1;
+            rows = min(kPanel, t.m - rb), cols = min(kPanel, j1 - cb);
         }
-        Bs[kk * kSmemLd + c] = (c < t.cols && kk < t.inner) ? B[(long long)kk * t.b_ks + (long long)c * t.b_cs] : 0.0;
     }
-    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wr = warp * 16, fr = lane >> 2, fk = lane & 3;
-    if (wr >= t.rows) return;
-    double acc[2][8][2];
+    // Shared strides of the operands: (row, inner) of A and (inner, column) of B.
+    const int a_i = a_rows ? 1 : kSmemLd, a_k = a_rows ? kSmemLd : 1;
+    const int b_k = b_cols ? kSmemLd : 1, b_c = b_cols ? 1 : kSmemLd;
+    const int groups = (t.b + 15) / 16;
+    const int x = threadIdx.x & 63, y = threadIdx.x >> 6;       // across: 64 outer x 2 inner a step
+    const int k = threadIdx.x & 15, outer = threadIdx.x >> 4;   // along: 16 inner x 8 outer a step
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int g = 0; g < 4; ++g) {
+        if (g < groups) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    const int col_groups = (t.cols + 7) / 8;
-    for (int k4 = 0; k4 < inner4; k4 += 4) {
-        double a[2], bv[8];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) a[i] = As[(wr + 8 * i + fr) * kSmemLd + k4 + fk];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) bv[j] = Bs[(k4 + fk) * kSmemLd + 8 * j + fr];
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (j < col_groups) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], bv[j]);
+            for (int step = 0; step < 8; ++step) {
+                if (a_rows) {
+                    const int kk = 16 * g + 2 * step + y;
+                    const bool in = x < rows && kk < t.b;
+                    copy_async_8(As + kk * kSmemLd + x, in ? A + (long long)kk * a_ks + x : A, in);
+                } else {
+                    const int kk = 16 * g + k, i = 8 * step + outer;
+                    const bool in = i < rows && kk < t.b;
+                    copy_async_8(As + i * kSmemLd + kk, in ? A + (long long)i * a_ks + kk : A, in);
+                }
+                if (b_cols) {
+                    const int kk = 16 * g + 2 * step + y;
+                    const bool in = x < cols && kk < t.b;
+                    copy_async_8(Bs + kk * kSmemLd + x, in ? B + (long long)kk * b_ld + x : B, in);
+                } else {
+                    const int kk = 16 * g + k, c = 8 * step + outer;
+                    const bool in = c < cols && kk < t.b;
+                    copy_async_8(Bs + c * kSmemLd + kk, in ? B + (long long)c * b_ld + kk : B, in);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
+    double acc[2][8][2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const int r = wr + 8 * i + fr;
-        if (r >= t.rows) continue;
 #pragma unroll
         for (int j = 0; j < 8; ++j)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int c = 8 * j + 2 * fk + h;
-                if (c >= t.cols) continue;
-                double* o = C + (long long)r * t.c_rs + (long long)c * t.c_cs;
-                *o = t.subtract ? *o - acc[i][j][h] : acc[i][j][h];
+                acc[i][j][h] = TRAILING && r < rows && c < cols ? C[(long long)r * c_rs + (long long)c * c_cs] : 0.0;
+            }
+    }
+    const int col_groups = (cols + 7) / 8;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        if (g == 0) copy_async_wait<3>();
+        if (g == 1) copy_async_wait<2>();
+        if (g == 2) copy_async_wait<1>();
+        if (g == 3) copy_async_wait<0>();
+        __syncthreads();
+        if (g >= groups || wr >= rows) continue;
+#pragma unroll
+        for (int k4 = 16 * g; k4 < 16 * g + 16; k4 += 4) {
+            double a[2], bv[8];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                a[i] = As[(wr + 8 * i + fr) * a_i + (k4 + fk) * a_k];
+                if (TRAILING) a[i] = -a[i];
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) bv[j] = Bs[(k4 + fk) * b_k + (8 * j + fr) * b_c];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j < col_groups) dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], bv[j]);
+        }
+    }
+    if (wr >= rows) return;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int r = wr + 8 * i + fr;
+        if (r >= rows) continue;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int c = 8 * j + 2 * fk + h;
+                if (c < cols) C[(long long)r * c_rs + (long long)c * c_cs] = acc[i][j][h];
             }
     }
 }
@@ -636,8 +728,8 @@ int allow_product_memory() {
     int device = 0;
     OB_CUDA(cudaGetDevice(&device));
     if (device >= 0 && device < 64 && allowed[device]) return OB_OK;
-    OB_CUDA(cudaFuncSetAttribute(front_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem));
-    OB_CUDA(cudaFuncSetAttribute(diag_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem));
+    OB_CUDA(cudaFuncSetAttribute(front_product_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem));
+    OB_CUDA(cudaFuncSetAttribute(front_product_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem));
     if (device >= 0 && device < 64) allowed[device] = 1;
     return OB_OK;
 }
@@ -703,14 +795,19 @@ int device_factor(CholAnalysis& A, const double* values, double sign, int pin_mo
                 OB_CHECK_LAUNCH("chol extend-add");
                 break;
             case kDiag:
-                diag_block_kernel<<<L.count, kDiagThreads, kTileSmem, stream>>>(static_cast<const DiagTask*>(L.tasks),
-                                                                        fronts, vals, status);
+                diag_block_kernel<<<L.count, kDiagThreads, 0, stream>>>(static_cast<const StepTask*>(L.tasks), fronts,
+                                                                        vals, status);
                 OB_CHECK_LAUNCH("chol diagonal blocks");
                 break;
+            case kPanelProduct:
+                front_product_kernel<false><<<L.count, kTileThreads, kTileSmem, stream>>>(
+                    static_cast<const StepTask*>(L.tasks), L.owner, fronts, vals);
+                OB_CHECK_LAUNCH("chol panel products");
+                break;
             default:
-                front_product_kernel<<<L.count, kTileThreads, kTileSmem, stream>>>(
-                    static_cast<const ProductTile*>(L.tasks), fronts, vals);
-                OB_CHECK_LAUNCH("chol front products");
+                front_product_kernel<true><<<L.count, kTileThreads, kTileSmem, stream>>>(
+                    static_cast<const StepTask*>(L.tasks), L.owner, fronts, vals);
+                OB_CHECK_LAUNCH("chol trailing products");
         }
     }
     int host_status = 0;

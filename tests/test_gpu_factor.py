@@ -236,3 +236,22 @@ def test_tile_widths_solve_alike(gpu, k: int) -> None:
     for got in answers:
         assert np.max(np.abs(got - answers[0])) <= 1e-12 * np.abs(answers[0]).max()
         assert np.max(np.abs(got - ref)) <= 1e-9 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 31, 33, 63, 64, 65, 127, 129, 200])
+def test_dense_operators_at_the_panel_edges(gpu, n: int) -> None:
+    """A complete graph is one front of n columns: panels of 64 and what is left of one (K1's block
+    and its 16 x 16 grid of threads), products of one tile and of several."""
+    import scipy.sparse as sp
+
+    rng = np.random.default_rng(n)
+    q = rng.normal(size=(n, n))
+    dense = q @ q.T + n * np.eye(n)  # a condition below 6
+    host = sp.csr_matrix(dense)
+    matrix = CsrMatrix.from_host(host.indptr, host.indices, host.data, host.shape)
+    factor = sparse_cholesky(matrix)
+    rhs = rng.normal(size=n)
+    x = DeviceArray.zeros(n, np.float64)
+    factor.solve(DeviceArray.from_host(rhs), x, refine=False)
+    # n eps times the condition, for the factorisation and the two passes.
+    np.testing.assert_allclose(x.numpy(), np.linalg.solve(dense, rhs), rtol=0, atol=30 * n * 2.2e-16 * np.abs(rhs).max())
