@@ -615,7 +615,10 @@ __global__ void shift_out_kernel(const double* __restrict__ phi, int n, int stri
 // large mesh is summed by many blocks and the grid does not wait on the largest mesh), each
 // chunk's per-column sums written apart, then folded per mesh in chunk order: a fixed order for a
 // given packing.
-constexpr int kPackedChunk = 2048;
+// 512 rows: a chunk is one block's serial sum, and at 16 columns 2 048 rows were 128 dependent
+// (numbering, value) loads deep, 137 blocks on 148 SMs (48 meshes, 91 k vertices: 101 us; see the
+// sum's own note for what is left).
+constexpr int kPackedChunk = 512;
 
 // The chunk table: chunk_first[m] = mesh m's first chunk (chunk_first[n_meshes] = the count) and
 // per chunk (mesh, first row, end row). One block; the meshes' chunk counts are scanned in
@@ -653,6 +656,7 @@ __global__ void packed_chunks_kernel(const int* __restrict__ vertex_offsets, int
 
 // A chunk's per-column sums of phi: threads own column t % stride (blockDim a multiple of
 // stride), rows t / stride + j (blockDim / stride) in order, then the row groups added in order.
+// Eight rows' places, then their values, are in flight a thread.
 __global__ void packed_partials_kernel(const double* __restrict__ phi, int stride, const int* __restrict__ iperm,
                                        const int* __restrict__ chunk_first, int n_meshes,
                                        const int4* __restrict__ chunks, double* __restrict__ partials) {
@@ -661,8 +665,15 @@ __global__ void packed_partials_kernel(const double* __restrict__ phi, int strid
     const int4 chunk = chunks[blockIdx.x];
     const int c = threadIdx.x % stride, rows_per_pass = blockDim.x / stride;
     double total = 0.0;
-    for (int v = chunk.y + threadIdx.x / stride; v < chunk.z; v += rows_per_pass)
-        total += phi[(size_t)row_of(iperm, v) * stride + c];
+    int v = chunk.y + threadIdx.x / stride;
+    for (; v + 7 * rows_per_pass < chunk.z; v += 8 * rows_per_pass) {
+        double value[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) value[q] = phi[(size_t)row_of(iperm, v + q * rows_per_pass) * stride + c];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) total += value[q];
+    }
+    for (; v < chunk.z; v += rows_per_pass) total += phi[(size_t)row_of(iperm, v) * stride + c];
     tree[threadIdx.x] = total;
     __syncthreads();
     if ((int)threadIdx.x < stride) {
@@ -681,7 +692,9 @@ __global__ void packed_fold_kernel(const double* __restrict__ phi, int stride, c
     const int m = blockIdx.x;
     for (int c = threadIdx.x; c < k; c += blockDim.x) {
         double column = 0.0;
-        for (int b = chunk_first[m]; b < chunk_first[m + 1]; ++b) column += partials[(size_t)b * stride + c];
+        const int end = chunk_first[m + 1];
+#pragma unroll 8
+        for (int b = chunk_first[m]; b < end; ++b) column += partials[(size_t)b * stride + c];
         const int s = sources[(size_t)m * k + c];
         const double at = s >= 0 ? phi[(size_t)row_of(iperm, vertex_offsets[m] + s) * stride + c] : 0.0;
         sums[(size_t)m * k + c] = make_double2(at, column);
