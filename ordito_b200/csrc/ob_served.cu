@@ -360,6 +360,121 @@ grad_div_records_kernel(const double2* __restrict__ records, const int4* __restr
     }
 }
 
+// ---- The divergence over corner planes ------------------------------------------------------
+// The record form's bound is its loads (the L1 pipe: 3 gathers of u and 112 bytes of record a corner)
+// and its 3-vector arithmetic. Both shrink in the face's own plane, where the whole gradient lies:
+// a, b and w are the normal crossed with the three edges, so they sum to zero and the gradient is
+// that of the two differences from the corner's own vertex, d1 = u_next - u_own and d2 = u_prev -
+// u_own (u_own is read once a vertex); and in the plane's orthonormal frame with its first axis
+// along u_next's term, it takes three numbers, s = (d1 b + d2 w_x, d2 w_y), and the corner's W two.
+// A corner is then 48 bytes -- those five numbers and its two other vertices -- read as three
+// 16-byte loads, and two gathers. The frame is float64 from the float64 terms (orthogonalised
+// twice), so the sums agree with the terms form's to its rounding.
+constexpr int kPlanePairs = 3;  // double2 a corner: b w_x | w_y W_x | W_y (next, prev)
+
+__global__ void corner_planes_kernel(const double* __restrict__ terms, const int* __restrict__ faces,
+                                     const int* __restrict__ corner_slots, long long n_corners,
+                                     double2* __restrict__ planes) {
+    const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (p >= n_corners) return;
+    const int q = corner_slots[p];
+    const int f = q / 3, e = q - 3 * f;
+    const int next = e == 2 ? 0 : e + 1, prev = e == 0 ? 2 : e - 1;
+    const double* T = terms + (size_t)kFaceTerms * f;
+    const d3 b{T[3 * next], T[3 * next + 1], T[3 * next + 2]};
+    const d3 w{T[3 * prev], T[3 * prev + 1], T[3 * prev + 2]};
+    const d3 W{T[9 + 3 * e], T[10 + 3 * e], T[11 + 3 * e]};
+    const auto dot = [](const d3& x, const d3& y) { return fma(x.x, y.x, fma(x.y, y.y, x.z * y.z)); };
+    // A length by its largest component, so no square leaves the range.
+    const auto length = [&](const d3& x) {
+        const double m = fmax(fabs(x.x), fmax(fabs(x.y), fabs(x.z)));
+        if (!(m > 0.0)) return 0.0;
+        const d3 y{x.x / m, x.y / m, x.z / m};
+        return m * sqrt(dot(y, y));
+    };
+    const double along = length(b);
+    d3 X{0.0, 0.0, 0.0}, Y{0.0, 0.0, 0.0};
+    double wx = 0.0, wy = 0.0;
+    if (along > 0.0) {
+        X = d3{b.x / along, b.y / along, b.z / along};
+        wx = dot(w, X);
+        d3 r{fma(-wx, X.x, w.x), fma(-wx, X.y, w.y), fma(-wx, X.z, w.z)};
+        const double again = dot(r, X);
+        r = d3{fma(-again, X.x, r.x), fma(-again, X.y, r.y), fma(-again, X.z, r.z)};
+        wx += again;
+        wy = length(r);
+        if (wy > 0.0) Y = d3{r.x / wy, r.y / wy, r.z / wy};
+    }
+    double2* P = planes + (size_t)kPlanePairs * p;
+    P[0] = make_double2(along, wx);
+    P[1] = make_double2(wy, dot(W, X));
+    P[2] = make_double2(dot(W, Y), __hiloint2double(faces[3 * f + next], faces[3 * f + prev]));
+}
+
+template <int CP>
+__global__ void __launch_bounds__(256)
+grad_div_planes_kernel(const double2* __restrict__ planes, const int* __restrict__ corner_offsets, int n, int k,
+                       const double* __restrict__ u, int u_stride, const int* __restrict__ u_iperm,
+                       double* __restrict__ out, int out_stride, const int* __restrict__ out_iperm,
+                       const char* __restrict__ out_pinned) {
+    const int groups = out_stride / CP;
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t >= (long long)n * groups) return;
+    const int v = (int)(t / groups), c0 = (int)(t % groups) * CP;
+    const int row = row_of(out_iperm, v);
+    double acc[CP];
+#pragma unroll
+    for (int j = 0; j < CP; ++j) acc[j] = 0.0;
+    auto load = [&](int r, double* dst) {
+        const double* src = u + (size_t)r * u_stride + c0;
+        if (CP == 1) {
+            dst[0] = src[0];
+        } else {
+#pragma unroll
+            for (int j = 0; j < CP; j += 2) {
+                // A pair starting below k lies inside the row (even strides).
+                const double2 p = (c0 + j < k) ? *reinterpret_cast<const double2*>(src + j) : make_double2(0.0, 0.0);
+                dst[j] = p.x;
+                dst[j + 1] = p.y;
+            }
+        }
+    };
+    if (c0 < k) {
+        const int end = corner_offsets[v + 1];
+        int p = corner_offsets[v];
+        double own[CP];
+        load(row_of(u_iperm, v), own);
+        for (; p < end; ++p) {
+            const double2* P = planes + (size_t)kPlanePairs * p;
+            const double2 p0 = P[0], p1 = P[1], p2 = P[2];
+            double u1[CP], u2[CP];
+            load(row_of(u_iperm, __double2hiint(p2.y)), u1);
+            load(row_of(u_iperm, __double2loint(p2.y)), u2);
+#pragma unroll
+            for (int j = 0; j < CP; ++j) {
+                const double d1 = u1[j] - own[j], d2 = u2[j] - own[j];
+                const double gx = fma(d1, p0.x, d2 * p0.y), gy = d2 * p1.x;
+                const double largest = fmax(fabs(gx), fabs(gy));
+                if (largest == 0.0) continue;  // no gradient: the unit gradient is zero
+                const double scale = inverse_power_of_two(largest);
+                const double sx = gx * scale, sy = gy * scale;
+                acc[j] += fma(sx, p1.y, sy * p2.x) * rsqrt(fma(sx, sx, sy * sy));
+            }
+        }
+    }
+    const bool pinned = out_pinned && out_pinned[row];
+    double* o = out + (size_t)row * out_stride + c0;
+#pragma unroll
+    for (int j = 0; j < CP; ++j)
+        if (pinned || c0 + j >= k) acc[j] = 0.0;
+    if (CP == 1) {
+        o[0] = acc[0];
+    } else {
+#pragma unroll
+        for (int j = 0; j < CP; j += 2) *reinterpret_cast<double2*>(o + j) = make_double2(acc[j], acc[j + 1]);
+    }
+}
+
 // ---- The divergence face by face over tiles of vertices ------------------------------------
 // The per-corner form above recomputes a face's unit gradient at each of its three corners. Here
 // a CTA takes kTileVertices consecutive vertices, forms the unit gradient of each distinct face
@@ -916,6 +1031,47 @@ int ob_grad_div_records(const double* records, const int32_t* ids, const int32_t
                                                                     u_stride, u_iperm, out, out_stride, out_iperm,
                                                                     out_pinned);
     OB_CHECK_LAUNCH("grad_div_records");
+    return OB_OK;
+}
+
+int ob_corner_planes(const double* terms, const int32_t* faces, const int32_t* corner_slots, int n_faces,
+                     double* planes, ob_stream_t stream_) {
+    cudaStream_t stream = as_stream(stream_);
+    OB_REQUIRE(n_faces >= 0, "ob_corner_planes: bad size");
+    if (n_faces == 0) return OB_OK;
+    OB_REQUIRE(terms && faces && corner_slots && planes, "ob_corner_planes: null pointer");
+    OB_REQUIRE(((uintptr_t)planes & 15) == 0, "ob_corner_planes: planes must start on 16 bytes");
+    const long long corners = 3LL * n_faces;
+    corner_planes_kernel<<<ceil_div(corners, kThreads), kThreads, 0, stream>>>(terms, faces, corner_slots, corners,
+                                                                               reinterpret_cast<double2*>(planes));
+    OB_CHECK_LAUNCH("corner_planes");
+    return OB_OK;
+}
+
+int ob_grad_div_planes(const double* planes, const int32_t* corner_offsets, int n_vertices, int n_columns,
+                       const double* u, int u_stride, const int32_t* u_iperm, double* out, int out_stride,
+                       const int32_t* out_iperm, const char* out_pinned, ob_stream_t stream_) {
+    cudaStream_t stream = as_stream(stream_);
+    OB_REQUIRE(n_vertices >= 0 && n_columns >= 1 && u_stride >= n_columns && out_stride >= n_columns,
+               "ob_grad_div_planes: bad size");
+    if (n_vertices == 0) return OB_OK;
+    OB_REQUIRE(planes && corner_offsets && u && out, "ob_grad_div_planes: null pointer");
+    OB_REQUIRE(((uintptr_t)planes & 15) == 0, "ob_grad_div_planes: planes must start on 16 bytes");
+    const bool paired = u_stride % 2 == 0 && out_stride % 2 == 0 && ((uintptr_t)u & 15) == 0 &&
+                        ((uintptr_t)out & 15) == 0;
+    const int cp = !paired ? 1 : (out_stride % 4 == 0 ? 4 : 2);
+    const int blocks = (int)ceil_div((long long)n_vertices * (out_stride / cp), kThreads);
+    const double2* P = reinterpret_cast<const double2*>(planes);
+    if (cp == 4)
+        grad_div_planes_kernel<4><<<blocks, kThreads, 0, stream>>>(P, corner_offsets, n_vertices, n_columns, u, u_stride,
+                                                                   u_iperm, out, out_stride, out_iperm, out_pinned);
+    else if (cp == 2)
+        grad_div_planes_kernel<2><<<blocks, kThreads, 0, stream>>>(P, corner_offsets, n_vertices, n_columns, u, u_stride,
+                                                                   u_iperm, out, out_stride, out_iperm, out_pinned);
+    else
+        grad_div_planes_kernel<1><<<blocks, kThreads, 0, stream>>>(P, corner_offsets, n_vertices, n_columns, u, u_stride,
+                                                                   u_iperm, out, out_stride, out_iperm, out_pinned);
+    OB_CHECK_LAUNCH("grad_div_planes");
     return OB_OK;
 }
 

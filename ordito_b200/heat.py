@@ -423,6 +423,16 @@ class HeatSolver:
         return self._gradient_terms
 
     @property
+    def corner_planes(self) -> DeviceArray:
+        """The divergence's corner planes over the mesh's own numbering (``ob_corner_planes``), built once."""
+        if getattr(self, "_corner_planes", None) is None:
+            mesh = self._mesh
+            planes = corner_planes(self.gradient_terms, mesh.faces, mesh.corner_index[1], mesh.n_faces)
+            _lib.call("ob_stream_synchronize", DEFAULT_STREAM)  # they serve other streams
+            self._corner_planes = planes
+        return self._corner_planes
+
+    @property
     def poisson_multigrid(self) -> Any:
         """The Poisson system's smoothed-aggregation hierarchy, built on first use and kept."""
         if getattr(self, "_poisson_multigrid", None) is None:
@@ -561,7 +571,7 @@ class HeatSolver:
                 matrix.release()
             self._operators = None
         self._systems.clear()
-        self._gradient_terms = None
+        self._gradient_terms = self._corner_planes = None
         self._mesh = None
 
     def release_factorizations(self) -> None:
@@ -583,13 +593,6 @@ class HeatSolver:
 def _require_sources(sources: Any, n_vertices: int) -> DeviceArray:
     src = as_device(sources, np.int32)
     return src.reshape(src.size)
-
-
-# The divergence's form: per corner (ob_grad_div_terms, the default: measured faster -- 3.7 against
-# 10.4 ms on icosphere(9) at 64 columns -- since a tile of 32 vertices still forms 1.7-2 times as
-# many face gradients as there are faces and its shared-memory passes hold fewer warps) or face by
-# face over vertex tiles (ob_grad_div_tiled).
-_TILED_DIVERGENCE = False
 
 
 def divergence_tiles(corner_offsets: DeviceArray, corner_slots: DeviceArray, n: int,
@@ -617,51 +620,41 @@ def corner_records(terms: DeviceArray, faces: DeviceArray, corner_slots: DeviceA
     return records, ids
 
 
-def _grad_div(solver: "HeatSolver", faces: DeviceArray, index: tuple, n: int, k: int, u: int,
-              u_stride: int, u_iperm: Any, out: int, out_stride: int, out_iperm: Any, out_pinned: Any,
-              stream: Any) -> None:
-    _grad_div_index(solver.gradient_terms, faces, index, n, k, u, u_stride, u_iperm, out,
-                    out_stride, out_iperm, out_pinned, stream)
-
-
-def _grad_div_index(terms: DeviceArray, faces: DeviceArray, index: tuple, n: int, k: int, u: int,
-                    u_stride: int, u_iperm: Any, out: int, out_stride: int, out_iperm: Any,
-                    out_pinned: Any, stream: Any) -> None:
-    """``-div`` of the per-face unit gradients of ``k`` heat columns over a corner index and its
-    tiles ``(offsets, slots, tile_faces, tile_counts, codes)``, from per-face terms: each vertex's
-    corners summed in ascending slot order (no atomics: the same bits on every run, the reference's
-    deterministic mode, ordito/heat.py:3170-3232, as the only mode), per corner
-    (``ob_grad_div_terms``) or face by face over the tiles (``ob_grad_div_tiled``)."""
-    corner_offsets, corner_slots, tile_faces, tile_counts, codes = index
-    if _TILED_DIVERGENCE:
-        _lib.call(
-            "ob_grad_div_tiled", terms.ptr, faces.ptr, corner_offsets.ptr,
-            corner_slots.ptr, tile_faces.ptr, tile_counts.ptr, codes.ptr, n, k, u, u_stride, u_iperm,
-            out, out_stride, out_iperm, out_pinned, stream,
-        )  # fmt: skip
-        return
-    _lib.call(
-        "ob_grad_div_terms", terms.ptr, faces.ptr, corner_offsets.ptr,
-        corner_slots.ptr, n, k, u, u_stride, u_iperm, out, out_stride, out_iperm, out_pinned,
-        stream,
-    )  # fmt: skip
+def corner_planes(terms: DeviceArray, faces: DeviceArray, corner_slots: DeviceArray,
+                  n_faces: int) -> DeviceArray:
+    """A corner index's ``ob_corner_planes``: each corner's gradient coefficients in its face's own
+    plane and its face's two other vertices, in the index's order, for ``ob_grad_div_planes``."""
+    planes = DeviceArray.empty(18 * max(n_faces, 1), np.float64)
+    _lib.call("ob_corner_planes", terms.ptr, faces.ptr, corner_slots.ptr, n_faces, planes.ptr, DEFAULT_STREAM)
+    return planes
 
 
 def _divergence(mesh: Trimesh, solver: "HeatSolver", k: int, u: int, u_stride: int, u_iperm: Any,
                 out: int, out_stride: int, out_iperm: Any, out_pinned: Any, stream: Any) -> None:
-    """``_grad_div`` over the mesh's own numbering (its corner index and tiles, made once)."""
-    _grad_div(solver, mesh.faces, mesh.corner_tiles, mesh.n_vertices, k, u, u_stride, u_iperm, out,
-              out_stride, out_iperm, out_pinned, stream)
+    """``-div`` of the per-face unit gradients of ``k`` heat columns over the mesh's own numbering,
+    each vertex's corners summed in ascending slot order (no atomics: the same bits on every run, the
+    reference's deterministic mode, ordito/heat.py:3170-3232, as the only mode): over the corner
+    planes for several columns (made once per solver), from the per-face terms for one (a query's
+    single pass does not pay for the planes)."""
+    corner_offsets, corner_slots = mesh.corner_index
+    if k > 1:
+        _lib.call("ob_grad_div_planes", solver.corner_planes.ptr, corner_offsets.ptr, mesh.n_vertices, k, u,
+                  u_stride, u_iperm, out, out_stride, out_iperm, out_pinned, stream)
+        return
+    _lib.call(
+        "ob_grad_div_terms", solver.gradient_terms.ptr, mesh.faces.ptr, corner_offsets.ptr,
+        corner_slots.ptr, mesh.n_vertices, k, u, u_stride, u_iperm, out, out_stride, out_iperm, out_pinned,
+        stream,
+    )  # fmt: skip
 
 
 def _corners_in_factor_rows(mesh: Trimesh, solver: "HeatSolver", h_iperm: int,
-                            p_iperm: int) -> tuple[DeviceArray, tuple, tuple] | None:
-    """The face buffer and the corner index renumbered into the factors' shared ordering (built
-    once per solver and ordering, outside any recording: the first eager pass builds it), with
-    the index's corner records (``corner_records``), so the served divergence reads the heat rows
-    and writes the Poisson rows with no inverse permutation per corner; None when the two
-    factors' orderings differ. A vertex's corners keep their ascending slot order, so the sums
-    are the same bits as in the vertex numbering."""
+                            p_iperm: int) -> tuple[DeviceArray, DeviceArray] | None:
+    """``(corner offsets, corner planes)`` of the mesh renumbered into the factors' shared ordering
+    (built once per solver and ordering, outside any recording: the first eager pass builds it), so
+    the served divergence reads the heat rows and writes the Poisson rows with no inverse
+    permutation per corner; None when the two factors' orderings differ. A vertex's corners keep
+    their ascending slot order, so the sums are the same bits as in the vertex numbering."""
     # Kept on the heat factor (its lifetime is the ordering's), keyed by both orderings.
     holder = solver.heat_factor
     key = (h_iperm, p_iperm, id(solver.poisson_factor))
@@ -684,10 +677,9 @@ def _corners_in_factor_rows(mesh: Trimesh, solver: "HeatSolver", h_iperm: int,
         workspace = DeviceArray.empty(int(size.value), np.uint8)
         _lib.call("ob_corner_index", faces.ptr, mesh.n_faces, n, offsets.ptr, slots.ptr,
                   workspace.ptr, int(size.value), DEFAULT_STREAM)
-        tiles = divergence_tiles(offsets, slots, n, mesh.n_faces)
-        records = corner_records(solver.gradient_terms, faces, slots, mesh.n_faces)
+        planes = corner_planes(solver.gradient_terms, faces, slots, mesh.n_faces)
         _lib.call("ob_stream_synchronize", DEFAULT_STREAM)  # the arrays serve other streams
-        result = (faces, (offsets, slots) + tiles, records)
+        result = (offsets, planes)
     holder._factor_row_corners = (key, result)
     return result
 
@@ -852,9 +844,9 @@ def _batch_columns(mesh: Trimesh, solver: "HeatSolver", src: DeviceArray, offset
             _divergence(mesh, solver, k, h_sol, h_stride, h_iperm, p_rhs, p_stride, p_iperm,
                         p_pinned, st)
         else:
-            _, index, (records, ids) = rows
-            _lib.call("ob_grad_div_records", records.ptr, ids.ptr, index[0].ptr, n, k, h_sol, h_stride, None,
-                      p_rhs, p_stride, None, p_pinned, st)
+            corner_offsets, planes = rows
+            _lib.call("ob_grad_div_planes", planes.ptr, corner_offsets.ptr, n, k, h_sol, h_stride, None, p_rhs,
+                      p_stride, None, p_pinned, st)
         poisson_factor.solve_in_place(k, st, work_set)
         if out is None:
             out = DeviceArray.empty((k, n), np.float64)

@@ -27,7 +27,7 @@ from ordito_b200 import _lib
 from ordito_b200.array import CsrMatrix
 from ordito_b200.cholesky import CholeskyAnalysis, SparseCholesky
 from ordito_b200.device import DEFAULT_STREAM, DeviceArray
-from ordito_b200.heat import _bounds_floor_length, capture_guard
+from ordito_b200.heat import _bounds_floor_length, capture_guard, corner_planes
 from ordito_b200.laplacian import face_terms, mesh_operator_pattern
 
 
@@ -120,22 +120,19 @@ class PackedMeshes:
         # packed pass takes milliseconds) serves both.
         self.tuning = tune_shared({"heat": self.heat_factor, "poisson": self.poisson_factor}, max_columns,
                                   reps=3)
-        # a8: the divergence's corner index and per-face terms over the union.
+        # a8: the divergence's corner index and corner planes over the union.
         self.corner_offsets = DeviceArray.empty(n + 1, np.int32)
-        self.corner_slots = DeviceArray.empty(max(3 * self.n_faces, 1), np.int32)
+        corner_slots = DeviceArray.empty(max(3 * self.n_faces, 1), np.int32)
         size = ctypes.c_size_t(0)
         _lib.call("ob_corner_index_workspace", n, self.n_faces, ctypes.byref(size))
         workspace = DeviceArray.empty(int(size.value), np.uint8)
         _lib.call("ob_corner_index", self.faces.ptr, self.n_faces, n, self.corner_offsets.ptr,
-                  self.corner_slots.ptr, workspace.ptr, int(size.value), DEFAULT_STREAM)
-        from ordito_b200.heat import divergence_tiles  # noqa: PLC0415
-
-        self.tile_faces, self.tile_counts, self.corner_codes = divergence_tiles(
-            self.corner_offsets, self.corner_slots, n, self.n_faces)
-        self.gradient_terms = DeviceArray.empty((max(self.n_faces, 1), 18), np.float64)
+                  corner_slots.ptr, workspace.ptr, int(size.value), DEFAULT_STREAM)
+        gradient_terms = DeviceArray.empty((max(self.n_faces, 1), 18), np.float64)
         _lib.call("ob_face_gradient_terms", self.xyz.ptr, self.faces.ptr, self.n_faces,
-                  terms.normals.ptr, terms.areas.ptr, terms.cot.ptr, self.gradient_terms.ptr,
+                  terms.normals.ptr, terms.areas.ptr, terms.cot.ptr, gradient_terms.ptr,
                   DEFAULT_STREAM)
+        self.corner_planes = corner_planes(gradient_terms, self.faces, corner_slots, self.n_faces)
         # Batch buffers at the widest batch: column sources, their offsets, the shift's table.
         K = self.max_columns
         self.d_sources = DeviceArray.empty(K * self.n_meshes, np.int32)
@@ -188,12 +185,8 @@ class PackedMeshes:
         _lib.call("ob_seed_permuted", self.d_sources.ptr, self.d_offsets.ptr, k, n, h_iperm, h_pinned,
                   h_stride, h_rhs, stream)
         hf.solve_in_place_sources(k, self.d_sources, self.d_offsets, stream)
-        from ordito_b200.heat import _grad_div_index  # noqa: PLC0415
-
-        _grad_div_index(self.gradient_terms, self.faces,
-                        (self.corner_offsets, self.corner_slots, self.tile_faces, self.tile_counts,
-                         self.corner_codes), n, k, h_sol, h_stride, h_iperm, p_rhs, p_stride, p_iperm,
-                        p_pinned, stream)
+        _lib.call("ob_grad_div_planes", self.corner_planes.ptr, self.corner_offsets.ptr, n, k, h_sol, h_stride,
+                  h_iperm, p_rhs, p_stride, p_iperm, p_pinned, stream)
         pf.solve_in_place(k, stream)
         _lib.call("ob_shift_packed", p_sol, n, p_stride, p_iperm, self.d_vertex_offsets.ptr,
                   self.n_meshes, self.d_shift.ptr, k, self.d_sums.ptr, self.out.ptr, stream)
