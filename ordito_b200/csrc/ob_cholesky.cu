@@ -839,9 +839,10 @@ struct TileOps {
         }
     }
 
-    // Issues (and commits as one group) the copies of the inner step from kb into a stage.
-    __device__ static void issue(const Tile& t, int c0, int kb, const int* in_row, const double* __restrict__ vals,
-                                 const double* in, int k, Stage<TC>& s) {
+    // Issues the copies of the inner step from kb into a stage: the matrix block's (the factor is
+    // constant, so they may start before the level below has finished), then the input rows' and
+    // the commit of both as one group.
+    __device__ static void issue_matrix(const Tile& t, int kb, const double* __restrict__ vals, Stage<TC>& s) {
         const double* M = vals + t.m;
 #pragma unroll
         for (int q = 0; q < kChunks; ++q) {
@@ -860,6 +861,9 @@ struct TileOps {
                 copy16(&s.a[i * kLdK + c2], src, 8 * valid);
             }
         }
+    }
+
+    __device__ static void issue_input(int c0, const int* in_row, const double* in, int k, Stage<TC>& s) {
 #pragma unroll
         for (int q = 0; q < kChunksB; ++q) {
             const int chunk = threadIdx.x + q * kThreads;
@@ -953,45 +957,70 @@ struct TileOps {
     }
 };
 
+// ---- Levels overlapped (programmatic dependent launch) -------------------------------------
+// A pass is a chain of levels, each short (5-35 us) against its launch, its tile's fetch and the
+// first trip of its factor block from DRAM. Every level but a pass's first is launched as
+// dependent on the one before with its start brought forward: its CTAs come in as that level's
+// leave, read what does not depend on it (the tile, its row lists, the factor block -- into the
+// first stage, and into L2) and only then wait for it. A level lets the next in after its own
+// wait, so what a CTA reads before its wait was written two launches back or earlier: the marks
+// are safe to read there, the work rows are not. Every CTA waits, also one with nothing to do, so
+// a level's end implies the end of all before it. The register kernel and the 16-column tiles are
+// launched so (the 131k torus at one column 0.437 -> 0.360 ms a query, the 41k sphere at 16 columns
+// 0.510 -> 0.451 ms, 48 packed meshes at 16 columns 0.545 -> 0.490 ms); the wide tiles are not: their
+// levels are bound by their products, and the start brought forward takes registers and issue
+// slots from them (the 131k torus at 64 columns 0.833 -> 0.857 ms a step).
 template <int TC>
-__device__ __forceinline__ void tile_product(const Tile& t, int k0, int c0, const double* __restrict__ vals,
-                                             const int* __restrict__ idx,
-                                             const double* in, double* out, int k, Stage<TC>* stage) {
+constexpr bool overlapped() { return TC <= kTileColsSixteen; }
+__device__ __forceinline__ void level_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void level_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// The tile's factor block from inner index k0 on into L2, a line (128 bytes) a request, `lanes`
+// threads to a stored row.
+__device__ __forceinline__ void prefetch_block(const Tile& t, int k0, const double* vals) {
+    constexpr int kLanes = 4;
+    const int first = t.trans ? k0 : t.r0, count = t.trans ? t.k1 - k0 : t.rows;
+    const int from = t.trans ? t.r0 : k0, width = t.trans ? t.rows : t.k1 - k0;
+    for (int o = threadIdx.x / kLanes; o < count; o += blockDim.x / kLanes) {
+        const double* row = vals + t.m + (size_t)(first + o) * t.ld + from;
+        for (int e = 16 * (threadIdx.x % kLanes); e < width; e += 16 * kLanes) prefetch_l2(row + e);
+    }
+}
+
+// A tile of an unmarked node in a forward pass over marked ones (see skip_inactive).
+__device__ __forceinline__ bool inactive(const Tile& t, const unsigned char* active) {
+    return active != nullptr && !active[t.node] && t.tri != 2;
+}
+
+// The stages of a tile whose first step's copies are under way.
+template <int TC>
+__device__ __forceinline__ void tile_product(const Tile& t, int k0, int steps, int c0, const int* out_row,
+                                             const double* __restrict__ vals,
+                                             const int* __restrict__ idx, const double* in, double* out, int k,
+                                             Stage<TC>* stage) {
     using Ops = TileOps<TC>;
     typename Ops::Acc acc;
     Ops::clear(acc);
-    // Inner steps from k0 (the tile's own, or past a zero Y block: first_inner).
-    const int steps = (t.k1 - k0 + kTileK - 1) / kTileK;
-    if (steps <= 0) {
-        // Nothing to multiply: an assigned output is zero, an accumulated one unchanged.
-        if (t.op == kAssign) {
-            int rows_out[2];
-            Ops::output_rows(t, idx, rows_out);
-            Ops::store(t, c0, rows_out, out, k, acc);
-        }
-        return;
-    }
     // The input rows of a step's chunks are read one step ahead of the copies that use them, so
     // a gathered index's load latency is not paid in front of every step's copies.
-    int first_rows[Ops::kChunksB], next_rows[Ops::kChunksB];
-    Ops::input_rows(t, k0, idx, first_rows);
-    Ops::issue(t, c0, k0, first_rows, vals, in, k, stage[0]);
+    int next_rows[Ops::kChunksB];
     if (steps > 1) Ops::input_rows(t, k0 + kTileK, idx, next_rows);
-    // The output rows, read before the products so the epilogue does not wait on them.
-    int out_row[2];
-    Ops::output_rows(t, idx, out_row);
     for (int st = 0; st < steps; ++st) {
         copy_wait<0>();
         // Every thread's copies of step st have landed, and every warp is past the products of
         // step st - 1, whose stage the next copies reuse: one barrier a step.
         __syncthreads();
         if (st + 1 < steps) {
-            Ops::issue(t, c0, k0 + (st + 1) * kTileK, next_rows, vals, in, k, stage[(st + 1) & 1]);
+            Ops::issue_matrix(t, k0 + (st + 1) * kTileK, vals, stage[(st + 1) & 1]);
+            Ops::issue_input(c0, next_rows, in, k, stage[(st + 1) & 1]);
             if (st + 2 < steps) Ops::input_rows(t, k0 + (st + 2) * kTileK, idx, next_rows);
         }
         Ops::compute(t, k0 + st * kTileK, stage[st & 1], acc);
     }
-    Ops::store(t, c0, out_row, out, k, acc);
+    // Nothing to multiply: an assigned output is zero, an accumulated one unchanged.
+    if (steps > 0 || t.op == kAssign) Ops::store(t, c0, out_row, out, k, acc);
 }
 
 // The two stages live in dynamic shared memory (stage_bytes, above the 48 KB static limit).
@@ -1000,23 +1029,20 @@ constexpr int stage_bytes() { return 2 * (int)sizeof(Stage<TC>); }
 
 // A forward pass over right-hand sides that are zero outside the marked supernodes (a batch of
 // source indicators: only a source's supernode and its ancestors receive anything): a tile of an
-// unmarked node has a zero input block. Its update rows of a deterministic factor are written as
-// zeros (the level's gather adds them), its Y rows too unless the backward pass is trimmed (and so
-// does not read them: first_inner), and a tile that accumulates is skipped. Returns whether the tile was
-// handled so.
-__device__ __forceinline__ bool skip_inactive(const Tile& t, const unsigned char* active, int trimmed, int c0,
-                                              int width, const int* idx, double* out, int k) {
-    // A backward tile of an unmarked node is trimmed instead (first_inner); when the backward pass
-    // trims, the Y rows of the forward diagonal tile, read by nothing else, are not written.
-    if (active == nullptr || active[t.node] || t.tri == 2) return false;
-    if (t.op == kAssign && (t.tri != 1 || !trimmed))
-        for (int e = threadIdx.x; e < t.rows * width; e += blockDim.x) {
-            const int i = e / width, c = c0 + e % width;
-            if (c >= k) continue;
-            const int r = t.out_rows < 0 ? t.out_base + t.r0 + i : idx[t.out_rows + t.r0 + i];
-            out[(size_t)r * k + c] = 0.0;
-        }
-    return true;
+// unmarked node (inactive) has a zero input block. Its update rows of a deterministic factor are
+// written as zeros (the level's gather adds them), its Y rows too unless the backward pass is
+// trimmed (and so does not read them: first_inner), and a tile that accumulates is skipped. A
+// backward tile of an unmarked node is trimmed instead; when the backward pass trims, the Y rows of
+// the forward diagonal tile, read by nothing else, are not written.
+__device__ __forceinline__ void clear_inactive(const Tile& t, int trimmed, int c0, int width, const int* idx,
+                                               double* out, int k) {
+    if (t.op != kAssign || (t.tri == 1 && trimmed)) return;
+    for (int e = threadIdx.x; e < t.rows * width; e += blockDim.x) {
+        const int i = e / width, c = c0 + e % width;
+        if (c >= k) continue;
+        const int r = t.out_rows < 0 ? t.out_base + t.r0 + i : idx[t.out_rows + t.r0 + i];
+        out[(size_t)r * k + c] = 0.0;
+    }
 }
 
 // The first inner index a tile's product runs from. The backward tile of an unmarked node (its Y
@@ -1041,8 +1067,35 @@ tile_product_kernel(const Tile* __restrict__ tiles, const double* __restrict__ v
     const int blocks = (k + TC - 1) / TC;
     const Tile t = tiles[blockIdx.x / blocks];
     const int c0 = (int)(blockIdx.x % blocks) * TC;
-    if (skip_inactive(t, active, trimmed, c0, TC, idx, rows, k)) return;
-    tile_product<TC>(t, first_inner(t, active), c0, vals, idx, rows, rows, k, stage);
+    using Ops = TileOps<TC>;
+    const bool idle = inactive(t, active);
+    if (!overlapped<TC>() && idle) {
+        clear_inactive(t, trimmed, c0, TC, idx, rows, k);
+        return;
+    }
+    // Inner steps from k0 (the tile's own, or past a zero Y block: first_inner).
+    const int k0 = first_inner(t, active), steps = idle ? 0 : (t.k1 - k0 + kTileK - 1) / kTileK;
+    int first_rows[Ops::kChunksB], out_row[2];
+    if (steps > 0) {
+        if (!overlapped<TC>()) Ops::input_rows(t, k0, idx, first_rows);
+        Ops::issue_matrix(t, k0, vals, stage[0]);
+        if (overlapped<TC>()) {
+            Ops::input_rows(t, k0, idx, first_rows);
+            prefetch_block(t, k0 + kTileK, vals);
+        }
+    }
+    if (overlapped<TC>()) {
+        level_wait();
+        level_release();
+        if (idle) {
+            clear_inactive(t, trimmed, c0, TC, idx, rows, k);
+            return;
+        }
+    }
+    if (steps > 0) Ops::issue_input(c0, first_rows, rows, k, stage[0]);
+    // The output rows, read before the products so the epilogue does not wait on them.
+    Ops::output_rows(t, idx, out_row);
+    tile_product<TC>(t, k0, steps, c0, out_row, vals, idx, rows, rows, k, stage);
 }
 
 // The same tile product for a narrow batch (KP = 2, 4, 6 or 8 columns, the even stride of 1-8
@@ -1059,11 +1112,22 @@ template <int KP>
 __global__ void __launch_bounds__(kNarrowThreads)
 narrow_tile_kernel(const Tile* __restrict__ tiles, const double* __restrict__ vals,
                    const int* __restrict__ idx, double* rows, const unsigned char* active, int trimmed) {
-    if (skip_inactive(tiles[blockIdx.x], active, trimmed, 0, KP, idx, rows, KP)) return;
     const double* in = rows;
     double* out = rows;
     __shared__ double other[kNarrowSlices - 1][kTileRows][KP];
     const Tile t = tiles[blockIdx.x];
+    const bool idle = inactive(t, active);
+    const int first = first_inner(t, active);
+    if (!idle) {
+        prefetch_block(t, first, vals);
+        if (t.in_rows >= 0 && first + 32 * (int)threadIdx.x < t.k1) prefetch_l2(idx + t.in_rows + first + 32 * threadIdx.x);
+    }
+    level_wait();
+    level_release();
+    if (idle) {
+        clear_inactive(t, trimmed, 0, KP, idx, rows, KP);
+        return;
+    }
     const int i = threadIdx.x % kTileRows, slice = threadIdx.x / kTileRows;
     double acc[KP];
 #pragma unroll
@@ -1087,7 +1151,7 @@ narrow_tile_kernel(const Tile* __restrict__ tiles, const double* __restrict__ va
             // Column-major reads: the 64 threads of a slice read 64 consecutive values. Values a
             // thread alone reads go through L2 only (`__ldcg`): caching them in L1 measured slower.
             constexpr int kStep = kNarrowSlices;
-            int kk = first_inner(t, active) + slice;
+            int kk = first + slice;
             for (; kk + 3 * kStep < t.k1; kk += 4 * kStep) {
                 const int r0 = row(kk), r1 = row(kk + kStep), r2 = row(kk + 2 * kStep), r3 = row(kk + 3 * kStep);
                 const double a0 = value(kk), a1 = value(kk + kStep), a2 = value(kk + 2 * kStep),
@@ -1634,9 +1698,12 @@ int triangular_solves(Factor* F, Factor::WorkSet& W, int k, cudaStream_t stream,
     OB_REQUIRE(W.BYX != nullptr && W.rows == 3LL * F->n + (F->deterministic ? F->n_update_rows : 0) &&
                    k <= even_columns(W.cap_k),
                "chol pass: work buffers not prepared for %d columns in this mode", k);
+    // The pass's first launch follows what is before it whole; the levels after overlap.
+    bool overlap = false;
     if (F->n_zero > 0) {
         zero_rows_kernel<<<F->n_zero, 256, 0, stream>>>(F->zero, F->n_zero, k, W.Y(k, F->n), W.X(k, F->n));
         OB_CHECK_LAUNCH("chol zero split rows");
+        overlap = true;
     }
     // A level's launch: the float64 tensor-core tiles, or for a narrow batch (stride 2-8) the
     // register kernel, which does not compute a 64-column tile's idle columns.
@@ -1645,26 +1712,45 @@ int triangular_solves(Factor* F, Factor::WorkSet& W, int k, cudaStream_t stream,
     // batch add (trimming changes how the tensor-core steps group the inner dimension).
     const int trimmed = forward_active != nullptr && !F->deterministic;
     auto level = [&](const Tile* tiles, int count, int cols, const unsigned char* active, const char* what) {
+        cudaLaunchAttribute early;
+        early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        early.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t config = {};
+        config.stream = stream;
+        config.attrs = &early;
+        config.numAttrs = overlap && k <= kTileColsSixteen ? 1 : 0;
+        overlap = true;
+        auto tensor = [&](auto kernel, int width, int threads, int shared) {
+            config.gridDim = dim3((unsigned)count * ceil_div(k, width));
+            config.blockDim = dim3((unsigned)threads);
+            config.dynamicSmemBytes = (size_t)shared;
+            return cudaLaunchKernelEx(&config, kernel, tiles, (const double*)F->vals, (const int*)F->idx, W.BYX, k,
+                                      active, trimmed);
+        };
+        auto narrow = [&](auto kernel) {
+            config.gridDim = dim3((unsigned)count);
+            config.blockDim = dim3(kNarrowThreads);
+            return cudaLaunchKernelEx(&config, kernel, tiles, (const double*)F->vals, (const int*)F->idx, W.BYX,
+                                      active, trimmed);
+        };
+        cudaError_t e;
         switch (k) {
-            case 2: narrow_tile_kernel<2><<<count, kNarrowThreads, 0, stream>>>(tiles, F->vals, F->idx, W.BYX, active, trimmed); break;
-            case 4: narrow_tile_kernel<4><<<count, kNarrowThreads, 0, stream>>>(tiles, F->vals, F->idx, W.BYX, active, trimmed); break;
-            case 6: narrow_tile_kernel<6><<<count, kNarrowThreads, 0, stream>>>(tiles, F->vals, F->idx, W.BYX, active, trimmed); break;
-            case 8: narrow_tile_kernel<8><<<count, kNarrowThreads, 0, stream>>>(tiles, F->vals, F->idx, W.BYX, active, trimmed); break;
+            case 2: e = narrow(narrow_tile_kernel<2>); break;
+            case 4: e = narrow(narrow_tile_kernel<4>); break;
+            case 6: e = narrow(narrow_tile_kernel<6>); break;
+            case 8: e = narrow(narrow_tile_kernel<8>); break;
             default:
                 if (k <= kTileColsSixteen)
-                    tile_product_kernel<kTileColsSixteen>
-                        <<<(unsigned)count, tile_threads<kTileColsSixteen>(), stage_bytes<kTileColsSixteen>(),
-                           stream>>>(tiles, F->vals, F->idx, W.BYX, k, active, trimmed);
+                    e = tensor(tile_product_kernel<kTileColsSixteen>, kTileColsSixteen,
+                               tile_threads<kTileColsSixteen>(), stage_bytes<kTileColsSixteen>());
                 else if (cols == kTileColsNarrow)
-                    tile_product_kernel<kTileColsNarrow>
-                        <<<(unsigned)count * ceil_div(k, kTileColsNarrow), tile_threads<kTileColsNarrow>(),
-                           stage_bytes<kTileColsNarrow>(),
-                           stream>>>(tiles, F->vals, F->idx, W.BYX, k, active, trimmed);
+                    e = tensor(tile_product_kernel<kTileColsNarrow>, kTileColsNarrow, tile_threads<kTileColsNarrow>(),
+                               stage_bytes<kTileColsNarrow>());
                 else
-                    tile_product_kernel<kTileCols><<<(unsigned)count * ceil_div(k, kTileCols), tile_threads<kTileCols>(),
-                                                      stage_bytes<kTileCols>(), stream>>>(tiles, F->vals, F->idx,
-                                                                                          W.BYX, k, active, trimmed);
+                    e = tensor(tile_product_kernel<kTileCols>, kTileCols, tile_threads<kTileCols>(),
+                               stage_bytes<kTileCols>());
         }
+        if (e != cudaSuccess) return cuda_status(e, what);
         OB_CHECK_LAUNCH(what);
         return OB_OK;
     };
@@ -1675,6 +1761,7 @@ int triangular_solves(Factor* F, Factor::WorkSet& W, int k, cudaStream_t stream,
             gather_updates_kernel<<<ceil_div(F->n_gather[l], 8), 256, 0, stream>>>(
                 F->gather_offsets[l], F->gather_rows[l], F->gather_src[l], F->n_gather[l], k, W.BYX);
             OB_CHECK_LAUNCH("chol deterministic gather");
+            overlap = false;  // the gather writes rows without waiting of its own
         }
     }
     // The backward pass starts past the zero Y block of every node the forward pass left unmarked.
