@@ -1268,6 +1268,7 @@ struct DeviceLevel {
     int* col = nullptr;
     float* val = nullptr;
     float* damped = nullptr;
+    float* scaled = nullptr;  // val with its columns scaled by damped (first_sweeps_kernel)
     int n_coarse = 0;
     long long pnnz = 0, rnnz = 0;  // stored entries of the prolongation and the restriction
     int *poff = nullptr, *pcol = nullptr, *roff = nullptr, *rcol = nullptr;
@@ -1376,6 +1377,18 @@ __device__ __forceinline__ float4 row_product(const int* __restrict__ off, const
     float4 acc = f4(0.0f);
     const int end = off[row + 1];
     int e = off[row];
+    // Four entries' places, then their values, in flight: a row's time is its loads' latency.
+    for (; e + 3 < end; e += 4) {
+        int j[4];
+        float a[4];
+        float4 v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) j[q] = col[e + q], a[q] = val[e + q];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = x[(size_t)j[q] * G + lane];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) fma4(a[q], v[q], acc);
+    }
     for (; e + 1 < end; e += 2) {
         const int j0 = col[e], j1 = col[e + 1];
         const float a0 = val[e], a1 = val[e + 1];
@@ -1464,6 +1477,31 @@ __global__ void __launch_bounds__(kThreads) scale_kernel(int n, int G, const flo
             C.beta = 0.0;
         }
     }
+}
+
+// The first two sweeps from zero in one: x = d .* b, then x + d .* (b - A x) = d .* (2 b - (A D) b)
+// with the columns of A scaled by d once at set-up (column_scale_kernel): b alone is gathered, and
+// the first sweep's write and second read of a vector (and its launch) go.
+__global__ void __launch_bounds__(kThreads) first_sweeps_kernel(int n, int G, const int* __restrict__ off,
+                                                                const int* __restrict__ col,
+                                                                const float* __restrict__ scaled,
+                                                                const float* __restrict__ d,
+                                                                const float4* __restrict__ b,
+                                                                float4* __restrict__ x) {
+    const int lane = threadIdx.x % G, groups = blockDim.x / G;
+    for (int row = blockIdx.x * groups + threadIdx.x / G; row < n; row += gridDim.x * groups) {
+        const float4 ax = row_product(off, col, scaled, b, G, row, lane);
+        const float4 v = b[(size_t)row * G + lane];
+        const float s = d[row];
+        x[(size_t)row * G + lane] = make_float4(s * (fmaf(2.0f, v.x, -ax.x)), s * (fmaf(2.0f, v.y, -ax.y)),
+                                                s * (fmaf(2.0f, v.z, -ax.z)), s * (fmaf(2.0f, v.w, -ax.w)));
+    }
+}
+
+__global__ void column_scale_kernel(long long nnz, const int* __restrict__ col, const float* __restrict__ val,
+                                    const float* __restrict__ d, float* __restrict__ scaled) {
+    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (e < nnz) scaled[e] = val[e] * d[col[e]];
 }
 
 // One damped-Jacobi sweep x_out = x_in + d .* (b - A x_in); kDot adds the top level's r.z fold.
@@ -1982,20 +2020,16 @@ int enqueue_cycle(Amg* M, Work* W, size_t l, const float* b, float* out, bool to
     }
     const int grid = grid_for((long long)L.n * G);
     float* other = W->y[l];
-    // Pre-smoothing: the first sweep from zero is a write; the second lands in `out`.
-    scale_kernel<false><<<grid, kThreads, 0, stream>>>(L.n, G, L.damped, f4p(b), f4m(other), nullptr,
-                                                         nullptr, nullptr);
-    OB_CHECK_LAUNCH("amg first sweep");
-    sweep_kernel<false><<<grid, kThreads, 0, stream>>>(L.n, G, L.off, L.col, L.val, L.damped, f4p(b),
-                                                        f4p(other), f4m(out), nullptr, nullptr, nullptr);
-    OB_CHECK_LAUNCH("amg sweep");
+    // Pre-smoothing: both sweeps from zero at once.
+    first_sweeps_kernel<<<grid, kThreads, 0, stream>>>(L.n, G, L.off, L.col, L.scaled, L.damped, f4p(b), f4m(out));
+    OB_CHECK_LAUNCH("amg first sweeps");
     residual_kernel<<<grid, kThreads, 0, stream>>>(L.n, G, L.off, L.col, L.val, f4p(b), f4p(out), f4m(W->r[l]));
     OB_CHECK_LAUNCH("amg residual");
     const DeviceLevel& C = M->levels[l + 1];
     spmm_kernel<false><<<grid_for((long long)C.n * G), kThreads, 0, stream>>>(
         C.n, G, L.roff, L.rcol, L.rval, f4p(W->r[l]), f4m(W->b[l + 1]));
     OB_CHECK_LAUNCH("amg restrict");
-    *launches += 4;
+    *launches += 3;
     int st = enqueue_cycle(M, W, l + 1, W->b[l + 1], W->x[l + 1], false, stream, launches);
     if (st) return st;
     spmm_kernel<true><<<grid, kThreads, 0, stream>>>(L.n, G, L.poff, L.pcol, L.pval, f4p(W->x[l + 1]), f4m(out));
@@ -2108,6 +2142,21 @@ extern "C" {
 std::atomic<int> g_build_on_device{1};
 bool amg_build_on_device() { return g_build_on_device.load() != 0; }
 
+// Each smoothed level's column-scaled values.
+int scale_levels(Amg* M, cudaStream_t stream) {
+    for (DeviceLevel& d : M->levels) {
+        if (d.damped == nullptr) continue;
+        void* p = nullptr;
+        OB_CUDA(cudaMalloc(&p, sizeof(float) * (size_t)std::max(d.nnz, 1LL)));
+        M->allocations.push_back(p);
+        d.scaled = static_cast<float*>(p);
+        if (d.nnz == 0) continue;
+        column_scale_kernel<<<grid_of(d.nnz), kThreads, 0, stream>>>(d.nnz, d.col, d.val, d.damped, d.scaled);
+        OB_CHECK_LAUNCH("amg column scale");
+    }
+    return OB_OK;
+}
+
 int setup_on_device(Amg* M, int n, long long nnz, const int32_t* offsets, const int32_t* columns,
                     const double* values, unsigned seed, cudaStream_t stream) {
     DevBuild B;
@@ -2206,6 +2255,7 @@ int setup_on_device(Amg* M, int n, long long nnz, const int32_t* offsets, const 
     if ((st = upload(M, slots, &M->slots, stream))) return st;
     if ((st = upload(M, narrow(H.inverse.empty() ? std::vector<double>(1, 0.0) : H.inverse), &M->inverse, stream)))
         return st;
+    if ((st = scale_levels(M, stream))) return st;
     OB_CUDA(cudaStreamSynchronize(stream));
     return OB_OK;
 }
@@ -2298,6 +2348,7 @@ int ob_amg_setup(int n, const int32_t* offsets, const int32_t* columns, const do
         if (st == OB_OK) st = upload(M.get(), narrow(H.inverse.empty() ? std::vector<double>(1, 0.0) : H.inverse),
                                      &M->inverse, stream);
     }
+    if (st == OB_OK && H.usable) st = scale_levels(M.get(), stream);
     if (st == OB_OK) {
         cudaError_t e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) st = cuda_status(e, "ob_amg_setup");
