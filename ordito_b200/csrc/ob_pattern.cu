@@ -3,15 +3,21 @@
 // Follows ordito/laplacian.py:1212-1299 (directed build), ordito/kernels/laplacian.py:707-748
 // (store_operator_keys) and ordito/array.py:1688-1807 (csr_from_keys). Keys are
 // row * V + col (uint64), sorted stably: equal keys keep the producer's slot order, so an entry's
-// contributors (its run of equal sorted keys) come out in face order. The sort is by row buckets:
-// each in-range key counted into its row and scattered into the row's bucket as (col, slot), each
-// bucket sorted by (col, slot) -- the order a stable sort by key gives, whatever order the scatter
-// filled the bucket in -- and the out-of-range (sentinel) keys placed after them in slot order.
-// That moves every key a few times, where a radix sort over the 2 log2 V bits of the keys makes a
-// pass a digit. No value is ever accumulated atomically: the runs are flagged, scanned and placed,
-// and each entry's value is formed later from its run.
+// contributors (its run of equal sorted keys) come out in face order. The sort is by row buckets,
+// straight from the faces: a corner counts its (at most two) keys into its vertex's row with one
+// atomic and later scatters them into the row's bucket with another, as (col, slot), each bucket is
+// sorted by (col, slot) -- the order a stable sort by key gives, whatever order the scatter filled it
+// in -- and its distinct columns counted; their scan is the row offsets, and one last pass writes the
+// keys, payloads, columns and run starts. The out-of-range (sentinel) keys follow in slot order. No
+// value is ever accumulated atomically: each entry's value is formed later from its run.
+//
+// What bounds it is traffic: the outputs (~16 bytes a key) and three trips of the buckets (8 bytes a
+// key), the faces twice, and two atomics a corner. The unsorted keys are never stored, and no scan or
+// pass runs over them: the form that stored them, with a general segmented sort and scans over
+// every slot, took 0.50 ms on a 655 k-vertex torus (14 launches).
 #include <cub/device/device_scan.cuh>
-#include <cub/device/device_segmented_sort.cuh>
+
+#include <algorithm>
 
 #include "ob_internal.cuh"
 
@@ -20,169 +26,303 @@ namespace {
 
 constexpr int kThreads = 256;
 
-__device__ __forceinline__ unsigned long long csr_key(int row, int col, int n) {
-    const unsigned long long sentinel = (unsigned long long)n * (unsigned long long)n;
-    if (row < 0 || row >= n || col < 0 || col >= n) return sentinel;
-    return (unsigned long long)row * (unsigned long long)n + (unsigned long long)col;
+// Slot 6 f + 2 e holds the key (i, j) of the edge opposite corner e (i = corner e + 1, j = corner
+// e + 2), slot 6 f + 2 e + 1 its reverse, payload 3 f + e; slot 6 F + v the diagonal of a referenced
+// vertex v (payload -1). A corner's own row so takes two of its face's slots: corner c's keys
+// (c, c - 1) and (c, c + 1).
+__device__ __forceinline__ int corner_column(const int* face, int c, int which) {
+    return face[which == 0 ? (c + 2) % 3 : (c + 1) % 3];
 }
-
-// Tail slots: the sentinel (an unreferenced vertex keeps an empty row).
-__global__ void fill_tail(unsigned long long* keys, long long tail, int n) {
-    const long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (v >= n) return;
-    keys[tail + v] = (unsigned long long)n * (unsigned long long)n;
-}
-
-// One thread per face: both directions of the edge opposite each corner (slots 6 f + 2 e and
-// + 1, payload 3 f + e: slot_payload), and the diagonal key of each in-range corner (every face
-// writes the same key into a shared vertex's tail slot, so the race is benign).
-__global__ void operator_keys(const int* __restrict__ faces, int n_faces, int n,
-                              unsigned long long* __restrict__ keys) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= n_faces) return;
-    const int c[3] = {faces[3 * f], faces[3 * f + 1], faces[3 * f + 2]};
-    const long long base = 6LL * f;
-    const long long tail = 6LL * n_faces;
-#pragma unroll
-    for (int e = 0; e < 3; ++e) {
-        const int i = c[(e + 1) % 3], j = c[(e + 2) % 3];
-        keys[base + 2 * e] = csr_key(i, j, n);
-        keys[base + 2 * e + 1] = csr_key(j, i, n);
-        const int v = c[e];
-        if (v >= 0 && v < n) keys[tail + v] = csr_key(v, v, n);
-    }
-}
-
-// The row of an in-range key row * n + col (< n^2, n < 2^31): the float64 quotient is within one of
-// it (its relative error is 2^-53 and the quotient is below 2^31), and one step each way makes it
-// exact -- the key's 64-bit integer division costs far more instructions than this.
-__device__ __forceinline__ int key_row(unsigned long long key, int n) {
-    long long r = (long long)((double)key / (double)n);
-    const unsigned long long un = (unsigned long long)n;
-    if ((unsigned long long)r * un > key) --r;
-    else if ((unsigned long long)(r + 1) * un <= key) ++r;
-    return (int)r;
+__device__ __forceinline__ int corner_slot(int c, int which) {
+    // (c, c - 1) is the reverse of the edge opposite c + 1, (c, c + 1) the edge opposite c - 1.
+    return which == 0 ? 2 * ((c + 1) % 3) + 1 : 2 * ((c + 2) % 3);
 }
 
 // The payload of slot i: the corner 3 f + e of an edge slot 6 f + 2 e (+ 1), -1 for a tail slot.
 __device__ __forceinline__ int slot_payload(long long i, long long tail) { return i < tail ? (int)(i / 2) : -1; }
 
-// Row counts of the in-range keys (integer atomics: the counts, not their order, are used) and each
-// slot's sentinel flag.
-__global__ void row_counts(const unsigned long long* __restrict__ keys, long long count, unsigned long long sentinel,
-                           int n, int* __restrict__ counts, int* __restrict__ sentinel_flag) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const unsigned long long key = keys[i];
-    const bool inside = key < sentinel;
-    sentinel_flag[i] = inside ? 0 : 1;
-    if (inside) atomicAdd(&counts[key_row(key, n)], 1);
-}
+__device__ __forceinline__ bool inside(int v, int n) { return v >= 0 && v < n; }
 
-// Each in-range key into its row's bucket as (col << 32 | slot); each sentinel key to its place
-// after every in-range one, in slot order.
-__global__ void scatter_rows(const unsigned long long* __restrict__ keys, long long count, unsigned long long sentinel,
-                             int n, const int* __restrict__ row_start, int* __restrict__ fill,
-                             const int* __restrict__ sentinel_before, long long tail,
-                             unsigned long long* __restrict__ bucket, unsigned long long* __restrict__ keys_out,
-                             int* __restrict__ order_out) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const unsigned long long key = keys[i];
-    if (key < sentinel) {
-        const int row = key_row(key, n);
-        const unsigned long long col = key - (unsigned long long)row * (unsigned long long)n;
-        const int at = row_start[row] + atomicAdd(&fill[row], 1);
-        bucket[at] = (col << 32) | (unsigned long long)i;
-    } else {
-        const long long at = (long long)row_start[n] + sentinel_before[i];
-        keys_out[at] = key;
-        order_out[at] = slot_payload(i, tail);
-    }
-}
-
-// The sorted buckets back to keys and payloads, a group of 8 lanes a row.
-__global__ void write_rows(const unsigned long long* __restrict__ sorted, const int* __restrict__ row_start, int n,
-                           long long tail, unsigned long long* __restrict__ keys_out, int* __restrict__ order_out) {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const int row = (int)(t / 8), lane = (int)(t % 8);
-    if (row >= n) return;
-    for (int p = row_start[row] + lane; p < row_start[row + 1]; p += 8) {
-        const unsigned long long v = sorted[p];
-        keys_out[p] = (unsigned long long)row * (unsigned long long)n + (v >> 32);
-        order_out[p] = slot_payload((long long)(v & 0xffffffffULL), tail);
-    }
-}
-
-__global__ void run_flags(const unsigned long long* __restrict__ keys, long long count,
-                          unsigned long long sentinel, int* __restrict__ flags) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const unsigned long long k = keys[i];
-    flags[i] = (k < sentinel && (i == 0 || keys[i - 1] != k)) ? 1 : 0;
-}
-
-// Places each run as one entry and writes the row bounds (ordito/kernels/array.py:1378-1418,
-// csr_row_offsets / csr_out_of_range): a run start that opens a row writes the bound of every row
-// from the previous entry's row up to its own, and the last in-range position closes the rest.
-__global__ void place_runs(const unsigned long long* __restrict__ keys,
-                           const int* __restrict__ inclusive, long long count,
-                           unsigned long long sentinel, int n, int* __restrict__ offsets,
-                           int* __restrict__ columns, int* __restrict__ run_start) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const unsigned long long key = keys[i];
-    if (key >= sentinel) {
-        if (i == 0)
-            for (int r = 0; r <= n; ++r) offsets[r] = 0;
+// Per face: its corners' in-range keys counted into their rows (integer atomics: the counts, not
+// their order, are used), the rows flagged as referenced, and its sentinel slots counted.
+__global__ void corner_counts(const int* __restrict__ faces, int n_faces, int n, int* __restrict__ counts,
+                              int* __restrict__ referenced, int* __restrict__ sentinels) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f > n_faces) return;
+    if (f == n_faces) {
+        sentinels[f] = 0;  // the scan's total
         return;
     }
-    const int row = key_row(key, n);
-    const int entry = inclusive[i] - 1;
-    if (i == 0 || keys[i - 1] != key) {
-        columns[entry] = (int)(key - (unsigned long long)row * (unsigned long long)n);
-        run_start[entry] = (int)i;
-        const int previous = (i == 0) ? -1 : key_row(keys[i - 1], n);
-        for (int r = previous + 1; r <= row; ++r) offsets[r] = entry;
+    const int c[3] = {faces[3 * f], faces[3 * f + 1], faces[3 * f + 2]};
+    int outside = 6;
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+        if (!inside(c[e], n)) continue;
+        const int keys = (int)inside(c[(e + 1) % 3], n) + (int)inside(c[(e + 2) % 3], n);
+        outside -= keys;
+        referenced[c[e]] = 1;
+        if (keys) atomicAdd(&counts[c[e]], keys);
     }
-    if (i + 1 == count || keys[i + 1] >= sentinel)
-        for (int r = row + 1; r <= n; ++r) offsets[r] = inclusive[i];
+    sentinels[f] = outside;
+}
+
+// Per row: its keys (the diagonal's among them) in the low half, whether its tail slot is a
+// sentinel (an unreferenced vertex: an empty row) in the high half; the scan of both is one.
+__global__ void row_totals(const int* __restrict__ counts, const int* __restrict__ referenced, int n,
+                           unsigned long long* __restrict__ totals) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v > n) return;
+    totals[v] = v == n            ? 0ULL
+                : referenced[v]   ? (unsigned long long)(counts[v] + 1)
+                                  : 1ULL << 32;
+}
+
+__device__ __forceinline__ int row_begin(const unsigned long long* starts, int row) {
+    return (int)(starts[row] & 0xffffffffULL);
+}
+
+// Each corner's keys into its row's bucket as (col << 32 | slot), the place after the row's first
+// (the diagonal's) taken by counting the row's counter down; each sentinel edge slot to its place
+// after every in-range key.
+__global__ void scatter_corners(const int* __restrict__ faces, int n_faces, int n,
+                                const unsigned long long* __restrict__ starts, int* __restrict__ counts,
+                                const int* __restrict__ sentinel_before, unsigned long long* __restrict__ bucket,
+                                unsigned long long* __restrict__ keys_out, int* __restrict__ order_out) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= n_faces) return;
+    const int c[3] = {faces[3 * f], faces[3 * f + 1], faces[3 * f + 2]};
+    const int before = sentinel_before[f];
+    const bool whole = before == sentinel_before[f + 1];
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+        if (!inside(c[e], n)) continue;
+        const int keys = (int)inside(c[(e + 1) % 3], n) + (int)inside(c[(e + 2) % 3], n);
+        if (keys == 0) continue;
+        int at = row_begin(starts, c[e]) + 1 + atomicSub(&counts[c[e]], keys) - keys;
+#pragma unroll
+        for (int which = 0; which < 2; ++which) {
+            const int col = corner_column(c, e, which);
+            if (!inside(col, n)) continue;
+            bucket[at++] = ((unsigned long long)col << 32) | (unsigned long long)(6LL * f + corner_slot(e, which));
+        }
+    }
+    if (whole) return;
+    const unsigned long long sentinel = (unsigned long long)n * (unsigned long long)n;
+    long long at = (long long)row_begin(starts, n) + before;
+    for (int slot = 0; slot < 6; ++slot) {
+        const int i = c[(slot / 2 + 1) % 3], j = c[(slot / 2 + 2) % 3];
+        if (inside(i, n) && inside(j, n)) continue;
+        keys_out[at] = sentinel;
+        order_out[at++] = slot_payload(6LL * f + slot, 6LL * n_faces);
+    }
+}
+
+// Each row's tail slot: the diagonal's key first in the row's bucket, or a sentinel in its place.
+__global__ void place_tail(const unsigned long long* __restrict__ starts, int n, int n_faces,
+                           const int* __restrict__ referenced, const int* __restrict__ sentinel_before,
+                           unsigned long long* __restrict__ bucket, unsigned long long* __restrict__ keys_out,
+                           int* __restrict__ order_out) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n) return;
+    if (referenced[v]) {
+        bucket[row_begin(starts, v)] = ((unsigned long long)v << 32) | (unsigned long long)(6LL * n_faces + v);
+        return;
+    }
+    const long long at = (long long)row_begin(starts, n) + sentinel_before[n_faces] + (long long)(starts[v] >> 32);
+    keys_out[at] = (unsigned long long)n * (unsigned long long)n;
+    order_out[at] = -1;
+}
+
+// A CTA sorts the buckets of kSortRows consecutive rows, which are consecutive in memory: staged in
+// shared memory with coalesced loads, a thread insertion-sorts its row there (13 keys on a mesh's
+// usual vertex; a warp a row spends five times the instructions), counts its distinct columns, and
+// the CTA writes the sorted segment back. Rows past kShortRow, and segments past the shared memory,
+// are left to sort_long_rows by a list.
+constexpr int kSortRows = 128;
+constexpr int kSortKeys = 3072;  // 24 KB: 24 keys a row on average
+constexpr int kShortRow = 96;
+
+__global__ void __launch_bounds__(kSortRows) sort_rows(const unsigned long long* __restrict__ starts, int n,
+                                                       unsigned long long* __restrict__ bucket,
+                                                       int* __restrict__ distinct, int* __restrict__ long_rows,
+                                                       int* __restrict__ n_long) {
+    __shared__ unsigned long long keys[kSortKeys];
+    const int first = blockIdx.x * kSortRows, row = first + threadIdx.x;
+    const int begin = row_begin(starts, first), end = row_begin(starts, min(n, first + kSortRows));
+    const bool staged = end - begin <= kSortKeys;
+    if (staged) {
+        for (int p = begin + threadIdx.x; p < end; p += kSortRows) keys[p - begin] = bucket[p];
+        __syncthreads();
+    }
+    if (row < n) {
+        const int from = row_begin(starts, row), count = row_begin(starts, row + 1) - from;
+        if (!staged || count > kShortRow) {
+            if (count > 1) long_rows[atomicAdd(n_long, 1)] = row;
+            else distinct[row] = count;
+        } else {
+            unsigned long long* mine = keys + (from - begin);
+            int columns = count > 0;
+            for (int i = 1; i < count; ++i) {
+                const unsigned long long key = mine[i];
+                int j = i;
+                for (; j > 0 && mine[j - 1] > key; --j) mine[j] = mine[j - 1];
+                mine[j] = key;
+            }
+            for (int i = 1; i < count; ++i) columns += (mine[i] >> 32) != (mine[i - 1] >> 32);
+            distinct[row] = columns;
+        }
+    }
+    if (!staged) return;
+    __syncthreads();
+    for (int p = begin + threadIdx.x; p < end; p += kSortRows) bucket[p] = keys[p - begin];
+}
+
+// The listed rows, a CTA a row: runs of kRun keys sorted by rank in shared memory, then merged
+// pairwise (a key's place is its own plus its rank in the other run, found by bisection), between
+// the buckets and a second buffer of their size.
+constexpr int kLongThreads = 1024;
+constexpr int kRun = 1024;
+
+__global__ void __launch_bounds__(kLongThreads) sort_long_rows(const unsigned long long* __restrict__ starts,
+                                                               const int* __restrict__ long_rows,
+                                                               const int* __restrict__ n_long,
+                                                               unsigned long long* bucket, unsigned long long* spare,
+                                                               int* __restrict__ distinct) {
+    __shared__ unsigned long long run[kRun];
+    __shared__ int scratch[32];
+    const int listed = *n_long;
+    for (int item = blockIdx.x; item < listed; item += gridDim.x) {
+        const int row = long_rows[item];
+        const int from = row_begin(starts, row), count = row_begin(starts, row + 1) - from;
+        unsigned long long *source = bucket + from, *target = spare + from;
+        for (int r = 0; r < count; r += kRun) {
+            const int size = min(kRun, count - r);
+            __syncthreads();
+            if ((int)threadIdx.x < size) run[threadIdx.x] = source[r + threadIdx.x];
+            __syncthreads();
+            if ((int)threadIdx.x < size) {
+                const unsigned long long key = run[threadIdx.x];
+                int rank = 0;
+                for (int i = 0; i < size; ++i) rank += run[i] < key;  // the keys differ by their slots
+                source[r + rank] = key;
+            }
+        }
+        __syncthreads();
+        for (long long width = kRun; width < count; width *= 2) {
+            for (int i = threadIdx.x; i < count; i += kLongThreads) {
+                const unsigned long long key = source[i];
+                const long long pair = i / (2 * width) * (2 * width), middle = min((long long)count, pair + width);
+                const bool left = i < middle;
+                long long lo = left ? middle : pair, hi = left ? min((long long)count, pair + 2 * width) : middle;
+                const long long other = lo;
+                while (lo < hi) {
+                    const long long m = (lo + hi) / 2;
+                    if (source[m] < key) lo = m + 1;
+                    else hi = m;
+                }
+                target[(left ? i : pair + i - middle) + (lo - other)] = key;
+            }
+            __syncthreads();
+            unsigned long long* swap = source;
+            source = target;
+            target = swap;
+        }
+        int columns = 0;
+        for (int i = threadIdx.x; i < count; i += kLongThreads) {
+            const unsigned long long key = source[i];
+            columns += i == 0 || (key >> 32) != (source[i - 1] >> 32);
+        }
+        const int total = block_sum(columns, scratch);
+        if (threadIdx.x == 0) distinct[row] = total;
+        __syncthreads();
+        if (source != bucket + from)
+            for (int i = threadIdx.x; i < count; i += kLongThreads) bucket[from + i] = source[i];
+        __syncthreads();
+    }
+}
+
+// The sorted buckets out, a CTA kSortRows rows: each position's key and payload, and each run of
+// one column as one entry (the entries of consecutive rows are consecutive: offsets of the CTA's
+// first row plus the runs counted so far).
+constexpr int kWriteThreads = 256;
+
+__global__ void __launch_bounds__(kWriteThreads) write_rows(const unsigned long long* __restrict__ bucket,
+                                                            const unsigned long long* __restrict__ starts,
+                                                            const int* __restrict__ offsets, int n, long long tail,
+                                                            unsigned long long* __restrict__ keys_out,
+                                                            int* __restrict__ order_out, int* __restrict__ columns,
+                                                            int* __restrict__ run_start) {
+    __shared__ int row_start[kSortRows + 1];
+    __shared__ int warp_runs[kWriteThreads / 32];
+    const int first = blockIdx.x * kSortRows, rows = min(kSortRows, n - first);
+    for (int i = threadIdx.x; i <= rows; i += kWriteThreads) row_start[i] = row_begin(starts, first + i);
+    __syncthreads();
+    const int begin = row_start[0], end = row_start[rows];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int entry = offsets[first];
+    for (int base = begin; base < end; base += kWriteThreads) {
+        const int p = base + threadIdx.x;
+        bool opens = false;
+        int col = 0;
+        if (p < end) {
+            // The row holding p: row_start[lo] <= p < row_start[lo + 1] (empty rows hold none).
+            int lo = 0, hi = rows - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) / 2;
+                if (row_start[mid] <= p) lo = mid;
+                else hi = mid - 1;
+            }
+            const unsigned long long v = bucket[p];
+            col = (int)(v >> 32);
+            opens = p == row_start[lo] || (int)(bucket[p - 1] >> 32) != col;
+            keys_out[p] = (unsigned long long)(first + lo) * (unsigned long long)n + (unsigned long long)col;
+            order_out[p] = slot_payload((long long)(v & 0xffffffffULL), tail);
+        }
+        const unsigned runs = __ballot_sync(0xffffffffu, opens);
+        if (lane == 0) warp_runs[warp] = __popc(runs);
+        __syncthreads();
+        int before = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < kWriteThreads / 32; ++w) {
+            before += w < warp ? warp_runs[w] : 0;
+            all += warp_runs[w];
+        }
+        if (opens) {
+            const int at = entry + before + __popc(runs & ((1u << lane) - 1u));
+            columns[at] = col;
+            run_start[at] = p;
+        }
+        entry += all;
+        __syncthreads();
+    }
 }
 
 struct PatternLayout {
-    size_t keys_in = 0, sentinel_before = 0, flags = 0, bucket = 0, sorted = 0, counts = 0, starts = 0, fill = 0,
-           sort_temp = 0, scan_temp = 0, total = 0;
+    size_t bucket = 0, spare = 0, counts = 0, totals = 0, starts = 0, sentinels = 0, distinct = 0, long_rows = 0,
+           scan_temp = 0, total = 0;
 };
 
 int pattern_layout(int n, int n_faces, PatternLayout* out) {
     const long long count = 6LL * n_faces + n;
     PatternLayout l;
-    size_t sort_bytes = 0, scan_bytes = 0, row_scan_bytes = 0;
+    size_t rows = 0, face = 0, entries = 0;
     if (count > 0) {
-        // The segmented sort's scratch depends on the in-range count, at most `count`.
-        OB_CUDA(cub::DeviceSegmentedSort::SortKeys(nullptr, sort_bytes, (const unsigned long long*)nullptr,
-                                                   (unsigned long long*)nullptr, (int)count, std::max(n, 1),
-                                                   (const int*)nullptr, (const int*)nullptr));
-        OB_CUDA(cub::DeviceScan::InclusiveSum(nullptr, scan_bytes, (const int*)nullptr,
-                                              (int*)nullptr, (int)count));
-        OB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, row_scan_bytes, (const int*)nullptr, (int*)nullptr,
-                                              n + 1));
-        size_t sentinel_scan = 0;
-        OB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, sentinel_scan, (const int*)nullptr, (int*)nullptr,
-                                              (int)count));
-        scan_bytes = std::max(std::max(scan_bytes, row_scan_bytes), sentinel_scan);
+        OB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, rows, (const unsigned long long*)nullptr,
+                                              (unsigned long long*)nullptr, n + 1));
+        OB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, face, (const int*)nullptr, (int*)nullptr, n_faces + 1));
+        OB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, entries, (const int*)nullptr, (int*)nullptr, n + 1));
     }
-    l.keys_in = 0;
-    l.sentinel_before = align_up(l.keys_in + 8 * (size_t)count);
-    l.flags = align_up(l.sentinel_before + 4 * (size_t)count);
-    l.bucket = align_up(l.flags + 4 * (size_t)count);
-    l.sorted = align_up(l.bucket + 8 * (size_t)count);
-    l.counts = align_up(l.sorted + 8 * (size_t)count);
-    l.starts = align_up(l.counts + 4 * (size_t)(n + 1));
-    l.fill = align_up(l.starts + 4 * (size_t)(n + 1));
-    l.sort_temp = align_up(l.fill + 4 * (size_t)(n + 1));
-    l.scan_temp = align_up(l.sort_temp + sort_bytes);
-    l.total = align_up(l.scan_temp + scan_bytes) + 256;
+    l.bucket = 0;
+    l.spare = align_up(l.bucket + 8 * (size_t)count);
+    // Zeroed at the start of a build, in one piece: the rows' counters, their flags, the list's length.
+    l.counts = align_up(l.spare + 8 * (size_t)count);
+    l.totals = align_up(l.counts + 4 * (2 * (size_t)n + 1));
+    l.starts = align_up(l.totals + 8 * ((size_t)n + 1));
+    l.sentinels = align_up(l.starts + 8 * ((size_t)n + 1));
+    l.distinct = align_up(l.sentinels + 4 * ((size_t)n_faces + 1));
+    l.long_rows = align_up(l.distinct + 4 * ((size_t)n + 1));
+    l.scan_temp = align_up(l.long_rows + 4 * (size_t)n);
+    l.total = align_up(l.scan_temp + std::max(rows, std::max(face, entries))) + 256;
     *out = l;
     return OB_OK;
 }
@@ -227,61 +367,52 @@ int ob_pattern_build(const int32_t* faces, int n_faces, int n_vertices, int32_t*
     OB_REQUIRE(workspace != nullptr && workspace_bytes >= l.total,
                "ob_pattern_build: workspace of %zu bytes, %zu needed", workspace_bytes, l.total);
     char* ws = reinterpret_cast<char*>(align_up(reinterpret_cast<size_t>(workspace)));
-    auto* keys_in = reinterpret_cast<unsigned long long*>(ws + l.keys_in);
-    auto* sentinel_before = reinterpret_cast<int*>(ws + l.sentinel_before);
-    auto* flags = reinterpret_cast<int*>(ws + l.flags);
     auto* bucket = reinterpret_cast<unsigned long long*>(ws + l.bucket);
-    auto* sorted = reinterpret_cast<unsigned long long*>(ws + l.sorted);
+    auto* spare = reinterpret_cast<unsigned long long*>(ws + l.spare);
     auto* counts = reinterpret_cast<int*>(ws + l.counts);
-    auto* starts = reinterpret_cast<int*>(ws + l.starts);
-    auto* fill = reinterpret_cast<int*>(ws + l.fill);
-    void* sort_temp = ws + l.sort_temp;
+    int *referenced = counts + n_vertices, *n_long = referenced + n_vertices;
+    auto* totals = reinterpret_cast<unsigned long long*>(ws + l.totals);
+    auto* starts = reinterpret_cast<unsigned long long*>(ws + l.starts);
+    auto* sentinels = reinterpret_cast<int*>(ws + l.sentinels);
+    auto* distinct = reinterpret_cast<int*>(ws + l.distinct);
+    auto* long_rows = reinterpret_cast<int*>(ws + l.long_rows);
     void* scan_temp = ws + l.scan_temp;
-    const long long tail = 6LL * n_faces;
-    if (n_vertices > 0) {
-        fill_tail<<<ceil_div(n_vertices, kThreads), kThreads, 0, stream>>>(keys_in, tail, n_vertices);
-        OB_CHECK_LAUNCH("fill_tail");
-    }
-    if (n_faces > 0) {
-        operator_keys<<<ceil_div(n_faces, kThreads), kThreads, 0, stream>>>(faces, n_faces, n_vertices, keys_in);
-        OB_CHECK_LAUNCH("operator_keys");
-    }
-    const unsigned long long sentinel = (unsigned long long)n_vertices * n_vertices;
-    auto* keys_out = reinterpret_cast<unsigned long long*>(keys);
-    const int blocks = ceil_div(count, kThreads);
     size_t scan_bytes = l.total - 256 - l.scan_temp;
-    OB_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)(n_vertices + 1), stream));
-    OB_CUDA(cudaMemsetAsync(fill, 0, sizeof(int) * (size_t)(n_vertices + 1), stream));
-    row_counts<<<blocks, kThreads, 0, stream>>>(keys_in, count, sentinel, std::max(n_vertices, 1), counts, flags);
-    OB_CHECK_LAUNCH("row_counts");
-    OB_CUDA(cub::DeviceScan::ExclusiveSum(scan_temp, scan_bytes, counts, starts, n_vertices + 1, stream));
+    auto* keys_out = reinterpret_cast<unsigned long long*>(keys);
+    const int n = n_vertices;
+    OB_CUDA(cudaMemsetAsync(counts, 0, sizeof(int) * (2 * (size_t)n + 1), stream));
+    corner_counts<<<ceil_div(n_faces + 1LL, kThreads), kThreads, 0, stream>>>(faces, n_faces, n, counts, referenced,
+                                                                             sentinels);
+    OB_CHECK_LAUNCH("corner_counts");
+    row_totals<<<ceil_div(n + 1LL, kThreads), kThreads, 0, stream>>>(counts, referenced, n, totals);
+    OB_CHECK_LAUNCH("row_totals");
+    OB_CUDA(cub::DeviceScan::ExclusiveSum(scan_temp, scan_bytes, totals, starts, n + 1, stream));
     count_launch(1);
     // The sentinel slots' places among themselves.
-    OB_CUDA(cub::DeviceScan::ExclusiveSum(scan_temp, scan_bytes, flags, sentinel_before, (int)count, stream));
+    OB_CUDA(cub::DeviceScan::ExclusiveSum(scan_temp, scan_bytes, sentinels, sentinels, n_faces + 1, stream));
     count_launch(1);
-    scatter_rows<<<blocks, kThreads, 0, stream>>>(keys_in, count, sentinel, std::max(n_vertices, 1), starts, fill,
-                                                  sentinel_before, tail, bucket, keys_out, order);
-    OB_CHECK_LAUNCH("scatter_rows");
-    if (n_vertices > 0) {
-        // Sorted by (col, slot) within each row: the sort covers the in-range keys, starts[n] of them
-        // (at most `count`, the size the scratch was sized for; the segments bound what is read).
-        size_t sort_bytes = l.scan_temp - l.sort_temp;
-        OB_CUDA(cub::DeviceSegmentedSort::SortKeys(sort_temp, sort_bytes, bucket, sorted, (int)count, n_vertices,
-                                                   starts, starts + 1, stream));
-        count_launch(1);
-        write_rows<<<ceil_div(8LL * n_vertices, kThreads), kThreads, 0, stream>>>(sorted, starts, n_vertices, tail,
-                                                                                 keys_out, order);
+    if (n_faces > 0) {
+        scatter_corners<<<ceil_div(n_faces, kThreads), kThreads, 0, stream>>>(faces, n_faces, n, starts, counts,
+                                                                             sentinels, bucket, keys_out, order);
+        OB_CHECK_LAUNCH("scatter_corners");
+    }
+    if (n > 0) {
+        place_tail<<<ceil_div(n, kThreads), kThreads, 0, stream>>>(starts, n, n_faces, referenced, sentinels, bucket,
+                                                                   keys_out, order);
+        OB_CHECK_LAUNCH("place_tail");
+        sort_rows<<<ceil_div(n, kSortRows), kSortRows, 0, stream>>>(starts, n, bucket, distinct, long_rows, n_long);
+        OB_CHECK_LAUNCH("sort_rows");
+        sort_long_rows<<<sm_count(), kLongThreads, 0, stream>>>(starts, long_rows, n_long, bucket, spare, distinct);
+        OB_CHECK_LAUNCH("sort_long_rows");
+    }
+    // (The scan reads distinct[n] and adds it to nothing.)
+    OB_CUDA(cub::DeviceScan::ExclusiveSum(scan_temp, scan_bytes, distinct, offsets, n + 1, stream));
+    count_launch(1);
+    if (n > 0) {
+        write_rows<<<ceil_div(n, kSortRows), kWriteThreads, 0, stream>>>(bucket, starts, offsets, n, 6LL * n_faces,
+                                                                         keys_out, order, columns, run_start);
         OB_CHECK_LAUNCH("write_rows");
     }
-    run_flags<<<blocks, kThreads, 0, stream>>>(reinterpret_cast<unsigned long long*>(keys), count,
-                                               sentinel, flags);
-    OB_CHECK_LAUNCH("run_flags");
-    OB_CUDA(cub::DeviceScan::InclusiveSum(scan_temp, scan_bytes, flags, flags, (int)count, stream));
-    count_launch(1);
-    place_runs<<<blocks, kThreads, 0, stream>>>(reinterpret_cast<unsigned long long*>(keys), flags,
-                                                count, sentinel, n_vertices, offsets, columns,
-                                                run_start);
-    OB_CHECK_LAUNCH("place_runs");
     return OB_OK;
 }
 
