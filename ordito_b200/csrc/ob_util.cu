@@ -95,15 +95,18 @@ __global__ void bounds_kernel(const float* __restrict__ xyz, int n, float* __res
         }
     }
     if (!last_block_arrived(counter, &last)) return;
-    if (threadIdx.x != 0) return;
     for (int d = 0; d < 3; ++d) {
         float a = INFINITY, b = -INFINITY;
-        for (int bx = 0; bx < (int)gridDim.x; ++bx) {
+        for (int bx = threadIdx.x; bx < (int)gridDim.x; bx += blockDim.x) {
             a = fminf(a, __ldcg(&partials[6 * bx + d]));
             b = fmaxf(b, __ldcg(&partials[6 * bx + 3 + d]));
         }
-        out[d] = a;
-        out[3 + d] = b;
+        a = -block_max(-a, scratch, -INFINITY);
+        b = block_max(b, scratch, -INFINITY);
+        if (threadIdx.x == 0) {
+            out[d] = a;
+            out[3 + d] = b;
+        }
     }
 }
 
