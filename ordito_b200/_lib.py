@@ -125,6 +125,9 @@ SIGNATURES: dict[str, list] = {
     "ob_log_map_outward_ball": [P, P, P, P, P, P, I, I, P, P],
     "ob_radial_divergence": [P, P, I, I, P, P, P, I, P, P, P, P, P, P],
     "ob_log_map_fields": [P, P, I, I, P, P],
+    "ob_chol_analyse_begin": [I, P, P, P, I, POINTER(c_void_p), P],
+    "ob_chol_analyse_end": [P, POINTER(c_void_p)],
+    "ob_chol_analyse_abandon": [P],
     "ob_chol_analyse_blocked": [I, I, P, P, P, I, POINTER(c_void_p), P],
     "ob_extend_ratio": [P, I, P, P, P],
     "ob_chol_set_deterministic": [P, I, P],

@@ -55,6 +55,15 @@ class CholeskyAnalysis:
         _lib.call("ob_chol_analyse_blocked", matrix.nrow, int(block), matrix.offsets.ptr,
                   matrix.columns.ptr, xyz, int(leaf_size), ctypes.byref(handle), DEFAULT_STREAM)
         del keep
+        self._bind(handle, matrix)
+
+    @classmethod
+    def _adopt(cls, handle: ctypes.c_void_p, matrix: CsrMatrix) -> "CholeskyAnalysis":
+        analysis = cls.__new__(cls)
+        analysis._bind(handle, matrix)
+        return analysis
+
+    def _bind(self, handle: ctypes.c_void_p, matrix: CsrMatrix) -> None:
         self.handle = handle
         info = (ctypes.c_longlong * 5)()
         _lib.call("ob_chol_analysis_info", handle, info)
@@ -269,6 +278,34 @@ def sparse_cholesky(matrix: CsrMatrix, coordinates: Any = None, *, negated: bool
     return SparseCholesky(matrix, analysis, singular=None, negated=not first)
 
 
+class _PendingAnalysis:
+    """An operator's analysis under way on a host thread (``ob_chol_analyse_begin``)."""
+
+    def __init__(self, matrix: CsrMatrix, coordinates: Any) -> None:
+        self.matrix = matrix
+        xyz, self._keep = device_pointer(coordinates, np.float32, 3 * matrix.nrow) if coordinates is not None else (0, None)
+        self.handle = ctypes.c_void_p(0)
+        _lib.call("ob_chol_analyse_begin", matrix.nrow, matrix.offsets.ptr, matrix.columns.ptr, xyz,
+                  CHOLESKY_LEAF_ROWS, ctypes.byref(self.handle), DEFAULT_STREAM)
+
+    def end(self) -> CholeskyAnalysis:
+        pending, self.handle = self.handle, ctypes.c_void_p(0)
+        handle = ctypes.c_void_p(0)
+        _lib.call("ob_chol_analyse_end", pending, ctypes.byref(handle))
+        return CholeskyAnalysis._adopt(handle, self.matrix)
+
+    def abandon(self) -> None:
+        if self.handle.value:
+            pending, self.handle = self.handle, ctypes.c_void_p(0)
+            _lib.lib.ob_chol_analyse_abandon(pending)
+
+    def __del__(self) -> None:
+        try:
+            self.abandon()
+        except Exception:
+            pass
+
+
 class OperatorFactorization:
     """The factorization slot of one operator (ordito/linalg.py:2191)."""
 
@@ -283,9 +320,18 @@ class OperatorFactorization:
         self.refused = False
         self.indefinite = False
         self.iterate_rejected = False
+        self._pending: _PendingAnalysis | None = None
+
+    def analyse_ahead(self) -> None:
+        """Start the analysis on a host thread now, for a ``factor`` that may follow."""
+        if self.analysis is None and self._pending is None and self.block == 1:
+            self._pending = _PendingAnalysis(self.matrix, self.coordinates)
 
     def exceeds_budget(self) -> bool:
         """Whether the factor would exceed ``CHOLESKY_MEMORY_BUDGET`` (asks the analysis)."""
+        if self.analysis is None and self._pending is not None:
+            pending, self._pending = self._pending, None
+            self.analysis = pending.end()
         if self.analysis is None:
             self.analysis = CholeskyAnalysis(self.matrix, self.coordinates, block=self.block)
         return self.analysis.factor_bytes > CHOLESKY_MEMORY_BUDGET
@@ -316,6 +362,9 @@ class OperatorFactorization:
         self.factorization.solve(rhs, solution, tol=tol, componentwise=componentwise)
 
     def release(self) -> None:
+        if self._pending is not None:
+            self._pending.abandon()
+            self._pending = None
         if self.factorization is not None:
             self.factorization.close()
             self.factorization = None

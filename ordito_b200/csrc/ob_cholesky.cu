@@ -17,10 +17,13 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <condition_variable>
 #include <cstring>
 #include <functional>
 #include <memory>
+#include <mutex>
 #include <numeric>
+#include <string>
 #include <thread>
 #include <vector>
 
@@ -53,9 +56,11 @@ struct Dissector {
     std::atomic<int> stamps{3};
     std::vector<Node> tree;  // built in postorder
     std::vector<int> order;  // new -> old, filled in postorder
+    const std::atomic<bool>* cancel;  // may be null; once true, what is left becomes leaves as it is
 
-    Dissector(const std::vector<int>& o, const std::vector<int>& c, const float* p, int n, int leaf)
-        : off(o), col(c), xyz(p), leaf_size(leaf), side(new std::atomic<int>[std::max(n, 1)]) {
+    Dissector(const std::vector<int>& o, const std::vector<int>& c, const float* p, int n, int leaf,
+              const std::atomic<bool>* stop = nullptr)
+        : off(o), col(c), xyz(p), leaf_size(leaf), side(new std::atomic<int>[std::max(n, 1)]), cancel(stop) {
         for (int v = 0; v < n; ++v) side[v].store(0, std::memory_order_relaxed);
     }
 
@@ -114,7 +119,7 @@ struct Dissector {
     // Builds the subtree of `verts` into `tree` / `order` (postorder, indices within the lists);
     // returns its root's index.
     int dissect(std::vector<int> verts, std::vector<Node>& tree_out, std::vector<int>& order_out, int depth) {
-        if ((int)verts.size() <= leaf_size) {
+        if ((int)verts.size() <= leaf_size || (cancel && cancel->load(std::memory_order_relaxed))) {
             std::sort(verts.begin(), verts.end());
             Node leaf;
             leaf.start = (int)order_out.size();
@@ -342,8 +347,9 @@ void amalgamate(Analysis& A, const std::vector<int>& adj_off, const std::vector<
 // vertex (xyz holds n / block points), as in a system of tangent vectors. The dissection then runs
 // over the vertices' graph and every vertex's rows stay together, consecutive in the ordering.
 int analyse(int n, std::vector<int> offsets, std::vector<int> columns, const float* xyz,
-            int leaf_size, Analysis* out, int block = 1) {
+            int leaf_size, Analysis* out, int block = 1, const std::atomic<bool>* cancel = nullptr) {
     Analysis& A = *out;
+    const auto cancelled = [cancel]() { return cancel && cancel->load(std::memory_order_relaxed); };
     A.n = n;
     A.offsets = std::move(offsets);
     A.columns = std::move(columns);
@@ -395,17 +401,20 @@ int analyse(int n, std::vector<int> offsets, std::vector<int> columns, const flo
             node.count *= block;
         }
     } else {
-        Dissector D(adj_off, adj, xyz, n, leaf_size);
+        Dissector D(adj_off, adj, xyz, n, leaf_size, cancel);
         std::vector<int> all(n);
         std::iota(all.begin(), all.end(), 0);
         D.dissect(std::move(all));
         A.perm = std::move(D.order);
         A.nodes = std::move(D.tree);
     }
+    if (cancelled()) return OB_ERR_INVALID;
     A.iperm.assign(n, 0);
     for (int i = 0; i < n; ++i) A.iperm[A.perm[i]] = i;
     symbolic(A, adj_off, adj);
+    if (cancelled()) return OB_ERR_INVALID;
     amalgamate(A, adj_off, adj);
+    if (cancelled()) return OB_ERR_INVALID;
     // Components (for pinning a singular operator): each vertex's component label and the last
     // vertex of each in the new order.
     A.component_last.assign(n, 0);
@@ -1839,6 +1848,114 @@ int solve_graph(Factor* F, Factor::WorkSet& W, int k, int refine, const int* off
 }
 
 
+// An analysis under way on a host thread of its own, beside the device's work (a query's settled
+// heat solve, whose iterate the factorisation may have to replace). The thread copies the operator's
+// pattern on its own stream, behind an event of the caller's, then works on its copies.
+struct Pending {
+    int device = 0;
+    cudaEvent_t ready = nullptr;
+    std::atomic<bool> cancel{false};
+    std::mutex mutex;
+    std::condition_variable signal;
+    bool copied = false;            // the caller's arrays are read no more
+    std::atomic<bool> done{false};
+    int status = OB_OK;
+    std::string error;
+    std::unique_ptr<Analysis> analysis;
+    std::thread worker;
+    ~Pending() {
+        if (ready) cudaEventDestroy(ready);
+    }
+};
+
+int copy_pattern(Pending& P, int n, const int* offsets, const int* columns, const float* xyz, std::vector<int>* off,
+                 std::vector<int>* col, std::vector<float>* pts) {
+    OB_CUDA(cudaSetDevice(P.device));
+    cudaStream_t stream = nullptr;
+    OB_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    auto copy = [&]() -> int {
+        OB_CUDA(cudaStreamWaitEvent(stream, P.ready, 0));
+        off->resize((size_t)n + 1);
+        OB_CUDA(cudaMemcpyAsync(off->data(), offsets, sizeof(int) * ((size_t)n + 1), cudaMemcpyDeviceToHost, stream));
+        OB_CUDA(cudaStreamSynchronize(stream));
+        col->resize((size_t)std::max((*off)[n], 0));
+        if (!col->empty())
+            OB_CUDA(cudaMemcpyAsync(col->data(), columns, sizeof(int) * col->size(), cudaMemcpyDeviceToHost, stream));
+        if (xyz != nullptr) {
+            pts->resize(3 * (size_t)n);
+            OB_CUDA(cudaMemcpyAsync(pts->data(), xyz, sizeof(float) * pts->size(), cudaMemcpyDeviceToHost, stream));
+        }
+        OB_CUDA(cudaStreamSynchronize(stream));
+        return OB_OK;
+    };
+    const int st = copy();
+    cudaStreamSynchronize(stream);  // nothing reads the caller's arrays past this point
+    cudaStreamDestroy(stream);
+    return st;
+}
+
+void run_pending(Pending& P, int n, const int* offsets, const int* columns, const float* xyz, int leaf_size) {
+    int st = OB_ERR_INVALID;
+    auto copies_done = [&P]() {
+        std::lock_guard<std::mutex> lock(P.mutex);
+        P.copied = true;
+        P.signal.notify_all();
+    };
+    try {
+        std::vector<int> off, col;
+        std::vector<float> pts;
+        if (!P.cancel.load()) st = copy_pattern(P, n, offsets, columns, xyz, &off, &col, &pts);
+        copies_done();
+        if (st == OB_OK) {
+            auto A = std::make_unique<Analysis>();
+            st = analyse(n, std::move(off), std::move(col), xyz ? pts.data() : nullptr, leaf_size, A.get(), 1, &P.cancel);
+            if (st == OB_OK) P.analysis = std::move(A);
+            else P.error = "the analysis was abandoned";
+        } else {
+            P.error = ob_last_error();
+        }
+    } catch (const std::exception& e) {
+        st = OB_ERR_NOMEM;
+        P.error = e.what();
+        copies_done();
+    }
+    P.status = st;
+    P.done.store(true);
+}
+
+// Abandoned analyses: their threads stop at their next step; each is joined when a later one is
+// abandoned after it has stopped, or at exit.
+class Abandoned {
+  public:
+    void add(std::shared_ptr<Pending> P) {
+        std::lock_guard<std::mutex> lock(mutex_);
+        for (size_t i = 0; i < list_.size();) {
+            if (list_[i]->done.load()) {
+                list_[i]->worker.join();
+                list_.erase(list_.begin() + (long)i);
+            } else {
+                ++i;
+            }
+        }
+        list_.push_back(std::move(P));
+    }
+    ~Abandoned() {
+        for (auto& P : list_) {
+            P->worker.join();
+            P->ready = nullptr;  // the driver may be gone by now
+        }
+    }
+
+  private:
+    std::mutex mutex_;
+    std::vector<std::shared_ptr<Pending>> list_;
+};
+
+Abandoned& abandoned() {
+    static Abandoned list;
+    return list;
+}
+
 }  // namespace
 }  // namespace ob
 
@@ -1880,6 +1997,56 @@ int ob_chol_analyse_blocked(int n, int block, const int32_t* offsets, const int3
         return st;
     }
     *analysis = A;
+    return OB_OK;
+}
+
+int ob_chol_analyse_begin(int n, const int32_t* offsets, const int32_t* columns, const float* xyz, int leaf_size,
+                          void** pending, ob_stream_t stream_) {
+    OB_REQUIRE(pending != nullptr, "ob_chol_analyse_begin: null output");
+    *pending = nullptr;
+    OB_REQUIRE(n >= 1 && offsets && columns, "ob_chol_analyse_begin: bad argument");
+    cudaStream_t stream = as_stream(stream_);
+    auto P = std::make_shared<Pending>();
+    OB_CUDA(cudaGetDevice(&P->device));
+    OB_CUDA(cudaEventCreateWithFlags(&P->ready, cudaEventDisableTiming));
+    cudaError_t e = cudaEventRecord(P->ready, stream);
+    if (e != cudaSuccess) return cuda_status(e, "ob_chol_analyse_begin: event");
+    try {
+        P->worker = std::thread([P, n, offsets, columns, xyz, leaf_size]() {
+            run_pending(*P, n, offsets, columns, xyz, leaf_size);
+        });
+        *pending = new std::shared_ptr<Pending>(P);
+    } catch (const std::exception&) {
+        if (P->worker.joinable()) P->worker.join();
+        return fail(OB_ERR_NOMEM, "ob_chol_analyse_begin: no host thread");
+    }
+    return OB_OK;
+}
+
+int ob_chol_analyse_end(void* pending, void** analysis) {
+    OB_REQUIRE(pending && analysis, "ob_chol_analyse_end: bad argument");
+    *analysis = nullptr;
+    auto* held = static_cast<std::shared_ptr<Pending>*>(pending);
+    std::shared_ptr<Pending> P = *held;
+    delete held;
+    P->worker.join();
+    if (P->status) return fail(P->status, "ob_chol_analyse_end: %s", P->error.c_str());
+    *analysis = P->analysis.release();
+    return OB_OK;
+}
+
+int ob_chol_analyse_abandon(void* pending) {
+    if (pending == nullptr) return OB_OK;
+    auto* held = static_cast<std::shared_ptr<Pending>*>(pending);
+    std::shared_ptr<Pending> P = *held;
+    delete held;
+    P->cancel.store(true);
+    {
+        // The caller's arrays are read no more once the copies are done (or were never started).
+        std::unique_lock<std::mutex> lock(P->mutex);
+        P->signal.wait(lock, [&]() { return P->copied; });
+    }
+    abandoned().add(P);
     return OB_OK;
 }
 

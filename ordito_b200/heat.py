@@ -43,6 +43,8 @@ _HEAT_CHECK_ROUNDS = 16  # :142
 _HEAT_CHANGE_TOLERANCE = 1e-6  # :146
 _HEAT_SETTLE_ROUNDS = 192  # :147
 _DIFFUSION_DECAY = 400.0  # :158
+# Rows from which a settled solve has its analysis started beside it.
+_ANALYSE_AHEAD_ROWS = 65536
 _GEOMETRY_CENTRAL_POISSON_SHIFT = 1e-6  # :193 (geometry-central's Poisson system -L + 1e-6 I)
 _TOLERANCE_MOLLIFY = 1e-5  # ordito/constants.py:31 (use_robust's margin, of the mean edge length)
 
@@ -460,6 +462,10 @@ class HeatSolver:
         operators = self.operators
         kept = self._kept("heat")
         held = kept["factorization"].factorization is not None
+        if not held and not kept["factorization"].refused and operators.heat_system.nrow >= _ANALYSE_AHEAD_ROWS:
+            # The settled iterate of a large mesh may be rejected: the analysis its factorization
+            # then needs runs on host threads while the device iterates.
+            kept["factorization"].analyse_ahead()
         twl.solve_spd_settled(
             operators.heat_system,
             rhs,
