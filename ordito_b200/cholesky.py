@@ -327,6 +327,12 @@ class OperatorFactorization:
         if self.analysis is None and self._pending is None and self.block == 1:
             self._pending = _PendingAnalysis(self.matrix, self.coordinates)
 
+    def drop_analysis_ahead(self) -> None:
+        """Give up an analysis started ahead that no ``factor`` has taken."""
+        if self._pending is not None:
+            pending, self._pending = self._pending, None
+            pending.abandon()
+
     def exceeds_budget(self) -> bool:
         """Whether the factor would exceed ``CHOLESKY_MEMORY_BUDGET`` (asks the analysis)."""
         if self.analysis is None and self._pending is not None:
@@ -362,9 +368,7 @@ class OperatorFactorization:
         self.factorization.solve(rhs, solution, tol=tol, componentwise=componentwise)
 
     def release(self) -> None:
-        if self._pending is not None:
-            self._pending.abandon()
-            self._pending = None
+        self.drop_analysis_ahead()
         if self.factorization is not None:
             self.factorization.close()
             self.factorization = None

@@ -43,8 +43,11 @@ _HEAT_CHECK_ROUNDS = 16  # :142
 _HEAT_CHANGE_TOLERANCE = 1e-6  # :146
 _HEAT_SETTLE_ROUNDS = 192  # :147
 _DIFFUSION_DECAY = 400.0  # :158
-# Rows from which a settled solve has its analysis started beside it.
-_ANALYSE_AHEAD_ROWS = 65536
+# Rows from which a settled solve has its analysis started beside it: the analysis then takes a
+# third of the call (0.26 s of 0.80 s at 2.6 M rows). On smaller meshes there is less to hide, and
+# the host threads of an analysis that turns out not to be needed delay the call's own launches
+# (a 200 k-vertex sheet whose iterate is kept: 22 -> 28 ms).
+_ANALYSE_AHEAD_ROWS = 1 << 20
 _GEOMETRY_CENTRAL_POISSON_SHIFT = 1e-6  # :193 (geometry-central's Poisson system -L + 1e-6 I)
 _TOLERANCE_MOLLIFY = 1e-5  # ordito/constants.py:31 (use_robust's margin, of the mean edge length)
 
@@ -476,6 +479,7 @@ class HeatSolver:
             factorization=kept["factorization"],
             narrow_values=True,
         )
+        kept["factorization"].drop_analysis_ahead()  # the iterate was accepted
         # A rejected settled iterate (answered by the factor or, past the budget, the march)
         # marks the mesh ill-conditioned for its Poisson solve (ordito/heat.py:4394-4404).
         if not held and (kept["factorization"].factorization is not None
