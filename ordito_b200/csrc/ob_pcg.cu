@@ -544,8 +544,10 @@ int next_pow2(int v) {
     return p;
 }
 
-constexpr size_t kStateBytes = 64;  // of the state in its allocation, the scalars after it
-static_assert(sizeof(LoopState) <= kStateBytes, "the state is followed by the columns' scalars");
+// The state's allocation: the state, the resident form's arrival counter and abort flag, the
+// columns' scalars.
+constexpr size_t kArrivalsAt = 32, kStateBytes = 64;
+static_assert(sizeof(LoopState) <= kArrivalsAt, "the state is followed by the arrivals");
 
 struct Solver {
     int n = 0, k_live = 0, k = 0, precond = 0, narrow = 0;
@@ -581,9 +583,10 @@ struct Solver {
     const void* resident = nullptr;
     int resident_form = 0, resident_threads = 0, resident_ctas = 0, resident_width = 0, resident_pushes = 0;
     size_t resident_smem = 0;
+    bool resident_settles = false;  // the form has the settle check
     double* published = nullptr;  // kGrid: two buffers of n
     double* resident_partials = nullptr;
-    unsigned int* arrivals = nullptr;  // the counter and the abort flag
+    unsigned int* arrivals = nullptr;  // the counter and the abort flag, in the state's allocation
     cudaStream_t capture = nullptr;
     // Cached loop graphs: key = (settle?, rounds per body, maxiter, params).
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
@@ -766,16 +769,18 @@ bool take_resident(Solver* S, int form, int rows_a_cta, int rows_a_thread) {
         return false;
     const size_t owned = (size_t)threads * rows_a_thread;
     const int registers = register_entries(rows_a_thread);
-    const int pushes = form == kCluster ? (int)(2 * owned) : 0;
+    const int pushes = form == kCluster ? (int)(owned * (registers ? kPushesARow : kPushesARow / 2)) : 0;
     const size_t fixed = (form == kGrid ? 0 : 16 * (owned + (form == kCluster ? kHalo : 0))) +
-                         8 * (6 * kClusterMax + 3 * 32 + 4) +
+                         8 * (6 * kClusterMax + 3 * 32 + 8 + 4 * kChebyshevDegree) +
+                         (far_vectors(rows_a_thread, S->precond == 1) ? 24 * owned : 0) +
                          (form == kCluster ? sizeof(int2) * pushes + sizeof(int) * (2 * kHaloTable + 4) : 0);
     const size_t entry = owned * (sizeof(unsigned) + sizeof(double));
-    if (fixed + (registers ? 0 : 7) * entry > (size_t)limit) return false;
+    if (fixed + (kBaseEntries - registers) * entry > (size_t)limit) return false;
     S->resident_form = form;
     S->resident_threads = threads;
     S->resident_ctas = (int)((S->n + owned - 1) / owned);
     S->resident_pushes = pushes;
+    S->resident_settles = !far_vectors(rows_a_thread, S->precond == 1);
     S->resident_width = (int)std::min<size_t>(kResidentWidth, registers + ((size_t)limit - fixed) / entry);
     S->resident_smem = fixed + (S->resident_width - registers) * entry;
     const bool cheb = S->precond == 1;
@@ -816,9 +821,9 @@ void choose_resident(Solver* S) {
     if (S->k != 1) return;
     if (S->n <= 1024 && take_resident(S, kBlock, S->n, 2)) return;
     const int cluster_rows = std::max((S->n + kClusterMax - 1) / kClusterMax, 64);
-    if (cluster_rows <= 2048 && take_resident(S, kCluster, cluster_rows, cluster_rows <= 1280 ? 2 : 4)) return;
+    if (cluster_rows <= 2048 && take_resident(S, kCluster, cluster_rows, cluster_rows <= 1024 ? 2 : 4)) return;
     const int grid_rows = std::max((S->n + sm_count() - 1) / sm_count(), 256);
-    if (grid_rows <= 2048) take_resident(S, kGrid, grid_rows, grid_rows <= 1280 ? 2 : 4);
+    if (grid_rows <= 2048) take_resident(S, kGrid, grid_rows, grid_rows <= 1024 ? 2 : 4);
 }
 
 // One solve by the resident form; check_rounds 0 stops by the residual.
@@ -829,7 +834,6 @@ int launch_resident(Solver* S, const double* rhs, double* x, double tol, int max
             if (int st = solver_alloc(S, (void**)&S->published, sizeof(double) * 2 * (size_t)S->n, stream)) return st;
             if (int st = solver_alloc(S, (void**)&S->resident_partials, sizeof(double) * 6 * S->resident_ctas, stream))
                 return st;
-            if (int st = solver_alloc(S, (void**)&S->arrivals, 2 * sizeof(int), stream)) return st;
         }
         OB_CUDA(cudaMemsetAsync(S->arrivals, 0, 2 * sizeof(int), stream));
     }
@@ -1061,7 +1065,7 @@ int read_back(Solver* S, cudaStream_t stream) {
     OB_CUDA(cudaMemcpyAsync(S->host_state, S->state, kStateBytes + sizeof(ColumnScalars) * S->k,
                             cudaMemcpyDeviceToHost, stream));
     OB_CUDA(cudaStreamSynchronize(stream));
-    if (S->host_state->status == kStatusAborted)
+    if (S->resident && reinterpret_cast<const int*>(reinterpret_cast<const char*>(S->host_state) + kArrivalsAt)[1] != 0)
         return fail(OB_ERR_TIMEOUT, "pcg: a wait between the solver's blocks gave up");
     return OB_OK;
 }
@@ -1134,6 +1138,7 @@ int ob_pcg_create(int n, const int32_t* offsets, const int32_t* columns, const d
         solver_release(S);
         return st;
     }
+    S->arrivals = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(S->state) + kArrivalsAt);
     S->scalars = reinterpret_cast<ColumnScalars*>(reinterpret_cast<char*>(S->state) + kStateBytes);
     if (cudaMallocHost((void**)&S->host_state, kStateBytes + sizeof(ColumnScalars) * S->k) != cudaSuccess) {
         cudaGetLastError();
@@ -1142,6 +1147,7 @@ int ob_pcg_create(int n, const int32_t* offsets, const int32_t* columns, const d
     }
     S->host_scalars = reinterpret_cast<ColumnScalars*>(reinterpret_cast<char*>(S->host_state) + kStateBytes);
     e = cudaMemsetAsync(S->counters, 0, sizeof(unsigned int) * 8, stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(S->state, 0, kStateBytes, stream);
     if (e != cudaSuccess) {
         solver_release(S);
         return cuda_status(e, "ob_pcg_create: memset");
@@ -1214,14 +1220,15 @@ int ob_pcg_settle(void* solver, const double* rhs, double* x, int check_rounds,
     OB_REQUIRE(check_rounds >= 1 && check_rounds <= 256, "ob_pcg_settle: check_rounds in [1, 256]");
     OB_REQUIRE(maxiter >= 0, "ob_pcg_settle: negative cap");
     Solver* S = static_cast<Solver*>(solver);
-    int st = S->resident ? launch_resident(S, rhs, x, 0.0, maxiter, check_rounds, change_tolerance, settle_rounds,
+    const bool resident = S->resident && S->resident_settles;
+    int st = resident ? launch_resident(S, rhs, x, 0.0, maxiter, check_rounds, change_tolerance, settle_rounds,
                                            stream)
                          : run_loop(S, rhs, x, 0.0, 1, check_rounds, maxiter, check_rounds, change_tolerance,
                                     settle_rounds, stream);
     if (st) return st;
     if (rounds || status) {
         if ((st = read_back(S, stream))) return st;
-        if (!S->resident) count_body_launches(S, check_rounds, 1);
+        if (!resident) count_body_launches(S, check_rounds, 1);
         if (rounds) *rounds = S->host_state->iterations;
         if (status) *status = S->host_state->status;
     }

@@ -13,14 +13,18 @@
 //   kCluster  up to 16 CTAs, each holding its rows' values and a copy of the other CTAs' values its
 //             rows read (its halo). A CTA publishes by storing its own values and pushing those
 //             other CTAs hold copies of into their shared memory (a list made at the start), so
-//             every gather is local; barrier.cluster between phases. (Gathering from the other
-//             CTAs instead took 3 us a mat-vec on a 10 k-vertex icosphere, whose edge rows read
-//             nothing local; what does not fit the halo is still read so.)
+//             every gather is local. The pushes are asynchronous stores that count themselves off at
+//             a barrier in the shared memory they arrive in (mbarrier transaction bytes), so a CTA
+//             waits for the values it reads and nothing else: barrier.cluster between the phases
+//             took 1.3 us each. (Gathering from the other CTAs took 3 us a mat-vec on a 10 k-vertex
+//             icosphere, whose edge rows read nothing local. Where a halo does not fit, or a CTA
+//             would push to one it does not read, the whole cluster gathers so, between
+//             barrier.clusters.)
 //   kGrid     up to one CTA an SM (a cooperative launch): global memory at L2, an arrival counter
-//             between phases. Its wait is bounded: a CTA that gives up raises `abort`, every CTA
-//             then leaves, and the host reports OB_ERR_TIMEOUT.
+//             between phases.
 //
-// Rows longer than the entries a thread holds read the rest from the CSR arrays. A round's float64
+// Every wait is bounded: a CTA that gives up raises `abort`, the others then give up as well, and the
+// host reports OB_ERR_TIMEOUT. Rows longer than the entries a thread holds read the rest from the CSR arrays. A round's float64
 // chain is kept short (two partial sums a row, one division behind the dots), since latency is what
 // is left: the sums a row and the scalars agree with the loop graph's to rounding. The dots are
 // folded thread, warp, CTA in a fixed order, so every run gives the same bits.
@@ -35,10 +39,15 @@ enum ResidentForm : int { kBlock = 0, kCluster = 1, kGrid = 2 };
 constexpr int kClusterMax = 16;
 constexpr int kHalo = 1024;      // other CTAs' values a cluster CTA holds copies of
 constexpr int kHaloTable = 2048; // the hash table that numbers them
+constexpr int kPushesARow = 4;   // a CTA's push list, of its rows (two rows a thread; half at four)
 constexpr int kResidentWidth = 16;      // entries a row kept on the chip, at most
-__host__ __device__ constexpr int register_entries(int rows_a_thread) { return rows_a_thread <= 2 ? 7 : 0; }
+constexpr int kBaseEntries = 7;  // a mesh row's usual count: every row is padded to it
+__host__ __device__ constexpr int register_entries(int rows_a_thread) { return rows_a_thread <= 2 ? kBaseEntries : 0; }
+// Whether x, p and s of a thread's rows lie in shared memory: four rows' vectors under the polynomial
+// take more than the 128 registers a thread has, and a step's loads then wait for one another (3 400
+// cycles a mat-vec of 1 250 rows, 2 200 without the polynomial). Such a solver has no settle check.
+__host__ __device__ constexpr bool far_vectors(int rows_a_thread, bool cheb) { return rows_a_thread == 4 && cheb; }
 __host__ __device__ constexpr int resident_threads(int) { return 512; }
-constexpr int kStatusAborted = -1;      // LoopState::status of a solve whose grid wait gave up
 constexpr unsigned kGridSpins = 1u << 22;  // polls (>= 0.3 us each) before a grid wait gives up
 
 struct ResidentArgs {
@@ -60,12 +69,12 @@ struct ResidentArgs {
     int narrow;  // the operator's values are rounded to float32
     int width;   // entries a row on the chip, those in registers among them
     int pushes;  // kCluster: the capacity of a CTA's push list
-    // kGrid: the published vector (two buffers of n), the CTAs' partial sums (6 a CTA), the
-    // arrival counter and the abort flag (both zero at the launch).
+    int* abort;  // 1 when a wait gave up (zero at the launch of kGrid, zeroed by the others)
+    // kGrid: the published vector (two buffers of n), the CTAs' partial sums (6 a CTA) and the
+    // arrival counter (zero at the launch).
     double* published;
     double* partials;
     unsigned int* counter;
-    int* abort;
 };
 
 __device__ __forceinline__ unsigned shared_address(const void* p) {
@@ -94,6 +103,37 @@ __device__ __forceinline__ double load_l2(const double* p) {
     double v;
     asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
     return v;
+}
+
+// Barriers in shared memory that count arriving bytes. A phase ends when the one arrival (which
+// says how many bytes are due) and that many bytes have come.
+__device__ __forceinline__ void arrivals_init(unsigned bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void arrivals_expect(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Waits for the phase of the given parity, kArrivalTries tries of 2 us at most (about a second);
+// false when it gave up.
+constexpr int kArrivalTries = 1 << 19;
+__device__ __forceinline__ bool arrivals_wait(unsigned bar, unsigned parity) {
+    for (int i = 0; i < kArrivalTries; ++i) {
+        unsigned done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, 2000;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+// A value into a CTA's shared memory, counted at that CTA's barrier when it is there.
+__device__ __forceinline__ void push_cluster(unsigned at, double v, unsigned bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(at), "d"(v), "r"(bar)
+                 : "memory");
 }
 
 // Arrives at a grid barrier and waits until `goal` arrivals (monotonic, wrap-safe). False when
@@ -169,7 +209,12 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
     double* scratch = parts + 6 * kClusterMax;
     double* totals = scratch + 3 * 32;
     int* alive = reinterpret_cast<int*>(totals + 3);
-    double* vals = totals + 4;
+    double* bars = totals + 4;  // kCluster: a barrier a buffer of the halo, then of the partial sums
+    double4* steps = reinterpret_cast<double4*>(bars + 4);
+    // x, p and s, which a round needs once, where the polynomial's steps need their registers.
+    constexpr bool kFar = far_vectors(R, CHEB);
+    double* far = bars + 4 + 4 * kChebyshevDegree;
+    double* vals = far + (kFar ? 3 * S : 0);
     const int more = a.width - E;
     int2* push = reinterpret_cast<int2*>(vals + (size_t)more * S);  // (own row, address); kCluster
     int* table = reinterpret_cast<int*>(push + (FORM == kCluster ? a.pushes : 0));
@@ -180,6 +225,12 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
     unsigned goal = 0;  // grid arrivals due
     bool ok = true, pulls = false;
     int pushed = 0;
+    // kCluster: exchanges so far of the published vector and of partial sums (each alternates between
+    // two buffers and their barriers, and a barrier between its two phases), and the halo's bytes.
+    unsigned sent = 0, summed = 0, due = 0;
+    const unsigned bars_at = FORM == kCluster ? shared_address(bars) : 0u;
+    if (FORM != kGrid && cta == 0 && tid == 0) *a.abort = 0;
+    if (CHEB && tid < kChebyshevDegree - 1) steps[tid] = a.steps[tid];  // read behind the start's barriers
 
     auto barrier = [&]() {
         if (FORM == kBlock) __syncthreads();
@@ -190,9 +241,9 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
         }
     };
     // Sums over every row of the system, in two halves around a barrier: `fold` leaves the CTA's
-    // three sums where `read` finds them after the next barrier(). `slot` 0: the dots; 1: the
-    // settle check's, a maximum and a sum -- the two may wait for the same barrier. (Between two
-    // folds lies a barrier() after which the first's scratch is not read; one CTA reads it later.)
+    // three sums where `read` finds them after the next barrier(), or what stands for it (below).
+    // `slot` 0: the dots; 1: the settle check's, a maximum and a sum. (Between two folds lies a
+    // barrier after which the first's scratch is not read; one CTA reads it later.)
     auto fold = [&](double v0, double v1, double v2, int slot) {
         if (FORM == kBlock && slot == 1) __syncthreads();
         if (slot == 0) {
@@ -207,7 +258,7 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
             }
         }
         if (FORM == kBlock) return;
-        __syncthreads();
+        ok = __syncthreads_and(ok);
         if (warp != 0) return;
         if (slot == 0) {
             row_sums(scratch, 32, warps, lane, v0, v1, v2);
@@ -217,17 +268,45 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
             v2 = 0.0;
         }
         if (FORM == kCluster) {
+            const unsigned b = summed & 1u;
+            if (!pulls && lane == 0) arrivals_expect(bars_at + 8u * (2u + b), 24u * (unsigned)ctas);
             if (lane < ctas) {
-                const unsigned at = cluster_address(shared_address(parts + 3 * kClusterMax * slot + cta), lane);
-                store_cluster(at, v0);
-                store_cluster(at + 8u * kClusterMax, v1);
-                store_cluster(at + 16u * kClusterMax, v2);
+                const unsigned at = cluster_address(shared_address(parts + 3 * kClusterMax * b + cta), lane);
+                if (pulls) {
+                    store_cluster(at, v0);
+                    store_cluster(at + 8u * kClusterMax, v1);
+                    store_cluster(at + 16u * kClusterMax, v2);
+                } else {
+                    const unsigned bar = cluster_address(bars_at + 8u * (2u + b), lane);
+                    push_cluster(at, v0, bar);
+                    push_cluster(at + 8u * kClusterMax, v1, bar);
+                    push_cluster(at + 16u * kClusterMax, v2, bar);
+                }
             }
         } else if (lane == 0) {
             double* at = a.partials + (size_t)3 * ctas * slot + cta;
             __stcg(at, v0);
             __stcg(at + ctas, v1);
             __stcg(at + 2 * ctas, v2);
+        }
+    };
+    // Where the cluster's exchanges count themselves off, a wait for one stands for the barrier. A
+    // thread that gave up waits no more; the CTA agrees on `ok` behind the sums and at its next
+    // barrier of its own (fold, publish), and leaves only where it has agreed.
+    auto await_sums = [&]() {
+        if (FORM == kCluster && !pulls) {
+            ok = ok && arrivals_wait(bars_at + 8u * (2u + (summed & 1u)), (summed >> 1) & 1u);
+            ok = __syncthreads_and(ok);
+        } else {
+            barrier();
+        }
+    };
+    auto await_published = [&]() {
+        if (FORM == kCluster && !pulls) {
+            ok = ok && arrivals_wait(bars_at + 8u * (sent & 1u), (sent >> 1) & 1u);
+            ++sent;
+        } else {
+            barrier();
         }
     };
     auto read = [&](double& v0, double& v1, double& v2, int slot) {
@@ -250,7 +329,8 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
             v0 = totals[0], v1 = totals[1], v2 = totals[2];
             return;
         }
-        const double* from = FORM == kBlock ? scratch : parts + 3 * kClusterMax * slot;
+        const double* from = FORM == kBlock ? scratch : parts + 3 * kClusterMax * (summed & 1u);
+        ++summed;
         const int stride = FORM == kBlock ? 32 : kClusterMax, count = FORM == kBlock ? warps : ctas;
         if (slot == 0) {
             row_sums(from, stride, count, lane, v0, v1, v2);
@@ -261,10 +341,11 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
     };
 
     // -- the rows: their entries, r = b - A x ----------------------------------------------------
-    double x[R], r[R], p[R], s[R], u[R], inv[R], scaled[R], previous[R];
+    constexpr int N = kFar ? 1 : R;
+    double x[N], r[R], p[N], s[N], u[R], inv[R], scaled[R], previous[N];
     double value[E ? E : 1][R];
     unsigned place[E ? E : 1][R];  // a column until the places are known
-    int over = 0, span = 0;
+    int over = 0, span = kBaseEntries;
     double bb = 0.0;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
@@ -295,11 +376,16 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
         span = max(span, min(d, a.width));
         const double b = live ? a.rhs[row] : 0.0;
         bb = fma(b, b, bb);
-        x[i] = live ? a.x[row] : 0.0;
-        previous[i] = x[i];
+        const double start = live ? a.x[row] : 0.0;
+        if constexpr (kFar) {
+            far[i * T + tid] = start;
+            far[S + i * T + tid] = far[2 * S + i * T + tid] = 0.0;
+        } else {
+            x[i] = previous[i] = start;
+            p[i] = s[i] = 0.0;
+        }
         r[i] = live ? b - ax : 0.0;
         inv[i] = live ? a.inv_diag[row] : 0.0;
-        p[i] = s[i] = 0.0;
         scaled[i] = u[i] = inv[i] * r[i];
     }
     // The warp's rows are padded to one span with zero entries on a live row.
@@ -339,9 +425,14 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
     if (FORM == kCluster) {
         for (int h = tid; h < kHaloTable; h += T) table[h] = -1;
         if (tid < 4) counters[tid] = 0;
+        if (tid == 0) {
+            for (unsigned b = 0; b < 4; ++b) arrivals_init(bars_at + 8u * b);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
         for (int i = tid; i < 2 * kHalo; i += T) pub[(i / kHalo) * buffer + S + i % kHalo] = 0.0;
-        cluster_barrier();  // every CTA of the cluster runs, its table and counters are ready
+        cluster_barrier();  // every CTA of the cluster runs, its table, counters and barriers are ready
         bool pulled = false;
+        unsigned from = 0;  // the CTAs this one holds copies from
 #pragma unroll
         for (int i = 0; i < R; ++i) {
 #pragma unroll
@@ -369,19 +460,33 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
                                  "r"(table[h] - owner * S), "r"((cta << 16) | slot)
                                  : "memory");
                     taken = slot;
+                    from |= 1u << owner;
                 }
             }
             table_slot[h] = taken;
             pulled |= taken < 0;
         }
         if (over) pulled = true;  // entries read from the CSR arrays may lie anywhere
-        if (__any_sync(0xffffffffu, pulled) && lane == 0) atomicOr(&counters[2], 1);
+        from = __reduce_or_sync(0xffffffffu, from);
+        if (lane == 0 && from) atomicOr(&counters[3], (int)from);
         cluster_barrier();  // every owner's list is whole
-        pulls = counters[2] != 0;
         pushed = min(counters[1], a.pushes);
+        due = 8u * (unsigned)min(counters[0], kHalo);
+        unsigned to_whom = 0;
+        for (int q = tid; q < pushed; q += T) to_whom |= 1u << (push[q].y >> 16);
+        to_whom = __reduce_or_sync(0xffffffffu, to_whom);
+        // A CTA pushes again once it holds what it waits for: safe where those it pushes to are
+        // those it reads. One that cannot takes the whole cluster back to barriers.
+        if (lane == 0 && (to_whom & ~(unsigned)counters[3])) pulled = true;
+        if (__any_sync(0xffffffffu, pulled) && lane < ctas)
+            asm volatile("red.shared::cluster.or.b32 [%0], 1;" ::"r"(cluster_address(shared_address(counters + 2), lane))
+                         : "memory");
+        cluster_barrier();
+        pulls = counters[2] != 0;
         for (int q = tid; q < pushed; q += T) {
-            const int2 to = push[q];
+            const int2 to = push[q];  // (own row, (CTA, slot)) to (own row, slot's address | CTA in the high bits)
             push[q].y = (int)cluster_address(pub_at + 8u * (unsigned)(S + (to.y & 0xffff)), to.y >> 16);
+            push[q].x = to.x | (to.y & 0x7fff0000);
         }
         __syncthreads();
     }
@@ -407,10 +512,15 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
                 __stcg(a.published + (size_t)parity * a.n + cta * S + at, v[i]);
         }
         if (FORM == kCluster) {
-            __syncthreads();
+            ok = __syncthreads_and(ok);
+            const unsigned bar = bars_at + 8u * (sent & 1u);
+            if (!pulls && tid == 0) arrivals_expect(bar, due);
             for (int q = tid; q < pushed; q += T) {
                 const int2 to = push[q];
-                store_cluster((unsigned)to.y + 8u * (unsigned)(parity * buffer), pub[parity * buffer + to.x]);
+                const unsigned at = (unsigned)to.y + 8u * (unsigned)(parity * buffer);
+                const double v = pub[parity * buffer + (to.x & 0xffff)];
+                if (pulls) store_cluster(at, v);
+                else push_cluster(at, v, cluster_address(bar, to.x >> 16));
             }
         }
     };
@@ -437,16 +547,31 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
             }
             out[i] = even + odd;
         }
-        for (int e0 = E; e0 < span; e0 += 4) {
+        // Four rows a thread: the base entries from shared memory, all their loads ahead of the sums.
+        if (E == 0) {
 #pragma unroll
-            for (int e1 = 0; e1 < 4; ++e1) {
-                const int e = e0 + e1;
-                if (e >= span) break;
+            for (int i = 0; i < R; ++i) {
+                double v[kBaseEntries], u_of[kBaseEntries];
 #pragma unroll
-                for (int i = 0; i < R; ++i) {
-                    const int at = ((e - E) * R + i) * T + tid;
-                    out[i] = fma(vals[at], gather(places[at]), out[i]);
+                for (int e = 0; e < kBaseEntries; ++e) {
+                    const int at = (e * R + i) * T + tid;
+                    v[e] = vals[at];
+                    u_of[e] = gather(places[at]);
                 }
+                double even = 0.0, odd = 0.0;
+#pragma unroll
+                for (int e = 0; e < kBaseEntries; ++e) {
+                    if (e & 1) odd = fma(v[e], u_of[e], odd);
+                    else even = fma(v[e], u_of[e], even);
+                }
+                out[i] = even + odd;
+            }
+        }
+        for (int e = kBaseEntries; e < span; ++e) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int at = ((e - E) * R + i) * T + tid;
+                out[i] = fma(vals[at], gather(places[at]), out[i]);
             }
         }
         if (over) {
@@ -468,8 +593,8 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
         double before[R], ax[R];
 #pragma unroll
         for (int i = 0; i < R; ++i) u[i] = before[i] = scaled[i];
-        for (int index = 0; index < kChebyshevDegree - 1 && ok; ++index) {
-            const double4 st = a.steps[index];
+        for (int index = 0; index < kChebyshevDegree - 1; ++index) {
+            const double4 st = steps[index];
             const double slope = st.w * st.x;
             double base[R];  // what the step takes from the vectors it has
 #pragma unroll
@@ -482,7 +607,8 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
 #pragma unroll
             for (int i = 0; i < R; ++i) u[i] = fma(-slope * inv[i], ax[i], base[i]);
             publish(u);
-            barrier();
+            if (!ok) break;
+            await_published();
         }
     };
 
@@ -490,7 +616,8 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
     double rr0 = 0.0, unused0, unused1;
     fold(bb, 0.0, 0.0, 0);
     publish(CHEB ? scaled : u);
-    barrier();
+    await_published();
+    if (FORM == kCluster) await_sums();
     read(rr0, unused0, unused1, 0);
     barrier();  // the sums are read before the next fold writes them
     precondition();
@@ -500,7 +627,7 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
     double settle_previous = 0.0, settle_reach = 0.0, settle_checks = 0.0;
     int round = 0, iterations = 0, status = OB_STATUS_CAPPED;
     bool done = false;
-    while (!done && ok) {
+    while (!done) {
         double w[R], ag = 0.0, ad = 0.0, ar = 0.0;
         matvec(w);
 #pragma unroll
@@ -511,7 +638,7 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
         }
         double gamma, delta;
         fold(ag, ad, ar, 0);
-        barrier();
+        await_sums();
         if (!ok) break;
         read(gamma, delta, rr, 0);
         double alpha = 0.0, beta = 0.0;
@@ -540,17 +667,26 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
         if (step) {
 #pragma unroll
             for (int i = 0; i < R; ++i) {
-                p[i] = fma(beta, p[i], u[i]);
-                s[i] = fma(beta, s[i], w[i]);
-                x[i] = fma(alpha, p[i], x[i]);
-                r[i] = fma(-alpha, s[i], r[i]);
+                if constexpr (kFar) {
+                    double* at = far + i * T + tid;
+                    const double pn = fma(beta, at[S], u[i]), sn = fma(beta, at[2 * S], w[i]);
+                    at[S] = pn;
+                    at[2 * S] = sn;
+                    at[0] = fma(alpha, pn, at[0]);
+                    r[i] = fma(-alpha, sn, r[i]);
+                } else {
+                    p[i] = fma(beta, p[i], u[i]);
+                    s[i] = fma(beta, s[i], w[i]);
+                    x[i] = fma(alpha, p[i], x[i]);
+                    r[i] = fma(-alpha, s[i], r[i]);
+                }
                 scaled[i] = inv[i] * r[i];
                 if (!CHEB) u[i] = scaled[i];
             }
         }
         if (done) break;
-        const bool check = a.check_rounds > 0 && round % a.check_rounds == 0;
-        if (check) {
+        const bool check = !kFar && a.check_rounds > 0 && round % a.check_rounds == 0;
+        if constexpr (!kFar) if (check) {
             double change = 0.0, reached = 0.0;
 #pragma unroll
             for (int i = 0; i < R; ++i) {
@@ -563,8 +699,10 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
             fold(change, reached, 0.0, 1);
         }
         publish(CHEB ? scaled : u);
-        barrier();
         if (!ok) break;
+        await_published();
+        if (FORM == kCluster && check) await_sums();
+        if ((FORM == kGrid || check) && !ok) break;
         if (check) {
             double change, reached;
             read(change, reached, unused0, 1);
@@ -584,16 +722,17 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
 #pragma unroll
     for (int i = 0; i < R; ++i) {
         const int row = cta * S + i * T + tid;
-        if (row < a.n) a.x[row] = x[i];
+        if (row < a.n) a.x[row] = kFar ? far[i * T + tid] : x[kFar ? 0 : i];
     }
     if (cta == 0 && tid == 0) {
         a.state->round = round;
         a.state->iterations = iterations;
         a.state->done = 1;
-        a.state->status = ok ? status : kStatusAborted;
+        a.state->status = status;
         a.scalars->rr = rr;
         a.scalars->rr0 = rr0;
     }
+    if (!ok) atomicExch(a.abort, 1);
     if (FORM == kCluster) cluster_barrier();  // no CTA leaves while another may still read its memory
 }
 
