@@ -1369,71 +1369,108 @@ __device__ __forceinline__ void fma4(float a, const float4& v, float4& acc) {
     acc.w = fmaf(a, v.w, acc.w);
 }
 
-// Row `row` of M x over a row group: lane reads columns [4 lane, 4 lane + 4).
+// The lanes of a row: `split` groups (a power of two, G * split <= 32) of G lanes, lane c of a group
+// on columns [4 c, 4 c + 4), group g on entries g, g + split, .. of the row.
+struct RowLanes {
+    int lane, part, row, stride;  // row: the team's first row, stride: rows between its rows
+};
+__device__ __forceinline__ RowLanes row_lanes(int G, int split) {
+    const int team = G * split, teams = blockDim.x / team;
+    return RowLanes{(int)threadIdx.x % G, (int)threadIdx.x % team / G,
+                    (int)(blockIdx.x * teams + threadIdx.x / team), (int)gridDim.x * teams};
+}
+
+__device__ __forceinline__ float4 shuffle_xor(unsigned mask, const float4& v, int m) {
+    return make_float4(__shfl_xor_sync(mask, v.x, m), __shfl_xor_sync(mask, v.y, m), __shfl_xor_sync(mask, v.z, m),
+                       __shfl_xor_sync(mask, v.w, m));
+}
+
+// Row `row` of M x over its lanes (every lane of the row gets the sum).
 __device__ __forceinline__ float4 row_product(const int* __restrict__ off, const int* __restrict__ col,
-                                              const float* __restrict__ val,
-                                              const float4* __restrict__ x, int G, int row,
-                                              int lane) {
+                                              const float* __restrict__ val, const float4* __restrict__ x, int G,
+                                              int split, int row, int lane, int part) {
     float4 acc = f4(0.0f);
     const int end = off[row + 1];
-    int e = off[row];
+    int e = off[row] + part;
     // Four entries' places, then their values, in flight: a row's time is its loads' latency.
-    for (; e + 3 < end; e += 4) {
+    for (; e + 3 * split < end; e += 4 * split) {
         int j[4];
         float a[4];
         float4 v[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) j[q] = col[e + q], a[q] = val[e + q];
+        for (int q = 0; q < 4; ++q) j[q] = col[e + q * split], a[q] = val[e + q * split];
 #pragma unroll
         for (int q = 0; q < 4; ++q) v[q] = x[(size_t)j[q] * G + lane];
 #pragma unroll
         for (int q = 0; q < 4; ++q) fma4(a[q], v[q], acc);
     }
-    for (; e + 1 < end; e += 2) {
-        const int j0 = col[e], j1 = col[e + 1];
-        const float a0 = val[e], a1 = val[e + 1];
+    for (; e + split < end; e += 2 * split) {
+        const int j0 = col[e], j1 = col[e + split];
+        const float a0 = val[e], a1 = val[e + split];
         const float4 v0 = x[(size_t)j0 * G + lane];
         const float4 v1 = x[(size_t)j1 * G + lane];
         fma4(a0, v0, acc);
         fma4(a1, v1, acc);
     }
     if (e < end) fma4(val[e], x[(size_t)col[e] * G + lane], acc);
+    if (split == 1) return acc;
+    const int team = G * split, at = threadIdx.x & 31 & ~(team - 1);
+    const unsigned mask = team == 32 ? 0xffffffffu : ((1u << team) - 1u) << at;
+    for (int m = G; m < team; m <<= 1) {
+        const float4 o = shuffle_xor(mask, acc, m);
+        acc.x += o.x;
+        acc.y += o.y;
+        acc.z += o.z;
+        acc.w += o.w;
+    }
     return acc;
 }
 
-// Per-thread column partial sums (4 columns a lane) -> block partials[block][kp] (fixed tree).
+// Per-thread column partial sums (4 columns a lane) -> block partials[block][kp] (fixed tree: the
+// lanes of a warp that share a column by shuffles, then the warps in order).
 __device__ __forceinline__ void store_column_partials(double4 mine, int G, double* partials,
                                                       double* smem) {
-    // smem: [groups][kp] doubles; groups = blockDim / G.
-    const int lane = threadIdx.x % G, group = threadIdx.x / G, kp = 4 * G;
-    const int groups = blockDim.x / G;
-    double* slot = smem + (size_t)group * kp + 4 * lane;
-    slot[0] = mine.x;
-    slot[1] = mine.y;
-    slot[2] = mine.z;
-    slot[3] = mine.w;
+    // smem: [warps][kp] doubles.
+    const int lane = threadIdx.x % G, warp = threadIdx.x >> 5, kp = 4 * G;
+    for (int m = G; m < 32; m <<= 1) {
+        mine.x += __shfl_xor_sync(0xffffffffu, mine.x, m);
+        mine.y += __shfl_xor_sync(0xffffffffu, mine.y, m);
+        mine.z += __shfl_xor_sync(0xffffffffu, mine.z, m);
+        mine.w += __shfl_xor_sync(0xffffffffu, mine.w, m);
+    }
+    if ((int)(threadIdx.x & 31) < G) {
+        double* slot = smem + (size_t)warp * kp + 4 * lane;
+        slot[0] = mine.x;
+        slot[1] = mine.y;
+        slot[2] = mine.z;
+        slot[3] = mine.w;
+    }
     __syncthreads();
     for (int c = threadIdx.x; c < kp; c += blockDim.x) {
         double s = 0.0;
-        for (int g = 0; g < groups; ++g) s += smem[(size_t)g * kp + c];
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; ++w) s += smem[(size_t)w * kp + c];
         partials[(size_t)blockIdx.x * kp + c] = s;
     }
     // Every writer publishes its partials before the block takes its last-block ticket.
     __threadfence();
 }
 
-// Last block: sums partials[blocks][kp] per column in block order into smem[kp].
+// Last block: sums partials[blocks][kp] per column (fixed order) into smem[blockDim + c].
 __device__ __forceinline__ void fold_columns(const double* partials, int blocks, int kp, double* smem) {
     const int subsets = blockDim.x / kp;  // kp divides blockDim (both powers of two, kp <= 128)
     const int c = threadIdx.x % kp, s = threadIdx.x / kp;
     double sum = 0.0;
+#pragma unroll 4
     for (int b = s; b < blocks; b += subsets) sum += partials[(size_t)b * kp + c];
+    for (int m = kp; m < 32; m <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
     __syncthreads();
     smem[threadIdx.x] = sum;
     __syncthreads();
     if (threadIdx.x < kp) {
+        // A column's sums stand at every kp-th thread, alike within a warp where kp < 32.
         double total = 0.0;
-        for (int t = 0; t < subsets; ++t) total += smem[t * kp + threadIdx.x];
+        for (int t = threadIdx.x; t < blockDim.x; t += max(kp, 32)) total += smem[t];
         smem[blockDim.x + threadIdx.x] = total;
     }
     __syncthreads();
@@ -1482,15 +1519,17 @@ __global__ void __launch_bounds__(kThreads) scale_kernel(int n, int G, const flo
 // The first two sweeps from zero in one: x = d .* b, then x + d .* (b - A x) = d .* (2 b - (A D) b)
 // with the columns of A scaled by d once at set-up (column_scale_kernel): b alone is gathered, and
 // the first sweep's write and second read of a vector (and its launch) go.
-__global__ void __launch_bounds__(kThreads) first_sweeps_kernel(int n, int G, const int* __restrict__ off,
+__global__ void __launch_bounds__(kThreads) first_sweeps_kernel(int n, int G, int split, const int* __restrict__ off,
                                                                 const int* __restrict__ col,
                                                                 const float* __restrict__ scaled,
                                                                 const float* __restrict__ d,
                                                                 const float4* __restrict__ b,
                                                                 float4* __restrict__ x) {
-    const int lane = threadIdx.x % G, groups = blockDim.x / G;
-    for (int row = blockIdx.x * groups + threadIdx.x / G; row < n; row += gridDim.x * groups) {
-        const float4 ax = row_product(off, col, scaled, b, G, row, lane);
+    const RowLanes at = row_lanes(G, split);
+    const int lane = at.lane;
+    for (int row = at.row; row < n; row += at.stride) {
+        const float4 ax = row_product(off, col, scaled, b, G, split, row, lane, at.part);
+        if (at.part) continue;
         const float4 v = b[(size_t)row * G + lane];
         const float s = d[row];
         x[(size_t)row * G + lane] = make_float4(s * (fmaf(2.0f, v.x, -ax.x)), s * (fmaf(2.0f, v.y, -ax.y)),
@@ -1506,7 +1545,7 @@ __global__ void column_scale_kernel(long long nnz, const int* __restrict__ col, 
 
 // One damped-Jacobi sweep x_out = x_in + d .* (b - A x_in); kDot adds the top level's r.z fold.
 template <bool kDot>
-__global__ void __launch_bounds__(kThreads) sweep_kernel(int n, int G, const int* __restrict__ off,
+__global__ void __launch_bounds__(kThreads) sweep_kernel(int n, int G, int split, const int* __restrict__ off,
                                                          const int* __restrict__ col,
                                                          const float* __restrict__ val,
                                                          const float* __restrict__ d,
@@ -1515,10 +1554,12 @@ __global__ void __launch_bounds__(kThreads) sweep_kernel(int n, int G, const int
                                                          float4* __restrict__ x_out, double* partials,
                                                          unsigned int* counter, ColumnState* cols) {
     extern __shared__ double smem[];
-    const int lane = threadIdx.x % G, groups = blockDim.x / G;
+    const RowLanes at = row_lanes(G, split);
+    const int lane = at.lane;
     double4 mine = make_double4(0, 0, 0, 0);
-    for (int row = blockIdx.x * groups + threadIdx.x / G; row < n; row += gridDim.x * groups) {
-        const float4 ax = row_product(off, col, val, x_in, G, row, lane);
+    for (int row = at.row; row < n; row += at.stride) {
+        const float4 ax = row_product(off, col, val, x_in, G, split, row, lane, at.part);
+        if (at.part) continue;
         const float4 bv = b[(size_t)row * G + lane];
         const float4 xv = x_in[(size_t)row * G + lane];
         const float s = d[row];
@@ -1585,15 +1626,17 @@ __global__ void __launch_bounds__(kThreads) column_dot_kernel(int n, int G, cons
 }
 
 // r = b - A x.
-__global__ void __launch_bounds__(kThreads) residual_kernel(int n, int G, const int* __restrict__ off,
+__global__ void __launch_bounds__(kThreads) residual_kernel(int n, int G, int split, const int* __restrict__ off,
                                                             const int* __restrict__ col,
                                                             const float* __restrict__ val,
                                                             const float4* __restrict__ b,
                                                             const float4* __restrict__ x,
                                                             float4* __restrict__ r) {
-    const int lane = threadIdx.x % G, groups = blockDim.x / G;
-    for (int row = blockIdx.x * groups + threadIdx.x / G; row < n; row += gridDim.x * groups) {
-        const float4 ax = row_product(off, col, val, x, G, row, lane);
+    const RowLanes at = row_lanes(G, split);
+    const int lane = at.lane;
+    for (int row = at.row; row < n; row += at.stride) {
+        const float4 ax = row_product(off, col, val, x, G, split, row, lane, at.part);
+        if (at.part) continue;
         const float4 bv = b[(size_t)row * G + lane];
         r[(size_t)row * G + lane] = make_float4(bv.x - ax.x, bv.y - ax.y, bv.z - ax.z, bv.w - ax.w);
     }
@@ -1601,14 +1644,16 @@ __global__ void __launch_bounds__(kThreads) residual_kernel(int n, int G, const 
 
 // y = M x (kAccumulate: y += M x), M rectangular (restriction or prolongation).
 template <bool kAccumulate>
-__global__ void __launch_bounds__(kThreads) spmm_kernel(int rows, int G, const int* __restrict__ off,
+__global__ void __launch_bounds__(kThreads) spmm_kernel(int rows, int G, int split, const int* __restrict__ off,
                                                         const int* __restrict__ col,
                                                         const float* __restrict__ val,
                                                         const float4* __restrict__ x,
                                                         float4* __restrict__ y) {
-    const int lane = threadIdx.x % G, groups = blockDim.x / G;
-    for (int row = blockIdx.x * groups + threadIdx.x / G; row < rows; row += gridDim.x * groups) {
-        float4 v = row_product(off, col, val, x, G, row, lane);
+    const RowLanes at = row_lanes(G, split);
+    const int lane = at.lane;
+    for (int row = at.row; row < rows; row += at.stride) {
+        float4 v = row_product(off, col, val, x, G, split, row, lane, at.part);
+        if (at.part) continue;
         if (kAccumulate) {
             const float4 o = y[(size_t)row * G + lane];
             v.x += o.x;
@@ -1633,13 +1678,20 @@ __global__ void __launch_bounds__(kThreads) coarse_kernel(int rows, int G, int m
     float4 acc = f4(0.0f);
     if (slot >= 0)
         for (int t = part; t < m; t += parts) fma4(inverse[(size_t)slot * m + t], b[(size_t)active[t] * G + lane], acc);
-    float* fs = reinterpret_cast<float*>(smem);
-    reinterpret_cast<float4*>(fs)[threadIdx.x] = acc;
+    for (int m = G; m < 32; m <<= 1) {
+        const float4 o = shuffle_xor(0xffffffffu, acc, m);
+        acc.x += o.x;
+        acc.y += o.y;
+        acc.z += o.z;
+        acc.w += o.w;
+    }
+    float4* warps = reinterpret_cast<float4*>(smem);
+    if ((int)(threadIdx.x & 31) < G) warps[(threadIdx.x >> 5) * G + lane] = acc;
     __syncthreads();
     if (part == 0) {
         float4 total = f4(0.0f);
-        for (int p = 0; p < parts; ++p) {
-            const float4 v = reinterpret_cast<float4*>(fs)[p * G + lane];
+        for (int w = 0; w < kThreads / 32; ++w) {
+            const float4 v = warps[w * G + lane];
             total.x += v.x;
             total.y += v.y;
             total.z += v.z;
@@ -1651,7 +1703,7 @@ __global__ void __launch_bounds__(kThreads) coarse_kernel(int rows, int G, int m
 
 // q = A z + beta q, p = z + beta p (the CG direction update folded into the product), and the
 // column dots p.q folded into alpha = rho / p.q by the last block.
-__global__ void __launch_bounds__(kThreads) direction_kernel(int n, int G, const int* __restrict__ off,
+__global__ void __launch_bounds__(kThreads) direction_kernel(int n, int G, int split, const int* __restrict__ off,
                                                              const int* __restrict__ col,
                                                              const float* __restrict__ val,
                                                              const float4* __restrict__ z,
@@ -1659,12 +1711,14 @@ __global__ void __launch_bounds__(kThreads) direction_kernel(int n, int G, const
                                                              double* partials, unsigned int* counter,
                                                              ColumnState* cols) {
     extern __shared__ double smem[];
-    const int lane = threadIdx.x % G, groups = blockDim.x / G;
+    const RowLanes team = row_lanes(G, split);
+    const int lane = team.lane;
     const float4 beta = make_float4((float)cols[4 * lane].beta, (float)cols[4 * lane + 1].beta,
                                     (float)cols[4 * lane + 2].beta, (float)cols[4 * lane + 3].beta);
     double4 mine = make_double4(0, 0, 0, 0);
-    for (int row = blockIdx.x * groups + threadIdx.x / G; row < n; row += gridDim.x * groups) {
-        const float4 az = row_product(off, col, val, z, G, row, lane);
+    for (int row = team.row; row < n; row += team.stride) {
+        const float4 az = row_product(off, col, val, z, G, split, row, lane, team.part);
+        if (team.part) continue;
         const size_t at = (size_t)row * G + lane;
         const float4 zv = z[at], pv = p[at], qv = q[at];
         float4 pn, qn;
@@ -1932,6 +1986,19 @@ int grid_for(long long threads) {
     return (int)std::max(1LL, std::min(cap, (threads + kThreads - 1) / kThreads));
 }
 
+// The lane groups a row of `nnz` / rows entries is split over: doubled while the launch has fewer
+// threads than the device holds and a lane at least two entries. A small level is bound by its rows'
+// serial chains (one group a row leaves 3 306 rows of ~30 entries, 8 columns, on 6 612 threads),
+// a large one has the threads without. With the folds below taken by shuffles and the reducing
+// kernels' grids at their occupancy, 8 queries on a 262 k-vertex hierarchy went from 8.13 to
+// 6.80 ms, a 64-column V-cycle from 425 to 394 us.
+int row_split(long long rows, long long nnz, int G) {
+    const long long resident = 2048LL * sm_count();
+    int split = 1;
+    while (2 * split * G <= 32 && rows * G * split < resident && nnz >= 4LL * split * rows) split *= 2;
+    return split;
+}
+
 size_t partial_smem(int G) { return sizeof(double) * std::max(2 * kThreads, (kThreads / G) * 4 * G); }
 
 int padded_columns(int k) {
@@ -1971,7 +2038,9 @@ int ensure_work(Amg* M, int kp, Work** out, cudaStream_t stream) {
         (st = alloc(f, (void**)&W->p)) || (st = alloc(f, (void**)&W->q)) || (st = alloc(dd, (void**)&W->b64)) ||
         (st = alloc(dd, (void**)&W->x64)) || (st = alloc(dd, (void**)&W->r64)))
         return st;
-    W->blocks = 2 * sm_count();
+    // The reducing kernels: as many blocks as an SM holds at their registers where the columns are few,
+    // fewer where the last block would have as many partials a column to fold by fewer threads.
+    W->blocks = (kp <= 16 ? 5 : kp <= 32 ? 4 : 2) * sm_count();
     if ((st = alloc(sizeof(double) * (size_t)W->blocks * kp, (void**)&W->partials)) ||
         (st = alloc(sizeof(unsigned int) * 8, (void**)&W->counters)) ||
         (st = alloc(sizeof(ColumnState) * kp, (void**)&W->cols)) ||
@@ -2018,32 +2087,34 @@ int enqueue_cycle(Amg* M, Work* W, size_t l, const float* b, float* out, bool to
         }
         return OB_OK;
     }
-    const int grid = grid_for((long long)L.n * G);
+    const int split = row_split(L.n, L.nnz, G), grid = grid_for((long long)L.n * G * split);
     float* other = W->y[l];
     // Pre-smoothing: both sweeps from zero at once.
-    first_sweeps_kernel<<<grid, kThreads, 0, stream>>>(L.n, G, L.off, L.col, L.scaled, L.damped, f4p(b), f4m(out));
+    first_sweeps_kernel<<<grid, kThreads, 0, stream>>>(L.n, G, split, L.off, L.col, L.scaled, L.damped, f4p(b), f4m(out));
     OB_CHECK_LAUNCH("amg first sweeps");
-    residual_kernel<<<grid, kThreads, 0, stream>>>(L.n, G, L.off, L.col, L.val, f4p(b), f4p(out), f4m(W->r[l]));
+    residual_kernel<<<grid, kThreads, 0, stream>>>(L.n, G, split, L.off, L.col, L.val, f4p(b), f4p(out), f4m(W->r[l]));
     OB_CHECK_LAUNCH("amg residual");
     const DeviceLevel& C = M->levels[l + 1];
-    spmm_kernel<false><<<grid_for((long long)C.n * G), kThreads, 0, stream>>>(
-        C.n, G, L.roff, L.rcol, L.rval, f4p(W->r[l]), f4m(W->b[l + 1]));
+    const int r_split = row_split(C.n, L.rnnz, G), p_split = row_split(L.n, L.pnnz, G);
+    spmm_kernel<false><<<grid_for((long long)C.n * G * r_split), kThreads, 0, stream>>>(
+        C.n, G, r_split, L.roff, L.rcol, L.rval, f4p(W->r[l]), f4m(W->b[l + 1]));
     OB_CHECK_LAUNCH("amg restrict");
     *launches += 3;
     int st = enqueue_cycle(M, W, l + 1, W->b[l + 1], W->x[l + 1], false, stream, launches);
     if (st) return st;
-    spmm_kernel<true><<<grid, kThreads, 0, stream>>>(L.n, G, L.poff, L.pcol, L.pval, f4p(W->x[l + 1]), f4m(out));
+    spmm_kernel<true><<<grid_for((long long)L.n * G * p_split), kThreads, 0, stream>>>(L.n, G, p_split, L.poff, L.pcol,
+                                                                                       L.pval, f4p(W->x[l + 1]), f4m(out));
     OB_CHECK_LAUNCH("amg prolong");
     // Post-smoothing: out -> other -> out.
-    sweep_kernel<false><<<grid, kThreads, 0, stream>>>(L.n, G, L.off, L.col, L.val, L.damped, f4p(b),
+    sweep_kernel<false><<<grid, kThreads, 0, stream>>>(L.n, G, split, L.off, L.col, L.val, L.damped, f4p(b),
                                                         f4p(out), f4m(other), nullptr, nullptr, nullptr);
     OB_CHECK_LAUNCH("amg sweep");
     if (top_dot)
-        sweep_kernel<true><<<W->blocks, kThreads, smem, stream>>>(L.n, G, L.off, L.col, L.val, L.damped, f4p(b),
+        sweep_kernel<true><<<W->blocks, kThreads, smem, stream>>>(L.n, G, split, L.off, L.col, L.val, L.damped, f4p(b),
                                                                   f4p(other), f4m(out), W->partials,
                                                                   W->counters + 0, W->cols);
     else
-        sweep_kernel<false><<<grid, kThreads, 0, stream>>>(L.n, G, L.off, L.col, L.val, L.damped, f4p(b),
+        sweep_kernel<false><<<grid, kThreads, 0, stream>>>(L.n, G, split, L.off, L.col, L.val, L.damped, f4p(b),
                                                             f4p(other), f4m(out), nullptr, nullptr, nullptr);
     OB_CHECK_LAUNCH("amg sweep");
     *launches += 3;
@@ -2057,7 +2128,8 @@ int enqueue_iteration(Amg* M, Work* W, cudaStream_t stream, int* launches) {
     const DeviceLevel& L = M->levels[0];
     auto f4p = [](const float* p) { return reinterpret_cast<const float4*>(p); };
     auto f4m = [](float* p) { return reinterpret_cast<float4*>(p); };
-    direction_kernel<<<W->blocks, kThreads, smem, stream>>>(M->n, G, L.off, L.col, L.val, f4p(W->z), f4m(W->p),
+    direction_kernel<<<W->blocks, kThreads, smem, stream>>>(M->n, G, row_split(M->n, L.nnz, G), L.off, L.col,
+                                                            L.val, f4p(W->z), f4m(W->p),
                                                             f4m(W->q), W->partials, W->counters + 1, W->cols);
     OB_CHECK_LAUNCH("amg direction");
     update_kernel<<<W->blocks, kThreads, smem, stream>>>(M->n, G, f4p(W->p), f4p(W->q), f4m(W->d), f4m(W->res),
@@ -2417,7 +2489,9 @@ int ob_amg_time_kernels(void* amg, int k, int reps, float* ms, long long* bytes,
     OB_CUDA(cudaMemsetAsync(W->r[0], 0, vec, stream));
     OB_CUDA(cudaMemsetAsync(W->x[1], 0, coarse, stream));
     const int G = W->G;
-    const int grid = grid_for((long long)L.n * G), coarse_grid = grid_for((long long)C.n * G);
+    const int split = row_split(L.n, L.nnz, G), r_split = row_split(C.n, L.rnnz, G), p_split = row_split(L.n, L.pnnz, G);
+    const int grid = grid_for((long long)L.n * G * split), coarse_grid = grid_for((long long)C.n * G * r_split),
+              prolong_grid = grid_for((long long)L.n * G * p_split);
     auto f4p = [](const float* p) { return reinterpret_cast<const float4*>(p); };
     auto f4m = [](float* p) { return reinterpret_cast<float4*>(p); };
     const long long matrix = 4LL * (L.n + 1) + 8LL * L.nnz;
@@ -2432,20 +2506,20 @@ int ob_amg_time_kernels(void* amg, int k, int reps, float* ms, long long* bytes,
     auto kernel = [&](int which) {
         switch (which) {
             case 0:
-                sweep_kernel<false><<<grid, kThreads, 0, stream>>>(L.n, G, L.off, L.col, L.val, L.damped, f4p(W->res),
+                sweep_kernel<false><<<grid, kThreads, 0, stream>>>(L.n, G, split, L.off, L.col, L.val, L.damped, f4p(W->res),
                                                                     f4p(W->y[0]), f4m(W->z), nullptr, nullptr,
                                                                     nullptr);
                 break;
             case 1:
-                residual_kernel<<<grid, kThreads, 0, stream>>>(L.n, G, L.off, L.col, L.val, f4p(W->res),
+                residual_kernel<<<grid, kThreads, 0, stream>>>(L.n, G, split, L.off, L.col, L.val, f4p(W->res),
                                                                f4p(W->z), f4m(W->r[0]));
                 break;
             case 2:
-                spmm_kernel<false><<<coarse_grid, kThreads, 0, stream>>>(C.n, G, L.roff, L.rcol, L.rval,
+                spmm_kernel<false><<<coarse_grid, kThreads, 0, stream>>>(C.n, G, r_split, L.roff, L.rcol, L.rval,
                                                                          f4p(W->r[0]), f4m(W->b[1]));
                 break;
             case 3:
-                spmm_kernel<true><<<grid, kThreads, 0, stream>>>(L.n, G, L.poff, L.pcol, L.pval, f4p(W->x[1]),
+                spmm_kernel<true><<<prolong_grid, kThreads, 0, stream>>>(L.n, G, p_split, L.poff, L.pcol, L.pval, f4p(W->x[1]),
                                                                  f4m(W->z));
                 break;
             default: {
