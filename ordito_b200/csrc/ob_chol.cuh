@@ -2,6 +2,7 @@
 // ob_chol_factor.cu: the numeric factorisation on the device).
 #pragma once
 
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -80,10 +81,17 @@ enum PinMode : int { kPinNone = 0, kPinAll = 1, kPinZeroSum = 2 };
 
 // Numeric factorisation of sign * values (CSR over the analysis' pattern, old numbering) on the
 // device, multifrontal over the tree, level by level: writes every supernode's [L11^-1; G] block
-// into vals (laid out by block_layout, zeroed here) and pinned[n] (new numbering). Returns
-// OB_ERR_INDEFINITE on a non-positive pivot (read back once at the end).
-int device_factor(CholAnalysis& A, const double* values, double sign, int pin_mode, double* vals,
-                  char* pinned, cudaStream_t stream);
+// into vals (laid out by block_layout, zeroed here) and pinned[n] (new numbering), and the solves'
+// tables of the analysis into `tables`. `meanwhile` is the host's own work on the factor, run once
+// everything is enqueued. Returns OB_ERR_INDEFINITE on a non-positive pivot (read back at the end).
+struct FactorTables {
+    long long n_vals;  // values in vals
+    int* idx;          // the row lists (BlockLayout)
+    int *perm, *iperm, *node_of;  // per row
+    int* parent;                  // per supernode
+};
+int device_factor(CholAnalysis& A, const double* values, double sign, int pin_mode, double* vals, char* pinned,
+                  const FactorTables& tables, const std::function<int()>& meanwhile, cudaStream_t stream);
 
 // D (8 x 8) += A (8 x 4) B (4 x 8) in float64 on the tensor cores (mma.sync m8n8k4 .f64, the
 // float64 matrix instruction sm_100 offers). Fragments: a = A[lane / 4][lane % 4],

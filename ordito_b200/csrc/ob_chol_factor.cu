@@ -10,8 +10,8 @@
 // front entry is summed in the same order on every run: no atomics). Its own columns are then
 // eliminated in panels of 64:
 //
-//   K1  the panel's diagonal block D (b x b, b <= 64): Cholesky and its inverse D^-1, in shared
-//       memory (one CTA a front); D^-1 goes straight into the stored block.
+//   K1  the panel's diagonal block D (b x b, b <= 64): Cholesky and its inverse D^-1, in registers
+//       (one CTA a front); D^-1 goes straight into the stored block.
 //   K2  the panel below the diagonal, L = F D^-T (in place), and the rows of the panel in the
 //       stored block, Z_p = D^-1 Z_p (in place).
 //   K3  the trailing update, F[j1:, j1:] -= L L^T (lower tiles), and Z[j1:, :j1] -= L Z_p.
@@ -82,6 +82,8 @@ struct FactorPlan {
     int* component = nullptr;        // per old row
     char* component_last = nullptr;  // per old row
     int* perm = nullptr;             // new -> old
+    int* iperm = nullptr;            // old -> new
+    int* node_of = nullptr;          // per new column: its supernode
     int* offsets = nullptr;          // the operator's row offsets (old numbering)
     // Per supernode: front offset, front leading dimension, own columns, off-diagonal rows, and
     // where its off-diagonal rows' positions in its parent's front start in `rel`.
@@ -91,6 +93,12 @@ struct FactorPlan {
     int* noff = nullptr;
     int* rel_at = nullptr;
     int* rel = nullptr;
+    int* rows = nullptr;  // the off-diagonal rows themselves, starting as in `rel`
+    // Per supernode: first column, parent, and where a factor's row lists of it start (BlockLayout).
+    int* start = nullptr;
+    int* parent = nullptr;
+    int* rows_at = nullptr;
+    int n_nodes = 0;
     struct Launch {
         int kind;
         const void* tasks;
@@ -224,6 +232,27 @@ __global__ void diag_dest_kernel(int n, const PlanTree T, long long* __restrict_
     diag_dest[j] = T.front_at[s] + lj * T.fld[s] + lj;
 }
 
+// A factor's row lists (a warp a supernode): its off-diagonal rows (rows of B), then the backward
+// product's inputs, its own rows of Y and its off-diagonal rows of X, in the stacked [B; Y; X].
+// The host filled and uploaded these lists before (as much as 60 MB at 2.6 M vertices), and made the
+// tile lists after the factorisation instead of beside it: a factor of the 2.6 M-vertex torus
+// took 102 ms where it now takes 57, of the 131k torus 3.81 and 3.08.
+__global__ void row_lists_kernel(int ns, int n, const int* __restrict__ start, const int* __restrict__ nc,
+                                 const int* __restrict__ row_at, const int* __restrict__ rows,
+                                 const int* __restrict__ rows_at, int* __restrict__ idx) {
+    const int s = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (s >= ns) return;
+    const int count = nc[s], first = row_at[s], noff = row_at[s + 1] - first;
+    int* off = idx + rows_at[s];
+    int* back = off + noff;
+    for (int i = lane; i < count; i += 32) back[i] = n + start[s] + i;
+    for (int i = lane; i < noff; i += 32) {
+        const int r = rows[first + i];
+        off[i] = r;
+        back[count + i] = 2 * n + r;
+    }
+}
+
 // The device tables and the launch schedule of an analysis (once). The per-entry and per-row
 // tables are built on the device from the tree; the host builds the launch schedule.
 int build_plan(const CholAnalysis& A, FactorPlan* P, cudaStream_t stream) {
@@ -256,10 +285,14 @@ int build_plan(const CholAnalysis& A, FactorPlan* P, cudaStream_t stream) {
     for (int i = 0; i < n; ++i) component_last[i] = (char)A.component_last[i];
     const long long nnz = A.offsets[n];
     P->n_entries = nnz;
+    P->n_nodes = ns;
     int st = OB_OK;
     if ((st = upload(P, &P->component, A.component, stream)) ||
         (st = upload(P, &P->component_last, component_last, stream)) ||
-        (st = upload(P, &P->perm, A.perm, stream)) || (st = upload(P, &P->offsets, A.offsets, stream)) ||
+        (st = upload(P, &P->perm, A.perm, stream)) || (st = upload(P, &P->iperm, A.iperm, stream)) ||
+        (st = upload(P, &P->offsets, A.offsets, stream)) || (st = upload(P, &P->start, start, stream)) ||
+        (st = upload(P, &P->parent, parent, stream)) || (st = upload(P, &P->rows, rows, stream)) ||
+        (st = upload(P, &P->rows_at, layout.rows_at, stream)) || (st = allocate(P, &P->node_of, (size_t)n, stream)) ||
         (st = upload(P, &P->front_at, front_at, stream)) ||
         (st = upload(P, &P->fld, fld, stream)) || (st = upload(P, &P->nc, nc, stream)) ||
         (st = upload(P, &P->noff, noff, stream)) || (st = upload(P, &P->rel_at, row_at, stream)) ||
@@ -270,26 +303,19 @@ int build_plan(const CholAnalysis& A, FactorPlan* P, cudaStream_t stream) {
         (st = allocate(P, &P->diag_dest, (size_t)n, stream)))
         return st;
     {
-        // The tree and the pattern, for the table kernels only.
+        // The pattern's columns, for the table kernels only.
         Scratch scratch(stream);
-        const int *d_start = nullptr, *d_parent = nullptr, *d_rows = nullptr, *d_iperm = nullptr,
-                  *d_columns = nullptr;
-        int* d_node_of = scratch.take<int>((size_t)n);
-        if ((st = scratch.commit()) || (st = upload_scratch(scratch, &d_start, start, stream)) ||
-            (st = upload_scratch(scratch, &d_parent, parent, stream)) ||
-            (st = upload_scratch(scratch, &d_rows, rows, stream)) ||
-            (st = upload_scratch(scratch, &d_iperm, A.iperm, stream)) ||
-            (st = upload_scratch(scratch, &d_columns, A.columns, stream)))
-            return st;
-        const PlanTree T{d_start, P->nc, P->front_at, P->fld, P->rel_at, d_rows, d_node_of};
+        const int* d_columns = nullptr;
+        if ((st = upload_scratch(scratch, &d_columns, A.columns, stream))) return st;
+        const PlanTree T{P->start, P->nc, P->front_at, P->fld, P->rel_at, P->rows, P->node_of};
         const int threads = 256;
-        node_of_kernel<<<ceil_div(32LL * ns, threads), threads, 0, stream>>>(ns, d_start, P->nc, d_node_of);
+        node_of_kernel<<<ceil_div(32LL * ns, threads), threads, 0, stream>>>(ns, P->start, P->nc, P->node_of);
         OB_CHECK_LAUNCH("chol plan node_of");
         OB_CUDA(cudaMemsetAsync(P->diag_pos, 0xFF, sizeof(int) * (size_t)n, stream));
         entries_kernel<<<ceil_div((long long)kEntryLanes * n, threads), threads, 0, stream>>>(
-            n, P->offsets, d_columns, d_iperm, T, P->entry_dest, P->entry_rc, P->diag_pos);
+            n, P->offsets, d_columns, P->iperm, T, P->entry_dest, P->entry_rc, P->diag_pos);
         OB_CHECK_LAUNCH("chol plan entries");
-        rel_kernel<<<ceil_div(32LL * ns, threads), threads, 0, stream>>>(ns, d_parent, T, P->rel);
+        rel_kernel<<<ceil_div(32LL * ns, threads), threads, 0, stream>>>(ns, P->parent, T, P->rel);
         OB_CHECK_LAUNCH("chol plan rel");
         diag_dest_kernel<<<ceil_div(n, threads), threads, 0, stream>>>(n, T, P->diag_dest);
         OB_CHECK_LAUNCH("chol plan diagonal slots");
@@ -757,7 +783,7 @@ int allow_product_memory() {
 }  // namespace
 
 int device_factor(CholAnalysis& A, const double* values, double sign, int pin_mode, double* vals, char* pinned,
-                  cudaStream_t stream) {
+                  const FactorTables& tables, const std::function<int()>& meanwhile, cudaStream_t stream) {
     if (int st = allow_product_memory()) return st;
     FactorPlan* P = nullptr;
     {
@@ -781,7 +807,8 @@ int device_factor(CholAnalysis& A, const double* values, double sign, int pin_mo
         P = A.plan;
     }
     const int n = A.n;
-    const long long vals_count = block_layout(A).total;
+    const long long vals_count = tables.n_vals;
+    const int ns = P->n_nodes;
     Scratch scratch(stream);
     double* fronts = scratch.take<double>((size_t)P->front_total);
     int* bad = scratch.take<int>((size_t)std::max(A.n_components, 1));
@@ -792,6 +819,19 @@ int device_factor(CholAnalysis& A, const double* values, double sign, int pin_mo
     OB_CUDA(cudaMemsetAsync(bad, 0, sizeof(int) * (size_t)std::max(A.n_components, 1), stream));
     OB_CUDA(cudaMemsetAsync(status, 0, sizeof(int), stream));
     const int threads = 256;
+    const struct {
+        int *to, *from;
+        int count;
+    } copies[] = {{tables.perm, P->perm, n}, {tables.iperm, P->iperm, n}, {tables.node_of, P->node_of, n},
+                  {tables.parent, P->parent, ns}};
+    for (const auto& c : copies)
+        if (c.count > 0)
+            OB_CUDA(cudaMemcpyAsync(c.to, c.from, sizeof(int) * (size_t)c.count, cudaMemcpyDeviceToDevice, stream));
+    if (ns > 0) {
+        row_lists_kernel<<<ceil_div(32LL * ns, threads), threads, 0, stream>>>(ns, n, P->start, P->nc, P->rel_at,
+                                                                               P->rows, P->rows_at, tables.idx);
+        OB_CHECK_LAUNCH("chol row lists");
+    }
     if (pin_mode == kPinZeroSum) {
         zero_sum_rows_kernel<<<ceil_div(n, threads), threads, 0, stream>>>(n, P->offsets, values, P->diag_pos,
                                                                            P->component, bad);
@@ -830,9 +870,12 @@ int device_factor(CholAnalysis& A, const double* values, double sign, int pin_mo
                 OB_CHECK_LAUNCH("chol trailing products");
         }
     }
+    // The launches above run while the host goes on.
+    const int beside = meanwhile();
     int host_status = 0;
     OB_CUDA(cudaMemcpyAsync(&host_status, status, sizeof(int), cudaMemcpyDeviceToHost, stream));
     OB_CUDA(cudaStreamSynchronize(stream));
+    if (beside) return beside;
     return host_status ? OB_ERR_INDEFINITE : OB_OK;
 }
 

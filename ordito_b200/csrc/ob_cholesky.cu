@@ -1589,40 +1589,16 @@ int setup_factor(Factor* F, const double* values, double sign, int pin_mode, cud
     // then its off-diagonal X rows, in the stacked [B; Y; X] numbering.
     BlockLayout layout = block_layout(A);
     OB_REQUIRE(layout.total_rows < (1LL << 31) && 3LL * n < (1LL << 31), "ob_chol_factor: factor too large");
-    std::vector<int> idx(std::max<long long>(layout.total_rows, 1));
-    for (int s = 0; s < ns; ++s) {
-        const Node& nd = A.nodes[s];
-        const int nc = nd.count, noff = (int)nd.off_rows.size();
-        std::copy(nd.off_rows.begin(), nd.off_rows.end(), idx.begin() + layout.rows_at[s]);
-        for (int i = 0; i < nc; ++i) idx[layout.back_at[s] + i] = n + nd.start + i;
-        for (int r = 0; r < noff; ++r) idx[layout.back_at[s] + nc + r] = 2 * n + nd.off_rows[r];
-    }
     F->n_vals = layout.total;
     int st = dev_alloc(F, (void**)&F->vals, sizeof(double) * std::max<long long>(layout.total, 1), stream);
-    if (!st) st = dev_alloc(F, (void**)&F->idx, sizeof(int) * idx.size(), stream);
+    if (!st) st = dev_alloc(F, (void**)&F->idx, sizeof(int) * (size_t)layout.total_rows, stream);
     if (!st) st = dev_alloc(F, (void**)&F->perm, sizeof(int) * A.n, stream);
     if (!st) st = dev_alloc(F, (void**)&F->iperm, sizeof(int) * A.n, stream);
     if (!st) st = dev_alloc(F, (void**)&F->pinned, std::max(A.n, 1), stream);
-    if (st) return st;
-    OB_CUDA(cudaMemcpyAsync(F->idx, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice,
-                            stream));
-    OB_CUDA(cudaMemcpyAsync(F->iperm, A.iperm.data(), sizeof(int) * A.n, cudaMemcpyHostToDevice,
-                            stream));
-    OB_CUDA(cudaMemcpyAsync(F->perm, A.perm.data(), sizeof(int) * A.n, cudaMemcpyHostToDevice,
-                            stream));
     // Each row's supernode and each supernode's parent, and a marking buffer per work set.
-    std::vector<int> node_of_row(std::max(n, 1), -1), parent(std::max(ns, 1), -1);
-    for (int s = 0; s < ns; ++s) {
-        parent[s] = A.nodes[s].parent;
-        for (int j = 0; j < A.nodes[s].count; ++j) node_of_row[A.nodes[s].start + j] = s;
-    }
-    if ((st = dev_alloc(F, (void**)&F->node_of_row, sizeof(int) * node_of_row.size(), stream)) ||
-        (st = dev_alloc(F, (void**)&F->parent_node, sizeof(int) * parent.size(), stream)))
-        return st;
-    OB_CUDA(cudaMemcpyAsync(F->node_of_row, node_of_row.data(), sizeof(int) * node_of_row.size(),
-                            cudaMemcpyHostToDevice, stream));
-    OB_CUDA(cudaMemcpyAsync(F->parent_node, parent.data(), sizeof(int) * parent.size(),
-                            cudaMemcpyHostToDevice, stream));
+    if (!st) st = dev_alloc(F, (void**)&F->node_of_row, sizeof(int) * std::max(n, 1), stream);
+    if (!st) st = dev_alloc(F, (void**)&F->parent_node, sizeof(int) * std::max(ns, 1), stream);
+    if (st) return st;
     F->n_nodes = ns;
     for (auto& W : F->sets)
         if ((st = dev_alloc(F, (void**)&W.active, std::max(ns, 1), stream))) return st;
@@ -1634,11 +1610,11 @@ int setup_factor(Factor* F, const double* values, double sign, int pin_mode, cud
     F->rows_at = std::move(layout.rows_at);
     F->back_at = std::move(layout.back_at);
     F->ld_at = std::move(layout.ld_at);
-    // The numeric factorisation (synchronises once, to read its pivot status).
-    if ((st = device_factor(A, values, sign, pin_mode, F->vals, F->pinned, stream))) return st;
-    if ((st = build_tiles(F, kSplitK, 2, stream))) return st;
-    OB_CUDA(cudaStreamSynchronize(stream));  // host staging buffers go out of scope
-    return OB_OK;
+    // The numeric factorisation, which fills these tables on the device and synchronises once, to
+    // read its pivot status; the host makes the tile lists while it runs.
+    const FactorTables tables{F->n_vals, F->idx, F->perm, F->iperm, F->node_of_row, F->parent_node};
+    return device_factor(A, values, sign, pin_mode, F->vals, F->pinned, tables,
+                         [&] { return build_tiles(F, kSplitK, 2, stream); }, stream);
 }
 
 // The internal column stride of B, Y and X: even, so every row starts on 16 bytes.

@@ -255,3 +255,22 @@ def test_dense_operators_at_the_panel_edges(gpu, n: int) -> None:
     factor.solve(DeviceArray.from_host(rhs), x, refine=False)
     # n eps times the condition, for the factorisation and the two passes.
     np.testing.assert_allclose(x.numpy(), np.linalg.solve(dense, rhs), rtol=0, atol=30 * n * 2.2e-16 * np.abs(rhs).max())
+
+
+@pytest.mark.parametrize(("parts", "length"), [(1, 1), (3, 1), (1, 40), (33, 2), (5, 70), (1, 700), (40, 33)])
+def test_row_lists_of_small_and_split_trees(gpu, parts: int, length: int) -> None:
+    """Separate paths: supernodes without off-diagonal rows, with one, and with more columns than a
+    warp lists at a time; two factors of one analysis, each with its own lists."""
+    import scipy.sparse as sp
+
+    path = sp.diags([np.full(length - 1, -1.0), np.full(length, 2.5), np.full(length - 1, -1.0)], [-1, 0, 1])
+    host = sp.block_diag([path] * parts, format="csr")
+    n = parts * length
+    matrix = CsrMatrix.from_host(host.indptr.astype(np.int32), host.indices.astype(np.int32), host.data, host.shape)
+    rhs = np.random.default_rng(n).normal(size=n)
+    expected = np.linalg.solve(host.toarray(), rhs)
+    for factor in (sparse_cholesky(matrix), sparse_cholesky(matrix)):
+        x = DeviceArray.zeros(n, np.float64)
+        factor.solve(DeviceArray.from_host(rhs), x, refine=False)
+        # Condition below 9; rows of three entries over the tree's levels.
+        np.testing.assert_allclose(x.numpy(), expected, rtol=0, atol=9 * 64 * 2.2e-16 * np.abs(rhs).max())
