@@ -1117,6 +1117,13 @@ tile_product_kernel(const Tile* __restrict__ tiles, const double* __restrict__ v
 constexpr int kNarrowThreads = 256;
 constexpr int kNarrowSlices = kNarrowThreads / kTileRows;
 
+// Four consecutive values, 32-byte aligned, as one load (read by one thread, so kept out of L1).
+__device__ __forceinline__ void load_four(const double* p, double (&a)[4]) {
+    asm volatile("ld.global.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(a[0]), "=d"(a[1]), "=d"(a[2]), "=d"(a[3])
+                 : "l"(p));
+}
+
 template <int KP>
 __global__ void __launch_bounds__(kNarrowThreads)
 narrow_tile_kernel(const Tile* __restrict__ tiles, const double* __restrict__ vals,
@@ -1172,20 +1179,21 @@ narrow_tile_kernel(const Tile* __restrict__ tiles, const double* __restrict__ va
             }
             for (; kk < t.k1; kk += kStep) add(value(kk), row(kk));
         } else {
-            // Row-major reads: a thread reads four consecutive values of its row as two 16-byte
-            // loads (every block row starts on 16 bytes and k0 is even), slice s taking elements
-            // 4 s .. 4 s + 3 of every 16; the one group that straddles k1 is read element by
-            // element by its slice.
+            // Row-major reads: a thread reads four consecutive values of its row as one 32-byte load,
+            // a sector (every block row starts on 64 bytes, and a tile's range on a multiple of
+            // four), slice s taking elements 4 s .. 4 s + 3 of every 16; the one group that straddles
+            // k1 is read element by element by its slice. As two 16-byte loads each sector crossed
+            // from L2 twice: a resident query on the 131k torus took 361 us, so 347.
             constexpr int kGroup = 4 * kNarrowSlices;
             int kk = t.k0 + 4 * slice;
             for (; kk + 3 < t.k1; kk += kGroup) {
-                const double2* p = reinterpret_cast<const double2*>(M + (size_t)(t.r0 + i) * t.ld + kk);
                 const int r0 = row(kk), r1 = row(kk + 1), r2 = row(kk + 2), r3 = row(kk + 3);
-                const double2 v01 = __ldcg(p), v23 = __ldcg(p + 1);
-                add(v01.x, r0);
-                add(v01.y, r1);
-                add(v23.x, r2);
-                add(v23.y, r3);
+                double a[4];
+                load_four(M + (size_t)(t.r0 + i) * t.ld + kk, a);
+                add(a[0], r0);
+                add(a[1], r1);
+                add(a[2], r2);
+                add(a[3], r3);
             }
             for (; kk < t.k1; ++kk) add(value(kk), row(kk));  // kk + 3 >= k1: at most 3
         }
