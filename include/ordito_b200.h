@@ -208,9 +208,12 @@ int ob_shift_noalloc(double* phi, int n_vertices, const int32_t* sources, int n_
  * Replaces ordito/linalg.py:3619 _BatchedCg with the kernels of
  * kernels/algorithms/conjugate_gradient.py (cg_matvec_dots :453, cg_update :797, settle
  * :1509/:1564) and the Jacobi-Chebyshev preconditioner (linalg.py:5135, multigrid.py:988).
- * A solver copies the CSR arrays into its own and owns its work vectors; its iteration's mat-vecs
- * read a sliced-ELL copy it builds from them (slices of 32 rows as wide as their widest row,
- * column-major within a slice, padded with zero entries on the row itself).
+ * A solver copies the CSR arrays into its own and owns its work vectors. One right-hand side of up
+ * to 2 048 rows an SM is solved by one kernel that keeps the rows on the chip; other solves replay
+ * a recorded loop whose mat-vecs read a sliced-ELL copy, built from the CSR arrays by the first of
+ * them (slices of 32 rows as wide as their widest row, column-major within a slice, padded with
+ * zero entries on the row itself). The resident kernel's waits are bounded: one that ran out is
+ * OB_ERR_TIMEOUT.
  * precond: 0 Jacobi, 1 Jacobi-Chebyshev (degree 12, interval [max(min(80/n, .5), 1-r), 1+r]).
  * narrow != 0 iterates on float32 copies of the values (vectors, dots, scalars stay float64).
  * n_columns right-hand sides are solved together; rhs/x are laid out [n][n_columns]. */
@@ -219,8 +222,9 @@ int ob_pcg_create(int n, const int32_t* offsets, const int32_t* columns, const d
 int ob_pcg_destroy(void* solver);
 /* A solver keeps its own copy of the operator it was created for. ob_pcg_rebind copies another
  * operator of the same shape (n, nnz) into it and redoes the value-dependent setup (inverse
- * diagonal, Chebyshev steps, sliced-ELL copy; reading back the copy's size synchronises the
- * stream, and a copy that must grow drops the recorded loops) -- its recorded loops replay unchanged,
+ * diagonal, Chebyshev steps); the sliced-ELL copy is built again by the next solve that reads it
+ * (its size is read back, which synchronises the stream, and a copy that must grow drops the
+ * recorded loops). The recorded loops otherwise replay unchanged,
  * which is how an operator rebuilt per call (ordito/linalg.py:1389-1396: "copied into a kept
  * state of that shape, which replays too") avoids a new state and a new recording. */
 int ob_pcg_rebind(void* solver, const int32_t* offsets, const int32_t* columns,
