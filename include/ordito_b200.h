@@ -52,6 +52,9 @@ int ob_get_device(int* device);
  * releases it in `stream` order, so pass the stream of the buffer's last use. */
 int ob_malloc(size_t bytes, void** ptr, ob_stream_t stream);
 int ob_free(void* ptr, ob_stream_t stream);
+/* Test hook (no counterpart in the reference): the calling thread's countdown-th device allocation
+ * from now is refused, once, as if the device were full (OB_ERR_NOMEM); 0 takes that back. */
+int ob_fail_allocation(int countdown);
 int ob_host_alloc(size_t bytes, void** ptr);             /* pinned host memory              */
 int ob_host_free(void* ptr);
 /* kind: 0 host->device, 1 device->host, 2 device->device, 3 host->host (cudaMemcpyKind order

@@ -42,6 +42,7 @@ SIGNATURES: dict[str, list] = {
     "ob_get_device": [POINTER(c_int)],
     "ob_malloc": [c_size_t, POINTER(c_void_p), P],
     "ob_free": [P, P],
+    "ob_fail_allocation": [I],
     "ob_host_alloc": [c_size_t, POINTER(c_void_p)],
     "ob_host_free": [P],
     "ob_memcpy": [P, P, c_size_t, I, P, I],

@@ -831,9 +831,13 @@ int launch_resident(Solver* S, const double* rhs, double* x, double tol, int max
                     double change_tolerance, int settle_rounds, cudaStream_t stream) {
     if (S->resident_form == kGrid) {
         if (S->published == nullptr) {
-            if (int st = solver_alloc(S, (void**)&S->published, sizeof(double) * 2 * (size_t)S->n, stream)) return st;
-            if (int st = solver_alloc(S, (void**)&S->resident_partials, sizeof(double) * 6 * S->resident_ctas, stream))
+            // One allocation, so a refused one leaves neither pointer set.
+            double* both = nullptr;
+            const size_t vectors = 2 * (size_t)S->n;
+            if (int st = solver_alloc(S, (void**)&both, sizeof(double) * (vectors + 6 * (size_t)S->resident_ctas), stream))
                 return st;
+            S->published = both;
+            S->resident_partials = both + vectors;
         }
         OB_CUDA(cudaMemsetAsync(S->arrivals, 0, 2 * sizeof(int), stream));
     }

@@ -69,7 +69,11 @@ cudaError_t kept_pool(cudaMemPool_t* pool) {
 
 }  // namespace
 
+// ob_fail_allocation: the calling thread's allocations left until one is refused (0: none is).
+thread_local int t_fail_allocation = 0;
+
 cudaError_t pool_malloc(void** p, size_t bytes, cudaStream_t stream) {
+    if (t_fail_allocation > 0 && --t_fail_allocation == 0) return cudaErrorMemoryAllocation;
     cudaMemPool_t pool;
     const cudaError_t e = kept_pool(&pool);
     if (e != cudaSuccess) return e;
@@ -119,6 +123,12 @@ int ob_malloc(size_t bytes, void** ptr, ob_stream_t stream) {
         return fail(e == cudaErrorMemoryAllocation ? OB_ERR_NOMEM : OB_ERR_CUDA,
                     "ob_malloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
     }
+    return OB_OK;
+}
+
+int ob_fail_allocation(int countdown) {
+    OB_REQUIRE(countdown >= 0, "ob_fail_allocation: negative countdown");
+    t_fail_allocation = countdown;
     return OB_OK;
 }
 

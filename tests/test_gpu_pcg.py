@@ -7,7 +7,7 @@ import pytest
 import scipy.sparse as sp
 import scipy.sparse.linalg as spla
 
-from ordito_b200 import linalg
+from ordito_b200 import _lib, linalg
 from ordito_b200.array import CsrMatrix
 from ordito_b200.device import DeviceArray
 
@@ -113,3 +113,25 @@ def test_rebound_state_solves_the_new_operator(gpu) -> None:
         linalg.solve_spd(matrix, DeviceArray.from_host(rhs), x, tol=1e-12)
         assert np.linalg.norm(rhs - host @ x.numpy()) <= 1e-11 * np.linalg.norm(rhs)
         matrix.release()
+
+
+@pytest.mark.parametrize("countdown", [1, 2, 3])
+def test_refused_allocation_leaves_the_state_whole(gpu, countdown: int) -> None:
+    """A first solve whose buffers are refused, then one on the same state, by the form that makes
+    buffers at its first solve (the grid's)."""
+    n = 40001
+    host = _operator(n, 5)
+    matrix = CsrMatrix.from_host(host.indptr, host.indices, host.data, host.shape)
+    solver = linalg._solver(matrix, "diag", False, 1)
+    rhs = np.random.default_rng(1).normal(size=n)
+    d_rhs, x = DeviceArray.from_host(rhs), DeviceArray.zeros(n, np.float64)
+    _lib.call("ob_fail_allocation", countdown)
+    try:
+        solver.solve(d_rhs.ptr, x.ptr, 1e-10, 1000)
+    except MemoryError:
+        pass
+    finally:
+        _lib.call("ob_fail_allocation", 0)
+    x.fill_zero()
+    solver.solve(d_rhs.ptr, x.ptr, 1e-10, 1000)
+    assert np.linalg.norm(rhs - host @ x.numpy()) <= 1.01e-10 * np.linalg.norm(rhs)
