@@ -245,7 +245,8 @@ int ob_pcg_settle(void* solver, const double* rhs, double* x, int check_rounds,
 /* Measurement hooks (no counterpart in the reference): the average duration of `reps` standalone
  * launches of the solver's round mat-vec-with-dots kernel on its current vectors (CUDA events on
  * `stream`), and the solver's shape: info[0..5] = n, padded columns, nnz, narrow, blocks, and the
- * sliced-ELL copy's entries (padding included). */
+ * sliced-ELL copy's entries (padding included; 0 while the bound operator has no such copy, which
+ * the first loop solve, or ob_pcg_time_matvec, makes). ob_pcg_info only reads: no device work. */
 int ob_pcg_time_matvec(void* solver, int reps, float* ms, ob_stream_t stream);
 int ob_pcg_info(void* solver, long long* info);
 /* backward_error_exceeds (kernels/linalg.py:1167): flag[0] = 1 when some row has

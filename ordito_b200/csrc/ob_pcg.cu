@@ -653,11 +653,11 @@ int build_sell(Solver* S, cudaStream_t stream) {
         S->sell_capacity = total;
     }
     S->sell_entries = total;
-    S->sell_bound = true;
     slice_fill_kernel<<<ceil_div(S->n, kThreads), kThreads, 0, stream>>>(
         S->n, S->offsets, S->columns, S->values, S->sell_start, S->sell_columns, S->sell_values,
         S->narrow ? S->sell_values32 : nullptr);
     OB_CHECK_LAUNCH("pcg slice fill");
+    S->sell_bound = true;
     return OB_OK;
 }
 
@@ -1286,13 +1286,12 @@ int ob_pcg_time_matvec(void* solver, int reps, float* ms, ob_stream_t stream_) {
 int ob_pcg_info(void* solver, long long* info) {
     OB_REQUIRE(solver && info, "ob_pcg_info: bad argument");
     Solver* S = static_cast<Solver*>(solver);
-    if (int st = ensure_loop(S, nullptr)) return st;
     info[0] = S->n;
     info[1] = S->k;
     info[2] = S->nnz;
     info[3] = S->narrow;
     info[4] = S->blocks;
-    info[5] = S->sell_entries;
+    info[5] = S->sell_bound ? S->sell_entries : 0;
     return OB_OK;
 }
 

@@ -2,6 +2,8 @@
 
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -135,3 +137,29 @@ def test_refused_allocation_leaves_the_state_whole(gpu, countdown: int) -> None:
     x.fill_zero()
     solver.solve(d_rhs.ptr, x.ptr, 1e-10, 1000)
     assert np.linalg.norm(rhs - host @ x.numpy()) <= 1.01e-10 * np.linalg.norm(rhs)
+
+
+def test_info_only_reads(gpu) -> None:
+    """The copy's entries are 0 until a call has made the copy, again 0 after a rebind, and asking
+    launches nothing (it has no stream to order work on)."""
+    host = _operator(5000, 2)
+    matrix = CsrMatrix.from_host(host.indptr, host.indices, host.data, host.shape)
+    solver = linalg._solver(matrix, "diag", False, 1)
+
+    def entries() -> int:
+        info = (ctypes.c_longlong * 6)()
+        launches = _lib.launch_count()
+        _lib.call("ob_pcg_info", solver.handle, info)
+        assert _lib.launch_count() == launches
+        assert (info[0], info[2]) == (5000, host.nnz)
+        return int(info[5])
+
+    assert entries() == 0
+    ms = ctypes.c_float(0.0)
+    _lib.call("ob_pcg_time_matvec", solver.handle, 1, ctypes.byref(ms), None)
+    built = entries()
+    assert built >= host.nnz
+    solver.rebind(matrix)
+    assert entries() == 0
+    _lib.call("ob_pcg_time_matvec", solver.handle, 1, ctypes.byref(ms), None)
+    assert entries() == built
