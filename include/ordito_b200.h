@@ -225,11 +225,11 @@ int ob_pcg_create(int n, const int32_t* offsets, const int32_t* columns, const d
 int ob_pcg_destroy(void* solver);
 /* A solver keeps its own copy of the operator it was created for. ob_pcg_rebind copies another
  * operator of the same shape (n, nnz) into it and redoes the value-dependent setup (inverse
- * diagonal, Chebyshev steps); the sliced-ELL copy is built again by the next solve that reads it
- * (its size is read back, which synchronises the stream, and a copy that must grow drops the
- * recorded loops). The recorded loops otherwise replay unchanged,
- * which is how an operator rebuilt per call (ordito/linalg.py:1389-1396: "copied into a kept
- * state of that shape, which replays too") avoids a new state and a new recording. */
+ * diagonal, Chebyshev steps), and returns once the caller's arrays have been copied; the sliced-ELL
+ * copy is built again by the next solve that reads it (its size is read back, which synchronises
+ * the stream, and a copy that must grow drops the recorded loops). The recorded loops otherwise
+ * replay unchanged, which is how an operator rebuilt per call (ordito/linalg.py:1389-1396: "copied
+ * into a kept state of that shape, which replays too") avoids a new state and a new recording. */
 int ob_pcg_rebind(void* solver, const int32_t* offsets, const int32_t* columns,
                   const double* values, long long nnz, ob_stream_t stream);
 /* solve_spd (linalg.py:1356): stops a column at |r| <= tol |b| (2-norm), or at maxiter rounds.

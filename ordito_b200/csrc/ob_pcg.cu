@@ -587,6 +587,7 @@ struct Solver {
     double* published = nullptr;  // kGrid: two buffers of n
     double* resident_partials = nullptr;
     unsigned int* arrivals = nullptr;  // the counter and the abort flag, in the state's allocation
+    cudaEvent_t copied = nullptr;  // behind the copies of the operator bound last
     cudaStream_t capture = nullptr;
     // Cached loop graphs: key = (settle?, rounds per body, maxiter, params).
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
@@ -685,6 +686,7 @@ int bind_operator(Solver* S, const int* offsets, const int* columns, const doubl
         OB_CUDA(cudaMemcpyAsync(const_cast<double*>(S->values), values, sizeof(double) * (size_t)nnz,
                                 cudaMemcpyDeviceToDevice, stream));
     }
+    OB_CUDA(cudaEventRecord(S->copied, stream));
     const int setup_blocks = std::max(1, std::min(ceil_div(n, kThreads), 4 * sm_count()));
     jacobi_setup_kernel<<<setup_blocks, kThreads, 0, stream>>>(
         n, S->offsets, S->columns, S->values, S->inv_diag, S->maxima, S->counters + 3,
@@ -706,6 +708,7 @@ void solver_release(Solver* S) {
     for (void* p : S->owned) cudaFree(p);
     if (S->host_state) cudaFreeHost(S->host_state);
     if (S->capture) cudaStreamDestroy(S->capture);
+    if (S->copied) cudaEventDestroy(S->copied);
     delete S;
 }
 
@@ -1150,7 +1153,8 @@ int ob_pcg_create(int n, const int32_t* offsets, const int32_t* columns, const d
         return fail(OB_ERR_NOMEM, "ob_pcg_create: host allocations failed");
     }
     S->host_scalars = reinterpret_cast<ColumnScalars*>(reinterpret_cast<char*>(S->host_state) + kStateBytes);
-    e = cudaMemsetAsync(S->counters, 0, sizeof(unsigned int) * 8, stream);
+    e = cudaEventCreateWithFlags(&S->copied, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaMemsetAsync(S->counters, 0, sizeof(unsigned int) * 8, stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(S->state, 0, kStateBytes, stream);
     if (e != cudaSuccess) {
         solver_release(S);
@@ -1179,7 +1183,11 @@ int ob_pcg_rebind(void* solver, const int32_t* offsets, const int32_t* columns, 
     Solver* S = static_cast<Solver*>(solver);
     OB_REQUIRE(nnz == S->nnz, "ob_pcg_rebind: %lld stored entries, the solver's shape has %lld", nnz,
                S->nnz);
-    return bind_operator(S, offsets, columns, values, as_stream(stream_));
+    if (int st = bind_operator(S, offsets, columns, values, as_stream(stream_))) return st;
+    // The caller's arrays are its own again once the copies are done; the set-up behind them is not
+    // waited for.
+    OB_CUDA(cudaEventSynchronize(S->copied));
+    return OB_OK;
 }
 
 int ob_pcg_destroy(void* solver) {

@@ -163,3 +163,34 @@ def test_info_only_reads(gpu) -> None:
     assert entries() == 0
     _lib.call("ob_pcg_time_matvec", solver.handle, 1, ctypes.byref(ms), None)
     assert entries() == built
+
+
+def test_rebind_returns_with_the_operator_copied(gpu) -> None:
+    """Another stream may overwrite the caller's arrays once ob_pcg_rebind has returned, however much
+    work its own stream still has before the copies."""
+    n = 30001
+    host = _operator(n, 4)
+    matrix = CsrMatrix.from_host(host.indptr, host.indices, host.data, host.shape)
+    other = CsrMatrix.from_host(host.indptr, host.indices, 3.0 * host.data, host.shape)
+    solver = linalg._solver(matrix, "diag", False, 1)
+    rhs = np.random.default_rng(2).normal(size=n)
+    d_rhs, x = DeviceArray.from_host(rhs), DeviceArray.zeros(n, np.float64)
+    busy_in, busy_out = DeviceArray.zeros(64 * n, np.float64), DeviceArray.zeros(64 * n, np.float64)
+    streams = [ctypes.c_void_p(0), ctypes.c_void_p(0)]
+    for stream in streams:
+        _lib.call("ob_stream_create", ctypes.byref(stream))
+    _lib.call("ob_device_synchronize")
+    try:
+        for _ in range(400):  # some tens of milliseconds ahead of the copies
+            _lib.call("ob_spmv", n, matrix.offsets.ptr, matrix.columns.ptr, matrix.values.ptr, busy_in.ptr,
+                      busy_out.ptr, 64, streams[0])
+        _lib.call("ob_pcg_rebind", solver.handle, other.offsets.ptr, other.columns.ptr, other.values.ptr, other.nnz,
+                  streams[0])
+        _lib.call("ob_memcpy", other.values.ptr, matrix.values.ptr, 8 * other.nnz, 2, streams[1], 0)
+        _lib.call("ob_pcg_solve", solver.handle, d_rhs.ptr, x.ptr, 1e-10, 1000, None, None, streams[0])
+        for stream in streams:
+            _lib.call("ob_stream_synchronize", stream)
+    finally:
+        for stream in streams:
+            _lib.call("ob_stream_destroy", stream)
+    assert np.linalg.norm(rhs - 3.0 * (host @ x.numpy())) <= 1.01e-10 * np.linalg.norm(rhs)
