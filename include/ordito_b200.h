@@ -215,8 +215,9 @@ int ob_shift_noalloc(double* phi, int n_vertices, const int32_t* sources, int n_
  * to 2 048 rows an SM is solved by one kernel that keeps the rows on the chip; other solves replay
  * a recorded loop whose mat-vecs read a sliced-ELL copy, built from the CSR arrays by the first of
  * them (slices of 32 rows as wide as their widest row, column-major within a slice, padded with
- * zero entries on the row itself). The resident kernel's waits are bounded: one that ran out is
- * OB_ERR_TIMEOUT.
+ * zero entries on the row itself). The resident kernel's waits are bounded: one that ran out leaves
+ * x unfinished and is reported as OB_ERR_TIMEOUT, once, by the solve itself where it reads anything
+ * back, otherwise by the solver's next solve that does.
  * precond: 0 Jacobi, 1 Jacobi-Chebyshev (degree 12, interval [max(min(80/n, .5), 1-r), 1+r]).
  * narrow != 0 iterates on float32 copies of the values (vectors, dots, scalars stay float64).
  * n_columns right-hand sides are solved together; rhs/x are laid out [n][n_columns]. */
@@ -249,6 +250,9 @@ int ob_pcg_settle(void* solver, const double* rhs, double* x, int check_rounds,
  * the first loop solve, or ob_pcg_time_matvec, makes). ob_pcg_info only reads: no device work. */
 int ob_pcg_time_matvec(void* solver, int reps, float* ms, ob_stream_t stream);
 int ob_pcg_info(void* solver, long long* info);
+/* Test hook (no counterpart in the reference): how often a wait between the resident kernel's blocks
+ * polls before it gives up (negative: the usual number, about a second; 0 or 1: at once). */
+int ob_pcg_wait_limit(void* solver, int polls);
 /* backward_error_exceeds (kernels/linalg.py:1167): flag[0] = 1 when some row has
  * |b - A x|_i > tol (|A| |x| + |b|)_i (or is NaN). flag is zeroed here. */
 int ob_backward_error(int n, const int32_t* offsets, const int32_t* columns, const double* values,

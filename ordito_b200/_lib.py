@@ -91,6 +91,7 @@ SIGNATURES: dict[str, list] = {
     "ob_pcg_settle": [P, P, P, I, D, I, I, POINTER(c_int), POINTER(c_int), P],
     "ob_pcg_time_matvec": [P, I, POINTER(c_float), P],
     "ob_pcg_info": [P, POINTER(ctypes.c_longlong)],
+    "ob_pcg_wait_limit": [P, I],
     "ob_backward_error": [I, P, P, P, P, P, I, D, P, P],
     "ob_spmv": [I, P, P, P, P, P, I, P],
     "ob_cast_scale": [P, I, P, I, ctypes.c_longlong, D, P],

@@ -544,9 +544,10 @@ int next_pow2(int v) {
     return p;
 }
 
-// The state's allocation: the state, the resident form's arrival counter and abort flag, the
-// columns' scalars.
+// The state's allocation: the state, the resident form's arrival counter, its abort flag of a launch
+// and its flag of a wait given up and not reported yet, the columns' scalars.
 constexpr size_t kArrivalsAt = 32, kStateBytes = 64;
+constexpr int kAbort = 1, kGaveUp = 2;  // ints from kArrivalsAt
 static_assert(sizeof(LoopState) <= kArrivalsAt, "the state is followed by the arrivals");
 
 struct Solver {
@@ -586,7 +587,8 @@ struct Solver {
     bool resident_settles = false;  // the form has the settle check
     double* published = nullptr;  // kGrid: two buffers of n
     double* resident_partials = nullptr;
-    unsigned int* arrivals = nullptr;  // the counter and the abort flag, in the state's allocation
+    unsigned int* arrivals = nullptr;  // the counter and the two flags, in the state's allocation
+    int polls = -1;                    // before a wait gives up (negative: the form's usual number)
     cudaEvent_t copied = nullptr;  // behind the copies of the operator bound last
     cudaStream_t capture = nullptr;
     // Cached loop graphs: key = (settle?, rounds per body, maxiter, params).
@@ -866,7 +868,9 @@ int launch_resident(Solver* S, const double* rhs, double* x, double tol, int max
     a.published = S->published;
     a.partials = S->resident_partials;
     a.counter = S->arrivals;
-    a.abort = reinterpret_cast<int*>(S->arrivals + 1);
+    a.polls = S->polls >= 0 ? S->polls : S->resident_form == kGrid ? kGridPolls : kClusterPolls;
+    a.abort = reinterpret_cast<int*>(S->arrivals + kAbort);
+    a.gave_up = reinterpret_cast<int*>(S->arrivals + kGaveUp);
     cudaLaunchAttribute attribute;
     const cudaLaunchConfig_t config = resident_config(S, &attribute, stream);
     void* args[] = {&a};
@@ -1072,8 +1076,12 @@ int read_back(Solver* S, cudaStream_t stream) {
     OB_CUDA(cudaMemcpyAsync(S->host_state, S->state, kStateBytes + sizeof(ColumnScalars) * S->k,
                             cudaMemcpyDeviceToHost, stream));
     OB_CUDA(cudaStreamSynchronize(stream));
-    if (S->resident && reinterpret_cast<const int*>(reinterpret_cast<const char*>(S->host_state) + kArrivalsAt)[1] != 0)
-        return fail(OB_ERR_TIMEOUT, "pcg: a wait between the solver's blocks gave up");
+    // A solve that reads nothing back leaves the flag to the next one that does.
+    if (reinterpret_cast<const int*>(reinterpret_cast<const char*>(S->host_state) + kArrivalsAt)[kGaveUp] != 0) {
+        OB_CUDA(cudaMemsetAsync(S->arrivals + kGaveUp, 0, sizeof(int), stream));
+        return fail(OB_ERR_TIMEOUT, "pcg: a wait between the solver's blocks gave up, in this solve or one "
+                                    "before it that read nothing back");
+    }
     return OB_OK;
 }
 
@@ -1288,6 +1296,12 @@ int ob_pcg_time_matvec(void* solver, int reps, float* ms, ob_stream_t stream_) {
     *ms = total / (float)reps;
     // Leave the state as a finished solve would.
     OB_CUDA(cudaMemsetAsync(S->state, 0, sizeof(LoopState), stream));
+    return OB_OK;
+}
+
+int ob_pcg_wait_limit(void* solver, int polls) {
+    OB_REQUIRE(solver, "ob_pcg_wait_limit: null solver");
+    static_cast<Solver*>(solver)->polls = polls;
     return OB_OK;
 }
 

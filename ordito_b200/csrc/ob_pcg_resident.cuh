@@ -23,8 +23,8 @@
 //   kGrid     up to one CTA an SM (a cooperative launch): global memory at L2, an arrival counter
 //             between phases.
 //
-// Every wait is bounded: a CTA that gives up raises `abort`, the others then give up as well, and the
-// host reports OB_ERR_TIMEOUT. Rows longer than the entries a thread holds read the rest from the CSR arrays. A round's float64
+// Every wait is bounded: a CTA that gives up raises `abort`, the others then give up as well, and
+// `gave_up` stays set until the host has reported OB_ERR_TIMEOUT. Rows longer than the entries a thread holds read the rest from the CSR arrays. A round's float64
 // chain is kept short (two partial sums a row, one division behind the dots), since latency is what
 // is left: the sums a row and the scalars agree with the loop graph's to rounding. The dots are
 // folded thread, warp, CTA in a fixed order, so every run gives the same bits.
@@ -48,7 +48,9 @@ __host__ __device__ constexpr int register_entries(int rows_a_thread) { return r
 // cycles a mat-vec of 1 250 rows, 2 200 without the polynomial). Such a solver has no settle check.
 __host__ __device__ constexpr bool far_vectors(int rows_a_thread, bool cheb) { return rows_a_thread == 4 && cheb; }
 __host__ __device__ constexpr int resident_threads(int) { return 512; }
-constexpr unsigned kGridSpins = 1u << 22;  // polls (>= 0.3 us each) before a grid wait gives up
+// Polls before a wait gives up, about a second: of a grid barrier (>= 0.3 us each), of a barrier in
+// shared memory (2 us at most each).
+constexpr int kGridPolls = 1 << 22, kClusterPolls = 1 << 19;
 
 struct ResidentArgs {
     int n;
@@ -69,7 +71,9 @@ struct ResidentArgs {
     int narrow;  // the operator's values are rounded to float32
     int width;   // entries a row on the chip, those in registers among them
     int pushes;  // kCluster: the capacity of a CTA's push list
+    int polls;   // before a wait gives up
     int* abort;  // 1 when a wait gave up (zero at the launch of kGrid, zeroed by the others)
+    int* gave_up;  // the same, but not zeroed by a launch
     // kGrid: the published vector (two buffers of n), the CTAs' partial sums (6 a CTA) and the
     // arrival counter (zero at the launch).
     double* published;
@@ -113,11 +117,9 @@ __device__ __forceinline__ void arrivals_init(unsigned bar) {
 __device__ __forceinline__ void arrivals_expect(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Waits for the phase of the given parity, kArrivalTries tries of 2 us at most (about a second);
-// false when it gave up.
-constexpr int kArrivalTries = 1 << 19;
-__device__ __forceinline__ bool arrivals_wait(unsigned bar, unsigned parity) {
-    for (int i = 0; i < kArrivalTries; ++i) {
+// Waits for the phase of the given parity, `polls` tries of 2 us at most; false when it gave up.
+__device__ __forceinline__ bool arrivals_wait(unsigned bar, unsigned parity, int polls) {
+    for (int i = 0; i < polls; ++i) {
         unsigned done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -138,17 +140,18 @@ __device__ __forceinline__ void push_cluster(unsigned at, double v, unsigned bar
 
 // Arrives at a grid barrier and waits until `goal` arrivals (monotonic, wrap-safe). False when
 // this wait, or another CTA's, gave up. Called by every thread.
-__device__ __forceinline__ bool grid_barrier(unsigned int* counter, unsigned int goal, int* abort, int* alive) {
+__device__ __forceinline__ bool grid_barrier(unsigned int* counter, unsigned int goal, int polls, int* abort,
+                                             int* alive) {
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         atomicAdd(counter, 1u);
-        unsigned seen, spins = 0;
-        int ok = 1;
+        unsigned seen;
+        int spins = 0, ok = 1;
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
             if ((int)(seen - goal) >= 0) break;
-            if (++spins >= kGridSpins || ((spins & 255u) == 0u && *(volatile int*)abort != 0)) {
+            if (++spins >= polls || ((spins & 255) == 0 && *(volatile int*)abort != 0)) {
                 atomicExch(abort, 1);
                 ok = 0;
                 break;
@@ -237,7 +240,7 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
         if (FORM == kCluster) cluster_barrier();
         if (FORM == kGrid) {
             goal += (unsigned)ctas;
-            ok = grid_barrier(a.counter, goal, a.abort, alive) && ok;
+            ok = grid_barrier(a.counter, goal, a.polls, a.abort, alive) && ok;
         }
     };
     // Sums over every row of the system, in two halves around a barrier: `fold` leaves the CTA's
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
     // barrier of its own (fold, publish), and leaves only where it has agreed.
     auto await_sums = [&]() {
         if (FORM == kCluster && !pulls) {
-            ok = ok && arrivals_wait(bars_at + 8u * (2u + (summed & 1u)), (summed >> 1) & 1u);
+            ok = ok && arrivals_wait(bars_at + 8u * (2u + (summed & 1u)), (summed >> 1) & 1u, a.polls);
             ok = __syncthreads_and(ok);
         } else {
             barrier();
@@ -303,7 +306,7 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
     };
     auto await_published = [&]() {
         if (FORM == kCluster && !pulls) {
-            ok = ok && arrivals_wait(bars_at + 8u * (sent & 1u), (sent >> 1) & 1u);
+            ok = ok && arrivals_wait(bars_at + 8u * (sent & 1u), (sent >> 1) & 1u, a.polls);
             ++sent;
         } else {
             barrier();
@@ -732,8 +735,22 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
         a.scalars->rr = rr;
         a.scalars->rr0 = rr0;
     }
-    if (!ok) atomicExch(a.abort, 1);
-    if (FORM == kCluster) cluster_barrier();  // no CTA leaves while another may still read its memory
+    if (!ok) {
+        atomicExch(a.abort, 1);
+        atomicExch(a.gave_up, 1);
+    }
+    if (FORM == kCluster) {
+        cluster_barrier();  // no CTA leaves while another may still read its memory
+        // Where every CTA waited for what was pushed to it, nothing is on its way any more. After a wait
+        // that was given up, pushes may be, and their sender cannot wait for them: none is sent past
+        // the barrier, and the CTAs stay for about 100 us, where a store to shared memory takes one.
+        if (*(volatile int*)a.abort != 0) {
+            const long long start = clock64();
+            while (clock64() - start < 200000) {
+            }
+            cluster_barrier();
+        }
+    }
 }
 
 }  // namespace

@@ -16,10 +16,10 @@ from ordito_b200.device import DeviceArray
 pytestmark = pytest.mark.gpu
 
 
-def _operator(n: int, seed: int) -> sp.csr_matrix:
+def _operator(n: int, seed: int, wide_row: bool = True) -> sp.csr_matrix:
     """A diagonally dominant symmetric operator of neighbours at distance 1 and ~sqrt(n) (a
-    dominance of 1.25: condition below 9) with one row and column of 40 entries, more than a
-    thread of the resident form keeps in shared memory."""
+    dominance of 1.25: condition below 9), with one row and column of 40 entries, more than a
+    thread of the resident form keeps in shared memory, or without."""
     rng = np.random.default_rng(seed)
     far = max(2, int(n**0.5))
     rows, cols = [], []
@@ -27,7 +27,7 @@ def _operator(n: int, seed: int) -> sp.csr_matrix:
         at = np.arange(max(0, n - step))
         rows.append(at)
         cols.append(at + step)
-    if n > 64:
+    if n > 64 and wide_row:
         to = rng.choice(np.arange(2, n), size=40, replace=False)
         rows.append(np.full(40, 0))
         cols.append(to)
@@ -194,3 +194,38 @@ def test_rebind_returns_with_the_operator_copied(gpu) -> None:
         for stream in streams:
             _lib.call("ob_stream_destroy", stream)
     assert np.linalg.norm(rhs - 3.0 * (host @ x.numpy())) <= 1.01e-10 * np.linalg.norm(rhs)
+
+
+@pytest.mark.parametrize(("n", "kind"), [(3000, "diag"), (20000, "diag"), (20000, "chebyshev"), (40001, "diag"),
+                                         (40001, "chebyshev")])
+def test_a_wait_given_up_is_reported_once(gpu, n: int, kind: str) -> None:
+    """Waits between a cluster's and a grid's blocks that run out at once: the solve returns, the
+    status says so, by the next solve that reads back where this one does not, and the state goes on
+    (its loop graph's settle too: 20 000 rows under Chebyshev)."""
+    host = _operator(n, 6, wide_row=False)
+    matrix = CsrMatrix.from_host(host.indptr, host.indices, host.data, host.shape)
+    solver = linalg._solver(matrix, kind, False, 1)
+    rhs = np.random.default_rng(3).normal(size=n)
+    d_rhs, x = DeviceArray.from_host(rhs), DeviceArray.zeros(n, np.float64)
+    rounds, residual = ctypes.c_int(0), ctypes.c_double(0.0)
+
+    def solve(read_back: bool = True) -> int:
+        x.fill_zero()
+        return _lib.lib.ob_pcg_solve(solver.handle, d_rhs.ptr, x.ptr, 1e-10, 1000,
+                                     ctypes.byref(rounds) if read_back else None,
+                                     ctypes.byref(residual) if read_back else None, None)
+
+    _lib.call("ob_pcg_wait_limit", solver.handle, 0)
+    try:
+        for _ in range(3):
+            assert solve() == _lib.OB_ERR_TIMEOUT
+        assert solve(read_back=False) == _lib.OB_OK
+    finally:
+        _lib.call("ob_pcg_wait_limit", solver.handle, -1)
+    assert solve(read_back=False) == _lib.OB_OK
+    assert solve() == _lib.OB_ERR_TIMEOUT  # the unread one's
+    assert solve() == _lib.OB_OK
+    assert np.linalg.norm(rhs - host @ x.numpy()) <= 1.01e-10 * np.linalg.norm(rhs)
+    x.fill_zero()
+    solver.settle(d_rhs.ptr, x.ptr, 16, 1e-6, 192, 1000)
+    assert np.linalg.norm(rhs - host @ x.numpy()) <= 1e-6 * np.linalg.norm(rhs)
