@@ -274,3 +274,21 @@ def test_row_lists_of_small_and_split_trees(gpu, parts: int, length: int) -> Non
         factor.solve(DeviceArray.from_host(rhs), x, refine=False)
         # Condition below 9; rows of three entries over the tree's levels.
         np.testing.assert_allclose(x.numpy(), expected, rtol=0, atol=9 * 64 * 2.2e-16 * np.abs(rhs).max())
+
+
+@pytest.mark.parametrize("exponent", [-1020, -1030, -1036, 1000])
+@pytest.mark.parametrize("n", [1, 2, 20, 65, 150])
+def test_operators_at_the_ends_of_the_range(gpu, n: int, exponent: int) -> None:
+    """Operators whose pivots are subnormal (their reciprocals are out of range) or near the largest."""
+    import scipy.sparse as sp
+
+    host = sp.diags([np.full(n - 1, -1.0), np.full(n, 2.5), np.full(n - 1, -1.0)], [-1, 0, 1]).tocsr()
+    rhs = np.random.default_rng(n).integers(-8, 9, size=n).astype(float)  # few bits: exact when scaled
+    matrix = CsrMatrix.from_host(host.indptr, host.indices, np.ldexp(host.data, exponent), host.shape)
+    factor = sparse_cholesky(matrix)
+    x = DeviceArray.zeros(n, np.float64)
+    factor.solve(DeviceArray.from_host(np.ldexp(rhs, exponent)), x, refine=False)
+    # A subnormal entry is rounded to 2^-1074, 2^(-1074 - exponent) of the operator; each pivot takes a
+    # few such roundings, and the condition is below 9.
+    rounding = max(2.0**-52, 2.0 ** (-1074 - exponent))
+    np.testing.assert_allclose(x.numpy(), np.linalg.solve(host.toarray(), rhs), rtol=0, atol=9 * 64 * rounding * 8)
