@@ -454,8 +454,8 @@ grad_div_planes_kernel(const double2* __restrict__ planes, const int* __restrict
             for (int j = 0; j < CP; ++j) {
                 const double d1 = u1[j] - own[j], d2 = u2[j] - own[j];
                 const double gx = fma(d1, p0.x, d2 * p0.y), gy = d2 * p1.x;
-                const double largest = fmax(fabs(gx), fabs(gy));
-                if (largest == 0.0) continue;  // no gradient: the unit gradient is zero
+                if (gx == 0.0 && gy == 0.0) continue;  // no gradient: the unit gradient is zero
+                const double largest = fmax(fabs(gx), fabs(gy));  // (a NaN beside a zero goes on as a NaN)
                 const double scale = inverse_power_of_two(largest);
                 const double sx = gx * scale, sy = gy * scale;
                 acc[j] += fma(sx, p1.y, sy * p2.x) * rsqrt(fma(sx, sx, sy * sy));

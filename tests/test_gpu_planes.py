@@ -69,6 +69,32 @@ def test_planes_match_the_terms(gpu, name: str, k: int, stride: int) -> None:
         np.testing.assert_allclose(outs["planes", 0], want, rtol=tolerance, atol=tolerance * np.abs(want).max())
 
 
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("k", [1, 2, 4])
+def test_planes_carry_what_is_not_finite(gpu, k: int, bad: float) -> None:
+    """A NaN or infinite value shows at every corner that reads it, as in the terms form, also where the
+    face's other two values are equal."""
+    v, f = creation.flat_grid((9, 7))
+    n = v.shape[0]
+    mesh = Trimesh(v, f.reshape(-1))
+    face = mesh.face_terms
+    offsets, slots = mesh.corner_index
+    terms = DeviceArray.empty((mesh.n_faces, 18), np.float64)
+    _lib.call("ob_face_gradient_terms", mesh.vertices.ptr, mesh.faces.ptr, mesh.n_faces, face.normals.ptr,
+              face.areas.ptr, face.cot.ptr, terms.ptr, None)
+    planes = corner_planes(terms, mesh.faces, slots, mesh.n_faces)
+    faces = f.reshape(-1, 3)
+    for at in range(0, n, 5):
+        field = np.zeros((n, k))
+        field[at, k - 1] = bad
+        u, out = DeviceArray.from_host(field.reshape(-1)), DeviceArray.empty(n * k, np.float64)
+        _lib.call("ob_grad_div_planes", planes.ptr, offsets.ptr, n, k, u.ptr, k, None, out.ptr, k, None, None, None)
+        got = ~np.isfinite(out.numpy().reshape(n, k))
+        want = np.zeros((n, k), dtype=bool)
+        want[np.unique(faces[(faces == at).any(axis=1)]), k - 1] = True  # the vertex and its neighbours
+        np.testing.assert_array_equal(got, want)
+
+
 # A chunk is 512 rows: one less, one, one more, and several, beside a mesh of three vertices.
 @pytest.mark.parametrize("k", [1, 3, 16])
 def test_packed_shift_over_chunk_edges(gpu, k: int) -> None:
