@@ -212,7 +212,9 @@ int ob_shift_noalloc(double* phi, int n_vertices, const int32_t* sources, int n_
  * kernels/algorithms/conjugate_gradient.py (cg_matvec_dots :453, cg_update :797, settle
  * :1509/:1564) and the Jacobi-Chebyshev preconditioner (linalg.py:5135, multigrid.py:988).
  * A solver copies the CSR arrays into its own and owns its work vectors. One right-hand side of up
- * to 2 048 rows an SM is solved by one kernel that keeps the rows on the chip; other solves replay
+ * to 2 048 rows an SM, few entries a row, is solved by one kernel that keeps the rows on the chip (the
+ * first such solve of a bound operator may wait for the kernel, which may leave an operator of
+ * scattered columns to another form); other solves replay
  * a recorded loop whose mat-vecs read a sliced-ELL copy, built from the CSR arrays by the first of
  * them (slices of 32 rows as wide as their widest row, column-major within a slice, padded with
  * zero entries on the row itself). The resident kernel's waits are bounded: one that ran out leaves

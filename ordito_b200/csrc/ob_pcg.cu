@@ -544,11 +544,20 @@ int next_pow2(int v) {
     return p;
 }
 
-// The state's allocation: the state, the resident form's arrival counter, its abort flag of a launch
-// and its flag of a wait given up and not reported yet, the columns' scalars.
+// The state's allocation: the state, the resident form's arrival counter, its abort flag and its count of
+// gathered lines of a launch, its flag of a wait given up and not reported yet, the columns' scalars.
 constexpr size_t kArrivalsAt = 32, kStateBytes = 64;
-constexpr int kAbort = 1, kGaveUp = 2;  // ints from kArrivalsAt
+constexpr int kAbort = 1, kScattered = 2, kGaveUp = 3;  // ints from kArrivalsAt (a launch zeroes the first three)
 static_assert(sizeof(LoopState) <= kArrivalsAt, "the state is followed by the arrivals");
+
+// One of the resident forms (ob_pcg_resident.cuh) for a system's size.
+struct ResidentPlan {
+    const void* kernel = nullptr;
+    int form = 0, threads = 0, ctas = 0, width = 0, more = 0, pushes = 0;
+    size_t smem = 0;
+    bool settles = false;      // the form has the settle check
+    bool may_decline = false;  // a launch may leave the system to another form
+};
 
 struct Solver {
     int n = 0, k_live = 0, k = 0, precond = 0, narrow = 0;
@@ -580,11 +589,14 @@ struct Solver {
     ColumnScalars* host_scalars = nullptr;
     int blocks = 0;
     bool loop_ready = false;  // the loop graph's vectors are allocated
-    // The resident form (ob_pcg_resident.cuh), when the system fits it.
-    const void* resident = nullptr;
-    int resident_form = 0, resident_threads = 0, resident_ctas = 0, resident_width = 0, resident_pushes = 0;
-    size_t resident_smem = 0;
-    bool resident_settles = false;  // the form has the settle check
+    // The resident form by the system's size (no kernel: the loop graph), and the one the bound operator
+    // takes, which is another where its rows' order scatters their columns over the cluster.
+    ResidentPlan by_size, resident;
+    bool undecided = false;  // a launch of `resident` may decline the bound operator
+    // The lists of further entries (12 bytes an entry, the rows' bounds).
+    double* more_values = nullptr;
+    unsigned* more_places = nullptr;
+    int* more_rows = nullptr;
     double* published = nullptr;  // kGrid: two buffers of n
     double* resident_partials = nullptr;
     unsigned int* arrivals = nullptr;  // the counter and the two flags, in the state's allocation
@@ -695,6 +707,8 @@ int bind_operator(Solver* S, const int* offsets, const int* columns, const doubl
         kChebyshevDegree - 1, S->steps);
     OB_CHECK_LAUNCH("pcg setup");
     S->sell_bound = false;
+    S->resident = S->by_size;
+    S->undecided = S->resident.may_decline;
     return OB_OK;
 }
 
@@ -742,19 +756,19 @@ const void* resident_kernel_of(bool cheb) {
     return cheb ? (const void*)resident_pcg_kernel<R, FORM, true> : (const void*)resident_pcg_kernel<R, FORM, false>;
 }
 
-cudaLaunchConfig_t resident_config(const Solver* S, cudaLaunchAttribute* attribute, cudaStream_t stream) {
+cudaLaunchConfig_t resident_config(const ResidentPlan& P, cudaLaunchAttribute* attribute, cudaStream_t stream) {
     cudaLaunchConfig_t config = {};
-    config.gridDim = dim3((unsigned)S->resident_ctas);
-    config.blockDim = dim3((unsigned)S->resident_threads);
-    config.dynamicSmemBytes = S->resident_smem;
+    config.gridDim = dim3((unsigned)P.ctas);
+    config.blockDim = dim3((unsigned)P.threads);
+    config.dynamicSmemBytes = P.smem;
     config.stream = stream;
     config.attrs = attribute;
-    if (S->resident_form == kCluster) {
+    if (P.form == kCluster) {
         attribute->id = cudaLaunchAttributeClusterDimension;
-        attribute->val.clusterDim.x = (unsigned)S->resident_ctas;
+        attribute->val.clusterDim.x = (unsigned)P.ctas;
         attribute->val.clusterDim.y = attribute->val.clusterDim.z = 1;
         config.numAttrs = 1;
-    } else if (S->resident_form == kGrid) {
+    } else if (P.form == kGrid) {
         attribute->id = cudaLaunchAttributeCooperative;
         attribute->val.cooperative = 1;
         config.numAttrs = 1;
@@ -762,33 +776,53 @@ cudaLaunchConfig_t resident_config(const Solver* S, cudaLaunchAttribute* attribu
     return config;
 }
 
-// Takes one form for the solver if the system fits it and the device can hold all its CTAs at once.
-bool take_resident(Solver* S, int form, int rows_a_cta, int rows_a_thread) {
+// A form for the solver's system if it fits it and the device can hold all its CTAs at once; otherwise
+// no kernel.
+ResidentPlan plan_resident(const Solver* S, int form, int rows_a_cta, int rows_a_thread) {
+    ResidentPlan P;
+    const bool cheb = S->precond == 1;
     const int per_warp = 32 * rows_a_thread;
     int threads = (rows_a_cta + per_warp - 1) / per_warp * 32;
     if (form == kGrid) threads = std::max(threads, 96);  // a warp for each of the three sums
-    if (threads > resident_threads(rows_a_thread)) return false;
+    if (threads > resident_threads(rows_a_thread)) return P;
     int device = 0, limit = 0;
     if (cudaGetDevice(&device) != cudaSuccess ||
         cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
-        return false;
+        return P;
     const size_t owned = (size_t)threads * rows_a_thread;
-    const int registers = register_entries(rows_a_thread);
-    const int pushes = form == kCluster ? (int)(owned * (registers ? kPushesARow : kPushesARow / 2)) : 0;
+    const int pushes = form == kCluster ? (int)(owned * (rows_a_thread == 2 ? kPushesARow : kPushesARow / 2)) : 0;
+    const size_t entry = sizeof(unsigned) + sizeof(double);
     const size_t fixed = (form == kGrid ? 0 : 16 * (owned + (form == kCluster ? kHalo : 0))) +
                          8 * (6 * kClusterMax + 3 * 32 + 8 + 4 * kChebyshevDegree) +
-                         (far_vectors(rows_a_thread, S->precond == 1) ? 24 * owned : 0) +
-                         (form == kCluster ? sizeof(int2) * pushes + sizeof(int) * (2 * kHaloTable + 4) : 0);
-    const size_t entry = owned * (sizeof(unsigned) + sizeof(double));
-    if (fixed + (kBaseEntries - registers) * entry > (size_t)limit) return false;
-    S->resident_form = form;
-    S->resident_threads = threads;
-    S->resident_ctas = (int)((S->n + owned - 1) / owned);
-    S->resident_pushes = pushes;
-    S->resident_settles = !far_vectors(rows_a_thread, S->precond == 1);
-    S->resident_width = (int)std::min<size_t>(kResidentWidth, registers + ((size_t)limit - fixed) / entry);
-    S->resident_smem = fixed + (S->resident_width - registers) * entry;
-    const bool cheb = S->precond == 1;
+                         (far_vectors(rows_a_thread, cheb) ? 24 * owned : 0) +
+                         (form == kCluster ? sizeof(int2) * pushes + sizeof(int) * 2 * kHaloTable
+                                           : sizeof(double) * kProducts * (threads / 32)) +
+                         (kBaseEntries - register_entries(rows_a_thread)) * owned * entry +
+                         sizeof(int) * (8 + 2 * 16 + 2);
+    if (fixed > (size_t)limit) return P;
+    // What is left: the bounds of the rows' listed entries, the entries in place, the list.
+    size_t left = (size_t)limit - fixed;
+    const size_t wanted = sizeof(int) * threads * (rows_a_thread + 1), bounds = left >= wanted ? wanted : 0;
+    left -= bounds;
+    const int mean = std::max(kBaseEntries, (int)((S->nnz + S->n - 1) / S->n));
+    const int in_place = (int)std::min<size_t>(most_in_place(form, mean) - kBaseEntries, left / 8 * 7 / (owned * entry));
+    left -= in_place * owned * entry;
+    P.form = form;
+    P.threads = threads;
+    P.ctas = (int)((S->n + owned - 1) / owned);
+    P.pushes = pushes;
+    P.settles = !far_vectors(rows_a_thread, cheb);
+    P.width = kBaseEntries + in_place;
+    // Operators whose rows are much longer than that on average go to the next form. us a settle round / a
+    // Chebyshev one of this form and the loop graph, the mean row in brackets: the cluster, 16 000 rows
+    // [21, 16 in place] 8.2 / 75 and 13.4 / 92, [31] 19 / 197 and 14.2 / 114 (the grid: 10.6 / 101); four
+    // rows a thread, 20 000 rows [11, 9 and 8 in place] 8.2 / 134 and 12.5 / 74, [15] 16.6 / 238 and
+    // 13.3 / 80.
+    if (mean > P.width + (rows_a_thread == 2 ? 5 : cheb ? 1 : 3)) return P;
+    P.more = bounds ? (int)std::min<size_t>((mean - kBaseEntries + 1) * owned, left / entry) : 0;
+    P.smem = fixed + bounds + (in_place * owned + P.more) * entry;
+    P.may_decline = form == kCluster || (form == kGrid && far_vectors(rows_a_thread, cheb) &&
+                                         (size_t)(256 << 10) < P.smem + kScatterLeaves);
     const void* kernel = form == kBlock ? resident_kernel_of<2, kBlock>(cheb)
                          : form == kCluster
                              ? (rows_a_thread == 2 ? resident_kernel_of<2, kCluster>(cheb)
@@ -800,82 +834,110 @@ bool take_resident(Solver* S, int form, int rows_a_cta, int rows_a_thread) {
     if (ok && form == kCluster) {
         ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
         cudaLaunchAttribute attribute;
-        const cudaLaunchConfig_t config = resident_config(S, &attribute, nullptr);
+        const cudaLaunchConfig_t config = resident_config(P, &attribute, nullptr);
         int clusters = 0;
         ok = ok && cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) == cudaSuccess && clusters >= 1;
     }
     if (ok && form == kGrid) {
         int per_sm = 0;
-        ok = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, S->resident_smem) ==
-                 cudaSuccess &&
-             (long long)per_sm * sm_count() >= S->resident_ctas;
+        ok = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, P.smem) == cudaSuccess &&
+             (long long)per_sm * sm_count() >= P.ctas;
     }
-    if (!ok) {
-        cudaGetLastError();
-        return false;
-    }
-    S->resident = kernel;
-    return true;
+    if (ok) P.kernel = kernel;
+    else cudaGetLastError();
+    return P;
+}
+
+ResidentPlan plan_grid(const Solver* S) {
+    const int rows = std::max((S->n + sm_count() - 1) / sm_count(), 256);
+    return rows <= 2048 ? plan_resident(S, kGrid, rows, rows <= 1024 ? 2 : 4) : ResidentPlan();
 }
 
 // The form by size: one CTA to 1 024 rows, a cluster of up to 16 CTAs while their shared memory holds
-// the rows (about 26 000), then a grid of one CTA an SM; two rows a thread (their entries in
-// registers) to 1 024 rows a CTA, four (in shared memory) to 2 048. Larger systems, and several
-// columns, take the loop graph, whose kernels then run for longer than their launch.
+// the rows (26 624, under the polynomial 22 528), then a grid of one CTA an SM; two rows a thread
+// (their entries in registers) to 1 024 rows a CTA, four (in shared memory) to 2 048. Larger systems,
+// and several columns, take the loop graph, whose kernels then run for longer than their launch.
 void choose_resident(Solver* S) {
     if (S->k != 1) return;
-    if (S->n <= 1024 && take_resident(S, kBlock, S->n, 2)) return;
+    ResidentPlan& P = S->by_size;
+    if (S->n <= 1024) P = plan_resident(S, kBlock, S->n, 2);
     const int cluster_rows = std::max((S->n + kClusterMax - 1) / kClusterMax, 64);
-    if (cluster_rows <= 2048 && take_resident(S, kCluster, cluster_rows, cluster_rows <= 1024 ? 2 : 4)) return;
-    const int grid_rows = std::max((S->n + sm_count() - 1) / sm_count(), 256);
-    if (grid_rows <= 2048) take_resident(S, kGrid, grid_rows, grid_rows <= 1024 ? 2 : 4);
+    if (P.kernel == nullptr && cluster_rows <= 2048)
+        P = plan_resident(S, kCluster, cluster_rows, cluster_rows <= 1024 ? 2 : 4);
+    if (P.kernel == nullptr) P = plan_grid(S);
+    S->resident = P;
+    S->undecided = P.may_decline;
 }
 
-// One solve by the resident form; check_rounds 0 stops by the residual.
+int read_back(Solver* S, cudaStream_t stream);
+
+// One solve by the resident form; check_rounds 0 stops by the residual. A form that may decline the
+// operator is waited for the first time; *taken says whether one has solved it, *read whether the
+// state has been read back.
 int launch_resident(Solver* S, const double* rhs, double* x, double tol, int maxiter, int check_rounds,
-                    double change_tolerance, int settle_rounds, cudaStream_t stream) {
-    if (S->resident_form == kGrid) {
-        if (S->published == nullptr) {
-            // One allocation, so a refused one leaves neither pointer set.
-            double* both = nullptr;
-            const size_t vectors = 2 * (size_t)S->n;
-            if (int st = solver_alloc(S, (void**)&both, sizeof(double) * (vectors + 6 * (size_t)S->resident_ctas), stream))
-                return st;
-            S->published = both;
-            S->resident_partials = both + vectors;
+                    double change_tolerance, int settle_rounds, cudaStream_t stream, bool* taken, bool* read) {
+    *taken = *read = false;
+    while (S->resident.kernel != nullptr && (check_rounds == 0 || S->resident.settles)) {
+        const ResidentPlan& P = S->resident;
+        if (P.form == kGrid) {
+            if (S->published == nullptr) {
+                // One allocation, so a refused one leaves neither pointer set.
+                double* both = nullptr;
+                const size_t vectors = 2 * (size_t)S->n;
+                if (int st = solver_alloc(S, (void**)&both, sizeof(double) * (vectors + 6 * (size_t)P.ctas), stream))
+                    return st;
+                S->published = both;
+                S->resident_partials = both + vectors;
+            }
+            OB_CUDA(cudaMemsetAsync(S->arrivals, 0, kGaveUp * sizeof(int), stream));
         }
-        OB_CUDA(cudaMemsetAsync(S->arrivals, 0, 2 * sizeof(int), stream));
+        ResidentArgs a = {};
+        a.n = S->n;
+        a.offsets = S->offsets;
+        a.columns = S->columns;
+        a.values = S->values;
+        a.inv_diag = S->inv_diag;
+        a.steps = S->steps;
+        a.rhs = rhs;
+        a.x = x;
+        a.tol = tol;
+        a.maxiter = maxiter;
+        a.check_rounds = check_rounds;
+        a.change_tolerance = change_tolerance;
+        a.settle_rounds = settle_rounds;
+        a.state = S->state;
+        a.scalars = S->scalars;
+        a.narrow = S->narrow;
+        a.width = P.width;
+        a.more = P.more;
+        a.pushes = P.pushes;
+        a.polls = S->polls >= 0 ? S->polls : P.form == kGrid ? kGridPolls : kClusterPolls;
+        a.abort = reinterpret_cast<int*>(S->arrivals + kAbort);
+        a.gave_up = reinterpret_cast<int*>(S->arrivals + kGaveUp);
+        a.scattered = S->undecided && P.form == kGrid ? reinterpret_cast<int*>(S->arrivals + kScattered) : nullptr;
+        a.more_values = S->more_values;
+        a.more_places = S->more_places;
+        a.more_rows = S->more_rows;
+        a.published = S->published;
+        a.partials = S->resident_partials;
+        a.counter = S->arrivals;
+        cudaLaunchAttribute attribute;
+        const cudaLaunchConfig_t config = resident_config(P, &attribute, stream);
+        void* args[] = {&a};
+        OB_CUDA(cudaLaunchKernelExC(&config, P.kernel, args));
+        OB_CHECK_LAUNCH("pcg resident solve");
+        *taken = true;
+        if (!S->undecided) return OB_OK;
+        const int st = read_back(S, stream);
+        if (st != OB_OK && st != OB_ERR_TIMEOUT) return st;
+        S->undecided = false;
+        *taken = *read = S->host_state->status != kDeclined;
+        if (!*taken) {
+            S->resident = P.form == kCluster ? plan_grid(S) : ResidentPlan();
+            S->undecided = S->resident.may_decline;
+        }
+        if (st || *taken) return st;
     }
-    ResidentArgs a = {};
-    a.n = S->n;
-    a.offsets = S->offsets;
-    a.columns = S->columns;
-    a.values = S->values;
-    a.inv_diag = S->inv_diag;
-    a.steps = S->steps;
-    a.rhs = rhs;
-    a.x = x;
-    a.tol = tol;
-    a.maxiter = maxiter;
-    a.check_rounds = check_rounds;
-    a.change_tolerance = change_tolerance;
-    a.settle_rounds = settle_rounds;
-    a.state = S->state;
-    a.scalars = S->scalars;
-    a.narrow = S->narrow;
-    a.width = S->resident_width;
-    a.pushes = S->resident_pushes;
-    a.published = S->published;
-    a.partials = S->resident_partials;
-    a.counter = S->arrivals;
-    a.polls = S->polls >= 0 ? S->polls : S->resident_form == kGrid ? kGridPolls : kClusterPolls;
-    a.abort = reinterpret_cast<int*>(S->arrivals + kAbort);
-    a.gave_up = reinterpret_cast<int*>(S->arrivals + kGaveUp);
-    cudaLaunchAttribute attribute;
-    const cudaLaunchConfig_t config = resident_config(S, &attribute, stream);
-    void* args[] = {&a};
-    OB_CUDA(cudaLaunchKernelExC(&config, S->resident, args));
-    OB_CHECK_LAUNCH("pcg resident solve");
     return OB_OK;
 }
 
@@ -1141,7 +1203,16 @@ int ob_pcg_create(int n, const int32_t* offsets, const int32_t* columns, const d
     double* own_values = nullptr;
     A((void**)&own_offsets, sizeof(int) * (size_t)(n + 1));
     A((void**)&own_columns, sizeof(int) * (size_t)std::max(nnz, 1));
-    A((void**)&own_values, sizeof(double) * (size_t)std::max(nnz, 1));
+    // Behind the values what the resident form's lists take at most: the entries' values, their places,
+    // and three bounds for every two rows of whole CTAs.
+    const size_t entries = (size_t)std::max(nnz, 1), rows = (size_t)n + 2048;
+    const bool lists = S->k == 1 && n <= 2048LL * sm_count();
+    A((void**)&own_values, sizeof(double) * entries + (lists ? 12 * entries + sizeof(int) * (rows * 3 / 2 + 64) : 0));
+    if (st == OB_OK && lists) {
+        S->more_values = own_values + entries;
+        S->more_places = reinterpret_cast<unsigned*>(S->more_values + entries);
+        S->more_rows = reinterpret_cast<int*>(S->more_places + entries);
+    }
     A((void**)&S->inv_diag, sizeof(double) * n);
     A((void**)&S->maxima, sizeof(double) * (size_t)S->blocks);
     A((void**)&S->steps, sizeof(double4) * kChebyshevDegree);
@@ -1215,12 +1286,13 @@ int ob_pcg_solve(void* solver, const double* rhs, double* x, double tol, int max
     OB_REQUIRE(solver && rhs && x, "ob_pcg_solve: null pointer");
     OB_REQUIRE(tol >= 0.0 && maxiter >= 0, "ob_pcg_solve: bad tolerance or cap");
     Solver* S = static_cast<Solver*>(solver);
-    int st = S->resident ? launch_resident(S, rhs, x, tol, maxiter, 0, 0.0, 0, stream)
-                         : run_loop(S, rhs, x, tol, 0, 4, maxiter, 0, 0.0, 0, stream);
+    bool resident, read;
+    int st = launch_resident(S, rhs, x, tol, maxiter, 0, 0.0, 0, stream, &resident, &read);
+    if (st == OB_OK && !resident) st = run_loop(S, rhs, x, tol, 0, 4, maxiter, 0, 0.0, 0, stream);
     if (st) return st;
     if (iterations || relative_residual) {
-        if ((st = read_back(S, stream))) return st;
-        if (!S->resident) count_body_launches(S, 4, 0);
+        if (!read && (st = read_back(S, stream))) return st;
+        if (!resident) count_body_launches(S, 4, 0);
         for (int c = 0; c < S->k_live; ++c) {
             if (iterations) iterations[c] = S->host_state->iterations;
             if (relative_residual) {
@@ -1240,14 +1312,14 @@ int ob_pcg_settle(void* solver, const double* rhs, double* x, int check_rounds,
     OB_REQUIRE(check_rounds >= 1 && check_rounds <= 256, "ob_pcg_settle: check_rounds in [1, 256]");
     OB_REQUIRE(maxiter >= 0, "ob_pcg_settle: negative cap");
     Solver* S = static_cast<Solver*>(solver);
-    const bool resident = S->resident && S->resident_settles;
-    int st = resident ? launch_resident(S, rhs, x, 0.0, maxiter, check_rounds, change_tolerance, settle_rounds,
-                                           stream)
-                         : run_loop(S, rhs, x, 0.0, 1, check_rounds, maxiter, check_rounds, change_tolerance,
-                                    settle_rounds, stream);
+    bool resident, read;
+    int st = launch_resident(S, rhs, x, 0.0, maxiter, check_rounds, change_tolerance, settle_rounds, stream, &resident,
+                             &read);
+    if (st == OB_OK && !resident)
+        st = run_loop(S, rhs, x, 0.0, 1, check_rounds, maxiter, check_rounds, change_tolerance, settle_rounds, stream);
     if (st) return st;
     if (rounds || status) {
-        if ((st = read_back(S, stream))) return st;
+        if (!read && (st = read_back(S, stream))) return st;
         if (!resident) count_body_launches(S, check_rounds, 1);
         if (rounds) *rounds = S->host_state->iterations;
         if (status) *status = S->host_state->status;

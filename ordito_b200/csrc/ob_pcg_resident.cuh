@@ -17,18 +17,25 @@
 //             a barrier in the shared memory they arrive in (mbarrier transaction bytes), so a CTA
 //             waits for the values it reads and nothing else: barrier.cluster between the phases
 //             took 1.3 us each. (Gathering from the other CTAs took 3 us a mat-vec on a 10 k-vertex
-//             icosphere, whose edge rows read nothing local. Where a halo does not fit, or a CTA
-//             would push to one it does not read, the whole cluster gathers so, between
-//             barrier.clusters.)
+//             icosphere, whose edge rows read nothing local. Where a halo does not quite fit, or a
+//             CTA would push to one it does not read, the whole cluster gathers so, between
+//             barrier.clusters; where far more is missing, the launch declines and the host takes
+//             the grid.)
 //   kGrid     up to one CTA an SM (a cooperative launch): global memory at L2, an arrival counter
 //             between phases.
 //
 // Every wait is bounded: a CTA that gives up raises `abort`, the others then give up as well, and
-// `gave_up` stays set until the host has reported OB_ERR_TIMEOUT. Rows longer than the entries a thread holds read the rest from the CSR arrays. A round's float64
-// chain is kept short (two partial sums a row, one division behind the dots), since latency is what
-// is left: the sums a row and the scalars agree with the loop graph's to rounding. The dots are
-// folded thread, warp, CTA in a fixed order, so every run gives the same bits.
+// `gave_up` stays set until the host has reported OB_ERR_TIMEOUT. A round's float64 chain is kept short
+// (two partial sums a row, one division behind the dots), since latency is what is left: the sums a
+// row and the scalars agree with the loop graph's to rounding. The dots are folded thread, warp, CTA
+// in a fixed order, so every run gives the same bits.
+//
+// Rows past the seven entries of a regular mesh (a scan has vertices of 7 to 20 neighbours, a pole any
+// number) have a few more in place where many of a warp's rows have them; the rest is a list, whose
+// entries all lanes of the warp take.
 #pragma once
+
+#include <type_traits>
 
 #include "ob_internal.cuh"
 
@@ -40,8 +47,25 @@ constexpr int kClusterMax = 16;
 constexpr int kHalo = 1024;      // other CTAs' values a cluster CTA holds copies of
 constexpr int kHaloTable = 2048; // the hash table that numbers them
 constexpr int kPushesARow = 4;   // a CTA's push list, of its rows (two rows a thread; half at four)
-constexpr int kResidentWidth = 16;      // entries a row kept on the chip, at most
-constexpr int kBaseEntries = 7;  // a mesh row's usual count: every row is padded to it
+constexpr int kBaseEntries = 7;  // a regular mesh's rows: every row is padded to it
+// The most entries a row has in place, of a system's `mean`: the longest row's where the CTA's gathers are
+// local, the mean's in the grid, whose loads in flight need the L1 that shared memory leaves (rows in
+// random order, us a Chebyshev round at 64 and at 8: 140 000 rows 115 and 81).
+constexpr int most_in_place(int form, int mean) { return form == kGrid ? mean : mean < 8 ? 16 : 2 * mean + 2; }
+constexpr int kProducts = 64;    // of those, a warp's products at a time
+constexpr int kLaneEntries = 16; // a row's listed entries that its own thread lists
+// Values a CTA of a cluster may gather from the others, in place of a copy, before the launch leaves the
+// system to the grid. Rows of a triangulation in random order, us a settle round / a Chebyshev one,
+// cluster and grid: 5 000 rows (some 600 such values a CTA) 5.6 / 44 and 6.8 / 50, 6 000 7.0 / 53 and
+// 6.7 / 51, 8 000 (1 500) 8.2 / 69 and 6.8 / 50, 10 000 10 / 84 and 7.3 / 52.
+constexpr int kMayLose = 768;
+// The same for the grid's four-row polynomial form where its shared memory leaves less than this of the
+// 256 KB it has with L1: lines of 16 values a warp's gather reads on average (2 or 3 where rows lie in
+// order, 31 in random order, which took 152 us a round of 200 000 rows where the loop graph takes 120;
+// 94 and 106 at 160 000, whose shared memory leaves 100 KB).
+constexpr size_t kScatterLeaves = 80 << 10;
+constexpr int kMayScatter = 16;
+constexpr int kDeclined = -1;    // LoopState::status of a launch that left the system to another form
 __host__ __device__ constexpr int register_entries(int rows_a_thread) { return rows_a_thread <= 2 ? kBaseEntries : 0; }
 // Whether x, p and s of a thread's rows lie in shared memory: four rows' vectors under the polynomial
 // take more than the 128 registers a thread has, and a step's loads then wait for one another (3 400
@@ -69,11 +93,17 @@ struct ResidentArgs {
     LoopState* state;
     ColumnScalars* scalars;
     int narrow;  // the operator's values are rounded to float32
-    int width;   // entries a row on the chip, those in registers among them
+    int width;   // entries a row has in place, at most, those in registers among them
+    int more;    // entries past those that a CTA's list holds on the chip
     int pushes;  // kCluster: the capacity of a CTA's push list
     int polls;   // before a wait gives up
     int* abort;  // 1 when a wait gave up (zero at the launch of kGrid, zeroed by the others)
     int* gave_up;  // the same, but not zeroed by a launch
+    int* scattered;  // kGrid: lines read by gathers (zero at the launch), null where the launch does not decline
+    // The lists of the CTAs that have more of them: nnz entries, and R + 1 bounds a thread.
+    double* more_values;
+    unsigned* more_places;
+    int* more_rows;
     // kGrid: the published vector (two buffers of n), the CTAs' partial sums (6 a CTA) and the
     // arrival counter (zero at the launch).
     double* published;
@@ -204,8 +234,10 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
     const int T = blockDim.x, S = T * R, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int warps = T >> 5, cta = blockIdx.x, ctas = gridDim.x;
     // Shared memory: the published vector's two buffers (own rows, then the halo), the cluster's
-    // partial sums (two rows of three values a CTA), the warps' (one), three totals, the entries past
-    // the registers' (values, places), then the halo's table and the push list.
+    // partial sums (two rows of three values a CTA), the warps' (one), three totals, the entries in
+    // place past the registers' (values, places), the warps' products and the list of further entries
+    // (values, places, the warps' and the rows' bounds), the push list and the halo's table (in a
+    // cluster the products' place once the set-up is over).
     const int buffer = FORM == kGrid ? 0 : S + (FORM == kCluster ? kHalo : 0);
     double* pub = resident_smem;
     double* parts = pub + 2 * buffer;
@@ -218,12 +250,20 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
     constexpr bool kFar = far_vectors(R, CHEB);
     double* far = bars + 4 + 4 * kChebyshevDegree;
     double* vals = far + (kFar ? 3 * S : 0);
-    const int more = a.width - E;
-    int2* push = reinterpret_cast<int2*>(vals + (size_t)more * S);  // (own row, address); kCluster
+    const int held = a.width - E;  // entries in place that lie in shared memory
+    double* own_products = vals + (size_t)held * S;
+    double* list_values = own_products + (FORM == kCluster ? 0 : kProducts * warps);
+    int2* push = reinterpret_cast<int2*>(list_values + a.more);  // (own row, address); kCluster
     int* table = reinterpret_cast<int*>(push + (FORM == kCluster ? a.pushes : 0));
-    int* table_slot = table + kHaloTable;
-    int* counters = table_slot + kHaloTable;  // halo values, pushes, pulled entries
-    unsigned* places = FORM == kCluster ? reinterpret_cast<unsigned*>(counters + 4) : reinterpret_cast<unsigned*>(push);
+    int* table_slot = table + (FORM == kCluster ? kHaloTable : 0);
+    // Halo values, pushes, the most values a CTA has no copy of, the CTAs read, this CTA's such values.
+    int* counters = table_slot + (FORM == kCluster ? kHaloTable : 0);
+    unsigned* places = reinterpret_cast<unsigned*>(counters + 8);
+    unsigned* list_places = places + (size_t)held * S;
+    int* list_warps = reinterpret_cast<int*>(list_places + a.more);  // each warp's first and last, in the CTA's
+    int* list_rows = list_warps + 2 * 16 + 1;                        // (then whether the list lies here)
+    double* products = (FORM == kCluster ? reinterpret_cast<double*>(table) : own_products) + kProducts * warp;
+    static_assert(sizeof(double) * kProducts * 16 <= 2 * sizeof(int) * kHaloTable, "the table holds the products");
     const unsigned pub_at = FORM == kGrid ? 0u : shared_address(pub);
     unsigned goal = 0;  // grid arrivals due
     bool ok = true, pulls = false;
@@ -348,60 +388,145 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
     double x[N], r[R], p[N], s[N], u[R], inv[R], scaled[R], previous[N];
     double value[E ? E : 1][R];
     unsigned place[E ? E : 1][R];  // a column until the places are known
-    int over = 0, span = kBaseEntries;
     double bb = 0.0;
+    // A warp's rows have `span` entries in place, and every shorter row is padded to it with zero entries
+    // on a live row: as many as the longest has where the gathers are local (a further entry a row is
+    // then cheaper than the list), otherwise as many as half of the rows have. What longer rows have past
+    // that is the warp's list, `listed` entries: in shared memory where the CTA's fit, otherwise in global
+    // memory (consecutive, read at L2).
+    int span = kBaseEntries, listed = 0;
+    bool long_rows, lists;  // whether any row of the CTA has more than its base entries in place, and listed
+    auto list = [&](double*& list_v, unsigned*& list_p, int*& bounds) {
+        const bool here = list_warps[2 * 16] != 0;
+        const size_t base = here ? 0 : (size_t)a.offsets[cta * S];  // entries of the CTAs before
+        const int first = list_warps[2 * warp];
+        list_v = (here ? list_values : a.more_values + base) + first;
+        list_p = (here ? list_places : a.more_places + base) + first;
+        bounds = (here ? list_rows : a.more_rows + (size_t)cta * T * (R + 1)) + tid * (R + 1);
+    };
+    {
+        double ax[R];
+        int from[R], length[R];
+        int longest = 0;
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-        const int row = cta * S + i * T + tid;
-        const bool live = row < a.n;
-        const int o = live ? a.offsets[row] : 0, d = live ? a.offsets[row + 1] - o : 0;
-        const unsigned self = (unsigned)min(row, a.n - 1);
-        double ax = 0.0;
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const bool has = e < d;
-            const int col = has ? a.columns[o + e] : (int)self;
-            const double v = has ? a.values[o + e] : 0.0;
-            if (has) ax = fma(v, a.x[col], ax);
-            value[e][i] = a.narrow ? (double)(float)v : v;
-            place[e][i] = (unsigned)col;
+        for (int i = 0; i < R; ++i) {
+            const int row = cta * S + i * T + tid;
+            const bool live = row < a.n;
+            from[i] = live ? a.offsets[row] : 0;
+            length[i] = live ? a.offsets[row + 1] - from[i] : 0;
+            longest = max(longest, length[i]);
         }
-        for (int e = E; e < d; ++e) {
-            const int col = a.columns[o + e];
-            const double v = a.values[o + e];
-            ax = fma(v, a.x[col], ax);
-            if (e < a.width) {
-                vals[((e - E) * R + i) * T + tid] = a.narrow ? (double)(float)v : v;
-                places[((e - E) * R + i) * T + tid] = (unsigned)col;
+        longest = __reduce_max_sync(0xffffffffu, longest);
+        if (FORM != kGrid && longest <= a.width) {
+            span = max(span, longest);
+        } else {
+            for (; span < min(longest, a.width); ++span) {
+                int have = 0;
+#pragma unroll
+                for (int i = 0; i < R; ++i) have += __popc(__ballot_sync(0xffffffffu, length[i] > span));
+                if (have < 16 * R) break;
             }
         }
-        over |= d > a.width;
-        span = max(span, min(d, a.width));
-        const double b = live ? a.rhs[row] : 0.0;
-        bb = fma(b, b, bb);
-        const double start = live ? a.x[row] : 0.0;
-        if constexpr (kFar) {
-            far[i * T + tid] = start;
-            far[S + i * T + tid] = far[2 * S + i * T + tid] = 0.0;
-        } else {
-            x[i] = previous[i] = start;
-            p[i] = s[i] = 0.0;
-        }
-        r[i] = live ? b - ax : 0.0;
-        inv[i] = live ? a.inv_diag[row] : 0.0;
-        scaled[i] = u[i] = inv[i] * r[i];
-    }
-    // The warp's rows are padded to one span with zero entries on a live row.
-    __syncwarp();
-    over = __any_sync(0xffffffffu, over);
-    span = __reduce_max_sync(0xffffffffu, span);
+        int mine = 0;
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-        const int row = cta * S + i * T + tid;
-        const int d = row < a.n ? a.offsets[row + 1] - a.offsets[row] : 0;
-        for (int e = max(d, E); e < span; ++e) {
-            vals[((e - E) * R + i) * T + tid] = 0.0;
-            places[((e - E) * R + i) * T + tid] = (unsigned)min(row, a.n - 1);
+        for (int i = 0; i < R; ++i) {
+            const unsigned self = (unsigned)min(cta * S + i * T + tid, a.n - 1);
+            auto entry = [&](int e, double& v, unsigned& at) {
+                const bool has = e < length[i];
+                at = has ? (unsigned)a.columns[from[i] + e] : self;
+                v = has ? a.values[from[i] + e] : 0.0;
+                if (has) ax[i] = fma(v, a.x[at], ax[i]);
+                v = a.narrow ? (double)(float)v : v;
+            };
+            ax[i] = 0.0;
+#pragma unroll
+            for (int e = 0; e < E; ++e) entry(e, value[e][i], place[e][i]);
+            for (int e = E; e < span; ++e)
+                entry(e, vals[((e - E) * R + i) * T + tid], places[((e - E) * R + i) * T + tid]);
+            mine += max(0, length[i] - span);
+        }
+        // Where the thread's listed entries start: the lanes' counts scanned, then the warps'.
+        int before = mine;
+#pragma unroll
+        for (int step = 1; step < 32; step *= 2) {
+            const int below = __shfl_up_sync(0xffffffffu, before, step);
+            if (lane >= step) before += below;
+        }
+        int* of_warps = reinterpret_cast<int*>(scratch);
+        listed = __shfl_sync(0xffffffffu, before, 31);
+        if (lane == 0) of_warps[warp] = listed;
+        long_rows = __syncthreads_or(span > kBaseEntries);
+        lists = __syncthreads_or(listed);
+        if (lists) {
+            int all = 0, first = 0;
+            for (int w = 0; w < warps; ++w) {
+                first += w < warp ? of_warps[w] : 0;
+                all += of_warps[w];
+            }
+            if (lane == 0) {
+                list_warps[2 * warp] = first;
+                list_warps[2 * warp + 1] = first + listed;
+                if (warp == 0) list_warps[2 * 16] = all <= a.more;
+            }
+            __syncthreads();
+        }
+        if (listed) {
+            double* list_v;
+            unsigned* list_p;
+            int* bounds;
+            list(list_v, list_p, bounds);
+            int at = before - mine;
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int past = max(0, length[i] - span);
+                bounds[i] = at;
+                if (past <= kLaneEntries) {
+                    for (int e = 0; e < past; ++e) {
+                        const int col = a.columns[from[i] + span + e];
+                        const double v = a.values[from[i] + span + e];
+                        ax[i] = fma(v, a.x[col], ax[i]);
+                        list_v[at + e] = a.narrow ? (double)(float)v : v;
+                        list_p[at + e] = (unsigned)col;
+                    }
+                }
+                // A long row by the whole warp.
+                for (unsigned left = __ballot_sync(0xffffffffu, past > kLaneEntries); left; left &= left - 1) {
+                    const int of = __ffs(left) - 1;
+                    const int start = __shfl_sync(0xffffffffu, from[i], of) + span;
+                    const int to = __shfl_sync(0xffffffffu, at, of), count = __shfl_sync(0xffffffffu, past, of);
+                    double part = 0.0;
+                    for (int e = lane; e < count; e += 32) {
+                        const int col = a.columns[start + e];
+                        const double v = a.values[start + e];
+                        part = fma(v, a.x[col], part);
+                        list_v[to + e] = a.narrow ? (double)(float)v : v;
+                        list_p[to + e] = (unsigned)col;
+                    }
+                    part = warp_sum(part);
+                    if (lane == of) ax[i] += part;
+                }
+                at += past;
+            }
+            bounds[R] = at;
+            __syncwarp();  // other lanes' entries are read below
+        }
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int row = cta * S + i * T + tid;
+            const bool live = row < a.n;
+            const double b = live ? a.rhs[row] : 0.0;
+            bb = fma(b, b, bb);
+            const double start = live ? a.x[row] : 0.0;
+            if constexpr (kFar) {
+                far[i * T + tid] = start;
+                far[S + i * T + tid] = far[2 * S + i * T + tid] = 0.0;
+            } else {
+                x[i] = previous[i] = start;
+                p[i] = s[i] = 0.0;
+            }
+            r[i] = live ? b - ax[i] : 0.0;
+            inv[i] = live ? a.inv_diag[row] : 0.0;
+            scaled[i] = u[i] = inv[i] * r[i];
         }
     }
 
@@ -427,24 +552,32 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
     };
     if (FORM == kCluster) {
         for (int h = tid; h < kHaloTable; h += T) table[h] = -1;
-        if (tid < 4) counters[tid] = 0;
+        if (tid < 8) counters[tid] = 0;
         if (tid == 0) {
             for (unsigned b = 0; b < 4; ++b) arrivals_init(bars_at + 8u * b);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         for (int i = tid; i < 2 * kHalo; i += T) pub[(i / kHalo) * buffer + S + i % kHalo] = 0.0;
         cluster_barrier();  // every CTA of the cluster runs, its table, counters and barriers are ready
-        bool pulled = false;
+        int lost = 0;
         unsigned from = 0;  // the CTAs this one holds copies from
 #pragma unroll
         for (int i = 0; i < R; ++i) {
 #pragma unroll
             for (int e = 0; e < E; ++e)
-                if (!mine((int)place[e][i])) pulled |= find((int)place[e][i], true) < 0;
+                if (!mine((int)place[e][i])) lost += find((int)place[e][i], true) < 0;
             for (int e = E; e < span; ++e) {
                 const int col = (int)places[((e - E) * R + i) * T + tid];
-                if (!mine(col)) pulled |= find(col, true) < 0;
+                if (!mine(col)) lost += find(col, true) < 0;
             }
+        }
+        if (listed) {
+            double* list_v;
+            unsigned* list_p;
+            int* bounds;
+            list(list_v, list_p, bounds);
+            for (int q = lane; q < listed; q += 32)
+                if (!mine((int)list_p[q])) lost += find((int)list_p[q], true) < 0;
         }
         __syncthreads();
         for (int h = tid; h < kHaloTable; h += T) {
@@ -467,9 +600,8 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
                 }
             }
             table_slot[h] = taken;
-            pulled |= taken < 0;
+            lost += taken < 0;
         }
-        if (over) pulled = true;  // entries read from the CSR arrays may lie anywhere
         from = __reduce_or_sync(0xffffffffu, from);
         if (lane == 0 && from) atomicOr(&counters[3], (int)from);
         cluster_barrier();  // every owner's list is whole
@@ -480,12 +612,21 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
         to_whom = __reduce_or_sync(0xffffffffu, to_whom);
         // A CTA pushes again once it holds what it waits for: safe where those it pushes to are
         // those it reads. One that cannot takes the whole cluster back to barriers.
-        if (lane == 0 && (to_whom & ~(unsigned)counters[3])) pulled = true;
-        if (__any_sync(0xffffffffu, pulled) && lane < ctas)
-            asm volatile("red.shared::cluster.or.b32 [%0], 1;" ::"r"(cluster_address(shared_address(counters + 2), lane))
+        if (lane == 0 && (to_whom & ~(unsigned)counters[3])) ++lost;
+        lost = __reduce_add_sync(0xffffffffu, lost);
+        if (lane == 0 && lost) atomicAdd(&counters[4], lost);
+        __syncthreads();
+        if (counters[4] && warp == 0 && lane < ctas)
+            asm volatile("red.shared::cluster.max.s32 [%0], %1;" ::"r"(cluster_address(shared_address(counters + 2), lane)),
+                         "r"(counters[4])
                          : "memory");
         cluster_barrier();
         pulls = counters[2] != 0;
+        if (counters[2] > kMayLose) {
+            // Every CTA leaves here: none reads or writes another's memory past the barrier.
+            if (cta == 0 && tid == 0) a.state->status = kDeclined;
+            return;
+        }
         for (int q = tid; q < pushed; q += T) {
             const int2 to = push[q];  // (own row, (CTA, slot)) to (own row, slot's address | CTA in the high bits)
             push[q].y = (int)cluster_address(pub_at + 8u * (unsigned)(S + (to.y & 0xffff)), to.y >> 16);
@@ -502,225 +643,287 @@ __global__ void __launch_bounds__(resident_threads(R), 1) resident_pcg_kernel(co
             *at = place_of((int)*at);
         }
     }
+    if (listed) {
+        double* list_v;
+        unsigned* list_p;
+        int* bounds;
+        list(list_v, list_p, bounds);
+        for (int q = lane; q < listed; q += 32) list_p[q] = place_of((int)list_p[q]);
+        __syncwarp();
+    }
 
-    int parity = 0;
-    auto publish = [&](const double* v) {
-        parity ^= 1;
+    // (Grid: the lines that a gather of the base entries reads, counted over all CTAs by the first barrier.)
+    const bool weighs = FORM == kGrid && kFar && a.scattered != nullptr;
+    if (weighs) {
+        int lines = 0;
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            const int at = i * T + tid;
-            if (FORM != kGrid)
-                pub[parity * buffer + at] = v[i];
-            else if (cta * S + at < a.n)
-                __stcg(a.published + (size_t)parity * a.n + cta * S + at, v[i]);
-        }
-        if (FORM == kCluster) {
-            ok = __syncthreads_and(ok);
-            const unsigned bar = bars_at + 8u * (sent & 1u);
-            if (!pulls && tid == 0) arrivals_expect(bar, due);
-            for (int q = tid; q < pushed; q += T) {
-                const int2 to = push[q];
-                const unsigned at = (unsigned)to.y + 8u * (unsigned)(parity * buffer);
-                const double v = pub[parity * buffer + (to.x & 0xffff)];
-                if (pulls) store_cluster(at, v);
-                else push_cluster(at, v, cluster_address(bar, to.x >> 16));
+            for (int e = 0; e < kBaseEntries; ++e) {
+                const unsigned line = places[(e * R + i) * T + tid] >> 4;
+                const unsigned same = __match_any_sync(0xffffffffu, line);
+                lines += __popc(__ballot_sync(0xffffffffu, __ffs(same) - 1 == lane));
             }
         }
-    };
-    auto gather = [&](unsigned at) -> double {
-        double v;
-        if (FORM == kGrid) {
-            v = load_l2(a.published + (size_t)parity * a.n + at);
-        } else if (FORM == kCluster && pulls) {
-            asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(at + 8u * (unsigned)(parity * buffer)));
-        } else {
-            asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(at + 8u * (unsigned)(parity * buffer)));
-        }
-        return v;
-    };
-    // out = A (the published vector): two partial sums a row halve the chain.
-    auto matvec = [&](double* out) {
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
-            double even = 0.0, odd = 0.0;
-#pragma unroll
-            for (int e = 0; e < E; ++e) {
-                if (e & 1) odd = fma(value[e][i], gather(place[e][i]), odd);
-                else even = fma(value[e][i], gather(place[e][i]), even);
-            }
-            out[i] = even + odd;
-        }
-        // Four rows a thread: the base entries from shared memory, all their loads ahead of the sums.
-        if (E == 0) {
+        if (lane == 0) atomicAdd(a.scattered, lines);
+    }
+
+    // The solve, in three copies: a CTA runs one without the code for the kinds of entries it does not have
+    // (beside which a cluster's Chebyshev round of 5 000 regular rows took 15.2 us, not 11.7).
+    double rr0 = 0.0, rr = 0.0;
+    int round = 0, iterations = 0, status = OB_STATUS_CAPPED;
+    bool declined = false;
+    auto solve = [&](auto kinds) {
+        constexpr int kKinds = decltype(kinds)::value;
+        int parity = 0;
+        auto publish = [&](const double* v) {
+            parity ^= 1;
 #pragma unroll
             for (int i = 0; i < R; ++i) {
-                double v[kBaseEntries], u_of[kBaseEntries];
-#pragma unroll
-                for (int e = 0; e < kBaseEntries; ++e) {
-                    const int at = (e * R + i) * T + tid;
-                    v[e] = vals[at];
-                    u_of[e] = gather(places[at]);
+                const int at = i * T + tid;
+                if (FORM != kGrid)
+                    pub[parity * buffer + at] = v[i];
+                else if (cta * S + at < a.n)
+                    __stcg(a.published + (size_t)parity * a.n + cta * S + at, v[i]);
+            }
+            if (FORM == kCluster) {
+                ok = __syncthreads_and(ok);
+                const unsigned bar = bars_at + 8u * (sent & 1u);
+                if (!pulls && tid == 0) arrivals_expect(bar, due);
+                for (int q = tid; q < pushed; q += T) {
+                    const int2 to = push[q];
+                    const unsigned at = (unsigned)to.y + 8u * (unsigned)(parity * buffer);
+                    const double v = pub[parity * buffer + (to.x & 0xffff)];
+                    if (pulls) store_cluster(at, v);
+                    else push_cluster(at, v, cluster_address(bar, to.x >> 16));
                 }
+            }
+        };
+        auto gather = [&](unsigned at) -> double {
+            double v;
+            if (FORM == kGrid) {
+                v = load_l2(a.published + (size_t)parity * a.n + at);
+            } else if (FORM == kCluster && pulls) {
+                asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(at + 8u * (unsigned)(parity * buffer)));
+            } else {
+                asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(at + 8u * (unsigned)(parity * buffer)));
+            }
+            return v;
+        };
+        // out = A (the published vector): two partial sums a row halve the chain.
+        auto matvec = [&](double* out) {
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
                 double even = 0.0, odd = 0.0;
 #pragma unroll
-                for (int e = 0; e < kBaseEntries; ++e) {
-                    if (e & 1) odd = fma(v[e], u_of[e], odd);
-                    else even = fma(v[e], u_of[e], even);
+                for (int e = 0; e < E; ++e) {
+                    if (e & 1) odd = fma(value[e][i], gather(place[e][i]), odd);
+                    else even = fma(value[e][i], gather(place[e][i]), even);
                 }
                 out[i] = even + odd;
             }
-        }
-        for (int e = kBaseEntries; e < span; ++e) {
+            // Four rows a thread: the base entries from shared memory, all their loads ahead of the sums.
+            if (E == 0) {
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
-                const int at = ((e - E) * R + i) * T + tid;
-                out[i] = fma(vals[at], gather(places[at]), out[i]);
-            }
-        }
-        if (over) {
+                for (int first = 0; first < R; first += 2) {
+                    double u_of[2][kBaseEntries];
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
-                const int row = cta * S + i * T + tid;
-                const int o = row < a.n ? a.offsets[row] : 0, d = row < a.n ? a.offsets[row + 1] - o : 0;
-                for (int e = a.width; e < d; ++e) {
-                    const double v = a.narrow ? (double)(float)a.values[o + e] : a.values[o + e];
-                    out[i] = fma(v, gather(place_of(a.columns[o + e])), out[i]);
+                    for (int i = first; i < first + 2; ++i)
+#pragma unroll
+                        for (int e = 0; e < kBaseEntries; ++e) u_of[i - first][e] = gather(places[(e * R + i) * T + tid]);
+#pragma unroll
+                    for (int i = first; i < first + 2; ++i) {
+                        double even = 0.0, odd = 0.0;
+#pragma unroll
+                        for (int e = 0; e < kBaseEntries; ++e) {
+                            const double v = vals[(e * R + i) * T + tid];
+                            if (e & 1) odd = fma(v, u_of[i - first][e], odd);
+                            else even = fma(v, u_of[i - first][e], even);
+                        }
+                        out[i] = even + odd;
+                    }
                 }
             }
-            __syncwarp();
-        }
-    };
-    // u = the polynomial of the published `scaled` (which is u itself under Jacobi), published.
-    auto precondition = [&]() {
-        if (!CHEB) return;
-        double before[R], ax[R];
+            if constexpr (kKinds >= 1) {
+                for (int e = kBaseEntries; e < span; ++e) {
 #pragma unroll
-        for (int i = 0; i < R; ++i) u[i] = before[i] = scaled[i];
-        for (int index = 0; index < kChebyshevDegree - 1; ++index) {
-            const double4 st = steps[index];
-            const double slope = st.w * st.x;
-            double base[R];  // what the step takes from the vectors it has
+                    for (int i = 0; i < R; ++i) {
+                        const int at = ((e - E) * R + i) * T + tid;
+                        out[i] = fma(vals[at], gather(places[at]), out[i]);
+                    }
+                }
+            }
+            // The listed entries: a lane an entry, then each row its own products in order.
+            if constexpr (kKinds == 2) {
+                if (listed) {
+                    double* list_v;
+                    unsigned* list_p;
+                    int* bounds;
+                    list(list_v, list_p, bounds);
+                    for (int from = 0; from < listed; from += kProducts) {
+                        double v[kProducts / 32], u_of[kProducts / 32];
+#pragma unroll
+                        for (int h = 0; h < kProducts / 32; ++h) {
+                            const int q = min(from + 32 * h + lane, listed - 1);
+                            v[h] = list_v[q];
+                            u_of[h] = gather(list_p[q]);
+                        }
+#pragma unroll
+                        for (int h = 0; h < kProducts / 32; ++h) products[32 * h + lane] = v[h] * u_of[h];
+                        __syncwarp();
+#pragma unroll
+                        for (int i = 0; i < R; ++i) {
+                            const int end = min(bounds[i + 1] - from, kProducts);
+#pragma unroll 4
+                            for (int q = max(bounds[i] - from, 0); q < end; ++q) out[i] += products[q];
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+        };
+        // u = the polynomial of the published `scaled` (which is u itself under Jacobi), published.
+        auto precondition = [&]() {
+            if (!CHEB) return;
+            double before[R], ax[R];
+#pragma unroll
+            for (int i = 0; i < R; ++i) u[i] = before[i] = scaled[i];
+            for (int index = 0; index < kChebyshevDegree - 1; ++index) {
+                const double4 st = steps[index];
+                const double slope = st.w * st.x;
+                double base[R];  // what the step takes from the vectors it has
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const double current = st.x * u[i];
+                    base[i] = fma(st.w, scaled[i], fma(st.z, current - st.y * before[i], current));
+                    before[i] = u[i];
+                }
+                matvec(ax);
+#pragma unroll
+                for (int i = 0; i < R; ++i) u[i] = fma(-slope * inv[i], ax[i], base[i]);
+                publish(u);
+                if (!ok) break;
+                await_published();
+            }
+        };
+
+        // -- the start: |b|^2, u published ---------------------------------------------------------
+        double unused0, unused1;
+        fold(bb, 0.0, 0.0, 0);
+        publish(CHEB ? scaled : u);
+        await_published();
+        if (FORM == kCluster) await_sums();
+        if (weighs && ok && *(volatile int*)a.scattered > kMayScatter * kBaseEntries * R * warps * ctas) {
+            declined = true;
+            return;
+        }
+        read(rr0, unused0, unused1, 0);
+        barrier();  // the sums are read before the next fold writes them
+        precondition();
+        const double atol_sq = a.tol * a.tol * rr0;
+        // 1 / gamma of the last step, formed beside its other division (0: its value has no such inverse).
+        double gamma_old = INFINITY, inverse_old = 0.0, denominator_old = 0.0;
+        rr = rr0;
+        double settle_previous = 0.0, settle_reach = 0.0, settle_checks = 0.0;
+        bool done = false;
+        while (!done) {
+            double w[R], ag = 0.0, ad = 0.0, ar = 0.0;
+            matvec(w);
 #pragma unroll
             for (int i = 0; i < R; ++i) {
-                const double current = st.x * u[i];
-                base[i] = fma(st.w, scaled[i], fma(st.z, current - st.y * before[i], current));
-                before[i] = u[i];
+                ag = fma(r[i], u[i], ag);
+                ad = fma(w[i], u[i], ad);
+                ar = fma(r[i], r[i], ar);
             }
-            matvec(ax);
+            double gamma, delta;
+            fold(ag, ad, ar, 0);
+            await_sums();
+            if (!ok) break;
+            read(gamma, delta, rr, 0);
+            double alpha = 0.0, beta = 0.0;
+            bool step = false;
+            if (rr > atol_sq && round <= a.maxiter && gamma != 0.0) {
+                // beta gamma / alpha_old of the loop graph, with alpha_old = gamma_old / denominator_old.
+                beta = inverse_old != 0.0 ? gamma * inverse_old : gamma / gamma_old;
+                const double denominator = delta - beta * beta * denominator_old;
+                if (denominator != 0.0) {
+                    alpha = gamma / denominator;
+                    const double inverse = 1.0 / gamma;
+                    step = true;
+                    inverse_old = gamma > 1e-290 && gamma < 1e290 ? inverse : 0.0;
+                    gamma_old = gamma;
+                    denominator_old = denominator;
+                }
+            }
+            iterations += step ? 1 : 0;
+            if (!step || round >= a.maxiter) {
+                done = true;
+                status = !(rr == rr) ? OB_STATUS_NONFINITE
+                         : (!step && round <= a.maxiter) ? OB_STATUS_CONVERGED
+                                                         : OB_STATUS_CAPPED;
+            }
+            ++round;
+            if (step) {
 #pragma unroll
-            for (int i = 0; i < R; ++i) u[i] = fma(-slope * inv[i], ax[i], base[i]);
-            publish(u);
+                for (int i = 0; i < R; ++i) {
+                    if constexpr (kFar) {
+                        double* at = far + i * T + tid;
+                        const double pn = fma(beta, at[S], u[i]), sn = fma(beta, at[2 * S], w[i]);
+                        at[S] = pn;
+                        at[2 * S] = sn;
+                        at[0] = fma(alpha, pn, at[0]);
+                        r[i] = fma(-alpha, sn, r[i]);
+                    } else {
+                        p[i] = fma(beta, p[i], u[i]);
+                        s[i] = fma(beta, s[i], w[i]);
+                        x[i] = fma(alpha, p[i], x[i]);
+                        r[i] = fma(-alpha, s[i], r[i]);
+                    }
+                    scaled[i] = inv[i] * r[i];
+                    if (!CHEB) u[i] = scaled[i];
+                }
+            }
+            if (done) break;
+            const bool check = !kFar && a.check_rounds > 0 && round % a.check_rounds == 0;
+            if constexpr (!kFar) if (check) {
+                double change = 0.0, reached = 0.0;
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    if (x[i] != 0.0) {
+                        change = fmax(change, fabs(x[i] - previous[i]) / fabs(x[i]));
+                        reached += 1.0;
+                    }
+                    previous[i] = x[i];
+                }
+                fold(change, reached, 0.0, 1);
+            }
+            publish(CHEB ? scaled : u);
             if (!ok) break;
             await_published();
+            if (FORM == kCluster && check) await_sums();
+            if ((FORM == kGrid || check) && !ok) break;
+            if (check) {
+                double change, reached;
+                read(change, reached, unused0, 1);
+                settle_checks += 1.0;
+                if (reached + 1.0 != settle_previous) {
+                    settle_previous = reached + 1.0;
+                    settle_reach = settle_checks;
+                } else if (change < a.change_tolerance ||
+                           (settle_checks - settle_reach) * (double)a.check_rounds >= (double)a.settle_rounds) {
+                    done = true;
+                    status = change < a.change_tolerance ? OB_STATUS_SETTLED : OB_STATUS_SETTLE_BOUND;
+                }
+                if (FORM == kBlock) __syncthreads();  // the scratch is read before the next fold
+            }
+            if (!done) precondition();
         }
     };
-
-    // -- the start: |b|^2, u published ---------------------------------------------------------
-    double rr0 = 0.0, unused0, unused1;
-    fold(bb, 0.0, 0.0, 0);
-    publish(CHEB ? scaled : u);
-    await_published();
-    if (FORM == kCluster) await_sums();
-    read(rr0, unused0, unused1, 0);
-    barrier();  // the sums are read before the next fold writes them
-    precondition();
-    const double atol_sq = a.tol * a.tol * rr0;
-    // 1 / gamma of the last step, formed beside its other division (0: its value has no such inverse).
-    double gamma_old = INFINITY, inverse_old = 0.0, denominator_old = 0.0, rr = rr0;
-    double settle_previous = 0.0, settle_reach = 0.0, settle_checks = 0.0;
-    int round = 0, iterations = 0, status = OB_STATUS_CAPPED;
-    bool done = false;
-    while (!done) {
-        double w[R], ag = 0.0, ad = 0.0, ar = 0.0;
-        matvec(w);
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
-            ag = fma(r[i], u[i], ag);
-            ad = fma(w[i], u[i], ad);
-            ar = fma(r[i], r[i], ar);
-        }
-        double gamma, delta;
-        fold(ag, ad, ar, 0);
-        await_sums();
-        if (!ok) break;
-        read(gamma, delta, rr, 0);
-        double alpha = 0.0, beta = 0.0;
-        bool step = false;
-        if (rr > atol_sq && round <= a.maxiter && gamma != 0.0) {
-            // beta gamma / alpha_old of the loop graph, with alpha_old = gamma_old / denominator_old.
-            beta = inverse_old != 0.0 ? gamma * inverse_old : gamma / gamma_old;
-            const double denominator = delta - beta * beta * denominator_old;
-            if (denominator != 0.0) {
-                alpha = gamma / denominator;
-                const double inverse = 1.0 / gamma;
-                step = true;
-                inverse_old = gamma > 1e-290 && gamma < 1e290 ? inverse : 0.0;
-                gamma_old = gamma;
-                denominator_old = denominator;
-            }
-        }
-        iterations += step ? 1 : 0;
-        if (!step || round >= a.maxiter) {
-            done = true;
-            status = !(rr == rr) ? OB_STATUS_NONFINITE
-                     : (!step && round <= a.maxiter) ? OB_STATUS_CONVERGED
-                                                     : OB_STATUS_CAPPED;
-        }
-        ++round;
-        if (step) {
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-                if constexpr (kFar) {
-                    double* at = far + i * T + tid;
-                    const double pn = fma(beta, at[S], u[i]), sn = fma(beta, at[2 * S], w[i]);
-                    at[S] = pn;
-                    at[2 * S] = sn;
-                    at[0] = fma(alpha, pn, at[0]);
-                    r[i] = fma(-alpha, sn, r[i]);
-                } else {
-                    p[i] = fma(beta, p[i], u[i]);
-                    s[i] = fma(beta, s[i], w[i]);
-                    x[i] = fma(alpha, p[i], x[i]);
-                    r[i] = fma(-alpha, s[i], r[i]);
-                }
-                scaled[i] = inv[i] * r[i];
-                if (!CHEB) u[i] = scaled[i];
-            }
-        }
-        if (done) break;
-        const bool check = !kFar && a.check_rounds > 0 && round % a.check_rounds == 0;
-        if constexpr (!kFar) if (check) {
-            double change = 0.0, reached = 0.0;
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-                if (x[i] != 0.0) {
-                    change = fmax(change, fabs(x[i] - previous[i]) / fabs(x[i]));
-                    reached += 1.0;
-                }
-                previous[i] = x[i];
-            }
-            fold(change, reached, 0.0, 1);
-        }
-        publish(CHEB ? scaled : u);
-        if (!ok) break;
-        await_published();
-        if (FORM == kCluster && check) await_sums();
-        if ((FORM == kGrid || check) && !ok) break;
-        if (check) {
-            double change, reached;
-            read(change, reached, unused0, 1);
-            settle_checks += 1.0;
-            if (reached + 1.0 != settle_previous) {
-                settle_previous = reached + 1.0;
-                settle_reach = settle_checks;
-            } else if (change < a.change_tolerance ||
-                       (settle_checks - settle_reach) * (double)a.check_rounds >= (double)a.settle_rounds) {
-                done = true;
-                status = change < a.change_tolerance ? OB_STATUS_SETTLED : OB_STATUS_SETTLE_BOUND;
-            }
-            if (FORM == kBlock) __syncthreads();  // the scratch is read before the next fold
-        }
-        if (!done) precondition();
+    if (lists) solve(std::integral_constant<int, 2>{});
+    else if (long_rows) solve(std::integral_constant<int, 1>{});
+    else solve(std::integral_constant<int, 0>{});
+    if (declined) {
+        if (cta == 0 && tid == 0) a.state->status = kDeclined;
+        return;
     }
 #pragma unroll
     for (int i = 0; i < R; ++i) {

@@ -68,7 +68,55 @@ def test_solve_at_every_form_edge(gpu, n: int, kind: str) -> None:
     assert np.linalg.norm(rhs - host @ results[0]) <= 1.01 * tol * np.linalg.norm(rhs)
 
 
-@pytest.mark.parametrize("n", [1500, 9000, 16384, 20000, 40000])
+# Every form on both sides of its edges, without a row that is longer than the others.
+@pytest.mark.parametrize("kind", ["diag", "chebyshev"])
+@pytest.mark.parametrize("n", [1024, 1025, 2049, 6144, 6145, 16384, 16385, 22528, 22529, 26624, 26625, 151553])
+def test_solve_of_short_rows(gpu, n: int, kind: str) -> None:
+    host = _operator(n, n, wide_row=False)
+    _solves(host, kind)
+
+
+def _solves(host: sp.csr_matrix, kind: str) -> None:
+    n = host.shape[0]
+    matrix = CsrMatrix.from_host(host.indptr, host.indices, host.data, host.shape)
+    preconditioner = (linalg.chebyshev_preconditioner if kind == "chebyshev"
+                      else linalg.jacobi_preconditioner)(matrix)
+    rng = np.random.default_rng(n + 1)
+    rhs, start = rng.normal(size=n), rng.normal(size=n)
+    results = []
+    for _ in range(2):
+        x = DeviceArray.from_host(start)
+        linalg.solve_spd(matrix, DeviceArray.from_host(rhs), x, tol=1e-10, preconditioner=preconditioner)
+        results.append(x.numpy())
+    np.testing.assert_array_equal(results[0], results[1])
+    assert np.linalg.norm(rhs - host @ results[0]) <= 1.01e-10 * np.linalg.norm(rhs)
+
+
+# Rows of 1 to ~40 entries (the last figure is the mean): past the seven every row has in place, past what
+# fits in place, past what a thread lists alone (16), more than the list in shared memory holds; and one
+# row of every column, of 3 000 in the larger ones.
+@pytest.mark.parametrize("kind", ["diag", "chebyshev"])
+@pytest.mark.parametrize(("n", "mean"), [(33, 8), (700, 9), (1024, 30), (1025, 9), (5000, 12), (16384, 20), (20000, 9),
+                                         (22528, 12), (30000, 30), (160000, 9)])
+def test_solve_of_irregular_rows(gpu, n: int, mean: int, kind: str) -> None:
+    rng = np.random.default_rng(n + mean)
+    per = np.minimum(rng.geometric(1.0 / (mean / 2), size=n), 40)
+    i = np.repeat(np.arange(n), per)
+    j = i + 1 + rng.integers(0, 60, size=i.size)
+    keep = j < n
+    i, j = i[keep], j[keep]
+    every = np.arange(n) if n <= 5000 else rng.choice(n, size=3000, replace=False)
+    every = every[every != n // 2]
+    off = sp.coo_matrix((-rng.uniform(0.5, 1.0, i.size), (i, j)), shape=(n, n)).tocsr()
+    off = off + sp.coo_matrix((np.full(every.size, -1e-3), (np.full(every.size, n // 2), every)), shape=(n, n)).tocsr()
+    off = off + off.T
+    diagonal = 1.25 * np.maximum(-np.asarray(off.sum(axis=1)).ravel(), 1.0)
+    host = (off + sp.diags(diagonal)).tocsr()
+    host.sort_indices()
+    _solves(host, kind)
+
+
+@pytest.mark.parametrize("n", [1500, 9000, 16384, 20000, 40000, 200000])
 def test_scattered_rows(gpu, n: int) -> None:
     """Rows in random order: every CTA reads the others' rows, past what its halo and push list hold."""
     rng = np.random.default_rng(n)
@@ -229,3 +277,30 @@ def test_a_wait_given_up_is_reported_once(gpu, n: int, kind: str) -> None:
     x.fill_zero()
     solver.settle(d_rhs.ptr, x.ptr, 16, 1e-6, 192, 1000)
     assert np.linalg.norm(rhs - host @ x.numpy()) <= 1e-6 * np.linalg.norm(rhs)
+
+
+def test_rebound_state_takes_its_form_anew(gpu) -> None:
+    """Operators of one shape whose rows lie in order and scattered: the cluster's, then the grid's form,
+    with and without reading anything back."""
+    n = 12000
+    rng = np.random.default_rng(0)
+    ordered = _operator(n, 8, wide_row=False)
+    order = rng.permutation(n)
+    scattered = ordered[order][:, order].tocsr()
+    scattered.sort_indices()
+    solver = None
+    rhs = rng.normal(size=n)
+    d_rhs = DeviceArray.from_host(rhs)
+    for host in (scattered, ordered, ordered, scattered, scattered, ordered):
+        matrix = CsrMatrix.from_host(host.indptr, host.indices, host.data, host.shape)
+        if solver is None:
+            solver = linalg._solver(matrix, "chebyshev", False, 1)
+        else:
+            solver.rebind(matrix)
+        for outputs in (False, True):
+            x = DeviceArray.zeros(n, np.float64)
+            if outputs:
+                solver.solve(d_rhs.ptr, x.ptr, 1e-10, 1000)
+            else:
+                _lib.call("ob_pcg_solve", solver.handle, d_rhs.ptr, x.ptr, 1e-10, 1000, None, None, None)
+            assert np.linalg.norm(rhs - host @ x.numpy()) <= 1.01e-10 * np.linalg.norm(rhs)
