@@ -420,14 +420,19 @@ int ob_corner_records(const double* terms, const int32_t* faces, const int32_t* 
 int ob_grad_div_records(const double* records, const int32_t* ids, const int32_t* corner_offsets, int n_vertices,
                         int n_columns, const double* u, int u_stride, const int32_t* u_iperm, double* out,
                         int out_stride, const int32_t* out_iperm, const char* out_pinned, ob_stream_t stream);
-/* ob_corner_planes / ob_grad_div_planes: ob_grad_div_terms in each face's own plane (no reference
+/* ob_corner_planes / ob_mesh_corner_planes / ob_grad_div_planes: ob_grad_div_terms in each face's own plane (no reference
  * counterpart: a layout of the same arithmetic, equal to its rounding). Set-up, once per face buffer
  * and corner index: planes[3 F][6] float64, 16-byte aligned, corner p's gradient coefficients and W_e
  * in the plane's frame and its face's two other vertices (two int32 in the last eight bytes) for
- * corner_slots[p]. ob_grad_div_planes then takes ob_grad_div_terms' arguments with the planes and
- * corner offsets in place of the terms, faces and corner index. */
+ * corner_slots[p]; from the face terms, or from what those are made of (ids: the faces in the
+ * numbering of the vectors, faces itself or a renumbered copy). ob_grad_div_planes then takes
+ * ob_grad_div_terms' arguments with the planes and corner offsets in place of the terms, faces and
+ * corner index. */
 int ob_corner_planes(const double* terms, const int32_t* faces, const int32_t* corner_slots, int n_faces,
                      double* planes, ob_stream_t stream);
+int ob_mesh_corner_planes(const float* xyz, const int32_t* faces, const int32_t* ids, const float* normals,
+                          const float* areas, const float* cot, const int32_t* corner_slots, int n_faces,
+                          double* planes, ob_stream_t stream);
 int ob_grad_div_planes(const double* planes, const int32_t* corner_offsets, int n_vertices, int n_columns,
                        const double* u, int u_stride, const int32_t* u_iperm, double* out, int out_stride,
                        const int32_t* out_iperm, const char* out_pinned, ob_stream_t stream);

@@ -151,6 +151,7 @@ SIGNATURES: dict[str, list] = {
     "ob_face_gradient_terms": [P, P, I, P, P, P, P, P],
     "ob_grad_div_terms": [P, P, P, P, I, I, P, I, P, P, I, P, P, P],
     "ob_corner_planes": [P, P, P, I, P, P],
+    "ob_mesh_corner_planes": [P, P, P, P, P, P, P, I, P, P],
     "ob_grad_div_planes": [P, P, I, I, P, I, P, P, I, P, P, P],
     "ob_corner_records": [P, P, P, I, P, P, P],
     "ob_grad_div_records": [P, P, P, I, I, P, I, P, P, I, P, P, P],

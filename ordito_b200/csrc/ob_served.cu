@@ -372,18 +372,9 @@ grad_div_records_kernel(const double2* __restrict__ records, const int4* __restr
 // twice), so the sums agree with the terms form's to its rounding.
 constexpr int kPlanePairs = 3;  // double2 a corner: b w_x | w_y W_x | W_y (next, prev)
 
-__global__ void corner_planes_kernel(const double* __restrict__ terms, const int* __restrict__ faces,
-                                     const int* __restrict__ corner_slots, long long n_corners,
-                                     double2* __restrict__ planes) {
-    const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (p >= n_corners) return;
-    const int q = corner_slots[p];
-    const int f = q / 3, e = q - 3 * f;
-    const int next = e == 2 ? 0 : e + 1, prev = e == 0 ? 2 : e - 1;
-    const double* T = terms + (size_t)kFaceTerms * f;
-    const d3 b{T[3 * next], T[3 * next + 1], T[3 * next + 2]};
-    const d3 w{T[3 * prev], T[3 * prev + 1], T[3 * prev + 2]};
-    const d3 W{T[9 + 3 * e], T[10 + 3 * e], T[11 + 3 * e]};
+// A corner's plane: b and w the bases of its face's next and previous corners, W its edge sum.
+__device__ __forceinline__ void store_plane(const d3& b, const d3& w, const d3& W, int next, int prev,
+                                            double2* __restrict__ P) {
     const auto dot = [](const d3& x, const d3& y) { return fma(x.x, y.x, fma(x.y, y.y, x.z * y.z)); };
     // A length by its largest component, so no square leaves the range.
     const auto length = [&](const d3& x) {
@@ -405,10 +396,51 @@ __global__ void corner_planes_kernel(const double* __restrict__ terms, const int
         wy = length(r);
         if (wy > 0.0) Y = d3{r.x / wy, r.y / wy, r.z / wy};
     }
-    double2* P = planes + (size_t)kPlanePairs * p;
     P[0] = make_double2(along, wx);
     P[1] = make_double2(wy, dot(W, X));
-    P[2] = make_double2(dot(W, Y), __hiloint2double(faces[3 * f + next], faces[3 * f + prev]));
+    P[2] = make_double2(dot(W, Y), __hiloint2double(next, prev));
+}
+
+// From the face terms.
+__global__ void corner_planes_kernel(const double* __restrict__ terms, const int* __restrict__ faces,
+                                     const int* __restrict__ corner_slots, long long n_corners,
+                                     double2* __restrict__ planes) {
+    const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (p >= n_corners) return;
+    const int q = corner_slots[p];
+    const int f = q / 3, e = q - 3 * f;
+    const int next = e == 2 ? 0 : e + 1, prev = e == 0 ? 2 : e - 1;
+    const double* T = terms + (size_t)kFaceTerms * f;
+    const d3 b{T[3 * next], T[3 * next + 1], T[3 * next + 2]};
+    const d3 w{T[3 * prev], T[3 * prev + 1], T[3 * prev + 2]};
+    const d3 W{T[9 + 3 * e], T[10 + 3 * e], T[11 + 3 * e]};
+    store_plane(b, w, W, faces[3 * f + next], faces[3 * f + prev], planes + (size_t)kPlanePairs * p);
+}
+
+// From the mesh itself: a batch on a fresh mesh has no use for the 144 bytes of terms a face otherwise.
+// `ids` holds the faces in the numbering of the vectors.
+__global__ void mesh_corner_planes_kernel(const float* __restrict__ xyz, const int* __restrict__ faces,
+                                          const int* __restrict__ ids, const float* __restrict__ normals,
+                                          const float* __restrict__ areas, const float* __restrict__ cot,
+                                          const int* __restrict__ corner_slots, long long n_corners,
+                                          double2* __restrict__ planes) {
+    const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (p >= n_corners) return;
+    const int q = corner_slots[p];
+    const int f = q / 3, e = q - 3 * f;
+    const int next = e == 2 ? 0 : e + 1, prev = e == 0 ? 2 : e - 1;
+    const d3 own = widen(load_f3(xyz, faces[q])), at_next = widen(load_f3(xyz, faces[3 * f + next])),
+             at_prev = widen(load_f3(xyz, faces[3 * f + prev])), normal = widen(load_f3(normals, f));
+    const d3 to_next = dsub(at_next, own), to_prev = dsub(at_prev, own);
+    d3 b{0, 0, 0}, w{0, 0, 0};
+    if ((double)areas[f] > 0.0) {
+        b = dcross(normal, dsub(own, at_prev));
+        w = dcross(normal, to_next);
+    }
+    const double c_next = (double)cot[3 * f + next], c_prev = (double)cot[3 * f + prev];
+    const d3 W{c_prev * to_next.x + c_next * to_prev.x, c_prev * to_next.y + c_next * to_prev.y,
+               c_prev * to_next.z + c_next * to_prev.z};
+    store_plane(b, w, W, ids[3 * f + next], ids[3 * f + prev], planes + (size_t)kPlanePairs * p);
 }
 
 template <int CP>
@@ -1045,6 +1077,22 @@ int ob_corner_planes(const double* terms, const int32_t* faces, const int32_t* c
     corner_planes_kernel<<<ceil_div(corners, kThreads), kThreads, 0, stream>>>(terms, faces, corner_slots, corners,
                                                                                reinterpret_cast<double2*>(planes));
     OB_CHECK_LAUNCH("corner_planes");
+    return OB_OK;
+}
+
+int ob_mesh_corner_planes(const float* xyz, const int32_t* faces, const int32_t* ids, const float* normals,
+                          const float* areas, const float* cot, const int32_t* corner_slots, int n_faces,
+                          double* planes, ob_stream_t stream_) {
+    cudaStream_t stream = as_stream(stream_);
+    OB_REQUIRE(n_faces >= 0, "ob_mesh_corner_planes: bad size");
+    if (n_faces == 0) return OB_OK;
+    OB_REQUIRE(xyz && faces && ids && normals && areas && cot && corner_slots && planes,
+               "ob_mesh_corner_planes: null pointer");
+    OB_REQUIRE(((uintptr_t)planes & 15) == 0, "ob_mesh_corner_planes: planes must start on 16 bytes");
+    const long long corners = 3LL * n_faces;
+    mesh_corner_planes_kernel<<<ceil_div(corners, kThreads), kThreads, 0, stream>>>(
+        xyz, faces, ids, normals, areas, cot, corner_slots, corners, reinterpret_cast<double2*>(planes));
+    OB_CHECK_LAUNCH("mesh_corner_planes");
     return OB_OK;
 }
 

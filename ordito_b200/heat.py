@@ -427,14 +427,18 @@ class HeatSolver:
             self._gradient_terms = terms
         return self._gradient_terms
 
-    @property
-    def corner_planes(self) -> DeviceArray:
-        """The divergence's corner planes over the mesh's own numbering (``ob_corner_planes``), built once."""
+    def corner_planes(self, stream: Any = DEFAULT_STREAM) -> DeviceArray:
+        """The divergence's corner planes over the mesh's own numbering (``ob_mesh_corner_planes``),
+        built once, for a pass on ``stream``."""
         if getattr(self, "_corner_planes", None) is None:
-            mesh = self._mesh
-            planes = corner_planes(self.gradient_terms, mesh.faces, mesh.corner_index[1], mesh.n_faces)
-            _lib.call("ob_stream_synchronize", DEFAULT_STREAM)  # they serve other streams
-            self._corner_planes = planes
+            mesh, ops = self._mesh, self.operators
+            planes = mesh_corner_planes(mesh.vertices, mesh.faces, mesh.faces, ops.face_normals, ops.face_areas,
+                                        ops.cot_entries, mesh.corner_index[1], mesh.n_faces)
+            if getattr(self, "_corner_planes", None) is None:
+                self._corner_planes, self._planes_waited = planes, False
+        if stream is not DEFAULT_STREAM and not self._planes_waited:
+            _lib.call("ob_stream_synchronize", DEFAULT_STREAM)  # where they are built
+            self._planes_waited = True
         return self._corner_planes
 
     @property
@@ -639,6 +643,17 @@ def corner_planes(terms: DeviceArray, faces: DeviceArray, corner_slots: DeviceAr
     return planes
 
 
+def mesh_corner_planes(vertices: DeviceArray, faces: DeviceArray, ids: DeviceArray, normals: DeviceArray,
+                       areas: DeviceArray, cot: DeviceArray, corner_slots: DeviceArray,
+                       n_faces: int) -> DeviceArray:
+    """``corner_planes`` from the mesh and its face tables (``ob_mesh_corner_planes``), with no face terms
+    in between; ``ids`` holds the faces in the vectors' numbering."""
+    planes = DeviceArray.empty(18 * max(n_faces, 1), np.float64)
+    _lib.call("ob_mesh_corner_planes", vertices.ptr, faces.ptr, ids.ptr, normals.ptr, areas.ptr, cot.ptr,
+              corner_slots.ptr, n_faces, planes.ptr, DEFAULT_STREAM)
+    return planes
+
+
 def _divergence(mesh: Trimesh, solver: "HeatSolver", k: int, u: int, u_stride: int, u_iperm: Any,
                 out: int, out_stride: int, out_iperm: Any, out_pinned: Any, stream: Any) -> None:
     """``-div`` of the per-face unit gradients of ``k`` heat columns over the mesh's own numbering,
@@ -648,7 +663,7 @@ def _divergence(mesh: Trimesh, solver: "HeatSolver", k: int, u: int, u_stride: i
     single pass does not pay for the planes)."""
     corner_offsets, corner_slots = mesh.corner_index
     if k > 1:
-        _lib.call("ob_grad_div_planes", solver.corner_planes.ptr, corner_offsets.ptr, mesh.n_vertices, k, u,
+        _lib.call("ob_grad_div_planes", solver.corner_planes(stream).ptr, corner_offsets.ptr, mesh.n_vertices, k, u,
                   u_stride, u_iperm, out, out_stride, out_iperm, out_pinned, stream)
         return
     _lib.call(
@@ -687,7 +702,9 @@ def _corners_in_factor_rows(mesh: Trimesh, solver: "HeatSolver", h_iperm: int,
         workspace = DeviceArray.empty(int(size.value), np.uint8)
         _lib.call("ob_corner_index", faces.ptr, mesh.n_faces, n, offsets.ptr, slots.ptr,
                   workspace.ptr, int(size.value), DEFAULT_STREAM)
-        planes = corner_planes(solver.gradient_terms, faces, slots, mesh.n_faces)
+        ops = solver.operators
+        planes = mesh_corner_planes(mesh.vertices, mesh.faces, faces, ops.face_normals, ops.face_areas,
+                                    ops.cot_entries, slots, mesh.n_faces)
         _lib.call("ob_stream_synchronize", DEFAULT_STREAM)  # the arrays serve other streams
         result = (offsets, planes)
     holder._factor_row_corners = (key, result)

@@ -27,7 +27,7 @@ from ordito_b200 import _lib
 from ordito_b200.array import CsrMatrix
 from ordito_b200.cholesky import CholeskyAnalysis, SparseCholesky
 from ordito_b200.device import DEFAULT_STREAM, DeviceArray
-from ordito_b200.heat import _bounds_floor_length, capture_guard, corner_planes
+from ordito_b200.heat import _bounds_floor_length, capture_guard, mesh_corner_planes
 from ordito_b200.laplacian import face_terms, mesh_operator_pattern
 
 
@@ -128,11 +128,8 @@ class PackedMeshes:
         workspace = DeviceArray.empty(int(size.value), np.uint8)
         _lib.call("ob_corner_index", self.faces.ptr, self.n_faces, n, self.corner_offsets.ptr,
                   corner_slots.ptr, workspace.ptr, int(size.value), DEFAULT_STREAM)
-        gradient_terms = DeviceArray.empty((max(self.n_faces, 1), 18), np.float64)
-        _lib.call("ob_face_gradient_terms", self.xyz.ptr, self.faces.ptr, self.n_faces,
-                  terms.normals.ptr, terms.areas.ptr, terms.cot.ptr, gradient_terms.ptr,
-                  DEFAULT_STREAM)
-        self.corner_planes = corner_planes(gradient_terms, self.faces, corner_slots, self.n_faces)
+        self.corner_planes = mesh_corner_planes(self.xyz, self.faces, self.faces, terms.normals, terms.areas,
+                                                terms.cot, corner_slots, self.n_faces)
         # Batch buffers at the widest batch: column sources, their offsets, the shift's table.
         K = self.max_columns
         self.d_sources = DeviceArray.empty(K * self.n_meshes, np.int32)

@@ -7,7 +7,7 @@ import pytest
 
 from ordito_b200 import _lib, creation
 from ordito_b200.device import DeviceArray
-from ordito_b200.heat import corner_planes
+from ordito_b200.heat import corner_planes, mesh_corner_planes
 from ordito_b200.mesh import Trimesh
 from tests import meshes
 
@@ -67,6 +67,29 @@ def test_planes_match_the_terms(gpu, name: str, k: int, stride: int) -> None:
         tolerance = 1e-10 if name == "sliver" else 1e-12
         want = outs["terms", 0]
         np.testing.assert_allclose(outs["planes", 0], want, rtol=tolerance, atol=tolerance * np.abs(want).max())
+
+
+@pytest.mark.parametrize("name", sorted(_MESHES))
+def test_planes_of_the_mesh_are_the_terms_planes(gpu, name: str) -> None:
+    """The planes made from the mesh itself against those from its face terms, and in another numbering."""
+    v, f = _MESHES[name]()
+    mesh = Trimesh(v, f.reshape(-1))
+    face = mesh.face_terms
+    slots = mesh.corner_index[1]
+    terms = DeviceArray.empty((mesh.n_faces, 18), np.float64)
+    _lib.call("ob_face_gradient_terms", mesh.vertices.ptr, mesh.faces.ptr, mesh.n_faces, face.normals.ptr,
+              face.areas.ptr, face.cot.ptr, terms.ptr, None)
+    order = np.random.default_rng(0).permutation(v.shape[0]).astype(np.int32)
+    for numbering in (np.arange(v.shape[0], dtype=np.int32), order):
+        ids = DeviceArray.from_host(numbering[f.reshape(-1)])
+        want = corner_planes(terms, ids, slots, mesh.n_faces).numpy().reshape(-1, 6)
+        got = mesh_corner_planes(mesh.vertices, mesh.faces, ids, face.normals, face.areas, face.cot, slots,
+                                 mesh.n_faces).numpy().reshape(-1, 6)
+        np.testing.assert_array_equal(got[:, 5].view(np.int64), want[:, 5].view(np.int64))
+        # The same float64 formulas: a few roundings of a corner's largest coefficient, which the frame's
+        # division by a sliver's height (1e-4 of its length) carries on.
+        scale = np.abs(want[:, :5]).max(axis=1, keepdims=True)
+        assert np.all(np.abs(got[:, :5] - want[:, :5]) <= 1e-11 * scale)
 
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
