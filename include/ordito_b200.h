@@ -326,11 +326,14 @@ int ob_chol_analyse_blocked(int n, int block, const int32_t* offsets, const int3
 /* ob_chol_analyse on a host thread, beside what the caller does next: begin returns at once (the
  * thread copies the pattern behind the work `stream` holds now, on a stream of its own; the arrays
  * must stay until end or abandon returns), end waits for it and returns the analysis, abandon gives it
- * up (it waits for the copies at most). Either releases `pending`. */
+ * up (it waits for the copies at most; the thread stops soon after). Either releases `pending`.
+ * ob_chol_analyses_held: the analyses that are in the process' memory, those under way among them (an
+ * inspection hook). */
 int ob_chol_analyse_begin(int n, const int32_t* offsets, const int32_t* columns, const float* xyz, int leaf_size,
                           void** pending, ob_stream_t stream);
 int ob_chol_analyse_end(void* pending, void** analysis);
 int ob_chol_analyse_abandon(void* pending);
+int ob_chol_analyses_held(int* count);
 int ob_chol_analysis_info(void* analysis, long long* info);
 /* The same analysis from host arrays (no device), and the supernodes of an analysis as
  * out[4 s .. 4 s + 3] = (tree level, own columns, off-diagonal rows, parent or -1), postorder.

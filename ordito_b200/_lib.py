@@ -130,6 +130,7 @@ SIGNATURES: dict[str, list] = {
     "ob_chol_analyse_begin": [I, P, P, P, I, POINTER(c_void_p), P],
     "ob_chol_analyse_end": [P, POINTER(c_void_p)],
     "ob_chol_analyse_abandon": [P],
+    "ob_chol_analyses_held": [POINTER(c_int)],
     "ob_chol_analyse_blocked": [I, I, P, P, P, I, POINTER(c_void_p), P],
     "ob_extend_ratio": [P, I, P, P, P],
     "ob_chol_set_deterministic": [P, I, P],

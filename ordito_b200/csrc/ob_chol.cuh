@@ -2,6 +2,7 @@
 // ob_chol_factor.cu: the numeric factorisation on the device).
 #pragma once
 
+#include <atomic>
 #include <functional>
 #include <memory>
 #include <mutex>
@@ -38,7 +39,12 @@ struct CholAnalysis {
     // operator of this pattern shares it: the heat and the Poisson systems).
     std::mutex plan_mutex;
     FactorPlan* plan = nullptr;
-    ~CholAnalysis() { release_plan(plan); }
+    CholAnalysis() { ++held; }
+    ~CholAnalysis() {
+        release_plan(plan);
+        --held;
+    }
+    static inline std::atomic<int> held{0};  // of the process
 };
 
 // Where each supernode's block [L11^-1; G] (nc + noff rows of ld = nc rounded up to 8 doubles)

@@ -183,7 +183,11 @@ struct Dissector {
 // neighbours plus its children's off-diagonal rows past its own columns; its level is its height
 // above the leaves. The nodes of one level depend only on the levels below, so each level's
 // nodes run across host threads (each node's rows sorted and deduplicated on its own).
-void symbolic(Analysis& A, const std::vector<int>& adj_off, const std::vector<int>& adj) {
+// (Once `cancel` is set, here and below, what is left is not done: analyse gives the analysis up.)
+using Cancel = std::atomic<bool>;
+bool given_up(const Cancel* cancel) { return cancel && cancel->load(std::memory_order_relaxed); }
+
+void symbolic(Analysis& A, const std::vector<int>& adj_off, const std::vector<int>& adj, const Cancel* cancel) {
     const int ns = (int)A.nodes.size();
     // Heights (the nodes are in postorder: children first), then the nodes bucketed by height.
     std::vector<int> height(ns, 0);
@@ -206,7 +210,7 @@ void symbolic(Analysis& A, const std::vector<int>& adj_off, const std::vector<in
         const long long count = first[l + 1] - first[l];
         parallel_range(count, A.n > (1 << 16), [&](long long lo, long long hi) {
             std::vector<int> rows;
-            for (long long i = lo; i < hi; ++i) {
+            for (long long i = lo; i < hi && !given_up(cancel); ++i) {
                 Node& node = A.nodes[nodes[i]];
                 const int end = node.start + node.count;
                 rows.clear();
@@ -246,7 +250,7 @@ void symbolic(Analysis& A, const std::vector<int>& adj_off, const std::vector<in
 constexpr long long kMergeValues = 1750000;
 constexpr double kMergeGrowth = 1.3;
 
-void amalgamate(Analysis& A, const std::vector<int>& adj_off, const std::vector<int>& adj) {
+void amalgamate(Analysis& A, const std::vector<int>& adj_off, const std::vector<int>& adj, const Cancel* cancel) {
     const int ns = (int)A.nodes.size();
     if (A.levels < 3) return;
     auto padded = [](long long c) { return (c + 7) / 8 * 8; };
@@ -265,6 +269,7 @@ void amalgamate(Analysis& A, const std::vector<int>& adj_off, const std::vector<
     std::vector<int> level(ns, 0);
     bool merged_any = false;
     for (;;) {
+        if (given_up(cancel)) return;
         int top = 0;
         for (int s = 0; s < ns; ++s) {
             if (!alive[s]) continue;
@@ -340,16 +345,15 @@ void amalgamate(Analysis& A, const std::vector<int>& adj_off, const std::vector<
     A.perm = std::move(order);
     A.nodes = std::move(tree);
     for (int i = 0; i < A.n; ++i) A.iperm[A.perm[i]] = i;
-    symbolic(A, adj_off, adj);
+    symbolic(A, adj_off, adj, cancel);
 }
 
 // `block` > 1: the operator's rows come in groups of `block` consecutive rows, one group a mesh
 // vertex (xyz holds n / block points), as in a system of tangent vectors. The dissection then runs
 // over the vertices' graph and every vertex's rows stay together, consecutive in the ordering.
 int analyse(int n, std::vector<int> offsets, std::vector<int> columns, const float* xyz,
-            int leaf_size, Analysis* out, int block = 1, const std::atomic<bool>* cancel = nullptr) {
+            int leaf_size, Analysis* out, int block = 1, const Cancel* cancel = nullptr) {
     Analysis& A = *out;
-    const auto cancelled = [cancel]() { return cancel && cancel->load(std::memory_order_relaxed); };
     A.n = n;
     A.offsets = std::move(offsets);
     A.columns = std::move(columns);
@@ -408,13 +412,13 @@ int analyse(int n, std::vector<int> offsets, std::vector<int> columns, const flo
         A.perm = std::move(D.order);
         A.nodes = std::move(D.tree);
     }
-    if (cancelled()) return OB_ERR_INVALID;
+    if (given_up(cancel)) return OB_ERR_INVALID;
     A.iperm.assign(n, 0);
     for (int i = 0; i < n; ++i) A.iperm[A.perm[i]] = i;
-    symbolic(A, adj_off, adj);
-    if (cancelled()) return OB_ERR_INVALID;
-    amalgamate(A, adj_off, adj);
-    if (cancelled()) return OB_ERR_INVALID;
+    symbolic(A, adj_off, adj, cancel);
+    if (given_up(cancel)) return OB_ERR_INVALID;
+    amalgamate(A, adj_off, adj, cancel);
+    if (given_up(cancel)) return OB_ERR_INVALID;
     // Components (for pinning a singular operator): each vertex's component label and the last
     // vertex of each in the new order.
     A.component_last.assign(n, 0);
@@ -1893,7 +1897,9 @@ void run_pending(Pending& P, int n, const int* offsets, const int* columns, cons
         if (st == OB_OK) {
             auto A = std::make_unique<Analysis>();
             st = analyse(n, std::move(off), std::move(col), xyz ? pts.data() : nullptr, leaf_size, A.get(), 1, &P.cancel);
-            if (st == OB_OK) P.analysis = std::move(A);
+            // One given up by now goes with this scope; abandon lets go of one that is not.
+            std::lock_guard<std::mutex> lock(P.mutex);
+            if (st == OB_OK && !P.cancel.load()) P.analysis = std::move(A);
             else P.error = "the analysis was abandoned";
         } else {
             P.error = ob_last_error();
@@ -1907,12 +1913,13 @@ void run_pending(Pending& P, int n, const int* offsets, const int* columns, cons
     P.done.store(true);
 }
 
-// Abandoned analyses: their threads stop at their next step; each is joined when a later one is
-// abandoned after it has stopped, or at exit.
+// Abandoned analyses, which hold none of their work any more: their threads stop at their next step; each
+// is joined once it has stopped, when it or a later one is abandoned, or at exit.
 class Abandoned {
   public:
     void add(std::shared_ptr<Pending> P) {
         std::lock_guard<std::mutex> lock(mutex_);
+        list_.push_back(std::move(P));
         for (size_t i = 0; i < list_.size();) {
             if (list_[i]->done.load()) {
                 list_[i]->worker.join();
@@ -1921,7 +1928,6 @@ class Abandoned {
                 ++i;
             }
         }
-        list_.push_back(std::move(P));
     }
     ~Abandoned() {
         for (auto& P : list_) {
@@ -2024,13 +2030,21 @@ int ob_chol_analyse_abandon(void* pending) {
     auto* held = static_cast<std::shared_ptr<Pending>*>(pending);
     std::shared_ptr<Pending> P = *held;
     delete held;
-    P->cancel.store(true);
+    std::unique_ptr<Analysis> finished;
     {
-        // The caller's arrays are read no more once the copies are done (or were never started).
         std::unique_lock<std::mutex> lock(P->mutex);
+        P->cancel.store(true);
+        // The caller's arrays are read no more once the copies are done (or were never started).
         P->signal.wait(lock, [&]() { return P->copied; });
+        finished = std::move(P->analysis);
     }
-    abandoned().add(P);
+    abandoned().add(std::move(P));
+    return OB_OK;
+}
+
+int ob_chol_analyses_held(int* count) {
+    OB_REQUIRE(count != nullptr, "ob_chol_analyses_held: null output");
+    *count = Analysis::held.load();
     return OB_OK;
 }
 

@@ -3,6 +3,8 @@
 from __future__ import annotations
 
 import ctypes
+import gc
+import time
 
 import numpy as np
 import pytest
@@ -45,6 +47,35 @@ def test_abandoned_analyses_leave_nothing_behind(gpu) -> None:
         slot.release()  # the mesh's arrays go right after
         mesh.dispose()
         del slot, mesh
+
+
+def _held() -> int:
+    count = ctypes.c_int(0)
+    _lib.call("ob_chol_analyses_held", ctypes.byref(count))
+    return count.value
+
+
+@pytest.mark.parametrize("wait", [0.0, 0.002, 0.02, 1.5])
+def test_abandoned_analysis_is_let_go(gpu, wait: float) -> None:
+    """One given up at once, under way, or after it has finished leaves no analysis behind, without
+    another being abandoned."""
+    v, f = creation.jittered_torus(300, 210, seed=3)
+    mesh = Trimesh(v, f.reshape(-1))
+    slot = OperatorFactorization(mesh.heat_solver(method="meshlab").operators.heat_system, mesh.vertices)
+    gc.collect()
+    before = _held()
+    slot.analyse_ahead()
+    time.sleep(wait)
+    if wait >= 1.0:
+        assert _held() == before + 1  # finished, and not taken
+    slot.drop_analysis_ahead()
+    for _ in range(200):
+        if _held() == before:
+            break
+        time.sleep(0.01)
+    assert _held() == before
+    assert slot.factor()  # its own analysis, made in place
+    slot.release()
 
 
 def test_large_queries_ahead_and_in_place_agree(gpu, monkeypatch) -> None:
