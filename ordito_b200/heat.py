@@ -473,17 +473,19 @@ class HeatSolver:
             # The settled iterate of a large mesh may be rejected: the analysis its factorization
             # then needs runs on host threads while the device iterates.
             kept["factorization"].analyse_ahead()
-        twl.solve_spd_settled(
-            operators.heat_system,
-            rhs,
-            solution,
-            check_rounds=_HEAT_CHECK_ROUNDS,
-            change_tolerance=_HEAT_CHANGE_TOLERANCE,
-            settle_rounds=self._vertex_time()[1],
-            factorization=kept["factorization"],
-            narrow_values=True,
-        )
-        kept["factorization"].drop_analysis_ahead()  # the iterate was accepted
+        try:
+            twl.solve_spd_settled(
+                operators.heat_system,
+                rhs,
+                solution,
+                check_rounds=_HEAT_CHECK_ROUNDS,
+                change_tolerance=_HEAT_CHANGE_TOLERANCE,
+                settle_rounds=self._vertex_time()[1],
+                factorization=kept["factorization"],
+                narrow_values=True,
+            )
+        finally:
+            kept["factorization"].drop_analysis_ahead()  # the iterate was accepted, or the solve failed
         # A rejected settled iterate (answered by the factor or, past the budget, the march)
         # marks the mesh ill-conditioned for its Poisson solve (ordito/heat.py:4394-4404).
         if not held and (kept["factorization"].factorization is not None

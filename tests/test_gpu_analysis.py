@@ -12,6 +12,7 @@ import pytest
 from ordito_b200 import _lib, creation
 from ordito_b200 import heat as gheat
 from ordito_b200.cholesky import CholeskyAnalysis, OperatorFactorization
+from ordito_b200.device import DeviceArray
 from ordito_b200.mesh import Trimesh
 
 pytestmark = pytest.mark.gpu
@@ -76,6 +77,22 @@ def test_abandoned_analysis_is_let_go(gpu, wait: float) -> None:
     assert _held() == before
     assert slot.factor()  # its own analysis, made in place
     slot.release()
+
+
+def test_a_failed_settled_solve_gives_its_analysis_up(gpu, monkeypatch) -> None:
+    v, f = creation.jittered_torus(300, 210, seed=4)
+    mesh = Trimesh(v, f.reshape(-1))
+    solver = mesh.heat_solver(method="meshlab")
+    rhs = DeviceArray.zeros(v.shape[0], np.float64)
+
+    def fail(*args, **kwargs):
+        raise RuntimeError("the solve failed")
+
+    monkeypatch.setattr(gheat, "_ANALYSE_AHEAD_ROWS", 1000)
+    monkeypatch.setattr(gheat.twl, "solve_spd_settled", fail)
+    with pytest.raises(RuntimeError, match="the solve failed"):
+        solver.diffuse(rhs, rhs)
+    assert solver._kept("heat")["factorization"]._pending is None
 
 
 def test_large_queries_ahead_and_in_place_agree(gpu, monkeypatch) -> None:
