@@ -28,15 +28,27 @@ _CASES = {
     "128": lambda: _random(250, 128, 0, 128, 1),
     "129": lambda: _random(250, 129, 0, 129, 2),
     "torus": lambda: (creation.torus(61, 37)[1], 61 * 37),
-    # Rows at, and one key past, the longest a thread sorts (96 keys: 2 x 47 + 1 = 95, 2 x 48 + 1 = 97).
+    # Rows a warp sorts.
     "fan47": lambda: _fan(47),
     "fan48": lambda: _fan(48),
-    # One run of 1 024 keys, two, and runs merged to an odd count.
+    # The longest row of 256 threads (1 023 keys), the shortest of a CTA (1 025), tiles merged to an odd count.
     "fan511": lambda: _fan(511),
     "fan512": lambda: _fan(512),
     "fan5000": lambda: _fan(5000),
     # A block of rows past the shared memory (60 keys a row).
     "crowded": lambda: _random(4000, 256, 0, 256, 3),
+    # The longest row a thread sorts and the shortest of a warp (23 and 25 keys), of a warp and of 256 threads
+    # (127 and 129), of one tile and of two (4 095 and 4 097).
+    "fan11": lambda: _fan(11),
+    "fan12": lambda: _fan(12),
+    "fan63": lambda: _fan(63),
+    "fan64": lambda: _fan(64),
+    "fan2047": lambda: _fan(2047),
+    "fan2048": lambda: _fan(2048),
+    "fan10300": lambda: _fan(10300),
+    # Rows of 3 to some hundreds of keys beside one another, in and past the shared memory.
+    "uneven": lambda: (np.concatenate([_fan(r)[0] + 1500 * (r > 40) for r in (20, 30, 200, 400, 700)]), 3000),
+    "crowded_hub": lambda: (np.concatenate((_random(9000, 300, 0, 300, 7)[0], _fan(299)[0])), 300),
     # Repeated corners, indices outside the vertices, unreferenced vertices.
     "degenerate": lambda: _random(600, 40, 0, 12, 4),
     "outside": lambda: _random(400, 100, -20, 130, 5),
