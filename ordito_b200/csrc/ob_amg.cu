@@ -1986,16 +1986,17 @@ int grid_for(long long threads) {
     return (int)std::max(1LL, std::min(cap, (threads + kThreads - 1) / kThreads));
 }
 
-// The lane groups a row of `nnz` / rows entries is split over: doubled while the launch has fewer
-// threads than the device holds and a lane at least two entries. A small level is bound by its rows'
-// serial chains (one group a row leaves 3 306 rows of ~30 entries, 8 columns, on 6 612 threads),
-// a large one has the threads without. With the folds below taken by shuffles and the reducing
-// kernels' grids at their occupancy, 8 queries on a 262 k-vertex hierarchy went from 8.13 to
-// 6.80 ms, a 64-column V-cycle from 425 to 394 us.
+// The lane groups a row of `nnz` / rows entries is split over: doubled while the launch stays within the
+// threads the device holds and a lane has at least two entries (a doubling past them: 12 000 rows at 64
+// columns 3.82 -> 4.25 ms a solve, 262 k at one 4.79 -> 5.59). A small level is bound by its rows' serial
+// chains (one group a row leaves 3 306 rows of ~30 entries, 8 columns, on 6 612 threads), a large one
+// has the threads without. With the folds below taken by shuffles and the reducing kernels' grids at
+// their occupancy, 8 queries on a 262 k-vertex hierarchy went from 8.13 to 6.80 ms, a 64-column
+// V-cycle from 425 to 394 us.
 int row_split(long long rows, long long nnz, int G) {
     const long long resident = 2048LL * sm_count();
     int split = 1;
-    while (2 * split * G <= 32 && rows * G * split < resident && nnz >= 4LL * split * rows) split *= 2;
+    while (2 * split * G <= 32 && 2 * rows * G * split <= resident && nnz >= 4LL * split * rows) split *= 2;
     return split;
 }
 
@@ -2039,8 +2040,10 @@ int ensure_work(Amg* M, int kp, Work** out, cudaStream_t stream) {
         (st = alloc(dd, (void**)&W->x64)) || (st = alloc(dd, (void**)&W->r64)))
         return st;
     // The reducing kernels: as many blocks as an SM holds at their registers where the columns are few,
-    // fewer where the last block would have as many partials a column to fold by fewer threads.
-    W->blocks = (kp <= 16 ? 5 : kp <= 32 ? 4 : 2) * sm_count();
+    // fewer where the last block would have as many partials a column to fold by fewer threads, and no
+    // more than have rows (5 000 rows at 16 columns 2.72 -> 2.37 ms a solve).
+    W->blocks = std::min((kp <= 16 ? 5 : kp <= 32 ? 4 : 2) * sm_count(),
+                         std::max(1, ceil_div((long long)M->n * (kp / 4), kThreads)));
     if ((st = alloc(sizeof(double) * (size_t)W->blocks * kp, (void**)&W->partials)) ||
         (st = alloc(sizeof(unsigned int) * 8, (void**)&W->counters)) ||
         (st = alloc(sizeof(ColumnState) * kp, (void**)&W->cols)) ||
