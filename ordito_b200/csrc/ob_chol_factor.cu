@@ -232,20 +232,30 @@ __global__ void diag_dest_kernel(int n, const PlanTree T, long long* __restrict_
     diag_dest[j] = T.front_at[s] + lj * T.fld[s] + lj;
 }
 
-// A factor's row lists (a warp a supernode): its off-diagonal rows (rows of B), then the backward
-// product's inputs, its own rows of Y and its off-diagonal rows of X, in the stacked [B; Y; X].
-// The host filled and uploaded these lists before (as much as 60 MB at 2.6 M vertices), and made the
-// tile lists after the factorisation instead of beside it: a factor of the 2.6 M-vertex torus
-// took 102 ms where it now takes 57, of the 131k torus 3.81 and 3.08.
-__global__ void row_lists_kernel(int ns, int n, const int* __restrict__ start, const int* __restrict__ nc,
-                                 const int* __restrict__ row_at, const int* __restrict__ rows,
-                                 const int* __restrict__ rows_at, int* __restrict__ idx) {
+// A factor's tables (a warp a supernode): its numbering, its rows' supernodes and the supernodes'
+// parents, then its row lists: a supernode's off-diagonal rows (rows of B), then the backward product's
+// inputs, its own rows of Y and its off-diagonal rows of X, in the stacked [B; Y; X]. The host filled
+// and uploaded these before (as much as 60 MB at 2.6 M vertices), and made the tile lists after the
+// factorisation instead of beside it: a factor of the 2.6 M-vertex torus took 102 ms where it now
+// takes 57, of the 131k torus 3.81 and 3.08. (One launch: with four copies beside it the two factors of
+// six vertices took 174 us, so 141.)
+__global__ void factor_tables_kernel(int ns, int n, const int* __restrict__ start, const int* __restrict__ nc,
+                                     const int* __restrict__ row_at, const int* __restrict__ rows,
+                                     const int* __restrict__ rows_at, const int* __restrict__ old_of,
+                                     const int* __restrict__ parent_of, const FactorTables to) {
     const int s = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (s >= ns) return;
-    const int count = nc[s], first = row_at[s], noff = row_at[s + 1] - first;
-    int* off = idx + rows_at[s];
+    const int count = nc[s], own = start[s], first = row_at[s], noff = row_at[s + 1] - first;
+    if (lane == 0) to.parent[s] = parent_of[s];
+    int* off = to.idx + rows_at[s];
     int* back = off + noff;
-    for (int i = lane; i < count; i += 32) back[i] = n + start[s] + i;
+    for (int i = lane; i < count; i += 32) {
+        const int old = old_of[own + i];
+        to.perm[own + i] = old;
+        to.iperm[old] = own + i;
+        to.node_of[own + i] = s;
+        back[i] = n + own + i;
+    }
     for (int i = lane; i < noff; i += 32) {
         const int r = rows[first + i];
         off[i] = r;
@@ -850,18 +860,10 @@ int device_factor(CholAnalysis& A, const double* values, double sign, int pin_mo
     OB_CUDA(cudaMemsetAsync(bad, 0, sizeof(int) * (size_t)std::max(A.n_components, 1), stream));
     OB_CUDA(cudaMemsetAsync(status, 0, sizeof(int), stream));
     const int threads = 256;
-    const struct {
-        int *to, *from;
-        int count;
-    } copies[] = {{tables.perm, P->perm, n}, {tables.iperm, P->iperm, n}, {tables.node_of, P->node_of, n},
-                  {tables.parent, P->parent, ns}};
-    for (const auto& c : copies)
-        if (c.count > 0)
-            OB_CUDA(cudaMemcpyAsync(c.to, c.from, sizeof(int) * (size_t)c.count, cudaMemcpyDeviceToDevice, stream));
     if (ns > 0) {
-        row_lists_kernel<<<ceil_div(32LL * ns, threads), threads, 0, stream>>>(ns, n, P->start, P->nc, P->rel_at,
-                                                                               P->rows, P->rows_at, tables.idx);
-        OB_CHECK_LAUNCH("chol row lists");
+        factor_tables_kernel<<<ceil_div(32LL * ns, threads), threads, 0, stream>>>(
+            ns, n, P->start, P->nc, P->rel_at, P->rows, P->rows_at, P->perm, P->parent, tables);
+        OB_CHECK_LAUNCH("chol factor tables");
     }
     if (pin_mode == kPinZeroSum) {
         zero_sum_rows_kernel<<<ceil_div(n, threads), threads, 0, stream>>>(n, P->offsets, values, P->diag_pos,
