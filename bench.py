@@ -541,12 +541,19 @@ def kernel_rooflines(mesh, solver, columns: int = 64, reps: int = 10) -> dict:
         out["amg_vcycle_ms"] = ms[4]
         out["amg_levels"] = amg.grid
 
-    # a8: the divergence from the per-face terms, `columns` fields in and out (float64).
+    # a8: the divergence, `columns` fields in and out (float64): over the corner planes, the form of the
+    # served, batched and packed passes, and the forms beside it.
     terms = solver.gradient_terms
     corner_offsets, corner_slots, tile_faces, tile_counts, codes = mesh.corner_tiles
     # A field with a gradient on every face (a zero field skips the normalisation).
     u = DeviceArray.from_host(np.random.default_rng(0).random(n * columns))
     div = DeviceArray.empty(n * columns, np.float64)
+    planes = solver.corner_planes()
+    timed("grad_div_planes", 144 * f + 4 * (n + 1) + 2 * 8 * n * columns,
+          lambda: _lib.call("ob_grad_div_planes", planes.ptr, corner_offsets.ptr, n, columns, u.ptr, columns, None,
+                            div.ptr, columns, None, None, None),
+          "corner-plane form (the served, batched and packed passes'): planes and corner offsets in, u in "
+          "and -div out (float64)")
     timed("grad_div_terms", 144 * f + 12 * f + 4 * (n + 1) + 12 * f + 2 * 8 * n * columns,
           lambda: _lib.call("ob_grad_div_terms", terms.ptr, mesh.faces.ptr, corner_offsets.ptr,
                             corner_slots.ptr, n, columns, u.ptr, columns, None, div.ptr, columns,
@@ -558,7 +565,7 @@ def kernel_rooflines(mesh, solver, columns: int = 64, reps: int = 10) -> dict:
     timed("grad_div_records", 144 * f + 12 * f + 4 * (n + 1) + 12 * f + 2 * 8 * n * columns,
           lambda: _lib.call("ob_grad_div_records", records.ptr, ids.ptr, corner_offsets.ptr, n, columns, u.ptr,
                             columns, None, div.ptr, columns, None, None, None),
-          "corner-record form (the served pass's): the per-corner form's algorithmic bytes (the records "
+          "corner-record form (measured beside it): the per-corner form's algorithmic bytes (the records "
           "themselves hold 336 B a face against the terms' 144), u in and -div out (float64)")
     del records, ids
     timed("grad_div_tiled", 144 * f + 12 * f + 4 * (n + 1) + 2 * 12 * f + 2 * 8 * n * columns,

@@ -2257,7 +2257,7 @@ int ob_chol_tile(void* factor, int chunk, int waves, ob_stream_t stream_) {
     cudaStream_t stream = as_stream(stream_);
     OB_REQUIRE(factor != nullptr && waves >= 0 && waves <= 64, "ob_chol_tile: bad argument");
     // A split tile's inner range starts at a multiple of chunk, and the tile kernels read the
-    // factor's rows from there in 16-byte pieces: chunk must keep every start on 16 bytes.
+    // factor's rows from there in 16- and 32-byte pieces: chunk must keep every start on 32 bytes.
     OB_REQUIRE(chunk == 0 || (chunk >= 16 && chunk <= 4096 && chunk % 8 == 0),
                "ob_chol_tile: chunk %d is not 0 or a multiple of 8 in [16, 4096]", chunk);
     Factor* F = static_cast<Factor*>(factor);

@@ -43,8 +43,8 @@ _HEAT_CHECK_ROUNDS = 16  # :142
 _HEAT_CHANGE_TOLERANCE = 1e-6  # :146
 _HEAT_SETTLE_ROUNDS = 192  # :147
 _DIFFUSION_DECAY = 400.0  # :158
-# Rows from which a settled solve has its analysis started beside it: the analysis then takes a
-# third of the call (0.26 s of 0.80 s at 2.6 M rows). On smaller meshes there is less to hide, and
+# Rows from which a settled solve has its analysis started beside it: in turn the two take 0.26 s and
+# 0.29 s of a call of 0.8 s at 2.6 M rows, beside one another 0.3 s of 0.5. On smaller meshes there is less to hide, and
 # the host threads of an analysis that turns out not to be needed delay the call's own launches
 # (a 200 k-vertex sheet whose iterate is kept: 22 -> 28 ms).
 _ANALYSE_AHEAD_ROWS = 1 << 20
@@ -614,7 +614,8 @@ def _require_sources(sources: Any, n_vertices: int) -> DeviceArray:
 def divergence_tiles(corner_offsets: DeviceArray, corner_slots: DeviceArray, n: int,
                      n_faces: int) -> tuple[DeviceArray, DeviceArray, DeviceArray]:
     """``(tile_faces, tile_counts, corner_codes)`` of a corner index (``ob_divergence_tiles``):
-    the distinct faces of every tile of 32 consecutive vertices, for ``ob_grad_div_tiled``."""
+    the distinct faces of every tile of 32 consecutive vertices, for ``ob_grad_div_tiled`` (a form
+    kept to be measured against: the path's passes take the corner planes)."""
     corners = max(3 * n_faces, 1)
     tile_faces = DeviceArray.empty(corners, np.int32)
     tile_counts = DeviceArray.empty(max((n + 31) // 32, 1), np.int32)
@@ -627,7 +628,8 @@ def divergence_tiles(corner_offsets: DeviceArray, corner_slots: DeviceArray, n: 
 def corner_records(terms: DeviceArray, faces: DeviceArray, corner_slots: DeviceArray,
                    n_faces: int) -> tuple[DeviceArray, DeviceArray]:
     """``(records, ids)`` of a corner index (``ob_corner_records``): each corner's twelve divergence
-    terms and its face's vertices, in the index's order, for ``ob_grad_div_records``."""
+    terms and its face's vertices, in the index's order, for ``ob_grad_div_records`` (a form kept to be
+    measured against: the path's passes take the corner planes)."""
     corners = max(3 * n_faces, 1)
     records = DeviceArray.empty(12 * corners, np.float64)
     ids = DeviceArray.empty(4 * corners, np.int32)
@@ -639,7 +641,8 @@ def corner_records(terms: DeviceArray, faces: DeviceArray, corner_slots: DeviceA
 def corner_planes(terms: DeviceArray, faces: DeviceArray, corner_slots: DeviceArray,
                   n_faces: int) -> DeviceArray:
     """A corner index's ``ob_corner_planes``: each corner's gradient coefficients in its face's own
-    plane and its face's two other vertices, in the index's order, for ``ob_grad_div_planes``."""
+    plane and its face's two other vertices, in the index's order, for ``ob_grad_div_planes``: from face
+    terms a caller holds (the path makes them from the mesh, ``mesh_corner_planes``)."""
     planes = DeviceArray.empty(18 * max(n_faces, 1), np.float64)
     _lib.call("ob_corner_planes", terms.ptr, faces.ptr, corner_slots.ptr, n_faces, planes.ptr, DEFAULT_STREAM)
     return planes

@@ -68,7 +68,8 @@ class Trimesh:
     @property
     def corner_tiles(self) -> tuple[DeviceArray, ...]:
         """The corner index and its divergence tiles, ``(corner_offsets, corner_slots, tile_faces,
-        tile_counts, corner_codes)`` (``ob_divergence_tiles``), made once."""
+        tile_counts, corner_codes)`` (``ob_divergence_tiles``), made once; read by the tiled form that
+        the benchmark measures beside the path's."""
         if getattr(self, "_corner_tiles", None) is None:
             from ordito_b200.heat import divergence_tiles  # noqa: PLC0415
 
