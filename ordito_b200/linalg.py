@@ -215,14 +215,19 @@ class NativeSolver:
 _KEPT: "collections.OrderedDict[tuple, NativeSolver]" = collections.OrderedDict()
 _KEPT_LIMIT = 16
 _KEPT_LOCK = threading.Lock()
+# States on their way into the pool. A garbage collection may retire one at any point of this thread,
+# between the statements under the lock too, so a retiring call never waits for the lock.
+_RETIRED: "collections.deque[NativeSolver]" = collections.deque()
 
 
 def _solver(matrix: CsrMatrix, kind: str, narrow: bool, n_columns: int) -> NativeSolver:
     key = (kind, bool(narrow), int(n_columns))
     solver = matrix._solvers.get(key)
     if solver is None:
+        shape_key = (matrix.nrow, matrix.nnz) + key  # (nnz may be read back: not under the lock)
         with _KEPT_LOCK:
-            solver = _KEPT.pop((matrix.nrow, matrix.nnz) + key, None)
+            solver = _KEPT.pop(shape_key, None)
+        _pool_retired()
         if solver is not None:
             solver.pooled = False
             solver.rebind(matrix)
@@ -237,18 +242,29 @@ def retire_solver(solver: Any) -> None:
     pool, least recently retired closed first), or closed."""
     if not isinstance(solver, NativeSolver) or not (solver.handle and solver.handle.value):
         return
-    closing = []
     solver.pooled = True
-    with _KEPT_LOCK:
-        previous = _KEPT.pop(solver.shape_key, None)
-        if previous is not None:
-            closing.append(previous)
-        _KEPT[solver.shape_key] = solver
-        while len(_KEPT) > _KEPT_LIMIT:
-            closing.append(_KEPT.popitem(last=False)[1])
+    _RETIRED.append(solver)
+    _pool_retired()
+
+
+def _pool_retired() -> None:
+    """Puts the retired states into the pool, unless a call below this one, or another thread's, is
+    at it: that one looks again before it leaves."""
+    closing = []
+    while _RETIRED and _KEPT_LOCK.acquire(blocking=False):
+        try:
+            while _RETIRED:
+                solver = _RETIRED.popleft()
+                closing.append(_KEPT.pop(solver.shape_key, None))
+                _KEPT[solver.shape_key] = solver
+                while len(_KEPT) > _KEPT_LIMIT:
+                    closing.append(_KEPT.popitem(last=False)[1])
+        finally:
+            _KEPT_LOCK.release()
     for old in closing:
-        old.pooled = False
-        old.close()
+        if old is not None:
+            old.pooled = False
+            old.close()
 
 
 def _kind(matrix: CsrMatrix, preconditioner: Preconditioner | None) -> str:
