@@ -275,7 +275,7 @@ __device__ __forceinline__ int rank_sort(const unsigned long long* from, int cou
 // tile of four keys a thread, then a CTA a row by such tiles, merged pairwise between the buckets and the
 // second buffer, each thread sixteen consecutive places of every output. A long row's runs up to each run
 // tile's end stay in the second buffer, for write_rows. ms a build: 20 000 fans of 30 faces 0.28, one million
-// random faces in rows of 60 keys 0.70, of 300 0.81, of 3 000 0.87, a fan of 200 000 faces 7.15; with every row past
+// random faces in rows of 60 keys 0.70, of 300 0.98, of 3 000 0.98, a fan of 200 000 faces 7.15; with every row past
 // 96 keys, or of a crowded block, by 1 024 threads, runs of 1 024 by rank and a bisection a key 0.60, 1.76,
 // 1.08, 3.20 and 18.7; by a general segmented sort of the stored keys 0.39, 3.1, 1.90, 1.50 and 7.1.
 constexpr int kListedThreads = 1024, kGroup = 256;
@@ -583,7 +583,7 @@ int ob_pattern_build(const int32_t* faces, int n_faces, int n_vertices, int32_t*
     OB_CUDA(cub::DeviceScan::ExclusiveSum(scan_temp, scan_bytes, distinct, offsets, n + 1, stream));
     count_launch(1);
     if (n > 0) {
-        const int helpers = std::min(ceil_div(count, kRunTile), 4 * sm_count());
+        const int helpers = std::min(ceil_div(count, kRunTile), sm_count());
         write_rows<<<ceil_div(n, kSortRows) + helpers, kWriteThreads, 0, stream>>>(
             bucket, spare, starts, offsets, n, 6LL * n_faces, lists.counts + 3, keys_out, order, columns, run_start);
         OB_CHECK_LAUNCH("write_rows");

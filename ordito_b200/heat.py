@@ -43,10 +43,10 @@ _HEAT_CHECK_ROUNDS = 16  # :142
 _HEAT_CHANGE_TOLERANCE = 1e-6  # :146
 _HEAT_SETTLE_ROUNDS = 192  # :147
 _DIFFUSION_DECAY = 400.0  # :158
-# Rows from which a settled solve has its analysis started beside it: in turn the two take 0.26 s and
-# 0.29 s of a call of 0.8 s at 2.6 M rows, beside one another 0.3 s of 0.5. On smaller meshes there is less to hide, and
-# the host threads of an analysis that turns out not to be needed delay the call's own launches
-# (a 200 k-vertex sheet whose iterate is kept: 22 -> 28 ms).
+# Rows from which a settled solve has its analysis started beside it: in turn the two take 0.26 s
+# and 0.29 s of a call of 0.8 s at 2.6 M rows, beside one another 0.3 s of 0.5. On smaller meshes
+# there is less to hide, and the host threads of an analysis that turns out not to be needed delay
+# the call's own launches (a 200 k-vertex sheet whose iterate is kept: 22 -> 28 ms).
 _ANALYSE_AHEAD_ROWS = 1 << 20
 _GEOMETRY_CENTRAL_POISSON_SHIFT = 1e-6  # :193 (geometry-central's Poisson system -L + 1e-6 I)
 _TOLERANCE_MOLLIFY = 1e-5  # ordito/constants.py:31 (use_robust's margin, of the mean edge length)
